@@ -383,7 +383,7 @@ vt_batch* vt_batch_create(const vt_mesh_desc* descs, int n, int device, int* sta
   }
   size_t max_inst_bytes = 0;
   for (auto& G : b->groups) {
-    G.kern = vt::select_kernel(G.p, G.nfq);
+    G.kern = vt::select_kernel(G.p, G.nfq, G.ops.data());
     int per_sm = 0;
     if ((e = vt::tensor_maps_available()) || (e = G.kern.configure(&per_sm))) {
       set(fail(VT_ERR_CUDA, vt::cuda_msg("stage kernel attributes", e)));
@@ -740,7 +740,7 @@ int vt_batch_autotune(vt_batch* b, int trials, int* blocks_per_sm_out, int* mapp
     int best_b = 1;
     float best_ms = 1e30f;
     for (int map : {vt::kMapComponent, vt::kMapPair}) {
-      const vt::StageKernel k = vt::select_kernel(G.p, G.nfq, map);
+      const vt::StageKernel k = vt::select_kernel(G.p, G.nfq, G.ops.data(), map);
       int limit = 0;
       if (k.configure(&limit)) continue;
       G.kern = k;
@@ -784,7 +784,7 @@ int vt_batch_set_mapping(vt_batch* b, const int* mapping) {
     if (mapping[gi] != vt::kMapComponent && mapping[gi] != vt::kMapPair)
       return fail(VT_ERR_INVALID, "vt_batch_set_mapping: mapping must be 0 (component) or 1 (pair)");
     vt::Group& G = b->groups[gi];
-    const vt::StageKernel k = vt::select_kernel(G.p, G.nfq, mapping[gi]);
+    const vt::StageKernel k = vt::select_kernel(G.p, G.nfq, G.ops.data(), mapping[gi]);
     int limit = 0;
     const cudaError_t e = k.configure(&limit);
     if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("vt_batch_set_mapping", e));

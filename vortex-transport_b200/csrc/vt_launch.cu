@@ -1,8 +1,10 @@
 // Kernel selection by (p, nfq, warp mapping) -- the instantiations are in
-// vt_stage_component.cu and vt_stage_pair.cu -- and the tile schedule kernels
-// (vt_launch.h).
+// vt_stage_component.cu, vt_stage_pair.cu and vt_stage_folded.cu -- and the
+// tile schedule kernels (vt_launch.h).
 #include <cuda.h>
 
+#include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 
@@ -50,8 +52,32 @@ cudaError_t encode_state_map(CUtensorMap* m, const void* base, long long Kpad, i
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-StageKernel select_kernel(int p, int nfq, int map) {
-  return map == kMapPair ? select_kernel_pair(p, nfq) : select_kernel_component(p, nfq);
+StageKernel select_kernel(int p, int nfq, const double* ops, int map) {
+  if (map != kMapPair) return select_kernel_component(p, nfq);
+  return operators_reflect(p, nfq, ops) ? select_kernel_folded(p, nfq) : select_kernel_pair(p, nfq);
+}
+
+bool operators_reflect(int p, int nfq, const double* ops) {
+  if (p < 1 || p > 3) return false;  // p = 0 has one node: nothing to fold
+  const int np = np_of_p(p);
+  auto D = [&](int d, int i, int j) { return ops[(d * np + i) * np + j]; };
+  auto lift = [&](int s, int i, int q) { return ops[2 * np * np + (s * np + i) * nfq + q]; };
+  double big_d = 0.0, off_d = 0.0, big_l = 0.0, off_l = 0.0;
+  bool finite = true;
+  auto take = [&](double x, double y, double* big, double* off) {
+    finite = finite && std::isfinite(x) && std::isfinite(y);
+    *big = std::max(*big, std::fabs(x));
+    *off = std::max(*off, std::fabs(x - y));
+  };
+  for (int i = 0; i < np; ++i) {
+    const int m = mirror_node(p, i);
+    for (int j = 0; j < np; ++j) take(D(0, i, j), D(1, m, mirror_node(p, j)), &big_d, &off_d);
+    for (int q = 0; q < nfq; ++q) {
+      take(lift(0, i, q), lift(2, m, nfq - 1 - q), &big_l, &off_l);
+      take(lift(1, i, q), lift(1, m, nfq - 1 - q), &big_l, &off_l);
+    }
+  }
+  return finite && off_d <= 1e-13 * big_d && off_l <= 1e-13 * big_l;
 }
 
 int stage_ops_doubles(int p, int nfq) {

@@ -23,14 +23,23 @@ struct StageKernel {
   int map = 0;
 };
 
-// The mapping a context uses unless told otherwise (the pair mapping: 8% faster
-// at p = 3 on the 768 x 768 mesh).
+// The mapping a context uses unless told otherwise.
 constexpr int kDefaultMap = kMapPair;
 
+// The kernel for the operator block `ops` (stage_ops_doubles(p, nfq) doubles).
+// kMapPair takes the folded form where operators_reflect says so.
 // Empty (null members) for p outside 0..3, nfq outside 1..10.
-StageKernel select_kernel(int p, int nfq, int map = kDefaultMap);
+StageKernel select_kernel(int p, int nfq, const double* ops, int map = kDefaultMap);
 StageKernel select_kernel_component(int p, int nfq);
 StageKernel select_kernel_pair(int p, int nfq);
+StageKernel select_kernel_folded(int p, int nfq);
+
+// Whether the operator block has the reference triangle's reflection symmetry
+// (vt_device.cuh) to 1e-13 of each operator's largest entry, a few roundings
+// of the tables it is folded from. The tables of the reference do (at most
+// 1e-14 apart wherever the area rule makes the mass matrix regular); a caller's own tables
+// need not.
+bool operators_reflect(int p, int nfq, const double* ops);
 
 // Number of doubles of the StageOps<P, NFQ> block for (p, nfq).
 int stage_ops_doubles(int p, int nfq);

@@ -153,7 +153,10 @@ int vt_step_rk4_noalloc(const vt_device_mesh* m, const double* dU_in, double* dU
       !vt::aligned_to(m->det_jacobian, 8) || !vt::aligned_to(m->inv_jacobian, 8) ||
       !vt::aligned_to(m->normals, 8) || !vt::aligned_to(m->side_lengths, 8))
     return fail(VT_ERR_INVALID, "vt_step_rk4_noalloc: a mesh array is misaligned for its element type");
-  const vt::StageKernel pk = vt::select_kernel(m->p, m->n_line_points);
+  double ops[vt::kMaxOps];
+  vt::fold_stage_operators(m->p, m->n_line_points, m->inv_mass_ref, m->stiffness_ref, m->line_quadrature,
+                           m->phi_plus, m->phi_minus, ops);
+  const vt::StageKernel pk = vt::select_kernel(m->p, m->n_line_points, ops);
 
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -192,10 +195,6 @@ int vt_step_rk4_noalloc(const vt_device_mesh* m, const double* dU_in, double* dU
   auto* Sb = reinterpret_cast<double2*>(base + cv.Sb);
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int K = m->n_elements, Np = vt::np_of(m->p);
-
-  double ops[vt::kMaxOps];
-  vt::fold_stage_operators(m->p, m->n_line_points, m->inv_mass_ref, m->stiffness_ref, m->line_quadrature,
-                           m->phi_plus, m->phi_minus, ops);
 
   // error key to "none", step and block counters and the neighbour flag to zero
   if ((e = cudaMemsetAsync(errw, 0xFF, sizeof(unsigned long long), st)) ||

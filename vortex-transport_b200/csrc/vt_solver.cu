@@ -443,7 +443,9 @@ vt_ctx* vt_create(const vt_mesh_desc* d, int device, int* status) {
   c->nfq = d->n_line_points;
   c->K = K;
   c->Kpad = (static_cast<long long>(K) + 127) / 128 * 128;
-  const vt::StageKernel sk = vt::select_kernel(c->p, c->nfq);
+  c->ops = vt::fold_operators(c->p, c->nfq, d->inv_mass_ref, d->stiffness_ref, d->line_quadrature,
+                              d->phi_plus, d->phi_minus);
+  const vt::StageKernel sk = vt::select_kernel(c->p, c->nfq, c->ops.data());
   c->launch = sk.launch;
   int per_sm = 0, sms = 0;
   if ((e = vt::tensor_maps_available()) || (e = sk.configure(&per_sm)) ||
@@ -453,8 +455,6 @@ vt_ctx* vt_create(const vt_mesh_desc* d, int device, int* status) {
     return nullptr;
   }
   c->max_blocks = sms * (per_sm > 0 ? per_sm : 1);
-  c->ops = vt::fold_operators(c->p, c->nfq, d->inv_mass_ref, d->stiffness_ref, d->line_quadrature,
-                              d->phi_plus, d->phi_minus);
   c->minv_ref.assign(d->inv_mass_ref, d->inv_mass_ref + c->Np * c->Np);
 
   // packed geometry and side-ordered neighbours (Evolve.cpp:167-202)
@@ -592,7 +592,8 @@ vt_ctx* vt_create_structured(const vt_params* prm, const vt_vortex* ic_in, int d
   c->nfq = nfq;
   c->K = 2 * nx * ny;
   c->Kpad = (static_cast<long long>(c->K) + 127) / 128 * 128;
-  const vt::StageKernel sk = vt::select_kernel(p, nfq);
+  c->ops = vt::fold_operators(p, nfq, minv.data(), stiff.data(), line.data(), pp.data(), pm.data());
+  const vt::StageKernel sk = vt::select_kernel(p, nfq, c->ops.data());
   c->launch = sk.launch;
   int per_sm = 0, sms = 0;
   if ((e = vt::tensor_maps_available()) || (e = sk.configure(&per_sm)) ||
@@ -602,7 +603,6 @@ vt_ctx* vt_create_structured(const vt_params* prm, const vt_vortex* ic_in, int d
     return nullptr;
   }
   c->max_blocks = sms * (per_sm > 0 ? per_sm : 1);
-  c->ops = vt::fold_operators(p, nfq, minv.data(), stiff.data(), line.data(), pp.data(), pm.data());
   c->minv_ref = minv;
   c->side_pairing = true;
   std::vector<double> m(minv), W(Np, 0.0);
@@ -970,7 +970,7 @@ int vt_set_stage_mapping(vt_ctx* c, int mapping) {
     return fail(VT_ERR_INVALID, "vt_set_stage_mapping: mapping must be 0 (component) or 1 (pair)");
   std::lock_guard<std::mutex> lk(c->mu);
   cudaSetDevice(c->device);
-  const vt::StageKernel sk = vt::select_kernel(c->p, c->nfq, mapping);
+  const vt::StageKernel sk = vt::select_kernel(c->p, c->nfq, c->ops.data(), mapping);
   int per_sm = 0, sms = 0;
   cudaError_t e = sk.configure(&per_sm);
   if (!e) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);

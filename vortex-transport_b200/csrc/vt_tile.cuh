@@ -190,8 +190,8 @@ __device__ __forceinline__ void run_sync(int t) {
 
 // ---- warp mappings -------------------------------------------------------------------
 // Thread t of a block holds element column el = t % 64 and group g = t / 64
-// (uniform per warp; warps of equal parity hold one run). Two mappings of the
-// work onto (el, g), chosen per order p (StageKernel, vt_launch.cu):
+// (uniform per warp; warps of equal parity hold one run). Mappings of the work
+// onto threads (StageKernel, vt_launch.cu):
 //   component (kMapComponent): g is the conserved component c; the thread
 //     forms every face point's trace and every node's update of component c;
 //   pair (kMapPair): g = (half, h) with h the component pair of the HBM
@@ -201,6 +201,8 @@ __device__ __forceinline__ void run_sync(int t) {
 //     QH = ceil(nfq / 2), NH = ceil(Np / 2). Shared- and global-memory
 //     accesses are then 16 bytes wide (half the load/store instructions) for
 //     the same floating-point work.
+//   folded (kMapFolded): below, taken instead of the pair mapping where the
+//     operators reflect.
 // The face buffer holds the same bytes either way: [s][c][q][el] doubles for
 // the component mapping, [s][q][h][el] double2 for the pair mapping (and the
 // nodal flux [j][8][el] doubles or [j][4][el] double2).
@@ -273,6 +275,178 @@ __device__ __forceinline__ void pair_fold(const double2* S, int h, int el, doubl
   for (int i = 0; i < NH; ++i)
     if (base + i < NP) r[i] = make_double2(fma(f, S[sidx<NP>(2 * (base + i) + h, el)].x, r[i].x),
                                            fma(f, S[sidx<NP>(2 * (base + i) + h, el)].y, r[i].y));
+}
+
+// The folded mapping. The FP64 pipe was the most used unit of the stage kernel
+// (54% busy), and the lift and the volume operator 44% of its instructions: the
+// even / odd split (FoldedOps) takes 117 + 128 FP64 instructions per element
+// and component at p = 3, nfq = 6 for the two, where the pair mapping takes
+// 216 + 200. With roe_flux2 and the shorter nodal flux the stage's FP64
+// instructions fell from about 3770 to 2630 per element (p = 3, nfq = 6), and
+// a pass of 5 RK4 steps at 768 x 768, p = 3 from 9.89 to 8.72 ms, 384 x 384,
+// p = 1 (20 steps) from 5.41 to 4.78 ms, 64 x 64, p = 2 (50 steps) from 1.68 to
+// 1.48 ms, all against the pair mapping on one GPU in turn.
+// A thread holds one component of one element and all its
+// nodes, as the even and odd parts of the node pairs (FoldedOps). Within a warp
+// the lanes are 16 consecutive elements x the two components of one pair, so
+// an 8-byte access of a warp to a row of component pairs (state rows in global
+// memory and in the state tile, the face and flux buffers) is 256 contiguous
+// bytes: no bank conflicts, whole sectors. Warp w works on run w & 1, pair
+// (w >> 1) & 1, elements 16 (w >> 2) ... + 15 of the run.
+__device__ __forceinline__ int folded_column(int t) {
+  return ((t >> 5) & 1) * kTileRun + (t >> 7) * 16 + ((t & 31) >> 1);
+}
+__device__ __forceinline__ int folded_component(int t) { return ((t >> 6) & 1) * 2 + (t & 1); }
+
+template <int P, int NFQ>
+__device__ __forceinline__ void folded_traces(const FoldedOps<P, NFQ>& ops, const double2* S, double* FB, int t) {
+  constexpr int NP = np_of_p(P), NE = P + 1, ES = kTileElems + 1;
+  const int el = folded_column(t), c = folded_component(t), h = c >> 1, part = c & 1;
+  const double* Sd = reinterpret_cast<const double*>(S) + sidx<NP>(h, el) * 2 + part;
+  double* out = FB + (h * ES + el) * 2 + part;
+  double u[NP];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) u[i] = Sd[i * 4 * kTileRun];
+#pragma unroll
+  for (int s = 0; s < 3; ++s)
+#pragma unroll
+    for (int q = 0; q < NFQ; ++q) {
+      double v = 0.0;
+#pragma unroll
+      for (int k = 0; k < NE; ++k) v = fma(ops.tp[s][q][k], u[edge_node(P, s, k)], v);
+      out[(s * NFQ + q) * 4 * ES] = v;
+    }
+}
+
+template <int P, int NFQ>
+__device__ __forceinline__ void folded_lift(const FoldedOps<P, NFQ>& ops, const double* FB, int el, int c,
+                                            double2 lsa, double2 lsb, double* r) {
+  constexpr int ES = kTileElems + 1, NS = FoldedOps<P, NFQ>::NS, NO = FoldedOps<P, NFQ>::NO;
+  const double* F = FB + ((c >> 1) * ES + el) * 2 + (c & 1);
+#pragma unroll
+  for (int a = 0; a < NS + NO; ++a) r[a] = 0.0;
+#pragma unroll
+  for (int q = 0; q < NFQ; ++q) {
+    const double f0 = lsa.x * F[q * 4 * ES], f2 = F[(2 * NFQ + NFQ - 1 - q) * 4 * ES];
+    const double fe = fma(lsb.x, f2, f0), fo = fma(-lsb.x, f2, f0);
+#pragma unroll
+    for (int a = 0; a < NS; ++a) r[a] = fma(ops.Le[a][q], fe, r[a]);
+#pragma unroll
+    for (int a = 0; a < NO; ++a) r[NS + a] = fma(ops.Lo[a][q], fo, r[NS + a]);
+  }
+#pragma unroll
+  for (int q = 0; q < (NFQ + 1) / 2; ++q) {
+    const double f1 = lsa.y * F[(NFQ + q) * 4 * ES];
+    double fe = f1, fo = 0.0;
+    if (q < NFQ / 2) {
+      const double fm = F[(NFQ + NFQ - 1 - q) * 4 * ES];
+      fe = fma(lsa.y, fm, f1);
+      fo = fma(-lsa.y, fm, f1);
+    }
+#pragma unroll
+    for (int a = 0; a < NS; ++a) r[a] = fma(ops.L1e[a][q], fe, r[a]);
+    if (q < NFQ / 2) {
+#pragma unroll
+      for (int a = 0; a < NO; ++a) r[NS + a] = fma(ops.L1o[a][q], fo, r[NS + a]);
+    }
+  }
+}
+
+// Stage 3's U3 / (3 c_out) (f = 1 / (3 c_out)) added to the even and odd parts.
+template <int P>
+__device__ __forceinline__ void folded_state(const double2* S, int el, int c, double f, double* r) {
+  constexpr int NP = np_of_p(P), NS = fold_nodes(P), NO = fold_pairs(P);
+  const double* Sd = reinterpret_cast<const double*>(S) + sidx<NP>(c >> 1, el) * 2 + (c & 1);
+#pragma unroll
+  for (int a = 0; a < NS; ++a) {
+    const double u = Sd[fold_node(P, a) * 4 * kTileRun];
+    if (a < NO) {
+      const double v = Sd[mirror_node(P, fold_node(P, a)) * 4 * kTileRun];
+      r[a] = fma(0.5 * f, u + v, r[a]);
+      r[NS + a] = fma(0.5 * f, u - v, r[NS + a]);
+    } else {
+      r[a] = fma(f, u, r[a]);
+    }
+  }
+}
+
+// The nodal flux in the form that folded_volume reads: for node j with mirror
+// image Pj, rows j*4 + h hold Gxi_j + Geta_Pj and rows j*4 + 2 + h
+// Gxi_j - Geta_Pj (component pair h). A thread takes both nodes of a pair, or
+// one fixed node, for column `col`.
+template <int P>
+__device__ __forceinline__ void folded_nodal_flux(const double2* S, double2* G2, int col, int grp, double2 j0,
+                                                  double2 j1) {
+  constexpr int NP = np_of_p(P), ES = kTileElems + 1, NS = fold_nodes(P), NO = fold_pairs(P);
+  auto flux = [&](int j, double* gxi, double* geta) {
+    const double2 s0 = S[sidx<NP>(2 * j, col)], s1 = S[sidx<NP>(2 * j + 1, col)];
+    const double sv[4] = {s0.x, s0.y, s1.x, s1.y};
+    contravariant_flux(sv, j0.x, j0.y, j1.x, j1.y, gxi, geta);
+  };
+  auto store = [&](int j, const double* gxi, const double* geta) {
+    double2* g = G2 + j * 4 * ES + col;
+    g[0] = make_double2(gxi[0] + geta[0], gxi[1] + geta[1]);
+    g[ES] = make_double2(gxi[2] + geta[2], gxi[3] + geta[3]);
+    g[2 * ES] = make_double2(gxi[0] - geta[0], gxi[1] - geta[1]);
+    g[3 * ES] = make_double2(gxi[2] - geta[2], gxi[3] - geta[3]);
+  };
+#pragma unroll
+  for (int u0 = 0; u0 < NS; u0 += 4) {
+    const int u = u0 + grp;  // uniform per warp
+    if (u >= NS) break;
+    int j = 0;
+#pragma unroll
+    for (int k = u0; k < u0 + 4 && k < NS; ++k)
+      if (u == k) j = fold_node(P, k);
+    double gxi[4], geta[4];
+    flux(j, gxi, geta);
+    if (u < NO) {
+      int m = 0;
+#pragma unroll
+      for (int k = u0; k < u0 + 4 && k < NO; ++k)
+        if (u == k) m = mirror_node(P, fold_node(P, k));
+      double hxi[4], heta[4];
+      flux(m, hxi, heta);
+      store(j, gxi, heta);
+      store(m, hxi, geta);
+    } else {
+      store(j, gxi, geta);
+    }
+  }
+}
+
+template <int P, int NFQ>
+__device__ __forceinline__ void folded_volume(const FoldedOps<P, NFQ>& ops, const double* FB, int el, int c,
+                                              double* r) {
+  constexpr int NP = np_of_p(P), ES = kTileElems + 1, NS = FoldedOps<P, NFQ>::NS, NO = FoldedOps<P, NFQ>::NO;
+  const double* G = FB + ((c >> 1) * ES + el) * 2 + (c & 1);
+#pragma unroll
+  for (int j = 0; j < NP; ++j) {
+    const double ge = G[j * 8 * ES], go = G[(j * 8 + 4) * ES];
+#pragma unroll
+    for (int a = 0; a < NS; ++a) r[a] = fma(ops.De[a][j], ge, r[a]);
+#pragma unroll
+    for (int a = 0; a < NO; ++a) r[NS + a] = fma(ops.Do[a][j], go, r[NS + a]);
+  }
+}
+
+// Even and odd parts -> the nodes' own values, in place.
+template <int P>
+__device__ __forceinline__ void unfold(double* r) {
+  constexpr int NP = np_of_p(P), NS = fold_nodes(P), NO = fold_pairs(P);
+  double v[NP];
+#pragma unroll
+  for (int a = 0; a < NS; ++a) {
+    const int j = fold_node(P, a);
+    if (a < NO) {
+      v[j] = r[a] + r[NS + a];
+      v[mirror_node(P, j)] = r[a] - r[NS + a];
+    } else {
+      v[j] = r[a];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NP; ++i) r[i] = v[i];
 }
 
 // Non-coherent loads issued where they are written, so that the stage
@@ -369,10 +543,21 @@ __device__ __forceinline__ void pair_update(const StageArgs& a, int e, int h, do
 }
 
 template <int P, int NFQ, int MAP>
+struct OpsOfMap {
+  using type = StageOps<P, NFQ>;
+};
+template <int P, int NFQ>
+struct OpsOfMap<P, NFQ, kMapFolded> {
+  using type = FoldedOps<P, NFQ>;
+};
+template <int P, int NFQ, int MAP>
+using OpsOf = typename OpsOfMap<P, NFQ, MAP>::type;
+
+template <int P, int NFQ, int MAP>
 // Three 256-thread blocks per SM (<= 80 registers per thread) keep 24 warps
 // resident alongside 3 x ~75 KB of shared memory.
 __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __grid_constant__ StageArgs a,
-                                                                        const StageOps<P, NFQ> ops) {
+                                                                        const OpsOf<P, NFQ, MAP> ops) {
   using L = TileLayout<P, NFQ>;
   constexpr int E = L::E;
   constexpr int NP = L::NP;
@@ -380,6 +565,8 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
   constexpr int ES = L::ES;
   constexpr int T = 4 * E;
   constexpr bool PAIR = MAP == kMapPair;
+  constexpr bool FOLD = MAP == kMapFolded;
+  constexpr bool D2 = PAIR || FOLD;  // the face and flux buffers hold component pairs
   extern __shared__ __align__(128) unsigned char smem[];
   double2* S = reinterpret_cast<double2*>(smem + L::kS);
   double2* H = reinterpret_cast<double2*>(smem + L::kH);
@@ -493,6 +680,8 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
     if constexpr (PAIR) {
       if (grp >> 1) pair_traces<P, NFQ, 1>(ops, S, FB2, grp & 1, col);
       else pair_traces<P, NFQ, 0>(ops, S, FB2, grp & 1, col);
+    } else if constexpr (FOLD) {
+      folded_traces<P, NFQ>(ops, S, FB, t);
     } else {
       const int cc = grp, el = col;
       const double* Sd = reinterpret_cast<const double*>(S);
@@ -525,7 +714,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
       const int e = EL[el];
       const double2 n = __ldg(a.geo + (2 + s) * KP + e);
       double up[4], um[4];
-      if constexpr (PAIR) {
+      if constexpr (D2) {
         const double2 x0 = FB2[((s * NFQ + q) * 2) * ES + el], x1 = FB2[((s * NFQ + q) * 2 + 1) * ES + el];
         up[0] = x0.x, up[1] = x0.y, up[2] = x1.x, up[3] = x1.y;
       } else {
@@ -533,7 +722,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
         for (int c = 0; c < 4; ++c) up[c] = FB[((s * 4 + c) * NFQ + q) * ES + el];
       }
       if (mirror) {
-        if constexpr (PAIR) {
+        if constexpr (D2) {
           const double2 y0 = FB2[((s * NFQ + qm) * 2) * ES + nl], y1 = FB2[((s * NFQ + qm) * 2 + 1) * ES + nl];
           um[0] = y0.x, um[1] = y0.y, um[2] = y1.x, um[3] = y1.y;
         } else {
@@ -564,9 +753,9 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
         }
       }
       double f[4];
-      const int code = roe_flux(up, um, n.x, n.y, f);
+      const int code = roe_flux2(up, um, n.x, n.y, f);
       if (code) record_error(a, NFQ, e, q, s, code);
-      if constexpr (PAIR) {
+      if constexpr (D2) {
         FB2[((s * NFQ + q) * 2) * ES + el] = make_double2(f[0], f[1]);
         FB2[((s * NFQ + q) * 2 + 1) * ES + el] = make_double2(f[2], f[3]);
         if (mirror) {
@@ -597,24 +786,30 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
     }
 
     // ---- 4. lift ---------------------------------------------------------------------------
-    const int el = col;
+    const int el = FOLD ? folded_column(t) : col;
     const int e = EL[el];
     const bool valid = e >= 0;
     const int eg = valid ? e : 0;
     constexpr int NH = (NP + 1) / 2;
-    constexpr int NR = PAIR ? NH : NP;  // accumulators: double2 per node pair, or one double per node
     double2 r2[PAIR ? NH : 1];
-    double r[PAIR ? 1 : NP];
+    double r[PAIR ? 1 : NP];  // FOLD: the even parts, then the odd parts, of the node pairs
+    const int cc = FOLD ? folded_component(t) : grp;  // this thread's component (not PAIR)
     {
-      const double2 lsa = __ldg(a.geo + 5 * KP + eg);
-      const double2 lsb = __ldg(a.geo + 6 * KP + eg);
-      if constexpr (PAIR) {
+      double2 lsa = __ldg(a.geo + 5 * KP + eg);
+      double2 lsb = __ldg(a.geo + 6 * KP + eg);
+      if constexpr (!FOLD) {  // half of the doubled flux (FoldedOps' lift carries the half)
+        lsa.x *= 0.5, lsa.y *= 0.5;
+        lsb.x *= 0.5;
+      }
+      if constexpr (FOLD) {
+        folded_lift<P, NFQ>(ops, FB, el, cc, lsa, lsb, r);
+      } else if constexpr (PAIR) {
 #pragma unroll
         for (int i = 0; i < NH; ++i) r2[i] = make_double2(0.0, 0.0);
         if (grp >> 1) pair_lift<P, NFQ, 1>(ops, FB2, grp & 1, el, lsa, lsb, r2);
         else pair_lift<P, NFQ, 0>(ops, FB2, grp & 1, el, lsa, lsb, r2);
       } else {
-        const int c = grp;
+        const int c = cc;
 #pragma unroll
         for (int i = 0; i < NP; ++i) r[i] = 0.0;
 #pragma unroll
@@ -637,14 +832,15 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
       if constexpr (PAIR) {
         if (grp >> 1) pair_fold<P, 1>(S, grp & 1, el, f, r2);
         else pair_fold<P, 0>(S, grp & 1, el, f, r2);
+      } else if constexpr (FOLD) {
+        folded_state<P>(S, el, cc, f, r);
       } else {
-        const int c = grp;
+        const int c = cc;
         const double* Sd = reinterpret_cast<const double*>(S);
 #pragma unroll
         for (int i = 0; i < NP; ++i) r[i] = fma(f, Sd[sidx<NP>(2 * i + (c >> 1), el) * 2 + (c & 1)], r[i]);
       }
     }
-    (void)NR;
     run_sync(t);
 
     // the next tile's neighbour table, now that the run's barrier has made its
@@ -658,23 +854,28 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
 
     // ---- 5. nodal flux of every node, once, contracted with the inverse Jacobian --------
     if (P > 0) {
-      const double2 j0 = __ldg(a.geo + 0 * KP + eg);
-      const double2 j1 = __ldg(a.geo + 1 * KP + eg);
-      for (int j = grp; j < NP; j += 4) {
-        const double2 s0 = S[sidx<NP>(2 * j, el)], s1 = S[sidx<NP>(2 * j + 1, el)];
-        const double sv[4] = {s0.x, s0.y, s1.x, s1.y};
-        double gxi[4], geta[4];
-        contravariant_flux(sv, j0.x, j0.y, j1.x, j1.y, gxi, geta);
-        if constexpr (PAIR) {  // G2[j][0..1] xi pairs, G2[j][2..3] eta pairs
-          FB2[(j * 4 + 0) * ES + el] = make_double2(gxi[0], gxi[1]);
-          FB2[(j * 4 + 1) * ES + el] = make_double2(gxi[2], gxi[3]);
-          FB2[(j * 4 + 2) * ES + el] = make_double2(geta[0], geta[1]);
-          FB2[(j * 4 + 3) * ES + el] = make_double2(geta[2], geta[3]);
-        } else {  // G[j][0..3] xi, G[j][4..7] eta
+      const int egc = FOLD ? max(EL[col], 0) : eg;  // this phase's column is `col` in every mapping
+      const double2 j0 = __ldg(a.geo + 0 * KP + egc);
+      const double2 j1 = __ldg(a.geo + 1 * KP + egc);
+      if constexpr (FOLD) {
+        folded_nodal_flux<P>(S, FB2, col, grp, j0, j1);
+      } else {
+        for (int j = grp; j < NP; j += 4) {
+          const double2 s0 = S[sidx<NP>(2 * j, el)], s1 = S[sidx<NP>(2 * j + 1, el)];
+          const double sv[4] = {s0.x, s0.y, s1.x, s1.y};
+          double gxi[4], geta[4];
+          contravariant_flux(sv, j0.x, j0.y, j1.x, j1.y, gxi, geta);
+          if constexpr (PAIR) {  // G2[j][0..1] xi pairs, G2[j][2..3] eta pairs
+            FB2[(j * 4 + 0) * ES + el] = make_double2(gxi[0], gxi[1]);
+            FB2[(j * 4 + 1) * ES + el] = make_double2(gxi[2], gxi[3]);
+            FB2[(j * 4 + 2) * ES + el] = make_double2(geta[0], geta[1]);
+            FB2[(j * 4 + 3) * ES + el] = make_double2(geta[2], geta[3]);
+          } else {  // G[j][0..3] xi, G[j][4..7] eta
 #pragma unroll
-          for (int cc = 0; cc < 4; ++cc) {
-            FB[(j * 8 + cc) * ES + el] = gxi[cc];
-            FB[(j * 8 + 4 + cc) * ES + el] = geta[cc];
+            for (int c = 0; c < 4; ++c) {
+              FB[(j * 8 + c) * ES + el] = gxi[c];
+              FB[(j * 8 + 4 + c) * ES + el] = geta[c];
+            }
           }
         }
       }
@@ -716,7 +917,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
       for (int i = 0; i < NH; ++i)
         pre2[i] = upd && half * NH + i < NP ? ld_early2(src + o + i * 2 * KP) : make_double2(0.0, 0.0);
     } else {
-      const int c = grp;
+      const int c = cc;
       const double* s1 = reinterpret_cast<const double*>(src) + ((c >> 1) * KP + eg) * 2 + (c & 1);
 #pragma unroll
       for (int i = 0; i < NP; ++i) pre[i] = upd ? ld_early(s1 + i * 4 * KP) : 0.0;
@@ -727,8 +928,10 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
       if constexpr (PAIR) {
         if (grp >> 1) pair_volume<P, NFQ, 1>(ops, FB2, grp & 1, el, r2);
         else pair_volume<P, NFQ, 0>(ops, FB2, grp & 1, el, r2);
+      } else if constexpr (FOLD) {
+        folded_volume<P, NFQ>(ops, FB, el, cc, r);
       } else {
-        const int c = grp;
+        const int c = cc;
 #pragma unroll
         for (int j = 0; j < NP; ++j) {
           const double gx = FB[(j * 8 + c) * ES + el];
@@ -739,6 +942,8 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
       }
     }
 
+    if constexpr (FOLD) unfold<P>(r);
+
     // ---- 6b. stage update ------------------------------------------------------------------
     if (valid) {
       const double dtt = a.tile_dt ? __ldg(a.tile_dt + tile) : 1.0;
@@ -747,7 +952,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
         if (grp >> 1) pair_update<P, 1>(a, e, grp & 1, c_acc, c_out, r2, pre2);
         else pair_update<P, 0>(a, e, grp & 1, c_acc, c_out, r2, pre2);
       } else {
-        const int c = grp, h = c >> 1, part = c & 1;
+        const int c = cc, h = c >> 1, part = c & 1;
         const long long off0 = (h * KP + e) * 2 + part;  // node 0; node i adds i * 4 * KP
         double* acc = reinterpret_cast<double*>(a.acc) + off0;
         double* out = reinterpret_cast<double*>(a.out) + off0;
