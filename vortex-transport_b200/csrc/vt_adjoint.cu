@@ -37,8 +37,8 @@ namespace {
 using FaceFn = cudaError_t (*)(const AdjArgs&, const double*, cudaStream_t);
 using TileFn = cudaError_t (*)(const AdjArgs&, const double*, int, cudaStream_t);
 using TileConfigFn = cudaError_t (*)(int*);
-using JvpFn = cudaError_t (*)(const double2*, const double2*, double2*, const double2*, const int4*, long long,
-                              int, const double*, cudaStream_t);
+using JvpFn = cudaError_t (*)(const double2*, const double2*, double2*, const double2*, const int4*, const int*,
+                              long long, const double*, cudaStream_t);
 
 struct AdjKernels {
   FaceFn face = nullptr;
@@ -52,7 +52,7 @@ template <int P, int NFQ>
 cudaError_t launch_face(const AdjArgs& a, const double* ops, cudaStream_t st) {
   StageOps<P, NFQ> o;
   std::memcpy(&o, ops, sizeof(o));
-  const dim3 grid((a.K + kAdjRun - 1) / kAdjRun, 3), block(kAdjRun, NFQ);
+  const dim3 grid(static_cast<unsigned>(a.ncols / kAdjRun), 3), block(kAdjRun, NFQ);
   adjoint_face_kernel<P, NFQ><<<grid, block, 0, st>>>(a, o);
   return cudaGetLastError();
 }
@@ -61,7 +61,7 @@ template <int P, int NFQ>
 cudaError_t launch_element(const AdjArgs& a, const double* ops, cudaStream_t st) {
   StageOps<P, NFQ> o;
   std::memcpy(&o, ops, sizeof(o));
-  const dim3 grid((a.K + kAdjRun - 1) / kAdjRun), block(kAdjRun, np_of_p(P));
+  const dim3 grid(static_cast<unsigned>(a.ncols / kAdjRun)), block(kAdjRun, np_of_p(P));
   adjoint_element_kernel<P, NFQ><<<grid, block, 0, st>>>(a, o);
   return cudaGetLastError();
 }
@@ -72,12 +72,9 @@ cudaError_t launch_tile(const AdjArgs& a, const double* ops, int max_blocks, cud
   StageOps<P, NFQ> o;
   std::memcpy(&o, ops, sizeof(o));
   const int grid = a.ntiles < max_blocks ? a.ntiles : max_blocks;
-  // the tensor maps of this launch's stage state and stage adjoint (host-side encoding, no allocation)
-  AdjArgs k = a;
-  cudaError_t e = encode_state_map(&k.map_U, a.U, a.Kpad, np_of_p(P));
-  if (!e) e = encode_state_map(&k.map_a, a.a, a.Kpad, np_of_p(P));
-  if (e) return e;
-  adjoint_tile_kernel<P, NFQ><<<grid, 4 * kTileElems, AdjTileLayout<P, NFQ>::kBytes, st>>>(k, o);
+  FoldedOps<P, NFQ> fo;
+  fold_operators(o, &fo);
+  adjoint_tile_kernel<P, NFQ><<<grid, 4 * kTileElems, AdjTileLayout<P, NFQ>::kBytes, st>>>(a, o, fo);
   return cudaGetLastError();
 }
 
@@ -92,10 +89,10 @@ cudaError_t configure_tile(int* blocks_per_sm) {
 
 template <int P, int NFQ>
 cudaError_t launch_jvp(const double2* U, const double2* V, double2* dR, const double2* geo, const int4* nbr,
-                       long long KP, int K, const double* ops, cudaStream_t st) {
+                       const int* elem, long long ncols, const double* ops, cudaStream_t st) {
   StageOps<P, NFQ> o;
   std::memcpy(&o, ops, sizeof(o));
-  rhs_jvp_kernel<P, NFQ><<<(K + 127) / 128, 128, 0, st>>>(U, V, dR, geo, nbr, KP, K, o);
+  rhs_jvp_kernel<P, NFQ><<<static_cast<unsigned>((ncols + 127) / 128), 128, 0, st>>>(U, V, dR, geo, nbr, elem, ncols, o);
   return cudaGetLastError();
 }
 
@@ -209,14 +206,16 @@ int setup(vt_ctx* c) {
   // other with opposite normals; a 2-colouring of the element adjacency
   // (breadth first) tells such meshes (the reference's type-0 / type-1
   // triangles) from ones with self-neighbours or odd cycles.
-  std::vector<int4> nb(static_cast<size_t>(c->K));
+  std::vector<int4> nb(static_cast<size_t>(c->ncols));
+  std::vector<int> elem(nb.size());
   cudaError_t e = cudaMemcpy(nb.data(), c->nbr, sizeof(int4) * nb.size(), cudaMemcpyDeviceToHost);
+  if (!e) e = cudaMemcpy(elem.data(), c->elem, sizeof(int) * elem.size(), cudaMemcpyDeviceToHost);
   if (e) return fail(VT_ERR_CUDA, cuda_msg("adjoint: neighbours", e));
   std::vector<signed char> col(nb.size(), -1);
   std::vector<int> queue;
   bool ok = true;
-  for (int start = 0; start < c->K && ok; ++start) {
-    if (col[start] >= 0) continue;
+  for (int start = 0; start < static_cast<int>(nb.size()) && ok; ++start) {
+    if (elem[start] < 0 || col[start] >= 0) continue;
     col[start] = 0;
     queue.assign(1, start);
     for (size_t h = 0; h < queue.size() && ok; ++h) {
@@ -232,11 +231,11 @@ int setup(vt_ctx* c) {
       }
     }
   }
-  // the fused reverse stage runs on the stage kernel's tiles
+  // the fused reverse stage runs on the stage kernel's tiles, with the folded operators
   int tile_blocks = 0;
-  if (ok) {
+  if (ok && operators_reflect(c->p, c->nfq, c->ops.data())) {
     int per_sm = 0, sms = 0;
-    if (c->tiles && c->ntiles > 0 && !k.tile_config(&per_sm) &&
+    if (c->ntiles > 0 && !k.tile_config(&per_sm) &&
         !cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) && per_sm > 0)
       tile_blocks = sms * per_sm;
     cudaGetLastError();
@@ -244,8 +243,8 @@ int setup(vt_ctx* c) {
   // eleven state vectors, plus the face adjoints of the two-launch form when
   // that form is the one used
   constexpr int kVectors = 11;
-  const size_t state_elems = static_cast<size_t>(2 * c->Np) * static_cast<size_t>(c->Kpad);
-  const size_t face_elems = tile_blocks > 0 ? 0 : static_cast<size_t>(6 * c->nfq) * static_cast<size_t>(c->Kpad);
+  const size_t state_elems = static_cast<size_t>(2 * c->Np) * static_cast<size_t>(c->ncols);
+  const size_t face_elems = tile_blocks > 0 ? 0 : static_cast<size_t>(6 * c->nfq) * static_cast<size_t>(c->ncols);
   const size_t total = kVectors * state_elems + 2 * face_elems;
   double2* bufs = nullptr;
   e = cudaMalloc(reinterpret_cast<void**>(&bufs), sizeof(double2) * total);
@@ -351,16 +350,14 @@ AdjArgs adj_args(vt_ctx* c) {
   AdjArgs a{};
   a.bp = c->adj->bp;
   a.bm = c->adj->bm;
-  a.elem_dt = c->elem_dt;
+  a.tile_dt = c->tile_dt;
   a.geo = c->geo;
   a.nbr = c->nbr;
-  a.tiles = c->tiles;
-  a.tile_items = c->tile_items;
-  a.tile_count = c->tile_count;
+  a.elem = c->elem;
+  a.lists = c->lists;
   a.ntiles = c->ntiles;
   a.err = c->err;
-  a.Kpad = c->Kpad;
-  a.K = c->K;
+  a.ncols = c->ncols;
   a.sa = 1.0;
   return a;
 }
@@ -485,15 +482,15 @@ cudaError_t run_plan_overlapped(vt_ctx* c, size_t begin, size_t end) {
 
 // Host or device AoS array -> SoA buffer on the context's stream.
 cudaError_t load_aos(vt_ctx* c, const double* src, int device_pointers, double2* dst) {
-  if (device_pointers) return aos_to_soa(c, src, dst);
+  if (device_pointers) return to_columns(c, src, dst);
   cudaError_t e = cudaMemcpyAsync(c->aos, src, sizeof(double) * 4 * static_cast<size_t>(c->K) * c->Np,
                                   cudaMemcpyHostToDevice, c->stream);
-  return e ? e : aos_to_soa(c, reinterpret_cast<const double*>(c->aos), dst);
+  return e ? e : to_columns(c, reinterpret_cast<const double*>(c->aos), dst);
 }
 
 cudaError_t store_aos(vt_ctx* c, const double2* src, double* dst, int device_pointers) {
-  if (device_pointers) return soa_to_aos(c, src, dst);
-  cudaError_t e = soa_to_aos(c, src, reinterpret_cast<double*>(c->aos));
+  if (device_pointers) return from_columns(c, src, dst);
+  cudaError_t e = from_columns(c, src, reinterpret_cast<double*>(c->aos));
   if (!e)
     e = cudaMemcpyAsync(dst, c->aos, sizeof(double) * 4 * static_cast<size_t>(c->K) * c->Np, cudaMemcpyDeviceToHost,
                         c->stream);
@@ -690,7 +687,7 @@ int vt_rhs_jvp(vt_ctx* c, const double* U, const double* V, double* dR, int devi
   s->fresh = false;
   cudaError_t e = vt::load_aos(c, U, device_pointers, s->s1);
   if (!e) e = vt::load_aos(c, V, device_pointers, s->s2);
-  if (!e) e = s->k.jvp(s->s1, s->s2, s->s3, c->geo, c->nbr, c->Kpad, c->K, c->ops.data(), c->stream);
+  if (!e) e = s->k.jvp(s->s1, s->s2, s->s3, c->geo, c->nbr, c->elem, c->ncols, c->ops.data(), c->stream);
   if (!e) e = vt::store_aos(c, s->s3, dR, device_pointers);
   if (!e) e = cudaStreamSynchronize(c->stream);
   return e ? fail(VT_ERR_CUDA, vt::cuda_msg("rhs jvp", e)) : VT_OK;
@@ -733,7 +730,7 @@ int vt_tangent_rk4(vt_ctx* c, double dt, int nsteps, const double* dU_0, double*
   double2 *dX = s->a0, *dS = s->a1, *dacc = s->acc, *dk = s->lam;
   const double2* X = c->U;
   auto jvp = [&](const double2* at, const double2* v) {
-    return s->k.jvp(at, v, dk, c->geo, c->nbr, c->Kpad, c->K, c->ops.data(), c->stream);
+    return s->k.jvp(at, v, dk, c->geo, c->nbr, c->elem, c->ncols, c->ops.data(), c->stream);
   };
   cudaError_t e = vt::load_aos(c, dU_0, device_pointers, dX);
   if (!e) e = vt::reset_error_words(c);

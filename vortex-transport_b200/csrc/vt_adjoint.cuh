@@ -1,10 +1,10 @@
 // Derivatives of the pointwise pieces of the right-hand side, for the
 // discrete adjoint and the tangent-linear model:
 //
-//   roe_flux_vjp         reverse sweep of roe_flux (vt_device.cuh): given the
-//                        adjoint of the flux, the adjoints of both states,
-//                        through the Roe averages, the c2^2 "sound speed" and
-//                        the entropy fix (Numericalflux.cpp:99-156);
+//   roe_flux2_vjp        reverse sweep of roe_flux2 (vt_device.cuh): given the
+//                        adjoint of the doubled flux, the adjoints of both
+//                        states, through the Roe averages, the c2^2 "sound
+//                        speed" and the entropy fix (Numericalflux.cpp:99-156);
 //   contravariant_vjp    reverse sweep of contravariant_flux (the nodal Euler
 //                        flux of Timestepping.cpp:141-158 contracted with J^-1);
 //   Dual<N>, roe_flux_t,
@@ -29,6 +29,15 @@ __host__ __device__ inline double rcp(double x) {
   return recip_nr(x);
 #else
   return 1.0 / x;
+#endif
+}
+
+// 1/sqrt(x), likewise: rsqrt_nr on the device, IEEE operations on the host.
+__host__ __device__ inline double rsq(double x) {
+#ifdef __CUDA_ARCH__
+  return rsqrt_nr(x);
+#else
+  return 1.0 / sqrt(x);
 #endif
 }
 
@@ -111,7 +120,7 @@ __host__ __device__ inline double val(double a) { return a; }
 __host__ __device__ inline double dsqrt(double a) { return sqrt(a); }
 __host__ __device__ inline double dabs(double a) { return fabs(a); }
 
-// ---- forward formulas on any scalar type (the algebra of roe_flux) --------------
+// ---- forward formulas on any scalar type ------------------------------------------
 template <typename T>
 __host__ __device__ inline int roe_flux_t(const T* uL, const T* uR, double nx, double ny, T* f) {
   const T rL = uL[0], rR = uR[0];
@@ -177,243 +186,154 @@ __host__ __device__ inline void contravariant_flux_t(const T* s, double j00, dou
 }
 
 // ---- reverse sweeps ------------------------------------------------------------------
-// bf: adjoint of the flux (4). Adds the adjoints of uL and uR to buL, buR.
-__host__ __device__ inline void roe_flux_vjp(const double* uL, const double* uR, double nx, double ny,
-                                             const double* bf, double* buL, double* buR) {
-  // forward recomputation of the intermediates
+// b: adjoint of roe_flux2's doubled flux (4); writes the adjoints of uL and uR
+// to buL, buR. The reverse sweep of roe_flux2's own arrangement: about 190 FP64
+// instructions, where the sweep of the flux written through both sides'
+// velocities and enthalpies took about 360 (the reverse stage is bound by
+// them: FP64 pipe 44% busy at two blocks per SM). What makes it short:
+//   C1 = A / ci, G1 = (gamma-1) X / ci: the adjoint of 1/ci is needed only as
+//     -(bA A + bG1 G1) / ci added to that of ci;
+//   the averages x = (g xR + xL) / s with s = rhoL + w: the adjoint of s is
+//     -sum (bx / s) x, and g = sqrt(rhoL/rhoR), w = sqrt(rhoL rhoR) have the
+//     logarithmic derivatives -+ 1/2 and 1/2;
+//   for |u_n| < 7/8 ci the acoustic part is (|l0| + |l1|)/2 = ci and
+//     (|l0| - |l1|)/2 = u_n.
+__host__ __device__ inline void roe_flux2_vjp(const double* uL, const double* uR, double nx, double ny,
+                                              const double* b, double* buL, double* buR) {
+  // forward
   const double rL = uL[0], rR = uR[0];
-  const double irLR = rcp(rL * rR);
+  const double rLR = rL * rR;
+  const double y = rsq(rLR);
+  const double irLR = y * y, w = rLR * y;
   const double irL = rR * irLR, irR = rL * irLR;
-  const double vxL = uL[1] * irL, vyL = uL[2] * irL;
-  const double unL = vxL * nx + vyL * ny;
-  const double pL = kGm1 * (uL[3] - 0.5 * (uL[1] * vxL + uL[2] * vyL));
-  const double rHL = uL[3] + pL;
-  const double HL = rHL * irL;
-  const double vxR = uR[1] * irR, vyR = uR[2] * irR;
-  const double unR = vxR * nx + vyR * ny;
-  const double pR = kGm1 * (uR[3] - 0.5 * (uR[1] * vxR + uR[2] * vyR));
-  const double rHR = uR[3] + pR;
-  const double HR = rHR * irR;
-  const double du0 = uR[0] - uL[0], du1 = uR[1] - uL[1], du2 = uR[2] - uL[2], du3 = uR[3] - uL[3];
-  const double di = sqrt(rR * irL);
-  const double d1 = rcp(1.0 + di);
-  const double ui = (di * vxR + vxL) * d1;
-  const double vi = (di * vyR + vyL) * d1;
-  const double Hi = (di * HR + HL) * d1;
-  const double af = 0.5 * (ui * ui + vi * vi);
+  const double unL = (uL[1] * nx + uL[2] * ny) * irL, unR = (uR[1] * nx + uR[2] * ny) * irR;
+  const double kinL = (uL[1] * uL[1] + uL[2] * uL[2]) * irL, kinR = (uR[1] * uR[1] + uR[2] * uR[2]) * irR;
+  const double rHL = uL[3] + kGm1 * (uL[3] - 0.5 * kinL), rHR = uR[3] + kGm1 * (uR[3] - 0.5 * kinR);
+  const double du0 = rR - rL, du1 = uR[1] - uL[1], du2 = uR[2] - uL[2], du3 = uR[3] - uL[3];
+  const double g = w * irR;
+  const double d1 = rcp(rL + w);
+  const double ui = (g * uR[1] + uL[1]) * d1, vi = (g * uR[2] + uL[2]) * d1, Hi = (g * rHR + rHL) * d1;
+  const double h = 0.5 * (ui * ui + vi * vi);
   const double ucp = ui * nx + vi * ny;
-  const double c2 = kGm1 * (Hi - af);
+  const double c2 = kGm1 * (Hi - h);
   const double ci = c2 * c2;
   const double ci1 = rcp(ci);
-  const double eps = 0.1 * ci;
-  const double ieps = 10.0 * ci1;
-  const double l0r = ucp + ci, l1r = ucp - ci, l3r = ucp;
-  const bool fx0 = fabs(l0r) < eps, fx1 = fabs(l1r) < eps, fx3 = fabs(l3r) < eps;
-  const double L0 = fx0 ? 0.5 * (eps + l0r * l0r * ieps) : fabs(l0r);
-  const double L1 = fx1 ? 0.5 * (eps + l1r * l1r * ieps) : fabs(l1r);
-  const double L3 = fx3 ? 0.5 * (eps + l3r * l3r * ieps) : fabs(l3r);
-  const double s1 = 0.5 * (L0 + L1);
-  const double s2 = 0.5 * (L0 - L1);
-  const double G1 = kGm1 * (af * du0 - ui * du1 - vi * du2 + du3);
-  const double G2 = -ucp * du0 + du1 * nx + du2 * ny;
-  const double A = G1 * (s1 - L3) * ci1 + G2 * s2;
+  const double t = ucp * ci1;
+  // l3 with its derivatives by u_n and ci
+  const bool fix = fabs(t) < 0.1;
+  const double l3 = fix ? 5.0 * ucp * t + 0.05 * ci : fabs(ucp);
+  const double l3u = fix ? 10.0 * t : (ucp < 0 ? -1.0 : 1.0);
+  const double l3c = fix ? 0.05 - 5.0 * t * t : 0.0;
+  const bool usual = fabs(t) < 0.875;
+  double s1 = ci, s2 = ucp;  // (|l0| + |l1|)/2 and (|l0| - |l1|)/2
+  double l0u = 1.0, l0c = 0.0, l1u = -1.0, l1c = 0.0;
+  if (!usual) {
+    const double l0r = ucp + ci, l1r = ucp - ci, eps = 0.1 * ci;
+    double l0 = fabs(l0r), l1 = fabs(l1r);
+    l0u = l0r < 0 ? -1.0 : 1.0;
+    l1u = l1r < 0 ? -1.0 : 1.0;
+    if (l0 < eps) {
+      const double z = l0r * ci1;
+      l0 = 5.0 * l0r * z + 0.05 * ci, l0u = 10.0 * z, l0c = 0.05 - 5.0 * z * z;
+    }
+    if (l1 < eps) {
+      const double z = l1r * ci1;
+      l1 = 5.0 * l1r * z + 0.05 * ci, l1u = 10.0 * z, l1c = 0.05 - 5.0 * z * z;
+    }
+    s1 = 0.5 * (l0 + l1);
+    s2 = 0.5 * (l0 - l1);
+  }
+  const double s1l3 = s1 - l3;
+  const double k1 = kGm1 * ci1;
+  const double G1 = k1 * (h * du0 - ui * du1 - vi * du2 + du3);
+  const double G2 = du1 * nx + du2 * ny - ucp * du0;
+  const double A = G1 * s1l3 + G2 * s2;
   const double C1 = A * ci1;
-  const double C2 = G1 * s2 * ci1 + G2 * (s1 - L3);
+  const double C2 = G1 * s2 + G2 * s1l3;
 
-  // flux assembly
-  double b_uL1 = 0.5 * bf[0] * nx + 0.5 * bf[1] * unL;
-  double b_uL2 = 0.5 * bf[0] * ny + 0.5 * bf[2] * unL;
-  double b_uR1 = 0.5 * bf[0] * nx + 0.5 * bf[1] * unR;
-  double b_uR2 = 0.5 * bf[0] * ny + 0.5 * bf[2] * unR;
-  double b_unL = 0.5 * (bf[1] * uL[1] + bf[2] * uL[2] + bf[3] * rHL);
-  double b_unR = 0.5 * (bf[1] * uR[1] + bf[2] * uR[2] + bf[3] * rHR);
-  double b_pL = 0.5 * (bf[1] * nx + bf[2] * ny);
-  double b_pR = b_pL;
-  double b_rHL = 0.5 * bf[3] * unL;
-  double b_rHR = 0.5 * bf[3] * unR;
-  double b_L3 = -0.5 * (bf[0] * du0 + bf[1] * du1 + bf[2] * du2 + bf[3] * du3);
-  double b_du0 = -0.5 * L3 * bf[0], b_du1 = -0.5 * L3 * bf[1];
-  double b_du2 = -0.5 * L3 * bf[2], b_du3 = -0.5 * L3 * bf[3];
-  const double b_C1 = -0.5 * (bf[0] + bf[1] * ui + bf[2] * vi + bf[3] * Hi);
-  const double b_C2 = -0.5 * (bf[1] * nx + bf[2] * ny + bf[3] * ucp);
-  double b_ui = -0.5 * bf[1] * C1;
-  double b_vi = -0.5 * bf[2] * C1;
-  double b_Hi = -0.5 * bf[3] * C1;
-  double b_ucp = -0.5 * bf[3] * C2;
-  // C2 = G1 s2 ci1 + G2 (s1 - L3)
-  double b_G1 = b_C2 * s2 * ci1;
-  double b_s2 = b_C2 * G1 * ci1;
-  double b_ci1 = b_C2 * G1 * s2;
-  double b_G2 = b_C2 * (s1 - L3);
-  double b_s1 = b_C2 * G2;
-  b_L3 -= b_C2 * G2;
-  // C1 = A ci1, A = G1 (s1 - L3) ci1 + G2 s2
+  // the flux's terms
+  const double bn = b[1] * nx + b[2] * ny;  // adjoint of both pressures
+  const double b_C2 = -(bn + b[3] * ucp);
+  const double b_C1 = -(b[0] + b[1] * ui + b[2] * vi + b[3] * Hi);
+  double b_l3 = -(b[0] * du0 + b[1] * du1 + b[2] * du2 + b[3] * du3);
+  double b_ucp = -C2 * b[3], b_ui = -C1 * b[1], b_vi = -C1 * b[2], b_Hi = -C1 * b[3];
   const double b_A = b_C1 * ci1;
-  b_ci1 += b_C1 * A;
-  b_G1 += b_A * (s1 - L3) * ci1;
-  b_s1 += b_A * G1 * ci1;
-  b_L3 -= b_A * G1 * ci1;
-  b_ci1 += b_A * G1 * (s1 - L3);
-  b_G2 += b_A * s2;
-  b_s2 += b_A * G2;
-  // G2 = -ucp du0 + du1 nx + du2 ny
+  const double b_G1 = b_A * s1l3 + b_C2 * s2, b_G2 = b_A * s2 + b_C2 * s1l3;
+  const double b_s1 = b_A * G1 + b_C2 * G2, b_s2 = b_A * G2 + b_C2 * G1;
+  double b_ci = -ci1 * (b_A * A + b_G1 * G1);
+  b_l3 -= b_s1;
+  if (usual) {
+    b_ci += b_s1;
+    b_ucp += b_s2;
+  } else {
+    const double b_l0 = 0.5 * (b_s1 + b_s2), b_l1 = 0.5 * (b_s1 - b_s2);
+    b_ucp += b_l0 * l0u + b_l1 * l1u;
+    b_ci += b_l0 * (l0u + l0c) + b_l1 * (l1c - l1u);
+  }
+  b_ucp += b_l3 * l3u;
+  b_ci += b_l3 * l3c;
+  const double b_X = k1 * b_G1;
+  const double b_du0 = b_X * h - l3 * b[0] - b_G2 * ucp;
+  const double b_du1 = b_G2 * nx - l3 * b[1] - b_X * ui;
+  const double b_du2 = b_G2 * ny - l3 * b[2] - b_X * vi;
+  const double b_du3 = b_X - l3 * b[3];
   b_ucp -= b_G2 * du0;
-  b_du0 -= b_G2 * ucp;
-  b_du1 += b_G2 * nx;
-  b_du2 += b_G2 * ny;
-  // G1 = (gamma-1) (af du0 - ui du1 - vi du2 + du3)
-  const double tg = kGm1 * b_G1;
-  double b_af = tg * du0;
-  b_du0 += tg * af;
-  b_ui -= tg * du1;
-  b_du1 -= tg * ui;
-  b_vi -= tg * du2;
-  b_du2 -= tg * vi;
-  b_du3 += tg;
-  // s1 = (L0 + L1) / 2, s2 = (L0 - L1) / 2
-  const double b_L0 = 0.5 * (b_s1 + b_s2);
-  const double b_L1 = 0.5 * (b_s1 - b_s2);
-  // entropy fix: L = |l| < eps ? (eps + l^2 ieps) / 2 : |l|
-  double b_eps = 0.0, b_ieps = 0.0;
-  double b_l0, b_l1, b_l3;
-  if (fx0) {
-    b_l0 = b_L0 * l0r * ieps;
-    b_eps += 0.5 * b_L0;
-    b_ieps += 0.5 * b_L0 * l0r * l0r;
-  } else {
-    b_l0 = l0r < 0 ? -b_L0 : b_L0;
-  }
-  if (fx1) {
-    b_l1 = b_L1 * l1r * ieps;
-    b_eps += 0.5 * b_L1;
-    b_ieps += 0.5 * b_L1 * l1r * l1r;
-  } else {
-    b_l1 = l1r < 0 ? -b_L1 : b_L1;
-  }
-  if (fx3) {
-    b_l3 = b_L3 * l3r * ieps;
-    b_eps += 0.5 * b_L3;
-    b_ieps += 0.5 * b_L3 * l3r * l3r;
-  } else {
-    b_l3 = l3r < 0 ? -b_L3 : b_L3;
-  }
-  // l0 = ucp + ci, l1 = ucp - ci, l3 = ucp; eps = ci / 10, ieps = 10 ci1
-  b_ucp += b_l0 + b_l1 + b_l3;
-  double b_ci = b_l0 - b_l1 + 0.1 * b_eps;
-  b_ci1 += 10.0 * b_ieps;
-  // ci1 = 1 / ci, ci = c2^2, c2 = (gamma-1) (Hi - af)
-  b_ci -= b_ci1 * ci1 * ci1;
-  const double b_c2 = 2.0 * c2 * b_ci;
-  b_Hi += kGm1 * b_c2;
-  b_af -= kGm1 * b_c2;
-  // ucp = ui nx + vi ny; af = (ui^2 + vi^2) / 2
-  b_ui += b_ucp * nx + b_af * ui;
-  b_vi += b_ucp * ny + b_af * vi;
-  // ui = (di vxR + vxL) d1 and likewise vi, Hi
-  const double b_d1 = b_ui * (di * vxR + vxL) + b_vi * (di * vyR + vyL) + b_Hi * (di * HR + HL);
-  double b_di = d1 * (b_ui * vxR + b_vi * vyR + b_Hi * HR);
-  double b_vxR = b_ui * di * d1, b_vxL = b_ui * d1;
-  double b_vyR = b_vi * di * d1, b_vyL = b_vi * d1;
-  const double b_HR = b_Hi * di * d1, b_HL = b_Hi * d1;
-  // d1 = 1 / (1 + di); di = sqrt(rR irL)
-  b_di -= b_d1 * d1 * d1;
-  const double b_q = b_di * 0.5 * rcp(di);
-  double b_rR = b_q * irL;
-  double b_irL = b_q * rR;
-  // du = uR - uL
-  double b_uR0 = b_du0, b_uL0 = -b_du0;
-  b_uR1 += b_du1;
-  b_uL1 -= b_du1;
-  b_uR2 += b_du2;
-  b_uL2 -= b_du2;
-  double b_uR3 = b_du3, b_uL3 = -b_du3;
-  // right state: HR = rHR irR, rHR = uR3 + pR, pR, unR, vxR, vyR
-  b_rHR += b_HR * irR;
-  double b_irR = b_HR * rHR;
-  b_uR3 += b_rHR;
-  b_pR += b_rHR;
-  const double tR = kGm1 * b_pR;
-  b_uR3 += tR;
-  b_uR1 -= 0.5 * tR * vxR;
-  b_vxR -= 0.5 * tR * uR[1];
-  b_uR2 -= 0.5 * tR * vyR;
-  b_vyR -= 0.5 * tR * uR[2];
-  b_vxR += b_unR * nx;
-  b_vyR += b_unR * ny;
-  b_uR1 += b_vxR * irR;
-  b_irR += b_vxR * uR[1];
-  b_uR2 += b_vyR * irR;
-  b_irR += b_vyR * uR[2];
-  // left state, the same
-  b_rHL += b_HL * irL;
-  b_irL += b_HL * rHL;
-  b_uL3 += b_rHL;
-  b_pL += b_rHL;
-  const double tL = kGm1 * b_pL;
-  b_uL3 += tL;
-  b_uL1 -= 0.5 * tL * vxL;
-  b_vxL -= 0.5 * tL * uL[1];
-  b_uL2 -= 0.5 * tL * vyL;
-  b_vyL -= 0.5 * tL * uL[2];
-  b_vxL += b_unL * nx;
-  b_vyL += b_unL * ny;
-  b_uL1 += b_vxL * irL;
-  b_irL += b_vxL * uL[1];
-  b_uL2 += b_vyL * irL;
-  b_irL += b_vyL * uL[2];
-  // irL = rR irLR, irR = rL irLR, irLR = 1 / (rL rR)
-  b_rR += b_irL * irLR;
-  const double b_irLR = b_irL * rR + b_irR * rL;
-  double b_rL = b_irR * irLR;
-  const double b_prod = -b_irLR * irLR * irLR;
-  b_rL += b_prod * rR;
-  b_rR += b_prod * rL;
-  b_uL0 += b_rL;
-  b_uR0 += b_rR;
-  buL[0] += b_uL0;
-  buL[1] += b_uL1;
-  buL[2] += b_uL2;
-  buL[3] += b_uL3;
-  buR[0] += b_uR0;
-  buR[1] += b_uR1;
-  buR[2] += b_uR2;
-  buR[3] += b_uR3;
+  // ci = c2^2, c2 = (gamma-1) (Hi - h), h = (ui^2 + vi^2)/2, u_n = ui nx + vi ny
+  const double z = 2.0 * kGm1 * c2 * b_ci;
+  b_Hi += z;
+  const double b_h = b_X * du0 - z;
+  b_ui += b_h * ui + b_ucp * nx - b_X * du1;
+  b_vi += b_h * vi + b_ucp * ny - b_X * du2;
+  // the averages
+  const double ai = b_ui * d1, av = b_vi * d1, aH = b_Hi * d1;
+  const double b_s = -(ai * ui + av * vi + aH * Hi);
+  const double gg = 0.5 * g * (ai * uR[1] + av * uR[2] + aH * rHR), ws = 0.5 * w * b_s;
+  // each side: rho H = rho E + p, p = (gamma-1) (rho E - kin/2), kin = |m|^2/rho, u_n = m.n/rho
+  const double rhL = b[3] * unL + aH, rhR = b[3] * unR + g * aH;
+  const double tL = kGm1 * (bn + rhL), tR = kGm1 * (bn + rhR);
+  const double eL = (b[1] * uL[1] + b[2] * uL[2] + b[3] * rHL) * irL;
+  const double eR = (b[1] * uR[1] + b[2] * uR[2] + b[3] * rHR) * irR;
+  const double cL = b[0] + eL, cR = b[0] + eR, mL = tL * irL, mR = tR * irR;
+  buL[0] = irL * (ws + gg + 0.5 * tL * kinL) - eL * unL + b_s - b_du0;
+  buL[1] = cL * nx + b[1] * unL + ai - mL * uL[1] - b_du1;
+  buL[2] = cL * ny + b[2] * unL + av - mL * uL[2] - b_du2;
+  buL[3] = rhL + tL - b_du3;
+  buR[0] = irR * (ws - gg + 0.5 * tR * kinR) - eR * unR + b_du0;
+  buR[1] = cR * nx + b[1] * unR + g * ai - mR * uR[1] + b_du1;
+  buR[2] = cR * ny + b[2] * unR + g * av - mR * uR[2] + b_du2;
+  buR[3] = rhR + tR + b_du3;
 }
 
-// bgxi, bgeta: adjoints of the contravariant flux (4 each); adds the state's adjoint to bs.
+// bf: adjoint of the flux itself (4). Adds the adjoints of uL and uR to buL, buR.
+__host__ __device__ inline void roe_flux_vjp(const double* uL, const double* uR, double nx, double ny,
+                                             const double* bf, double* buL, double* buR) {
+  const double b[4] = {0.5 * bf[0], 0.5 * bf[1], 0.5 * bf[2], 0.5 * bf[3]};
+  double bl[4], br[4];
+  roe_flux2_vjp(uL, uR, nx, ny, b, bl, br);
+  for (int c = 0; c < 4; ++c) {
+    buL[c] += bl[c];
+    buR[c] += br[c];
+  }
+}
+
+// bgxi, bgeta: adjoints of the contravariant flux (4 each); writes the state's adjoint to bs.
 __host__ __device__ inline void contravariant_vjp(const double* s, double j00, double j01, double j10, double j11,
                                                   const double* bgxi, const double* bgeta, double* bs) {
   const double ir = rcp(s[0]);
   const double vx = s[1] * ir, vy = s[2] * ir;
-  const double p = kGm1 * (s[3] - 0.5 * (s[1] * vx + s[2] * vy));
-  const double rH = s[3] + p;
-  double bfx[4], bfy[4];
-  for (int c = 0; c < 4; ++c) {
-    bfx[c] = j00 * bgxi[c] + j10 * bgeta[c];
-    bfy[c] = j01 * bgxi[c] + j11 * bgeta[c];
-  }
-  // fx = (s1, s1 vx + p, s2 vx, rH vx), fy = (s2, s1 vy, s2 vy + p, rH vy)
-  double b_s1 = bfx[0] + bfx[1] * vx + bfy[1] * vy;
-  double b_s2 = bfx[2] * vx + bfy[0] + bfy[2] * vy;
-  double b_vx = bfx[1] * s[1] + bfx[2] * s[2] + bfx[3] * rH;
-  double b_vy = bfy[1] * s[1] + bfy[2] * s[2] + bfy[3] * rH;
-  double b_p = bfx[1] + bfy[2];
-  const double b_rH = bfx[3] * vx + bfy[3] * vy;
-  double b_s3 = b_rH;
-  b_p += b_rH;
-  const double t = kGm1 * b_p;
-  b_s3 += t;
-  b_s1 -= 0.5 * t * vx;
-  b_vx -= 0.5 * t * s[1];
-  b_s2 -= 0.5 * t * vy;
-  b_vy -= 0.5 * t * s[2];
-  b_s1 += b_vx * ir;
-  b_s2 += b_vy * ir;
-  const double b_ir = b_vx * s[1] + b_vy * s[2];
-  bs[0] += -b_ir * ir * ir;
-  bs[1] += b_s1;
-  bs[2] += b_s2;
-  bs[3] += b_s3;
+  const double kin = s[1] * vx + s[2] * vy;
+  const double rH = s[3] + kGm1 * (s[3] - 0.5 * kin);
+  const double vxi = j00 * vx + j01 * vy, veta = j10 * vx + j11 * vy;
+  // g[0] = rho v, g[1] = m1 v + j0 p, g[2] = m2 v + j1 p, g[3] = rho H v for v = vxi, veta
+  const double b_vxi = bgxi[1] * s[1] + bgxi[2] * s[2] + bgxi[3] * rH;
+  const double b_veta = bgeta[1] * s[1] + bgeta[2] * s[2] + bgeta[3] * rH;
+  const double b_rH = bgxi[3] * vxi + bgeta[3] * veta;
+  const double t = kGm1 * (bgxi[1] * j00 + bgxi[2] * j01 + bgeta[1] * j10 + bgeta[2] * j11 + b_rH);
+  const double wxi = bgxi[0] + b_vxi * ir, weta = bgeta[0] + b_veta * ir;  // m.j = rho v
+  bs[0] = ir * (0.5 * t * kin - b_vxi * vxi - b_veta * veta);
+  bs[1] = wxi * j00 + weta * j10 + bgxi[1] * vxi + bgeta[1] * veta - t * vx;
+  bs[2] = wxi * j01 + weta * j11 + bgxi[2] * vxi + bgeta[2] * veta - t * vy;
+  bs[3] = b_rH + t;
 }
 
 }  // namespace vt

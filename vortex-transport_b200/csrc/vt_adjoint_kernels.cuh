@@ -21,10 +21,11 @@
 // On meshes whose faces take the edge-once form the whole reverse stage is
 // one launch instead, adjoint_tile_kernel (vt_adjoint_tile.cuh).
 //
-// Both read the state through the SoA-of-double2 layout of the stage kernel,
-// so a warp's 32 consecutive elements are contiguous 512-byte rows. The
-// face adjoints bp/bm hold 2 double2 rows per (s, q) face point:
-//   bp[((s * NFQ + q) * 2 + h) * Kpad + e]
+// Both read the state through the column layout of the stage kernel
+// (vt_device.cuh), so a warp's 32 columns are contiguous 512-byte rows; e below
+// is a column. The face adjoints bp/bm hold 2 double2 rows per (s, q) face
+// point:
+//   bp[((s * NFQ + q) * 2 + h) * ncols + e]
 #pragma once
 
 #include "vt_adjoint.cuh"
@@ -43,23 +44,17 @@ struct AdjArgs {
   double2* bm;            // face adjoints, neighbour trace
   const double2* geo;
   const int4* nbr;
-  // Per-element time steps (a batch group with uneven steps), or null: then
-  // sa (when sa_dt is set), cl and cg are fractions of the element's step.
-  const double* elem_dt;
+  const int* elem;  // element of each column (-1: empty)
+  // Per-tile time steps (a batch group with uneven steps), or null: then sa
+  // (when sa_dt is set), cl and cg are fractions of the tile's step.
+  const double* tile_dt;
   int sa_dt;
   // The stage kernel's tile schedule (adjoint_tile_kernel) and error words.
-  const int4* tiles;
-  const int* tile_items;
-  const int* tile_count;
+  const unsigned char* lists;
   int ntiles;
   unsigned long long* err;
-  long long Kpad;
-  int K;
+  long long ncols;
   double sa, lam_coef, cl, cg;
-  // 2-D tensor maps of U and a (adjoint_tile_kernel only), as the stage
-  // kernel's: [2 Np rows] x [2 Kpad doubles], a box of one 32-element run;
-  // encoded on the host by the launcher
-  CUtensorMap map_U, map_a;
 };
 
 constexpr int kAdjRun = 32;  // elements per block (one per lane)
@@ -69,10 +64,10 @@ __global__ void __launch_bounds__(kAdjRun * NFQ)
     adjoint_face_kernel(const AdjArgs a, const StageOps<P, NFQ> o) {
   constexpr int NP = np_of_p(P), NE = P + 1;
   const int e = blockIdx.x * kAdjRun + threadIdx.x;
-  if (e >= a.K) return;
+  if (__ldg(a.elem + e) < 0) return;
   const int s = blockIdx.y, q = threadIdx.y;  // uniform per block / warp
   const int w = s * NFQ + q;
-  const long long KP = a.Kpad;
+  const long long KP = a.ncols;
   const int4 nb4 = __ldg(a.nbr + e);
   const int nb = s == 0 ? nb4.x : (s == 1 ? nb4.y : nb4.z);
   double up[4] = {0.0, 0.0, 0.0, 0.0}, um[4] = {0.0, 0.0, 0.0, 0.0};
@@ -80,8 +75,9 @@ __global__ void __launch_bounds__(kAdjRun * NFQ)
   for (int k = 0; k < NE; ++k) {
     const int node = edge_node(P, s, k);
     const double cp = o.tp[s][q][k], cm = o.tm[s][q][k];
-    const double2 x0 = __ldg(a.U + (2 * node) * KP + e), x1 = __ldg(a.U + (2 * node + 1) * KP + e);
-    const double2 y0 = __ldg(a.U + (2 * node) * KP + nb), y1 = __ldg(a.U + (2 * node + 1) * KP + nb);
+    const double2 *pe = a.U + state_index(NP, e, 2 * node), *pn = a.U + state_index(NP, nb, 2 * node);
+    const double2 x0 = __ldg(pe), x1 = __ldg(pe + kTileRun);
+    const double2 y0 = __ldg(pn), y1 = __ldg(pn + kTileRun);
     up[0] = fma(cp, x0.x, up[0]);
     up[1] = fma(cp, x0.y, up[1]);
     up[2] = fma(cp, x1.x, up[2]);
@@ -95,18 +91,19 @@ __global__ void __launch_bounds__(kAdjRun * NFQ)
 #pragma unroll
   for (int i = 0; i < NP; ++i) {
     const double l = o.lift[s][i][q];
-    const double2 a0 = __ldg(a.a + (2 * i) * KP + e), a1 = __ldg(a.a + (2 * i + 1) * KP + e);
+    const double2* pa = a.a + state_index(NP, e, 2 * i);
+    const double2 a0 = __ldg(pa), a1 = __ldg(pa + kTileRun);
     bf[0] = fma(l, a0.x, bf[0]);
     bf[1] = fma(l, a0.y, bf[1]);
     bf[2] = fma(l, a1.x, bf[2]);
     bf[3] = fma(l, a1.y, bf[3]);
   }
-  const double2 lsa = __ldg(a.geo + 5 * KP + e), lsb = __ldg(a.geo + 6 * KP + e);
-  const double sa = (a.elem_dt && a.sa_dt) ? a.sa * __ldg(a.elem_dt + e) : a.sa;
+  const double2 lsa = __ldg(a.geo + geo_index(e, 2)), lsb = __ldg(a.geo + geo_index(e, 3));
+  const double sa = (a.tile_dt && a.sa_dt) ? a.sa * __ldg(a.tile_dt + e / kTileElems) : a.sa;
   const double sc = -(s == 0 ? lsa.x : (s == 1 ? lsa.y : lsb.x)) * sa;
 #pragma unroll
   for (int c = 0; c < 4; ++c) bf[c] *= sc;
-  const double2 n = __ldg(a.geo + (2 + s) * KP + e);
+  const double2 n = __ldg(a.geo + geo_index(e, 4 + s));
   double bu[4] = {0.0, 0.0, 0.0, 0.0}, bv[4] = {0.0, 0.0, 0.0, 0.0};
   roe_flux_vjp(up, um, n.x, n.y, bf, bu, bv);
   const long long r0 = static_cast<long long>(2 * w) * KP + e;
@@ -123,19 +120,20 @@ __global__ void __launch_bounds__(kAdjRun * np_of_p(P), 3)
   __shared__ double2 sA[2 * NP][kAdjRun];  // the block's stage adjoints, row pair j loaded by warp j
   const int e = blockIdx.x * kAdjRun + threadIdx.x;
   const int j = threadIdx.y;  // node, uniform per warp
-  const long long KP = a.Kpad;
+  const long long KP = a.ncols;
+  const bool valid = __ldg(a.elem + e) >= 0;
   // every global operand of this thread is requested before the barrier
-  const long long r0 = (2 * j) * KP + e, r1 = r0 + KP;
+  const long long r0 = state_index(NP, e, 2 * j), r1 = r0 + kTileRun;
   double2 u0 = make_double2(1.0, 0.0), u1 = make_double2(0.0, 0.0), j0 = u1, j1 = u1, l0 = u1, l1 = u1, c0 = u1,
           c1 = u1;
   int4 nb4 = make_int4(0, 0, 0, 0);
-  if (e < a.K) {
-    sA[2 * j][threadIdx.x] = __ldg(a.a + (2 * j) * KP + e);
-    sA[2 * j + 1][threadIdx.x] = __ldg(a.a + (2 * j + 1) * KP + e);
+  if (valid) {
+    sA[2 * j][threadIdx.x] = __ldg(a.a + r0);
+    sA[2 * j + 1][threadIdx.x] = __ldg(a.a + r1);
     u0 = __ldg(a.U + r0);
     u1 = __ldg(a.U + r1);
-    j0 = __ldg(a.geo + 0 * KP + e);
-    j1 = __ldg(a.geo + 1 * KP + e);
+    j0 = __ldg(a.geo + geo_index(e, 0));
+    j1 = __ldg(a.geo + geo_index(e, 1));
     nb4 = __ldg(a.nbr + e);
     if (a.lam_coef != 0.0 || a.a_out) {
       l0 = a.lam[r0];
@@ -147,7 +145,7 @@ __global__ void __launch_bounds__(kAdjRun * np_of_p(P), 3)
     }
   }
   __syncthreads();
-  if (e >= a.K) return;
+  if (!valid) return;
   double g[4] = {0.0, 0.0, 0.0, 0.0};
   if (P > 0) {
     double bx[4] = {0.0, 0.0, 0.0, 0.0}, by[4] = {0.0, 0.0, 0.0, 0.0};
@@ -164,7 +162,7 @@ __global__ void __launch_bounds__(kAdjRun * np_of_p(P), 3)
       by[2] = fma(d1, a1.x, by[2]);
       by[3] = fma(d1, a1.y, by[3]);
     }
-    const double sa = (a.elem_dt && a.sa_dt) ? a.sa * __ldg(a.elem_dt + e) : a.sa;
+    const double sa = (a.tile_dt && a.sa_dt) ? a.sa * __ldg(a.tile_dt + e / kTileElems) : a.sa;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       bx[c] *= sa;
@@ -202,8 +200,8 @@ __global__ void __launch_bounds__(kAdjRun * np_of_p(P), 3)
 #pragma unroll
   for (int c = 0; c < 4; ++c) acc[c] = fma(a.lam_coef, lam[c], acc[c]) + g[c];
   if (a.a_out) {
-    const double h = a.elem_dt ? __ldg(a.elem_dt + e) : 1.0;
-    const double cl = a.elem_dt ? a.cl * h : a.cl, cg = a.elem_dt ? a.cg * h : a.cg;
+    const double h = a.tile_dt ? __ldg(a.tile_dt + e / kTileElems) : 1.0;
+    const double cl = a.tile_dt ? a.cl * h : a.cl, cg = a.tile_dt ? a.cg * h : a.cg;
     double an[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) an[c] = fma(cl, lam[c], cg * g[c]);
@@ -220,16 +218,16 @@ __global__ void __launch_bounds__(kAdjRun * np_of_p(P), 3)
 template <int P, int NFQ>
 __global__ void __launch_bounds__(128)
     rhs_jvp_kernel(const double2* __restrict__ U, const double2* __restrict__ V, double2* __restrict__ dR,
-                   const double2* __restrict__ geo, const int4* __restrict__ nbr, long long KP, int K,
-                   const StageOps<P, NFQ> o) {
+                   const double2* __restrict__ geo, const int4* __restrict__ nbr, const int* __restrict__ elem,
+                   long long ncols, const StageOps<P, NFQ> o) {
   constexpr int NP = np_of_p(P), NE = P + 1;
   using D1 = Dual<1>;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= K) return;
+  if (e >= ncols || elem[e] < 0) return;
   D1 u[NP][4], r[NP][4];
   for (int i = 0; i < NP; ++i) {
-    const double2 x0 = U[(2 * i) * KP + e], x1 = U[(2 * i + 1) * KP + e];
-    const double2 v0 = V[(2 * i) * KP + e], v1 = V[(2 * i + 1) * KP + e];
+    const long long r0 = state_index(NP, e, 2 * i), r1 = r0 + kTileRun;
+    const double2 x0 = U[r0], x1 = U[r1], v0 = V[r0], v1 = V[r1];
     const double xs[4] = {x0.x, x0.y, x1.x, x1.y}, vs[4] = {v0.x, v0.y, v1.x, v1.y};
     for (int c = 0; c < 4; ++c) {
       u[i][c] = D1(xs[c]);
@@ -238,7 +236,7 @@ __global__ void __launch_bounds__(128)
     }
   }
   if (P > 0) {
-    const double2 j0 = geo[0 * KP + e], j1 = geo[1 * KP + e];
+    const double2 j0 = geo[geo_index(e, 0)], j1 = geo[geo_index(e, 1)];
     for (int j = 0; j < NP; ++j) {
       D1 gxi[4], geta[4];
       contravariant_flux_t(u[j], j0.x, j0.y, j1.x, j1.y, gxi, geta);
@@ -247,16 +245,16 @@ __global__ void __launch_bounds__(128)
     }
   }
   const int4 nb4 = nbr[e];
-  const double2 lsa = geo[5 * KP + e], lsb = geo[6 * KP + e];
+  const double2 lsa = geo[geo_index(e, 2)], lsb = geo[geo_index(e, 3)];
   for (int s = 0; s < 3; ++s) {
     const int nb = s == 0 ? nb4.x : (s == 1 ? nb4.y : nb4.z);
     const double ls = s == 0 ? lsa.x : (s == 1 ? lsa.y : lsb.x);
-    const double2 n = geo[(2 + s) * KP + e];
+    const double2 n = geo[geo_index(e, 4 + s)];
     D1 un[NE][4];
     for (int k = 0; k < NE; ++k) {
       const int node = edge_node(P, s, k);
-      const double2 x0 = U[(2 * node) * KP + nb], x1 = U[(2 * node + 1) * KP + nb];
-      const double2 v0 = V[(2 * node) * KP + nb], v1 = V[(2 * node + 1) * KP + nb];
+      const long long r0 = state_index(NP, nb, 2 * node), r1 = r0 + kTileRun;
+      const double2 x0 = U[r0], x1 = U[r1], v0 = V[r0], v1 = V[r1];
       const double xs[4] = {x0.x, x0.y, x1.x, x1.y}, vs[4] = {v0.x, v0.y, v1.x, v1.y};
       for (int c = 0; c < 4; ++c) {
         un[k][c] = D1(xs[c]);
@@ -278,8 +276,8 @@ __global__ void __launch_bounds__(128)
     }
   }
   for (int i = 0; i < NP; ++i) {
-    dR[(2 * i) * KP + e] = make_double2(r[i][0].d[0], r[i][1].d[0]);
-    dR[(2 * i + 1) * KP + e] = make_double2(r[i][2].d[0], r[i][3].d[0]);
+    dR[state_index(NP, e, 2 * i)] = make_double2(r[i][0].d[0], r[i][1].d[0]);
+    dR[state_index(NP, e, 2 * i + 1)] = make_double2(r[i][2].d[0], r[i][3].d[0]);
   }
 }
 

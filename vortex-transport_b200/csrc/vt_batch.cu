@@ -35,23 +35,6 @@ cudaError_t dalloc(T** p, size_t bytes) {
   return cudaMalloc(reinterpret_cast<void**>(p), bytes);
 }
 
-// instance AoS (K_i x Np x 4) <-> group SoA rows at an element offset
-__global__ void batch_aos_to_soa(const double2* __restrict__ aos, double2* __restrict__ soa, int K, int Np,
-                                 long long Kpad, long long offset) {
-  const long long l = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (l >= static_cast<long long>(K) * 2 * Np) return;
-  const int e = static_cast<int>(l / (2 * Np)), r = static_cast<int>(l % (2 * Np));
-  soa[r * Kpad + offset + e] = aos[l];
-}
-
-__global__ void batch_soa_to_aos(const double2* __restrict__ soa, double2* __restrict__ aos, int K, int Np,
-                                 long long Kpad, long long offset) {
-  const long long l = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (l >= static_cast<long long>(K) * 2 * Np) return;
-  const int e = static_cast<int>(l / (2 * Np)), r = static_cast<int>(l % (2 * Np));
-  aos[l] = soa[r * Kpad + offset + e];
-}
-
 std::vector<double> fold(int p, int nfq, const vt_mesh_desc& d) {
   std::vector<double> ops(static_cast<size_t>(stage_ops_doubles(p, nfq)));
   fold_stage_operators(p, nfq, d.inv_mass_ref, d.stiffness_ref, d.line_quadrature, d.phi_plus, d.phi_minus,
@@ -73,17 +56,19 @@ std::vector<double> table_key(const vt_mesh_desc& d) {
 
 struct Group {
   int p = 0, nfq = 0, Np = 0;
-  long long K = 0, Kpad = 0;
+  long long K = 0, ncols = 0;
   int ntiles = 0;
   std::vector<int> members;
   std::vector<long long> offset;  // element offset of each member
   std::vector<int> tile_begin;    // first tile of each member
+  std::vector<Numbering> num;     // of each member's own elements and columns
   std::vector<double> ops;
   StageKernel kern;
   int max_blocks = 0;
   double2 *U = nullptr, *A = nullptr, *Sa = nullptr, *Sb = nullptr, *geo = nullptr;
-  int4 *nbr = nullptr, *tiles = nullptr;
-  int *items = nullptr, *count = nullptr;
+  int4* nbr = nullptr;
+  int* elem = nullptr;
+  unsigned char* lists = nullptr;
   double* tile_dt = nullptr;
   unsigned long long* err = nullptr;
 };
@@ -111,10 +96,8 @@ struct vt_batch {
   std::vector<double> dt;  // per instance
   int last_instance = -1;
   vt_error_info last{};
-  // one solver context per group over the group's own buffers, for the adjoint,
-  // with each group's per-element time steps
+  // one solver context per group over the group's own buffers, for the adjoint
   std::vector<vt_ctx*> views;
-  std::vector<double*> view_dt;
 };
 
 namespace {
@@ -129,8 +112,6 @@ void release(vt_batch* b) {
     if (v->aos) cudaFree(v->aos);
     delete v;
   }
-  for (double* p : b->view_dt)
-    if (p) cudaFree(p);
   if (b->graph) cudaGraphExecDestroy(b->graph);
   for (cudaStream_t st : b->gstreams)
     if (st) cudaStreamDestroy(st);
@@ -138,7 +119,7 @@ void release(vt_batch* b) {
     if (ev) cudaEventDestroy(ev);
   if (b->fork) cudaEventDestroy(b->fork);
   for (auto& g : b->groups) {
-    void* bufs[] = {g.U, g.A, g.Sa, g.Sb, g.geo, g.nbr, g.tiles, g.items, g.count, g.tile_dt, g.err};
+    void* bufs[] = {g.U, g.A, g.Sa, g.Sb, g.geo, g.nbr, g.elem, g.lists, g.tile_dt, g.err};
     for (void* p : bufs)
       if (p) cudaFree(p);
   }
@@ -155,12 +136,10 @@ vt::StageArgs group_args(vt::Group& g, const double2* in, double2* out, int stag
   a.out = out;
   a.geo = g.geo;
   a.nbr = g.nbr;
-  a.tiles = g.tiles;
-  a.tile_items = g.items;
-  a.tile_count = g.count;
+  a.elem = g.elem;
+  a.lists = g.lists;
   a.tile_dt = g.tile_dt;
   a.err = g.err;
-  a.Kpad = g.Kpad;
   a.K = static_cast<int>(g.K);
   a.ntiles = g.ntiles;
   a.stage = stage;
@@ -195,6 +174,21 @@ cudaError_t enqueue_step(vt_batch* b) {
   }
   for (size_t gi = 0; gi < b->groups.size() && !e; ++gi) e = cudaStreamWaitEvent(b->stream, b->join[gi], 0);
   return e;
+}
+
+// elem of every member's columns (elements numbered across the group).
+cudaError_t number_members(vt_batch* b, const vt::Group& G) {
+  cudaError_t e = cudaSuccess;
+  for (size_t m = 0; m < G.members.size() && !e; ++m)
+    e = vt::launch_number_columns(G.num[m], G.elem, vt::kTileElems * G.tile_begin[m], static_cast<int>(G.offset[m]),
+                                  b->stream);
+  return e;
+}
+
+// Member i's block of a group's state vector.
+double2* member_columns(const vt_batch* b, int i, double2* group) {
+  const vt::Group& G = b->groups[b->group_of[i]];
+  return group + 2ll * G.Np * vt::kTileElems * G.tile_begin[b->index_in_group[i]];
 }
 
 cudaError_t reset_errors(vt_batch* b) {
@@ -252,7 +246,9 @@ int ensure_views(vt_batch* b) {
     c->Np = G.Np;
     c->nfq = G.nfq;
     c->K = static_cast<int>(G.K);
-    c->Kpad = G.Kpad;
+    c->ncols = G.ncols;
+    for (size_t m = 0; m < G.members.size(); ++m)
+      c->parts.push_back({G.num[m], static_cast<long long>(vt::kTileElems) * G.tile_begin[m], G.offset[m]});
     c->max_blocks = G.max_blocks;
     c->stream = b->stream;
     c->U = G.U;
@@ -261,34 +257,26 @@ int ensure_views(vt_batch* b) {
     c->Sb = G.Sb;
     c->geo = G.geo;
     c->nbr = G.nbr;
-    c->tiles = G.tiles;
-    c->tile_items = G.items;
-    c->tile_count = G.count;
+    c->elem = G.elem;
+    c->lists = G.lists;
     c->ntiles = G.ntiles;
     c->err = G.err;
     c->ops = G.ops;
     c->launch = G.kern.launch;
     c->map = G.kern.map;
     c->tile_dt = G.tile_dt;
-    double* edt = nullptr;
-    const cudaError_t ea = cudaMalloc(reinterpret_cast<void**>(&edt), sizeof(double) * static_cast<size_t>(G.K));
-    if (ea) {
-      delete c;
-      return fail(ea == cudaErrorMemoryAllocation ? VT_ERR_NO_MEMORY : VT_ERR_CUDA,
-                  vt::cuda_msg("batch adjoint set-up", ea));
-    }
-    c->elem_dt = edt;
-    b->view_dt.push_back(edt);
-    std::vector<int4> nb(static_cast<size_t>(G.K));
-    const cudaError_t e = cudaMemcpy(nb.data(), G.nbr, sizeof(int4) * nb.size(), cudaMemcpyDeviceToHost);
+    std::vector<int4> nb(static_cast<size_t>(G.ncols));
+    std::vector<int> el(static_cast<size_t>(G.ncols));
+    cudaError_t e = cudaMemcpy(nb.data(), G.nbr, sizeof(int4) * nb.size(), cudaMemcpyDeviceToHost);
+    if (!e) e = cudaMemcpy(el.data(), G.elem, sizeof(int) * el.size(), cudaMemcpyDeviceToHost);
     if (e) {
       delete c;
       return fail(VT_ERR_CUDA, vt::cuda_msg("batch adjoint set-up", e));
     }
     c->side_pairing = true;
     for (size_t n = 0; n < nb.size() && c->side_pairing; ++n)
-      c->side_pairing = nb[nb[n].x].x == static_cast<int>(n) && nb[nb[n].y].y == static_cast<int>(n) &&
-                        nb[nb[n].z].z == static_cast<int>(n);
+      c->side_pairing = el[n] < 0 || (nb[nb[n].x].x == static_cast<int>(n) && nb[nb[n].y].y == static_cast<int>(n) &&
+                                     nb[nb[n].z].z == static_cast<int>(n));
     b->views.push_back(c);
   }
   return VT_OK;
@@ -385,56 +373,33 @@ vt_batch* vt_batch_create(const vt_mesh_desc* descs, int n, int device, int* sta
   for (auto& G : b->groups) {
     G.kern = vt::select_kernel(G.p, G.nfq, G.ops.data());
     int per_sm = 0;
-    if ((e = vt::tensor_maps_available()) || (e = G.kern.configure(&per_sm))) {
+    if ((e = G.kern.configure(&per_sm))) {
       set(fail(VT_ERR_CUDA, vt::cuda_msg("stage kernel attributes", e)));
       release(b);
       return nullptr;
     }
     G.max_blocks = b->sms * (per_sm > 0 ? per_sm : 1);
-    G.Kpad = (G.K + 127) / 128 * 128;
-    const long long KP = G.Kpad;
-    // packed geometry, shifted neighbours and per-member tiles
-    std::vector<double2> geo(7 * static_cast<size_t>(KP), make_double2(0.0, 0.0));
-    std::vector<int4> nbr(static_cast<size_t>(KP), make_int4(0, 0, 0, 0));
-    std::vector<int4> tiles;
+    // each member's columns, and so its tiles, follow the previous member's
     for (size_t m = 0; m < G.members.size(); ++m) {
       const vt_mesh_desc& d = descs[G.members[m]];
-      const int off = static_cast<int>(G.offset[m]);
       max_inst_bytes = std::max(max_inst_bytes, sizeof(double) * 4 * static_cast<size_t>(d.n_elements) * G.Np);
-      for (int k = 0; k < d.n_elements; ++k) {
-        const long long n_ = off + k;
-        const double* ji = d.inv_jacobian + 4 * static_cast<size_t>(k);
-        const double* nv = d.normals + 6 * static_cast<size_t>(k);
-        const double* ln = d.side_lengths + 3 * static_cast<size_t>(k);
-        const double det = d.det_jacobian[k];
-        geo[0 * KP + n_] = make_double2(ji[0], ji[1]);
-        geo[1 * KP + n_] = make_double2(ji[2], ji[3]);
-        for (int s = 0; s < 3; ++s) geo[(2 + s) * KP + n_] = make_double2(nv[2 * s], nv[2 * s + 1]);
-        geo[5 * KP + n_] = make_double2(ln[0] / det, ln[1] / det);
-        geo[6 * KP + n_] = make_double2(ln[2] / det, det);
-        const int right = d.neighbours[3 * k] + off, left = d.neighbours[3 * k + 1] + off,
-                  vert = d.neighbours[3 * k + 2] + off;
-        nbr[n_] = d.element_type[k] == 0 ? make_int4(vert, right, left, 0) : make_int4(vert, left, right, 0);
-      }
-      G.tile_begin.push_back(static_cast<int>(tiles.size()));
-      std::vector<int4> runs = vt::structured_tile_runs(d.n_elements, d.element_type, d.neighbours);
-      if (runs.empty())
-        for (int s0 = 0; s0 < d.n_elements; s0 += vt::kTileElems) {
-          const int l0 = std::min(vt::kTileRun, d.n_elements - s0);
-          const int l1 = std::max(0, std::min(vt::kTileRun, d.n_elements - s0 - vt::kTileRun));
-          runs.push_back(make_int4(s0, l0, s0 + vt::kTileRun, l1));
-        }
-      for (const int4& r : runs) tiles.push_back(make_int4(r.x + off, r.y, r.z + off, r.w));
+      G.num.push_back(vt::number_mesh(d.n_elements, d.element_type, d.neighbours));
+      G.tile_begin.push_back(G.ntiles);
+      G.ntiles += G.num.back().ntiles;
     }
-    G.ntiles = static_cast<int>(tiles.size());
-    const size_t state_bytes = sizeof(double2) * 2 * G.Np * static_cast<size_t>(KP);
+    G.ncols = static_cast<long long>(vt::kTileElems) * G.ntiles;
+    std::vector<double2> geo(vt::kGeoRows * static_cast<size_t>(G.ncols), make_double2(0.0, 0.0));
+    std::vector<int4> nbr(static_cast<size_t>(G.ncols), make_int4(0, 0, 0, 0));
+    for (size_t m = 0; m < G.members.size(); ++m)
+      vt::pack_mesh(descs[G.members[m]], G.num[m], geo.data(), nbr.data(),
+                    static_cast<long long>(vt::kTileElems) * G.tile_begin[m]);
+    const size_t state_bytes = sizeof(double2) * 2 * G.Np * static_cast<size_t>(G.ncols);
     if ((e = vt::dalloc(&G.U, state_bytes)) || (e = vt::dalloc(&G.A, state_bytes)) ||
         (e = vt::dalloc(&G.Sa, state_bytes)) || (e = vt::dalloc(&G.Sb, state_bytes)) ||
         (e = vt::dalloc(&G.geo, geo.size() * sizeof(double2))) || (e = vt::dalloc(&G.nbr, nbr.size() * sizeof(int4))) ||
-        (e = vt::dalloc(&G.tiles, tiles.size() * sizeof(int4))) ||
-        (e = vt::dalloc(&G.items, sizeof(int) * vt::kMaxItems * tiles.size())) ||
-        (e = vt::dalloc(&G.count, sizeof(int) * tiles.size())) ||
-        (e = vt::dalloc(&G.tile_dt, sizeof(double) * tiles.size())) ||
+        (e = vt::dalloc(&G.elem, sizeof(int) * G.ncols)) ||
+        (e = vt::dalloc(&G.lists, vt::kTileListBytes * static_cast<size_t>(G.ntiles))) ||
+        (e = vt::dalloc(&G.tile_dt, sizeof(double) * G.ntiles)) ||
         (e = vt::dalloc(&G.err, 4 * sizeof(unsigned long long)))) {
       set(fail(e == cudaErrorMemoryAllocation ? VT_ERR_NO_MEMORY : VT_ERR_CUDA, vt::cuda_msg("vt_batch_create", e)));
       release(b);
@@ -442,11 +407,10 @@ vt_batch* vt_batch_create(const vt_mesh_desc* descs, int n, int device, int* sta
     }
     if ((e = cudaMemcpy(G.geo, geo.data(), geo.size() * sizeof(double2), cudaMemcpyHostToDevice)) ||
         (e = cudaMemcpy(G.nbr, nbr.data(), nbr.size() * sizeof(int4), cudaMemcpyHostToDevice)) ||
-        (e = cudaMemcpy(G.tiles, tiles.data(), tiles.size() * sizeof(int4), cudaMemcpyHostToDevice)) ||
         (e = cudaMemset(G.U, 0, state_bytes)) || (e = cudaMemset(G.A, 0, state_bytes)) ||
         (e = cudaMemset(G.Sa, 0, state_bytes)) || (e = cudaMemset(G.Sb, 0, state_bytes)) ||
-        (e = cudaMemset(G.tile_dt, 0, sizeof(double) * tiles.size())) ||
-        (e = vt::launch_build_tile_items(G.tiles, G.nbr, G.items, G.count, G.ntiles, G.nfq, b->stream)) ||
+        (e = cudaMemset(G.tile_dt, 0, sizeof(double) * G.ntiles)) || (e = number_members(b, G)) ||
+        (e = vt::launch_build_tile_lists(G.nbr, G.elem, static_cast<int>(G.K), G.ntiles, G.nfq, G.lists, b->stream)) ||
         (e = cudaStreamSynchronize(b->stream))) {
       set(fail(VT_ERR_CUDA, vt::cuda_msg("vt_batch_create upload", e)));
       release(b);
@@ -477,12 +441,9 @@ int vt_batch_upload_state(vt_batch* b, int i, const double* U) {
   const int K = b->K_of[i];
   const size_t bytes = sizeof(double) * 4 * static_cast<size_t>(K) * G.Np;
   cudaError_t e = cudaMemcpyAsync(b->staging, U, bytes, cudaMemcpyHostToDevice, b->stream);
-  const long long nrow = static_cast<long long>(K) * 2 * G.Np;
-  if (!e) {
-    vt::batch_aos_to_soa<<<static_cast<int>((nrow + 255) / 256), 256, 0, b->stream>>>(
-        b->staging, G.U, K, G.Np, G.Kpad, G.offset[b->index_in_group[i]]);
-    e = cudaGetLastError();
-  }
+  if (!e)
+    e = vt::launch_to_columns(reinterpret_cast<const double*>(b->staging), member_columns(b, i, G.U),
+                              G.num[b->index_in_group[i]], G.Np, b->stream);
   if (!e) e = cudaStreamSynchronize(b->stream);
   return e ? fail(VT_ERR_CUDA, vt::cuda_msg("vt_batch_upload_state", e)) : VT_OK;
 }
@@ -494,10 +455,8 @@ int vt_batch_download_state(vt_batch* b, int i, double* U, double* F) {
   vt::Group& G = b->groups[b->group_of[i]];
   const int K = b->K_of[i];
   const size_t bytes = sizeof(double) * 4 * static_cast<size_t>(K) * G.Np;
-  const long long nrow = static_cast<long long>(K) * 2 * G.Np;
-  vt::batch_soa_to_aos<<<static_cast<int>((nrow + 255) / 256), 256, 0, b->stream>>>(
-      G.U, b->staging, K, G.Np, G.Kpad, G.offset[b->index_in_group[i]]);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = vt::launch_from_columns(member_columns(b, i, G.U), reinterpret_cast<double*>(b->staging),
+                                          G.num[b->index_in_group[i]], G.Np, b->stream);
   if (!e) e = cudaMemcpyAsync(U, b->staging, bytes, cudaMemcpyDeviceToHost, b->stream);
   if (!e) e = cudaStreamSynchronize(b->stream);
   if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("vt_batch_download_state", e));
@@ -511,11 +470,7 @@ int vt_batch_upload_state_device(vt_batch* b, int i, const double* dU) {
   std::lock_guard<std::mutex> lk(b->mu);
   cudaSetDevice(b->device);
   vt::Group& G = b->groups[b->group_of[i]];
-  const int K = b->K_of[i];
-  const long long nrow = static_cast<long long>(K) * 2 * G.Np;
-  vt::batch_aos_to_soa<<<static_cast<int>((nrow + 255) / 256), 256, 0, b->stream>>>(
-      reinterpret_cast<const double2*>(dU), G.U, K, G.Np, G.Kpad, G.offset[b->index_in_group[i]]);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = vt::launch_to_columns(dU, member_columns(b, i, G.U), G.num[b->index_in_group[i]], G.Np, b->stream);
   if (!e) e = cudaStreamSynchronize(b->stream);
   return e ? fail(VT_ERR_CUDA, vt::cuda_msg("vt_batch_upload_state_device", e)) : VT_OK;
 }
@@ -526,11 +481,7 @@ int vt_batch_download_state_device(vt_batch* b, int i, double* dU) {
   std::lock_guard<std::mutex> lk(b->mu);
   cudaSetDevice(b->device);
   vt::Group& G = b->groups[b->group_of[i]];
-  const int K = b->K_of[i];
-  const long long nrow = static_cast<long long>(K) * 2 * G.Np;
-  vt::batch_soa_to_aos<<<static_cast<int>((nrow + 255) / 256), 256, 0, b->stream>>>(
-      G.U, reinterpret_cast<double2*>(dU), K, G.Np, G.Kpad, G.offset[b->index_in_group[i]]);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = vt::launch_from_columns(member_columns(b, i, G.U), dU, G.num[b->index_in_group[i]], G.Np, b->stream);
   if (!e) e = cudaStreamSynchronize(b->stream);
   return e ? fail(VT_ERR_CUDA, vt::cuda_msg("vt_batch_download_state_device", e)) : VT_OK;
 }
@@ -594,14 +545,6 @@ int vt_batch_adjoint_forward(vt_batch* b, int nsteps, int nsnapshots) {
   for (size_t gi = 0; gi < b->groups.size(); ++gi) {
     vt::Group& G = b->groups[gi];
     vt_ctx* c = b->views[gi];
-    // each element steps with its instance's time step (the tiles already carry it)
-    std::vector<double> edt(static_cast<size_t>(G.K));
-    for (size_t m = 0; m < G.members.size(); ++m)
-      std::fill(edt.begin() + G.offset[m], edt.begin() + G.offset[m] + b->K_of[G.members[m]], b->dt[G.members[m]]);
-    cudaError_t e = cudaMemcpyAsync(b->view_dt[gi], edt.data(), sizeof(double) * edt.size(), cudaMemcpyHostToDevice,
-                                    b->stream);
-    if (!e) e = cudaStreamSynchronize(b->stream);
-    if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("batch adjoint time steps", e));
     c->max_blocks = G.max_blocks;
     st = vt_adjoint_forward(c, 1.0, nsteps, nsnapshots);
     if (st > 0) {  // map the group element to its instance
@@ -726,7 +669,7 @@ int vt_batch_autotune(vt_batch* b, int trials, int* blocks_per_sm_out, int* mapp
   // tuning does not advance the solution
   std::vector<std::vector<double2>> saved;
   for (auto& G : b->groups) {
-    const size_t state = 2 * G.Np * static_cast<size_t>(G.Kpad);
+    const size_t state = 2 * G.Np * static_cast<size_t>(G.ncols);
     saved.emplace_back(state);
     if (cudaMemcpy(saved.back().data(), G.U, state * sizeof(double2), cudaMemcpyDeviceToHost))
       return fail(VT_ERR_CUDA, "autotune save");
@@ -739,7 +682,7 @@ int vt_batch_autotune(vt_batch* b, int trials, int* blocks_per_sm_out, int* mapp
     vt::StageKernel best_k = G.kern;
     int best_b = 1;
     float best_ms = 1e30f;
-    for (int map : {vt::kMapComponent, vt::kMapPair}) {
+    for (int map : {vt::kMapComponent, vt::kMapDefault}) {
       const vt::StageKernel k = vt::select_kernel(G.p, G.nfq, G.ops.data(), map);
       int limit = 0;
       if (k.configure(&limit)) continue;
@@ -781,7 +724,7 @@ int vt_batch_set_mapping(vt_batch* b, const int* mapping) {
   std::lock_guard<std::mutex> lk(b->mu);
   cudaSetDevice(b->device);
   for (size_t gi = 0; gi < b->groups.size(); ++gi) {
-    if (mapping[gi] != vt::kMapComponent && mapping[gi] != vt::kMapPair)
+    if (mapping[gi] != vt::kMapComponent && mapping[gi] != vt::kMapDefault)
       return fail(VT_ERR_INVALID, "vt_batch_set_mapping: mapping must be 0 (component) or 1 (pair)");
     vt::Group& G = b->groups[gi];
     const vt::StageKernel k = vt::select_kernel(G.p, G.nfq, G.ops.data(), mapping[gi]);
@@ -810,7 +753,7 @@ int vt_batch_time_groups(vt_batch* b, int reps, float* ms_per_step) {
   for (size_t gi = 0; gi < b->groups.size() && !st; ++gi) {
     vt::Group& G = b->groups[gi];
     // the group's state is saved and restored, so timing does not advance the solution
-    const size_t state = 2 * G.Np * static_cast<size_t>(G.Kpad);
+    const size_t state = 2 * G.Np * static_cast<size_t>(G.ncols);
     std::vector<double2> saved(state);
     cudaError_t e = cudaMemcpy(saved.data(), G.U, state * sizeof(double2), cudaMemcpyDeviceToHost);
     if (!e) e = enqueue_group_step(G, b->stream);  // warm-up

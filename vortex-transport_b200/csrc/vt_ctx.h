@@ -18,15 +18,15 @@ struct AdjointState;  // vt_adjoint.cu
 struct vt_ctx {
   std::mutex mu;
   int device = 0, p = 0, Np = 0, nfq = 0, K = 0;
-  long long Kpad = 0;
+  vt::Numbering num;
+  long long ncols = 0;  // columns: 64 per tile
   int max_blocks = 0;  // persistent grid: SMs x resident blocks per SM
   cudaStream_t stream = nullptr;
   double2 *U = nullptr, *A = nullptr, *Sa = nullptr, *Sb = nullptr, *R = nullptr;
   double2* geo = nullptr;
   int4* nbr = nullptr;
-  int4* tiles = nullptr;      // tile runs
-  int* tile_items = nullptr;  // per-tile face lists
-  int* tile_count = nullptr;
+  int* elem = nullptr;              // element of each column
+  unsigned char* lists = nullptr;   // per-tile face lists
   int ntiles = 0;
   unsigned long long* err = nullptr;
   double2* aos = nullptr;
@@ -42,10 +42,16 @@ struct vt_ctx {
   int pending_steps = 0;
   double pending_dt = 0.0;
   bool side_pairing = false;  // nbr(nbr(e, s), s) == e for every element and side
-  // Per-tile / per-element time steps (a batch group's view; null otherwise):
-  // stage and adjoint coefficients are then fractions scaled on the device.
+  // Per-tile time steps (a batch group's view; null otherwise): stage and
+  // adjoint coefficients are then fractions scaled on the device.
   const double* tile_dt = nullptr;
-  const double* elem_dt = nullptr;
+  // A batch group's view: the numbering of each instance, at its first column
+  // and its first element (else empty: num numbers everything).
+  struct Part {
+    vt::Numbering num;
+    long long column, element;
+  };
+  std::vector<Part> parts;
   vt::AdjointState* adj = nullptr;
   // vt_test_bulk_wait: the stage kernels' wait bound and test flags
   unsigned test_wait_tries = 0;
@@ -55,6 +61,10 @@ struct vt_ctx {
 namespace vt {
 
 std::string cuda_msg(const char* what, cudaError_t e);
+
+// A mesh's geometry rows and side-ordered neighbour columns (StageArgs), its
+// columns starting at `column` of the arrays.
+void pack_mesh(const vt_mesh_desc& d, const Numbering& num, double2* geo, int4* nbr, long long column);
 
 // Arguments of one stage launch on this context's mesh and schedule.
 StageArgs stage_args(vt_ctx* c, const double2* in, const double2* base, double2* acc, double2* out, int stage,
@@ -68,9 +78,9 @@ cudaError_t reset_error_words(vt_ctx* c);
 int finish(vt_ctx* c, int nsteps, double dt);
 // Device AoS staging buffer (K x Np x 4 doubles), allocated on first use.
 int ensure_aos(vt_ctx* c);
-// AoS (K x Np x 4, device memory) <-> the SoA-of-double2 state layout.
-cudaError_t aos_to_soa(vt_ctx* c, const double* src, double2* dst);
-cudaError_t soa_to_aos(vt_ctx* c, const double2* src, double* dst);
+// AoS (K x Np x 4, device memory) <-> the columns of a state vector.
+cudaError_t to_columns(vt_ctx* c, const double* src, double2* dst);
+cudaError_t from_columns(vt_ctx* c, const double2* src, double* dst);
 
 // Frees the adjoint's buffers (no-op without them).
 void adjoint_release(vt_ctx* c);

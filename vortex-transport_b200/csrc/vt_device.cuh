@@ -1,15 +1,18 @@
 // Device-side building blocks of the stepper: state layout, folded operators,
 // Roe flux, nodal flux and the first-error record.
 //
-// HBM layout of a state vector (U, a stage, the RK accumulator): structure of
-// arrays of double2, row r = 2*i + h for node i and component pair h
-// (h = 0: rho, rho u; h = 1: rho v, rho E), element e in the column:
-//   state[r * Kpad + e]
-// A warp touching 32 consecutive elements of one row reads 512 contiguous
-// bytes; one element's state is 2*Np 16-byte loads.
+// Layout in HBM. The elements are renumbered into columns: a tile is 64
+// columns (some may be empty), and half a tile, 32 columns, is a block. A state
+// vector (U, a stage, the RK accumulator) holds each block's 2 Np rows of 32
+// double2, row 2*i + h for node i and component pair h (h = 0: rho, rho u;
+// h = 1: rho v, rho E): a block is contiguous (10 KB at p = 3), so a tile
+// arrives by two bulk copies, a thread's rows lie at constant distances (the
+// loads and stores of a phase share one address computation), and a warp
+// touching the 32 columns of one row reads 512 contiguous bytes. The geometry
+// has the same form with 7 rows. Columns follow the mesh: the triangles of
+// type 0 of a tile are its first block, those of type 1 its second, so that
+// the faces of one kind join consecutive columns (Numbering).
 #pragma once
-
-#include <cuda.h>
 
 #include <cstdint>
 
@@ -73,7 +76,7 @@ __host__ __device__ constexpr int mirror_node(int p, int node) {
 }
 
 // StageOps split into the parts that are even and odd under the reflection
-// (fold_operators, vt_stage_inst.cuh). With Pj the mirror image of node j and
+// (fold_operators). With Pj the mirror image of node j and
 // r_i the residual of node i, the even part e_a = (r_a + r_Pa) / 2 and the odd
 // part o_a = (r_a - r_Pa) / 2 of a node pair are
 //   e_a = sum_j Dxi_e[a][j] (Gxi_j + Geta_Pj) + sum_q lift_e ...
@@ -98,16 +101,97 @@ struct FoldedOps {
   double tm[3][NFQ][NE];
 };
 
-// What one stage launch reads and writes. Geometry rows (double2, Kpad each):
-//   0: (Jinv00, Jinv01)  1: (Jinv10, Jinv11)  2..4: normal of side 0..2
-//   5: (len0/detJ, len1/detJ)  6: (len2/detJ, 0)
-// nbr[e] = (neighbour across side 0, 1, 2, unused).
+// Even and odd parts of the operators under the reflection (FoldedOps). Each
+// coefficient takes both of the entries that the symmetry makes equal, so the
+// rounding of the two is averaged.
+template <int P, int NFQ>
+inline void fold_operators(const StageOps<P, NFQ>& o, FoldedOps<P, NFQ>* f) {
+  constexpr int NP = np_of_p(P), NS = fold_nodes(P), NO = fold_pairs(P);
+  *f = FoldedOps<P, NFQ>{};
+  for (int a = 0; a < NS; ++a) {
+    const int i = fold_node(P, a), m = mirror_node(P, i);
+    for (int j = 0; j < NP; ++j) {
+      const int mj = mirror_node(P, j);
+      const double x = 0.5 * (o.D[0][i][j] + o.D[1][m][mj]), y = 0.5 * (o.D[0][m][j] + o.D[1][i][mj]);
+      f->De[a][j] = 0.5 * (x + y);
+      if (a < NO) f->Do[a][j] = 0.5 * (x - y);
+    }
+    for (int q = 0; q < NFQ; ++q) {
+      const int r = NFQ - 1 - q;
+      const double x = 0.5 * (o.lift[0][i][q] + o.lift[2][m][r]), y = 0.5 * (o.lift[0][m][q] + o.lift[2][i][r]);
+      f->Le[a][q] = -0.25 * (x + y);
+      if (a < NO) f->Lo[a][q] = -0.25 * (x - y);
+      if (q <= r) {
+        const double v = 0.5 * (o.lift[1][i][q] + o.lift[1][m][r]), z = 0.5 * (o.lift[1][m][q] + o.lift[1][i][r]);
+        f->L1e[a][q] = -0.25 * (v + z);
+        if (a < NO) f->L1o[a][q] = -0.25 * (v - z);
+      }
+    }
+  }
+  for (int s = 0; s < 3; ++s)
+    for (int q = 0; q < NFQ; ++q)
+      for (int k = 0; k < FoldedOps<P, NFQ>::NE; ++k) {
+        f->tp[s][q][k] = o.tp[s][q][k];
+        f->tm[s][q][k] = o.tm[s][q][k];
+      }
+}
+
+constexpr int kTileRun = 32;              // columns per block (half a tile)
+constexpr int kTileElems = 2 * kTileRun;  // columns per tile
+constexpr int kGeoRows = 7;
+
+// Index (in double2) of row `row` of column x of a state vector / the geometry.
+__host__ __device__ __forceinline__ long long state_index(int np, long long x, int row) {
+  return ((x >> 5) * 2 * np + row) * kTileRun + (x & 31);
+}
+__host__ __device__ __forceinline__ long long geo_index(long long x, int row) {
+  return ((x >> 5) * kGeoRows + row) * kTileRun + (x & 31);
+}
+
+// Which column holds which element. On the reference's structured mesh of nx x
+// ny cells (Meshgeneration.cpp:57-117: cell (j, row) holds elements
+// 2(row*nx + j) and +1, of types 0 and 1) a tile is a block of W x H cells, W H
+// <= 32, narrower at the mesh's right and upper edge; cell k of the tile has
+// its type-0 triangle in column k and its type-1 triangle in column 32 + k. On
+// any other mesh (nx = 0) a tile is 64 consecutive elements, the even ones in
+// its first block and the odd ones in its second. The elements' own order
+// (error reports, the callers' arrays) is never the columns' order.
+struct Numbering {
+  int K = 0, nx = 0, ny = 0, W = 0, H = 0, ntx = 0, ntiles = 0;
+  __host__ __device__ int column(int e) const {
+    if (nx == 0) return (e & ~63) | ((e & 1) << 5) | ((e & 63) >> 1);
+    const int cell = e >> 1, r = cell / nx, j = cell - r * nx;
+    const int ti = j / W, tj = r / H, w = W < nx - ti * W ? W : nx - ti * W;
+    return (tj * ntx + ti) * kTileElems + (e & 1) * kTileRun + (r - tj * H) * w + (j - ti * W);
+  }
+  // -1 for an empty column
+  __host__ __device__ int element(int x) const {
+    const int tile = x / kTileElems, half = (x >> 5) & 1, k = x & 31;
+    if (nx == 0) {
+      const int e = tile * kTileElems + 2 * k + half;
+      return e < K ? e : -1;
+    }
+    const int tj = tile / ntx, ti = tile - tj * ntx;
+    const int w = W < nx - ti * W ? W : nx - ti * W, r = k / w, j = k - r * w;
+    return r < H && tj * H + r < ny ? 2 * ((tj * H + r) * nx + ti * W + j) + half : -1;
+  }
+};
+
+// What one stage launch reads and writes. Geometry rows (double2 per column):
+//   0: (Jinv00, Jinv01)  1: (Jinv10, Jinv11)  2: (len0/detJ, len1/detJ)
+//   3: (len2/detJ, detJ)  4..6: normal of side 0..2
+// nbr[x] = (column across side 0, 1, 2, unused).
 //
-// Tiles: tiles[t] = (start0, len0, start1, len1), two runs of consecutive
-// elements (local columns 0..31 and 32..63). tile_items[t * kMaxItems + i],
-// i < tile_count[t], lists the (element, side) faces tile t evaluates:
-//   bits 0-7 local element, 8-9 side, 10 mirror (the neighbour is in the tile
-//   and receives -F), 11-18 the neighbour's local column when mirrored.
+// lists holds kTileListBytes per tile, built once per mesh (vt_schedule.cuh):
+//   uint16 [kMaxItems]  the (column, side) faces the tile evaluates, by class:
+//     both columns in the tile, the neighbour staged in a slot, the neighbour
+//     read from global memory (no slot left). Bits 0-5 the column in the tile,
+//     6-7 the side, 8 both in the tile, 9-15 the neighbour's column in the tile
+//     or its slot (kNoSlot: none);
+//   uint32 [4]  their number n, the face points per work item and a factor
+//     that divides by n (face_part);
+//   uint32 [2][kSlots]  per block, the neighbours to stage: 4 * column + side,
+//     kNoNeighbour where a slot is empty (the used slots come first).
 struct StageArgs {
   const double2* in;    // state the right-hand side is evaluated on
   const double2* base;  // U_n (RK4 stages 1, 2)
@@ -115,12 +199,10 @@ struct StageArgs {
   double2* out;         // next stage state / new U / the right-hand side itself
   const double2* geo;
   const int4* nbr;
-  const int4* tiles;
-  const int* tile_items;
-  const int* tile_count;
+  const int* elem;      // element of each column (-1: empty), or null: Numbering with nx = 0
+  const unsigned char* lists;
   const double* tile_dt;  // per-tile time step (batched problems), or null: c_* hold dt
   unsigned long long* err;  // [0] first-error key, [1] steps done, [2] blocks done
-  long long Kpad;
   int K;
   int ntiles;
   int stage;     // 0..3 RK4 stages, 4 forward Euler, 5 right-hand side only
@@ -128,31 +210,45 @@ struct StageArgs {
   double c_out;  // output coefficient
   // Test hook of the bounded waits (vt_test_bulk_wait): polls of the tile's
   // mbarrier before a wait gives up (0: the default bound), and bit 0 of
-  // test_flags issues no state copies at all, so every wait gives up.
+  // test_flags issues no copies at all, so every wait gives up.
   unsigned wait_tries = 0;
   int test_flags = 0;
   // RK4 stages 0-2 that only produce the next stage state (a step rerun to
   // keep its stage states): stage 1 does not form the accumulator
   int no_acc = 0;
-  // 2-D tensor maps of in / acc / base, [2 Np rows] x [2 Kpad doubles], box of
-  // 2 Np rows x 64 doubles (one 32-element run); encoded on the host by the
-  // launcher, read by the tensor copies through this grid-constant parameter
-  CUtensorMap map_in, map_acc, map_base;
 };
 
 enum : int { kTestNoCopies = 1 };
 
-constexpr int kTileRun = 32;            // elements per run
-constexpr int kTileElems = 2 * kTileRun;  // elements per tile
 constexpr int kMaxItems = 3 * kTileElems;
+// A block of a W x H tile has W + H faces that leave the tile, one of 64
+// consecutive elements in a row of the reference's mesh 33.
+constexpr int kSlots = 32;
+constexpr int kListCount = 2 * kMaxItems;      // byte offset of the counts
+constexpr int kListOuter = kListCount + 16;    // byte offset of the slots
+constexpr int kTileListBytes = kListOuter + 2 * kSlots * 4;
+static_assert(kListCount % 16 == 0 && kTileListBytes % 16 == 0, "16-byte copies");
+constexpr unsigned kNoNeighbour = 0xffffffffu;
+constexpr int kNoSlot = 127;
+
+__host__ __device__ constexpr unsigned face_item(int col, int side, bool inside, int x) {
+  return static_cast<unsigned>(col | (side << 6) | (inside ? 1 << 8 : 0) | (x << 9));
+}
+
+// The work items of a face list are its n faces times the parts of their nfq
+// points, part-major: item w is part w / n of face w % n. The factor 2^20 / n +
+// 1 makes w / n one multiplication, exact while w n < 2^20 (w < 10 n, n <= 192).
+__host__ __device__ constexpr unsigned face_factor(int n) { return n > 0 ? (1u << 20) / n + 1 : 0; }
+__device__ __forceinline__ int face_part(int w, unsigned factor) { return static_cast<int>((w * factor) >> 20); }
 
 enum : int { kStageEuler = 4, kStageRhs = 5 };
 
-// Warp mappings of the stage kernel (vt_tile.cuh): one thread per (element,
-// component), or per (element, component pair, node half). kMapFolded is the
-// form that kMapPair takes where the operators have the reference triangle's
-// reflection symmetry (select_kernel, vt_launch.cu).
-enum : int { kMapComponent = 0, kMapPair = 1, kMapFolded = 2 };
+// Mappings of the stage kernel (vt_tile.cuh), one thread per (element,
+// component) in each: kMapComponent applies the operators as they are;
+// kMapDefault takes the form kMapFolded where the operators have the reference
+// triangle's reflection symmetry, else kMapComponent's (select_kernel,
+// vt_launch.cu).
+enum : int { kMapComponent = 0, kMapDefault = 1, kMapFolded = 2 };
 
 // First-error key: (stage epoch << 40) | (((e * nfq + q) * 3 + s) * 4 + code).
 // The minimum over all failures is the failure the reference's serial loop
@@ -230,10 +326,13 @@ __device__ __forceinline__ int flux_error_code(const double* uL, const double* u
 //   the pressure sum and C2 share the normal's coefficients.
 // The checks look at the sign words of both densities, both pressures and c2
 // with integer instructions; only when one is not positive does
-// flux_error_code decide as the reference does.
-// Equal to the reference's expression up to rounding. Returns the reference's
-// error code (1 left state, 2 right state, 3 c2 <= 0) or 0.
-__device__ __forceinline__ int roe_flux2(const double* uL, const double* uR, double nx, double ny, double* f) {
+// flux_error_code decide as the reference does; one branch serves this and the
+// eigenvalue test. Equal to the reference's expression up to rounding.
+// on_error is called with the reference's error code (1 left state, 2 right
+// state, 3 c2 <= 0).
+template <typename OnError>
+__device__ __forceinline__ void roe_flux2(const double* uL, const double* uR, double nx, double ny, double* f,
+                                          OnError&& on_error) {
   const double rL = uL[0], rR = uR[0];
   const double rLR = rL * rR;
   const double y = rsqrt_nr(rLR);
@@ -261,18 +360,15 @@ __device__ __forceinline__ int roe_flux2(const double* uL, const double* uR, dou
   const double ci = c2 * c2;
   const double ci1 = recip_nr(ci);
 
-  const int sign = min(min(min(__double2hiint(rL), __double2hiint(rR)), min(__double2hiint(pL), __double2hiint(pR))),
-                       __double2hiint(c2));
-  int code = 0;
-  if (__builtin_expect(sign <= 0, 0)) code = flux_error_code(uL, uR, c2);
-
   const double t = ucp * ci1;
   const double l3 = fabs(t) < 0.1 ? fma(5.0 * ucp, t, 0.05 * ci) : fabs(ucp);
-  double s1l3, s2;  // (|l0| + |l1|)/2 - l3 and (|l0| - |l1|)/2
-  if (__builtin_expect((__double2hiint(t) & 0x7fffffff) < 0x3fec0000, 1)) {  // |t| < 7/8
-    s1l3 = ci - l3;
-    s2 = ucp;
-  } else {
+  double s1l3 = ci - l3, s2 = ucp;  // (|l0| + |l1|)/2 - l3 and (|l0| - |l1|)/2
+  // positive where |t| < 7/8 and the checked values are positive
+  const int usual = min(min(min(__double2hiint(rL), __double2hiint(rR)), min(__double2hiint(pL), __double2hiint(pR))),
+                        min(__double2hiint(c2), 0x3fec0000 - (__double2hiint(t) & 0x7fffffff)));
+  if (__builtin_expect(usual <= 0, 0)) {
+    const int code = flux_error_code(uL, uR, c2);
+    if (code) on_error(code);
     const double l0r = ucp + ci, l1r = ucp - ci, eps = 0.1 * ci;
     const double l0 = fabs(l0r) < eps ? fma(l0r * l0r, 5.0 * ci1, 0.05 * ci) : fabs(l0r);
     const double l1 = fabs(l1r) < eps ? fma(l1r * l1r, 5.0 * ci1, 0.05 * ci) : fabs(l1r);
@@ -288,7 +384,6 @@ __device__ __forceinline__ int roe_flux2(const double* uL, const double* uR, dou
   f[1] = fma(uL[1], unL, fma(uR[1], unR, fma(pC, nx, -fma(l3, du1, C1 * ui))));
   f[2] = fma(uL[2], unL, fma(uR[2], unR, fma(pC, ny, -fma(l3, du2, C1 * vi))));
   f[3] = fma(rHL, unL, fma(rHR, unR, -fma(l3, du3, fma(C1, Hi, C2 * ucp))));
-  return code;
 }
 
 // Nodal Euler flux of one node's state (the formula of Timestepping.cpp:141-158)

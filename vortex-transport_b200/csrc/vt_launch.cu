@@ -1,64 +1,24 @@
 // Kernel selection by (p, nfq, warp mapping) -- the instantiations are in
-// vt_stage_component.cu, vt_stage_pair.cu and vt_stage_folded.cu -- and the
-// tile schedule kernels (vt_launch.h).
-#include <cuda.h>
-
+// vt_stage_component.cu and vt_stage_folded.cu -- and the tile schedule kernels
+// (vt_launch.h).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <mutex>
 
 #include "vt_launch.h"
 #include "vt_schedule.cuh"
 
 namespace vt {
 
-namespace {
-
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q{};
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  });
-  return fn;
-}
-
-}  // namespace
-
-cudaError_t tensor_maps_available() { return encode_tiled() ? cudaSuccess : cudaErrorNotSupported; }
-
-// Tensor map of one SoA state vector: [2 Np rows] x [2 Kpad doubles], a box of
-// one 32-element run. No L2 promotion: a box row is 512 contiguous bytes, whole
-// sectors already (promotion to 256-byte lines was 0.2% slower at 768 x 768).
-cudaError_t encode_state_map(CUtensorMap* m, const void* base, long long Kpad, int Np) {
-  const EncodeTiledFn fn = encode_tiled();
-  if (!fn) return cudaErrorNotSupported;
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(2 * Kpad), static_cast<cuuint64_t>(2 * Np)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(2 * Kpad * sizeof(double))};
-  const cuuint32_t box[2] = {2 * kTileRun, static_cast<cuuint32_t>(2 * Np)};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<void*>(base), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
-}
-
 StageKernel select_kernel(int p, int nfq, const double* ops, int map) {
-  if (map != kMapPair) return select_kernel_component(p, nfq);
-  return operators_reflect(p, nfq, ops) ? select_kernel_folded(p, nfq) : select_kernel_pair(p, nfq);
+  const bool fold = map == kMapDefault && operators_reflect(p, nfq, ops);
+  StageKernel k = fold ? select_kernel_folded(p, nfq) : select_kernel_component(p, nfq);
+  k.map = map;
+  return k;
 }
 
 bool operators_reflect(int p, int nfq, const double* ops) {
-  if (p < 1 || p > 3) return false;  // p = 0 has one node: nothing to fold
+  if (p < 0 || p > 3) return false;
   const int np = np_of_p(p);
   auto D = [&](int d, int i, int j) { return ops[(d * np + i) * np + j]; };
   auto lift = [&](int s, int i, int q) { return ops[2 * np * np + (s * np + i) * nfq + q]; };
@@ -111,20 +71,68 @@ void fold_stage_operators(int p, int nfq, const double* minv, const double* stif
       for (int k = 0; k < NE; ++k) ops[o++] = phi_minus[(sd * Np + edge_node(p, sd, k)) * nfq + q];
 }
 
-std::vector<int4> structured_tile_runs(int K, const int32_t* type, const int32_t* conn) {
-  return structured_tiles(K, type, conn);
-}
+Numbering number_mesh(int K, const int32_t* type, const int32_t* conn) { return mesh_numbering(K, type, conn); }
+Numbering number_grid(int nx, int ny) { return grid_numbering(nx, ny); }
+Numbering number_contiguous(int K) { return contiguous_numbering(K); }
 
-std::vector<int4> grid_tile_runs(int nx, int ny) { return grid_tiles(nx, ny); }
-
-cudaError_t launch_contiguous_tiles(int4* tiles, int K, int ntiles, cudaStream_t st) {
-  contiguous_tiles_kernel<<<(ntiles + 255) / 256, 256, 0, st>>>(tiles, K, ntiles);
+cudaError_t launch_number_columns(const Numbering& num, int* elem, int x0, int e0, cudaStream_t st) {
+  number_columns_kernel<<<(num.ntiles * kTileElems + 255) / 256, 256, 0, st>>>(num, elem, x0, e0);
   return cudaGetLastError();
 }
 
-cudaError_t launch_build_tile_items(const int4* tiles, const int4* nbr, int* items, int* count, int ntiles, int nfq,
+cudaError_t launch_build_tile_lists(const int4* nbr, const int* elem, int K, int ntiles, int nfq, unsigned char* lists,
                                     cudaStream_t st) {
-  build_tile_items_kernel<<<ntiles, 256, 0, st>>>(tiles, nbr, items, count, nfq);
+  build_tile_lists_kernel<<<ntiles, 256, 0, st>>>(nbr, elem, K, nfq, lists);
+  return cudaGetLastError();
+}
+
+namespace {
+
+// A block of 32 columns at a time, through shared memory, so that the rows of
+// the block and the elements' own rows (2 Np double2 each) are both read and
+// written in order.
+__global__ void to_columns_kernel(const double2* __restrict__ aos, double2* __restrict__ blocks, const Numbering num,
+                                  int Np) {
+  extern __shared__ double2 tile[];
+  const int R = 2 * Np, b = blockIdx.x;
+  for (int l = threadIdx.x; l < kTileRun * R; l += blockDim.x) {
+    const int k = l / R, r = l - k * R, e = num.element(b * kTileRun + k);
+    if (e >= 0) tile[k * (R + 1) + r] = aos[static_cast<long long>(e) * R + r];
+  }
+  __syncthreads();
+  for (int l = threadIdx.x; l < kTileRun * R; l += blockDim.x) {
+    const int r = l / kTileRun, k = l % kTileRun;
+    if (num.element(b * kTileRun + k) >= 0)
+      blocks[(static_cast<long long>(b) * R + r) * kTileRun + k] = tile[k * (R + 1) + r];
+  }
+}
+
+__global__ void from_columns_kernel(const double2* __restrict__ blocks, double2* __restrict__ aos, const Numbering num,
+                                    int Np) {
+  extern __shared__ double2 tile[];
+  const int R = 2 * Np, b = blockIdx.x;
+  for (int l = threadIdx.x; l < kTileRun * R; l += blockDim.x) {
+    const int r = l / kTileRun, k = l % kTileRun;
+    tile[k * (R + 1) + r] = blocks[static_cast<long long>(b) * R * kTileRun + l];
+  }
+  __syncthreads();
+  for (int l = threadIdx.x; l < kTileRun * R; l += blockDim.x) {
+    const int k = l / R, r = l - k * R, e = num.element(b * kTileRun + k);
+    if (e >= 0) aos[static_cast<long long>(e) * R + r] = tile[k * (R + 1) + r];
+  }
+}
+
+}  // namespace
+
+cudaError_t launch_to_columns(const double* aos, double2* columns, const Numbering& num, int Np, cudaStream_t st) {
+  to_columns_kernel<<<2 * num.ntiles, 256, sizeof(double2) * kTileRun * (2 * Np + 1), st>>>(
+      reinterpret_cast<const double2*>(aos), columns, num, Np);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_from_columns(const double2* columns, double* aos, const Numbering& num, int Np, cudaStream_t st) {
+  from_columns_kernel<<<2 * num.ntiles, 256, sizeof(double2) * kTileRun * (2 * Np + 1), st>>>(
+      columns, reinterpret_cast<double2*>(aos), num, Np);
   return cudaGetLastError();
 }
 

@@ -4,8 +4,6 @@
 
 #include <cuda_runtime.h>
 
-#include <vector>
-
 #include "vt_device.cuh"
 
 namespace vt {
@@ -19,19 +17,19 @@ struct StageKernel {
   // Sets the dynamic shared-memory attribute on the current device and
   // reports resident blocks per SM. Call before any launch or capture.
   ConfigFn configure = nullptr;
-  // Warp mapping of the instantiation (kMapComponent or kMapPair, vt_tile.cuh).
+  // The mapping it was selected for (kMapComponent or kMapDefault).
   int map = 0;
 };
 
 // The mapping a context uses unless told otherwise.
-constexpr int kDefaultMap = kMapPair;
+constexpr int kDefaultMap = kMapDefault;
 
-// The kernel for the operator block `ops` (stage_ops_doubles(p, nfq) doubles).
-// kMapPair takes the folded form where operators_reflect says so.
+// The kernel for the operator block `ops` (stage_ops_doubles(p, nfq) doubles):
+// kMapDefault takes the folded form where operators_reflect says so, else the
+// same kernel as kMapComponent.
 // Empty (null members) for p outside 0..3, nfq outside 1..10.
 StageKernel select_kernel(int p, int nfq, const double* ops, int map = kDefaultMap);
 StageKernel select_kernel_component(int p, int nfq);
-StageKernel select_kernel_pair(int p, int nfq);
 StageKernel select_kernel_folded(int p, int nfq);
 
 // Whether the operator block has the reference triangle's reflection symmetry
@@ -53,24 +51,21 @@ int stage_ops_doubles(int p, int nfq);
 void fold_stage_operators(int p, int nfq, const double* minv, const double* stiff, const double* line,
                           const double* phi_plus, const double* phi_minus, double* ops);
 
-// Two-row tiles for the reference's structured mesh, empty if `conn` is not it.
-std::vector<int4> structured_tile_runs(int K, const int32_t* type, const int32_t* conn);
-// The same runs from the grid size alone (empty unless nx, ny suit them).
-std::vector<int4> grid_tile_runs(int nx, int ny);
+// Column numberings (vt_device.cuh): of a mesh (the reference's structured
+// mesh is recognised by its connectivity), of the reference's mesh of nx x ny
+// cells, and without knowledge of the mesh.
+Numbering number_mesh(int K, const int32_t* type, const int32_t* conn);
+Numbering number_grid(int nx, int ny);
+Numbering number_contiguous(int K);
 
-// Encodes the 2-D tensor map of a state vector for the stage kernel's tensor
-// copies: [2 Np rows] x [2 Kpad doubles], box of 2 Np rows x 64 doubles (one
-// run of 32 elements). Host only; a pure encoding (cuTensorMapEncodeTiled,
-// reached through the runtime's driver entry point), no allocation.
-cudaError_t encode_state_map(CUtensorMap* map, const void* base, long long Kpad, int Np);
-// cudaSuccess when the driver provides the tensor-map encoder (looked up once;
-// call before any stream capture).
-cudaError_t tensor_maps_available();
-
-// Device-side: tiles of 64 consecutive elements, then the per-tile face lists.
-cudaError_t launch_contiguous_tiles(int4* tiles, int K, int ntiles, cudaStream_t st);
-// nfq decides where the face items that read global memory are placed (vt_schedule.cuh).
-cudaError_t launch_build_tile_items(const int4* tiles, const int4* nbr, int* items, int* count, int ntiles, int nfq,
+// elem[x0 + x] = e0 + element of the numbering's column x (-1: empty).
+cudaError_t launch_number_columns(const Numbering& num, int* elem, int x0, int e0, cudaStream_t st);
+// The tiles' face lists (kTileListBytes each, 16-byte aligned) from the columns'
+// neighbours and elements (elem null: contiguous numbering of K elements).
+cudaError_t launch_build_tile_lists(const int4* nbr, const int* elem, int K, int ntiles, int nfq, unsigned char* lists,
                                     cudaStream_t st);
+// The callers' layout (K x Np x 4 doubles, 16-byte aligned) <-> a state vector's columns.
+cudaError_t launch_to_columns(const double* aos, double2* columns, const Numbering& num, int Np, cudaStream_t st);
+cudaError_t launch_from_columns(const double2* columns, double* aos, const Numbering& num, int Np, cudaStream_t st);
 
 }  // namespace vt

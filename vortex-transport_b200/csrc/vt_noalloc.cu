@@ -50,33 +50,34 @@ std::mutex g_setup_mu;
 size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
 struct Carve {
-  long long Kpad;
-  int ntiles;
-  size_t err, geo, nbr, tiles, items, count, U, A, Sa, Sb, total;
+  Numbering num;
+  size_t err, geo, nbr, lists, U, A, Sa, Sb, total;
 };
 
 Carve carve(int p, int K) {
   Carve c;
-  c.Kpad = (static_cast<long long>(K) + 127) / 128 * 128;
-  const size_t state = sizeof(double2) * 2 * np_of(p) * static_cast<size_t>(c.Kpad);
+  c.num = number_contiguous(K);
+  // sizes are those of 128-column multiples and of a list record of 788 bytes
+  // per tile, which is more than the columns need: the size limit stays where
+  // callers know it
+  const size_t cols = (static_cast<size_t>(K) + 127) / 128 * 128, tiles = static_cast<size_t>(c.num.ntiles);
+  const size_t state = sizeof(double2) * 2 * np_of(p) * cols;
   c.err = 0;
   c.geo = align256(c.err + 4 * sizeof(unsigned long long));
-  c.nbr = align256(c.geo + sizeof(double2) * 7 * static_cast<size_t>(c.Kpad));
-  c.ntiles = (K + kTileElems - 1) / kTileElems;
-  c.tiles = align256(c.nbr + sizeof(int4) * static_cast<size_t>(c.Kpad));
-  c.items = align256(c.tiles + sizeof(int4) * static_cast<size_t>(c.ntiles));
-  c.count = align256(c.items + sizeof(int) * kMaxItems * static_cast<size_t>(c.ntiles));
-  c.U = align256(c.count + sizeof(int) * static_cast<size_t>(c.ntiles));
+  c.nbr = align256(c.geo + sizeof(double2) * kGeoRows * cols);
+  c.lists = align256(c.nbr + sizeof(int4) * cols);
+  c.U = align256(align256(align256(c.lists + 16 * tiles) + 768 * tiles) + 4 * tiles);
   c.A = align256(c.U + state);
   c.Sa = align256(c.A + state);
   c.Sb = align256(c.Sa + state);
   c.total = align256(c.Sb + state);
   return c;
 }
+static_assert(kTileListBytes <= 768, "a tile's list fits its share of the scratch");
 
 // Packs the caller's per-element device arrays (vt_mesh_desc layouts) into the
 // kernel's geometry and side-ordered neighbour rows; flags bad neighbour ids.
-__global__ void pack_geometry_kernel(vt_device_mesh m, double2* geo, int4* nbr, long long KP,
+__global__ void pack_geometry_kernel(vt_device_mesh m, const Numbering num, double2* geo, int4* nbr,
                                      unsigned long long* err) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= m.n_elements) return;
@@ -84,34 +85,20 @@ __global__ void pack_geometry_kernel(vt_device_mesh m, double2* geo, int4* nbr, 
   const double* nv = m.normals + 6 * static_cast<size_t>(n);
   const double* ln = m.side_lengths + 3 * static_cast<size_t>(n);
   const double det = m.det_jacobian[n];
-  geo[0 * KP + n] = make_double2(ji[0], ji[1]);
-  geo[1 * KP + n] = make_double2(ji[2], ji[3]);
-  for (int s = 0; s < 3; ++s) geo[(2 + s) * KP + n] = make_double2(nv[2 * s], nv[2 * s + 1]);
-  geo[5 * KP + n] = make_double2(ln[0] / det, ln[1] / det);
-  geo[6 * KP + n] = make_double2(ln[2] / det, det);
+  const int x = num.column(n);
+  geo[geo_index(x, 0)] = make_double2(ji[0], ji[1]);
+  geo[geo_index(x, 1)] = make_double2(ji[2], ji[3]);
+  geo[geo_index(x, 2)] = make_double2(ln[0] / det, ln[1] / det);
+  geo[geo_index(x, 3)] = make_double2(ln[2] / det, det);
+  for (int s = 0; s < 3; ++s) geo[geo_index(x, 4 + s)] = make_double2(nv[2 * s], nv[2 * s + 1]);
   int right = m.neighbours[3 * n], left = m.neighbours[3 * n + 1], vert = m.neighbours[3 * n + 2];
   const int K = m.n_elements;
   if (right < 0 || right >= K || left < 0 || left >= K || vert < 0 || vert >= K) {
     atomicOr(&err[3], 1ull);
     right = left = vert = n;
   }
-  nbr[n] = m.element_type[n] == 0 ? make_int4(vert, right, left, 0) : make_int4(vert, left, right, 0);
-}
-
-__global__ void gather_soa_kernel(const double2* __restrict__ aos, double2* __restrict__ soa, int K, int Np,
-                                  long long KP) {
-  const long long l = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (l >= static_cast<long long>(K) * 2 * Np) return;
-  const int r = static_cast<int>(l / K), e = static_cast<int>(l % K);
-  soa[r * KP + e] = aos[static_cast<long long>(e) * 2 * Np + r];
-}
-
-__global__ void scatter_aos_kernel(const double2* __restrict__ soa, double2* __restrict__ aos, int K, int Np,
-                                   long long KP) {
-  const long long l = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (l >= static_cast<long long>(K) * 2 * Np) return;
-  const int r = static_cast<int>(l / K), e = static_cast<int>(l % K);
-  aos[static_cast<long long>(e) * 2 * Np + r] = soa[r * KP + e];
+  right = num.column(right), left = num.column(left), vert = num.column(vert);
+  nbr[x] = m.element_type[n] == 0 ? make_int4(vert, right, left, 0) : make_int4(vert, left, right, 0);
 }
 
 // The operator block of StageOps<P, NFQ> (at most 740 doubles), folded on the
@@ -178,7 +165,7 @@ int vt_step_rk4_noalloc(const vt_device_mesh* m, const double* dU_in, double* dU
   if (e || !scratch_ptr)
     return fail(VT_ERR_CUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
   int per_sm = 0;
-  if ((e = vt::tensor_maps_available()) || (e = pk.configure(&per_sm)))
+  if ((e = pk.configure(&per_sm)))
     return fail(VT_ERR_CUDA, std::string("kernel attributes: ") + cudaGetErrorString(e));
   const int max_blocks = ds->sms * (per_sm > 0 ? per_sm : 1);
 
@@ -186,9 +173,7 @@ int vt_step_rk4_noalloc(const vt_device_mesh* m, const double* dU_in, double* dU
   auto* errw = reinterpret_cast<unsigned long long*>(base + cv.err);
   auto* geo = reinterpret_cast<double2*>(base + cv.geo);
   auto* nbr = reinterpret_cast<int4*>(base + cv.nbr);
-  auto* tiles = reinterpret_cast<int4*>(base + cv.tiles);
-  auto* items = reinterpret_cast<int*>(base + cv.items);
-  auto* count = reinterpret_cast<int*>(base + cv.count);
+  unsigned char* lists = base + cv.lists;
   auto* U = reinterpret_cast<double2*>(base + cv.U);
   auto* A = reinterpret_cast<double2*>(base + cv.A);
   auto* Sa = reinterpret_cast<double2*>(base + cv.Sa);
@@ -200,14 +185,10 @@ int vt_step_rk4_noalloc(const vt_device_mesh* m, const double* dU_in, double* dU
   if ((e = cudaMemsetAsync(errw, 0xFF, sizeof(unsigned long long), st)) ||
       (e = cudaMemsetAsync(errw + 1, 0, 3 * sizeof(unsigned long long), st)))
     return fail(VT_ERR_CUDA, std::string("scratch reset: ") + cudaGetErrorString(e));
-  vt::pack_geometry_kernel<<<(K + 255) / 256, 256, 0, st>>>(*m, geo, nbr, cv.Kpad, errw);
-  if ((e = vt::launch_contiguous_tiles(tiles, K, cv.ntiles, st)) ||
-      (e = vt::launch_build_tile_items(tiles, nbr, items, count, cv.ntiles, m->n_line_points, st)))
+  vt::pack_geometry_kernel<<<(K + 255) / 256, 256, 0, st>>>(*m, cv.num, geo, nbr, errw);
+  if ((e = vt::launch_build_tile_lists(nbr, nullptr, K, cv.num.ntiles, m->n_line_points, lists, st)))
     return fail(VT_ERR_CUDA, std::string("tile schedule: ") + cudaGetErrorString(e));
-  const long long nrow = static_cast<long long>(K) * 2 * Np;
-  const int tb = static_cast<int>((nrow + 255) / 256);
-  vt::gather_soa_kernel<<<tb, 256, 0, st>>>(reinterpret_cast<const double2*>(dU_in), U, K, Np, cv.Kpad);
-  if ((e = cudaGetLastError())) return fail(VT_ERR_CUDA, std::string("pack: ") + cudaGetErrorString(e));
+  if ((e = vt::launch_to_columns(dU_in, U, cv.num, Np, st))) return fail(VT_ERR_CUDA, std::string("pack: ") + cudaGetErrorString(e));
 
   auto args = [&](const double2* in, double2* out, int stage, double c_acc, double c_out) {
     vt::StageArgs a;
@@ -217,13 +198,11 @@ int vt_step_rk4_noalloc(const vt_device_mesh* m, const double* dU_in, double* dU
     a.out = out;
     a.geo = geo;
     a.nbr = nbr;
-    a.tiles = tiles;
-    a.tile_items = items;
+    a.elem = nullptr;
+    a.lists = lists;
     a.tile_dt = nullptr;
-    a.tile_count = count;
-    a.ntiles = cv.ntiles;
+    a.ntiles = cv.num.ntiles;
     a.err = errw;
-    a.Kpad = cv.Kpad;
     a.K = K;
     a.stage = stage;
     a.c_acc = c_acc;
@@ -236,10 +215,7 @@ int vt_step_rk4_noalloc(const vt_device_mesh* m, const double* dU_in, double* dU
     if (!e) e = pk.launch(args(Sb, Sa, 2, (1.0 / 3) * dt, dt), ops, max_blocks, st);
     if (!e) e = pk.launch(args(Sa, U, 3, 0.0, (1.0 / 6) * dt), ops, max_blocks, st);
   }
-  if (!e) {
-    vt::scatter_aos_kernel<<<tb, 256, 0, st>>>(U, reinterpret_cast<double2*>(dU_out), K, Np, cv.Kpad);
-    e = cudaGetLastError();
-  }
+  if (!e) e = vt::launch_from_columns(U, dU_out, cv.num, Np, st);
   unsigned long long words[4] = {~0ull, 0, 0, 0};
   if (!e) e = cudaMemcpyAsync(words, errw, sizeof(words), cudaMemcpyDeviceToHost, st);
   if (!e) e = cudaStreamSynchronize(st);

@@ -1,40 +1,50 @@
-// Tile schedule of the stage kernel: which elements form each tile and which
-// faces each tile evaluates. Built once per mesh.
-//
-// A tile is two runs of up to 32 consecutive elements. On the reference's
-// structured mesh (Meshgeneration.cpp:57-117: cell (j, row) holds elements
-// 2(row*nx + j) and +1) a tile is 16 cells of two adjacent rows, so the faces
-// between the two rows are evaluated once inside the tile; on any other mesh a
-// tile is 64 consecutive elements.
+// Tile schedule of the stage kernel: which elements form each tile (Numbering,
+// vt_device.cuh) and which faces each tile evaluates. Built once per mesh.
 #pragma once
-
-#include <vector>
 
 #include "vt_device.cuh"
 
 namespace vt {
 
-// Two-row tiles of the reference's structured mesh with nx x ny cells (nx a
-// multiple of kTileRun / 2 and ny even); empty otherwise.
-inline std::vector<int4> grid_tiles(int nx, int ny) {
-  std::vector<int4> tiles;
-  constexpr int cells = kTileRun / 2;  // cells per run
-  if (nx < 1 || ny < 1 || nx % cells || ny % 2) return tiles;
-  for (int rp = 0; rp < ny / 2; ++rp)
-    for (int j = 0; j < nx / cells; ++j) {
-      const int s0 = 2 * nx * (2 * rp) + kTileRun * j;
-      tiles.push_back(make_int4(s0, kTileRun, s0 + 2 * nx, kTileRun));
+// Tiles of the reference's structured mesh of nx x ny cells. The stage kernel
+// does every phase for all 64 columns of a tile, filled or not, except the
+// faces: 3 W H + W + H of them (W H diagonals, the ones between its cells once,
+// the 2 W + 2 H on its rim by each side). So the shape is the one with the
+// least tiles x (158 + faces), 158 faces' worth of FP64 instructions being
+// what the other phases take at p = 3, nfq = 6; 8 x 4 cells (108 faces, 24 of
+// them on the rim) where nx and ny allow, where two rows of 16 have 114 and 36.
+// It depends on nothing but nx and ny, so that a problem has the same tiles,
+// and rounds the same way, alone and in a batch.
+inline Numbering grid_numbering(int nx, int ny) {
+  Numbering best;
+  double least = 0.0;
+  for (int H = 1; H <= kTileRun && H <= ny; ++H)
+    for (int W = 1; W * H <= kTileRun && W <= nx; ++W) {
+      const int ntx = (nx + W - 1) / W, nty = (ny + H - 1) / H;
+      const double cost = static_cast<double>(ntx) * nty * (158.0 + 3 * W * H + W + H);
+      if (best.ntiles == 0 || cost < least || (cost == least && W > best.W)) {
+        least = cost;
+        best.K = 2 * nx * ny;
+        best.nx = nx, best.ny = ny, best.W = W, best.H = H, best.ntx = ntx, best.ntiles = ntx * nty;
+      }
     }
-  return tiles;
+  return best;
 }
 
-// grid_tiles when `conn`/`type` are exactly the reference's periodic
-// structured mesh; empty otherwise.
-inline std::vector<int4> structured_tiles(int K, const int32_t* type, const int32_t* conn) {
-  std::vector<int4> tiles;
-  if (K < 2 || conn[1] < 1) return tiles;
+inline Numbering contiguous_numbering(int K) {
+  Numbering n;
+  n.K = K;
+  n.ntiles = (K + kTileElems - 1) / kTileElems;
+  return n;
+}
+
+// grid_numbering when `conn`/`type` are exactly the reference's periodic
+// structured mesh, else contiguous_numbering.
+inline Numbering mesh_numbering(int K, const int32_t* type, const int32_t* conn) {
+  const Numbering other = contiguous_numbering(K);
+  if (K < 2 || conn[1] < 1) return other;
   const int nx = (conn[1] + 1) / 2;  // element 0's left neighbour is 2 nx - 1
-  if (nx < 1 || K % (2 * nx)) return tiles;
+  if (nx < 1 || K % (2 * nx)) return other;
   const int ny = K / (2 * nx);
   for (int i = 0; i < K; ++i) {
     const int left = i % (2 * nx) == 0 ? i - 1 + 2 * nx : i - 1;
@@ -44,83 +54,105 @@ inline std::vector<int4> structured_tiles(int K, const int32_t* type, const int3
     if (i >= 2 * nx * (ny - 1)) vert = i % 2 == 0 ? i + 1 - 2 * nx : i - 1 - 2 * nx * (ny - 1);
     else if (i >= 2 * nx) vert = i % 2 == 0 ? i + 1 - 2 * nx : i - 1 + 2 * nx;
     else vert = i % 2 == 0 ? i + 1 + 2 * nx * (ny - 1) : i - 1 + 2 * nx;
-    if (type[i] != i % 2 || conn[3 * i] != right || conn[3 * i + 1] != left || conn[3 * i + 2] != vert)
-      return tiles;
+    if (type[i] != i % 2 || conn[3 * i] != right || conn[3 * i + 1] != left || conn[3 * i + 2] != vert) return other;
   }
-  return grid_tiles(nx, ny);
+  return grid_numbering(nx, ny);
 }
 
-__global__ void contiguous_tiles_kernel(int4* tiles, int K, int ntiles) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ntiles) return;
-  const int s0 = t * kTileElems, s1 = s0 + kTileRun;
-  const int l0 = min(kTileRun, K - s0), l1 = max(0, min(kTileRun, K - s1));
-  tiles[t] = make_int4(s0, l0, s1, l1);
+// elem[x] of the numbering's columns, for columns x0 .. x0 + 64 ntiles - 1 of
+// the array (elements e0 .. of it).
+__global__ void number_columns_kernel(const Numbering num, int* __restrict__ elem, int x0, int e0) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= num.ntiles * kTileElems) return;
+  const int e = num.element(x);
+  elem[x0 + x] = e < 0 ? -1 : e0 + e;
 }
 
-// One block of 256 threads per tile: every (element, side) of the tile is a
+__device__ __forceinline__ int side_of(const int4& n, int s) { return s == 0 ? n.x : (s == 1 ? n.y : n.z); }
+
+// One block of 256 threads per tile: every (side, column) of the tile is a
 // candidate; it is evaluated here when the neighbour is outside the tile or
-// has a larger index. Grouped by how the outer state is found -- a partner in
-// the tile, a side-0 neighbour staged in shared memory, any other neighbour
-// read from global memory -- so that a warp's work items take one path, and
-// in (element, side) order within a group.
+// is a later element (`elem` null: columns are numbered contiguously).
+// Grouped by how the outer state is found (a partner in the tile whose side
+// faces this one, a neighbour staged in a slot, a neighbour read from global
+// memory), and in (side, column) order within a group, so that the lanes of a
+// warp, which take consecutive faces, follow one path and read consecutive
+// columns of the shared buffers.
 //
-// The stage kernel gives work item w = item * nfq + q to thread w mod 256, so
-// with nw = n * nfq > 256 the threads below L = nw mod 256 (or all, when L is
-// 0) take one item more than the rest. The items of the last group wait on
-// global loads; they are placed on threads with one item fewer (item indices
-// from ceil(L / nfq) on, in the first round) when they fit there, so that
-// their latency does not lengthen the face phase.
-__global__ void build_tile_items_kernel(const int4* __restrict__ tiles, const int4* __restrict__ nbr,
-                                        int* __restrict__ items, int* __restrict__ count, int nfq) {
-  __shared__ int warp_n[3][8];
+// A work item is `points` face points of one face. The block's 256 threads
+// take ceil(n ceil(nfq / points) / 256) items each, so the points each
+// evaluates one after another are that times `points`: the list's `points` is
+// the one that makes this least (the largest among equals, since a list entry
+// and a normal are read per item): at nfq = 6, 3 for the 108 faces of 8 x 4
+// cells, 2 for up to 85, 1 for up to 42 faces.
+__global__ void build_tile_lists_kernel(const int4* __restrict__ nbr, const int* __restrict__ elem, int K, int nfq,
+                                        unsigned char* __restrict__ lists) {
+  __shared__ int warp_n[3][8], warp_out[2][8];
   const int tile = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int4 run = tiles[tile];
-  bool take = false;
-  int code = 0, cls = 0;
-  if (t < kMaxItems) {
-    const int el = t / 3, s = t % 3;
-    const int pos = el % kTileRun;
-    const bool second = el >= kTileRun;
-    const int e = (second ? run.z : run.x) + pos;
-    if (pos < (second ? run.w : run.y)) {
-      const int4 n4 = nbr[e];
-      const int nb = s == 0 ? n4.x : (s == 1 ? n4.y : n4.z);
-      int nl = -1;
-      if (nb >= run.x && nb < run.x + run.y) nl = nb - run.x;
-      else if (nb >= run.z && nb < run.z + run.w) nl = kTileRun + nb - run.z;
-      const bool inside = nl >= 0 && nb != e;
-      take = !inside || e < nb;
-      code = el | (s << 8) | (inside ? (1 << 10) | (nl << 11) : 0);
-      cls = inside ? 0 : (s == 0 ? 1 : 2);
-    }
+  unsigned char* list = lists + static_cast<long long>(tile) * kTileListBytes;
+  unsigned short* items = reinterpret_cast<unsigned short*>(list);
+  unsigned* counts = reinterpret_cast<unsigned*>(list + kListCount);
+  unsigned* outer = reinterpret_cast<unsigned*>(list + kListOuter);
+  if (t < 2 * kSlots) outer[t] = kNoNeighbour;
+  auto element = [&](int x) {
+    if (elem) return elem[x];
+    Numbering c;
+    c.K = K;
+    return c.element(x);
+  };
+  const int col = t % kTileElems, s = t / kTileElems, x = tile * kTileElems + col;
+  const bool second = col >= kTileRun;
+  bool take = false, inside = false;
+  int nb = 0;
+  const int e = t < kMaxItems ? element(x) : -1;
+  if (e >= 0) {
+    nb = side_of(nbr[x], s);
+    inside = nb / kTileElems == tile && nb != x && side_of(nbr[nb], s) == x;
+    take = !inside || e < element(nb);
   }
+  // slots: rank among the block's leaving faces (a warp holds one side of one block's columns)
+  const bool out = take && !inside;
+  const unsigned mo = __ballot_sync(0xffffffffu, out);
+  if (lane == 0) {
+    warp_out[0][warp] = second ? 0 : __popc(mo);
+    warp_out[1][warp] = second ? __popc(mo) : 0;
+  }
+  __syncthreads();
+  int slot = __popc(mo & ((1u << lane) - 1u));
+  for (int w = 0; w < warp; ++w) slot += warp_out[second][w];
+  const int cls = inside ? 0 : (slot < kSlots ? 1 : 2);
   unsigned m[3];
   for (int k = 0; k < 3; ++k) {
     m[k] = __ballot_sync(0xffffffffu, take && cls == k);
     if (lane == 0) warp_n[k][warp] = __popc(m[k]);
   }
   __syncthreads();
-  int n_cls[3] = {0, 0, 0};
+  int n = 0, rank = 0;  // position within the (class 0, class 1, class 2) order
   for (int k = 0; k < 3; ++k)
-    for (int w = 0; w < 8; ++w) n_cls[k] += warp_n[k][w];
-  const int n = n_cls[0] + n_cls[1] + n_cls[2];
-  // where the global-gather group goes: item index k0, or after the others
-  const int T = 4 * kTileElems, nw = n * nfq;
-  const int L = nw % T;
-  const int k0 = nfq > 0 ? (L + nfq - 1) / nfq : 0;
-  const bool move = nw > T && L > 0 && (k0 + n_cls[2]) * nfq <= T && k0 <= n_cls[0] + n_cls[1];
-  int rank = 0;  // position within the (class 0, class 1, class 2) order
-  for (int k = 0; k < cls; ++k) rank += n_cls[k];
-  for (int w = 0; w < warp; ++w) rank += warp_n[cls][w];
+    for (int w = 0; w < 8; ++w) {
+      n += warp_n[k][w];
+      if (k < cls || (k == cls && w < warp)) rank += warp_n[k][w];
+    }
   rank += __popc(m[cls] & ((1u << lane) - 1u));
-  int slot = rank;
-  if (move) {
-    if (cls == 2) slot = k0 + (rank - n_cls[0] - n_cls[1]);
-    else if (rank >= k0) slot = rank + n_cls[2];
+  if (take) {
+    const int y = inside ? nb % kTileElems : (cls == 1 ? second * kSlots + slot : kNoSlot);
+    items[rank] = static_cast<unsigned short>(face_item(col, s, inside, y));
+    if (cls == 1) outer[second * kSlots + slot] = 4u * static_cast<unsigned>(nb) + static_cast<unsigned>(s);
   }
-  if (take) items[static_cast<long long>(tile) * kMaxItems + slot] = code;
-  if (t == 0) count[tile] = n;
+  if (t == 0) {
+    int points = 1, least = 0;
+    for (int k = 1; k <= nfq; ++k) {
+      const int rounds = (n * ((nfq + k - 1) / k) + 4 * kTileElems - 1) / (4 * kTileElems);
+      if (k == 1 || rounds * k <= least) {
+        least = rounds * k;
+        points = k;
+      }
+    }
+    counts[0] = n;
+    counts[1] = points;
+    counts[2] = face_factor(n);
+    counts[3] = 0;
+  }
 }
 
 }  // namespace vt

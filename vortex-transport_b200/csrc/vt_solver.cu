@@ -20,7 +20,7 @@
 namespace vt {
 namespace {
 
-std::vector<double> fold_operators(int p, int nfq, const double* minv, const double* stiff,
+std::vector<double> host_operators(int p, int nfq, const double* minv, const double* stiff,
                                    const double* line, const double* phi_plus,
                                    const double* phi_minus) {
   std::vector<double> ops(static_cast<size_t>(stage_ops_doubles(p, nfq)));
@@ -28,50 +28,18 @@ std::vector<double> fold_operators(int p, int nfq, const double* minv, const dou
   return ops;
 }
 
-// Host AoS (K x Np x 4) <-> device SoA-of-double2 rows, through a shared
-// memory tile of 32 elements so both sides stay coalesced.
-constexpr int kTileE = 32;
-
-__global__ void aos_to_soa_kernel(const double2* __restrict__ aos, double2* __restrict__ soa, int K,
-                                  int Np, long long Kpad) {
-  extern __shared__ double2 tile[];
-  const int R = 2 * Np;
-  const int e0 = blockIdx.x * kTileE;
-  const int ne = min(kTileE, K - e0);
-  for (int l = threadIdx.x; l < ne * R; l += blockDim.x) tile[l] = aos[static_cast<long long>(e0) * R + l];
-  __syncthreads();
-  for (int l = threadIdx.x; l < kTileE * R; l += blockDim.x) {
-    const int r = l / kTileE, j = l % kTileE;
-    if (j < ne) soa[r * Kpad + e0 + j] = tile[j * R + r];
-  }
-}
-
-__global__ void soa_to_aos_kernel(const double2* __restrict__ soa, double2* __restrict__ aos, int K,
-                                  int Np, long long Kpad) {
-  extern __shared__ double2 tile[];
-  const int R = 2 * Np;
-  const int e0 = blockIdx.x * kTileE;
-  const int ne = min(kTileE, K - e0);
-  for (int l = threadIdx.x; l < kTileE * R; l += blockDim.x) {
-    const int r = l / kTileE, j = l % kTileE;
-    if (j < ne) tile[j * R + r] = soa[r * Kpad + e0 + j];
-  }
-  __syncthreads();
-  for (int l = threadIdx.x; l < ne * R; l += blockDim.x) aos[static_cast<long long>(e0) * R + l] = tile[l];
-}
-
-// Conservation totals: per block, sum over its elements of detJ * W . U in a
+// Conservation totals: per block, sum over its columns of detJ * W . U in a
 // fixed order; a second single-block pass sums the partials in a fixed order.
 __global__ void totals_partial_kernel(const double2* __restrict__ U, const double2* __restrict__ geo,
-                                      const double* __restrict__ W, int K, int Np, long long Kpad,
+                                      const double* __restrict__ W, const int* __restrict__ elem, int ncols, int Np,
                                       double* __restrict__ partial) {
   __shared__ double red[4][256];
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
   double acc[4] = {0, 0, 0, 0};
-  if (e < K) {
-    const double detj = geo[6 * Kpad + e].y;
+  if (x < ncols && elem[x] >= 0) {
+    const double detj = geo[geo_index(x, 3)].y;
     for (int i = 0; i < Np; ++i) {
-      const double2 a = U[(2 * i) * Kpad + e], b = U[(2 * i + 1) * Kpad + e];
+      const double2 a = U[state_index(Np, x, 2 * i)], b = U[state_index(Np, x, 2 * i + 1)];
       acc[0] += W[i] * a.x;
       acc[1] += W[i] * a.y;
       acc[2] += W[i] * b.x;
@@ -96,18 +64,19 @@ __global__ void totals_partial_kernel(const double2* __restrict__ U, const doubl
 // sums in a fixed order, summed by totals_final_kernel.
 __global__ void l2_partial_kernel(const double2* __restrict__ U, const double2* __restrict__ V,
                                   const double2* __restrict__ geo, const double* __restrict__ bq,
-                                  const double* __restrict__ wq, int nq, int K, int Np, long long Kpad,
-                                  double* __restrict__ partial) {
+                                  const double* __restrict__ wq, const int* __restrict__ elem, int nq, int ncols,
+                                  int Np, double* __restrict__ partial) {
   __shared__ double red[4][256];
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
   double acc[4] = {0, 0, 0, 0};
-  if (e < K) {
+  if (x < ncols && elem[x] >= 0) {
     double del[10][4];
     for (int j = 0; j < Np; ++j) {
-      const double2 a = U[(2 * j) * Kpad + e], b = U[(2 * j + 1) * Kpad + e];
-      const double2 c = V[(2 * j) * Kpad + e], d = V[(2 * j + 1) * Kpad + e];
-      const double x[4] = {a.x - c.x, a.y - c.y, b.x - d.x, b.y - d.y};
-      for (int k = 0; k < 4; ++k) del[j][k] = x[k] * x[k];
+      const long long i0 = state_index(Np, x, 2 * j), i1 = i0 + kTileRun;
+      const double2 a = U[i0], b = U[i1];
+      const double2 c = V[i0], d = V[i1];
+      const double dv[4] = {a.x - c.x, a.y - c.y, b.x - d.x, b.y - d.y};
+      for (int k = 0; k < 4; ++k) del[j][k] = dv[k] * dv[k];
     }
     for (int k = 0; k < 4; ++k) {
       double s = 0.0;
@@ -116,7 +85,7 @@ __global__ void l2_partial_kernel(const double2* __restrict__ U, const double2* 
         for (int j = 0; j < Np; ++j) v += del[j][k] * bq[q * Np + j];
         s += wq[q] * v;
       }
-      acc[k] = geo[6 * Kpad + e].y * s;
+      acc[k] = geo[geo_index(x, 3)].y * s;
     }
   }
   for (int c = 0; c < 4; ++c) red[c][threadIdx.x] = acc[c];
@@ -148,20 +117,21 @@ __device__ void vortex_point(const vt_vortex& c, double x, double y, double t, d
 
 // L2 projection of the vortex onto each element's basis (Element.cpp:180-326):
 // b_i = sum_q detJ phi_i(q) u(x_q) w_q, U_i = sum_j (M_ref^-1_ij / detJ) b_j, with
-// x_q the affine image of the area-rule point. One thread per element; tab
+// x_q the affine image of the area-rule point. One thread per column; tab
 // holds the basis at the points (nq x Np), the weights (nq), the points (nq x 2)
 // and M_ref^-1 (Np x Np).
 __global__ void project_vortex_kernel(const double* __restrict__ verts, const double2* __restrict__ geo,
-                                      const double* __restrict__ tab, int nq, const vt_vortex ic, double t, int K,
-                                      int Np, long long Kpad, double2* __restrict__ U) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= K) return;
+                                      const double* __restrict__ tab, int nq, const vt_vortex ic, double t,
+                                      const int* __restrict__ elem, int ncols, int Np, double2* __restrict__ U) {
+  const int col = blockIdx.x * blockDim.x + threadIdx.x;
+  const int e = col < ncols ? elem[col] : -1;
+  if (e < 0) return;
   const double* bq = tab;
   const double* wq = tab + nq * Np;
   const double* pq = wq + nq;
   const double* minv = pq + 2 * nq;
   const double* v = verts + 6 * static_cast<long long>(e);
-  const double det = geo[6 * Kpad + e].y;
+  const double det = geo[geo_index(col, 3)].y;
   double b[10][4];
   for (int i = 0; i < Np; ++i)
     for (int k = 0; k < 4; ++k) b[i][k] = 0.0;
@@ -179,8 +149,8 @@ __global__ void project_vortex_kernel(const double* __restrict__ verts, const do
     double r[4] = {0, 0, 0, 0};
     for (int j = 0; j < Np; ++j)
       for (int k = 0; k < 4; ++k) r[k] += (minv[i * Np + j] / det) * b[j][k];
-    U[(2 * i) * Kpad + e] = make_double2(r[0], r[1]);
-    U[(2 * i + 1) * Kpad + e] = make_double2(r[2], r[3]);
+    U[state_index(Np, col, 2 * i)] = make_double2(r[0], r[1]);
+    U[state_index(Np, col, 2 * i + 1)] = make_double2(r[2], r[3]);
   }
 }
 
@@ -210,7 +180,7 @@ __device__ void grid_point(const GridSpec& g, int a, int b, double* x, double* y
 
 // One thread per element: vertices, packed geometry rows, side-ordered
 // neighbours, and (when U is given) the nodal vortex state at the nodes.
-__global__ void structured_mesh_kernel(const GridSpec g, int Np, long long Kpad, double* __restrict__ verts,
+__global__ void structured_mesh_kernel(const GridSpec g, const Numbering num, int Np, double* __restrict__ verts,
                                        double2* __restrict__ geo, int4* __restrict__ nbr, const vt_vortex ic,
                                        double2* __restrict__ U) {
   const int K = 2 * g.nx * g.ny;
@@ -234,20 +204,22 @@ __global__ void structured_mesh_kernel(const GridSpec g, int Np, long long Kpad,
   const double l0 = pow(__dadd_rn(__dmul_rn(x1 - x0, x1 - x0), __dmul_rn(y1 - y0, y1 - y0)), 0.5);
   const double l1 = pow(__dadd_rn(__dmul_rn(x2 - x1, x2 - x1), __dmul_rn(y2 - y1, y2 - y1)), 0.5);
   const double l2 = pow(__dadd_rn(__dmul_rn(x0 - x2, x0 - x2), __dmul_rn(y0 - y2, y0 - y2)), 0.5);
-  geo[0 * Kpad + e] = make_double2(i00, i01);
-  geo[1 * Kpad + e] = make_double2(i10, i11);
-  geo[2 * Kpad + e] = make_double2((y1 - y0) / l0, -1 * (x1 - x0) / l0);
-  geo[3 * Kpad + e] = make_double2((y2 - y1) / l1, -1 * (x2 - x1) / l1);
-  geo[4 * Kpad + e] = make_double2((y0 - y2) / l2, -1 * (x0 - x2) / l2);
-  geo[5 * Kpad + e] = make_double2(l0 / det, l1 / det);
-  geo[6 * Kpad + e] = make_double2(l2 / det, det);
+  const int col = num.column(e);
+  geo[geo_index(col, 0)] = make_double2(i00, i01);
+  geo[geo_index(col, 1)] = make_double2(i10, i11);
+  geo[geo_index(col, 2)] = make_double2(l0 / det, l1 / det);
+  geo[geo_index(col, 3)] = make_double2(l2 / det, det);
+  geo[geo_index(col, 4)] = make_double2((y1 - y0) / l0, -1 * (x1 - x0) / l0);
+  geo[geo_index(col, 5)] = make_double2((y2 - y1) / l1, -1 * (x2 - x1) / l1);
+  geo[geo_index(col, 6)] = make_double2((y0 - y2) / l2, -1 * (x0 - x2) / l2);
   const int left = e % (2 * nx) == 0 ? e - 1 + 2 * nx : e - 1;
   const int right = (e + 1) % (2 * nx) == 0 ? e + 1 - 2 * nx : e + 1;
   int vert;
   if (e >= 2 * nx * (ny - 1)) vert = even ? e + 1 - 2 * nx : e - 1 - 2 * nx * (ny - 1);
   else if (e >= 2 * nx) vert = even ? e + 1 - 2 * nx : e - 1 + 2 * nx;
   else vert = even ? e + 1 + 2 * nx * (ny - 1) : e - 1 + 2 * nx;
-  nbr[e] = even ? make_int4(vert, right, left, 0) : make_int4(vert, left, right, 0);
+  const int cv = num.column(vert), cl = num.column(left), cr = num.column(right);
+  nbr[col] = even ? make_int4(cv, cr, cl, 0) : make_int4(cv, cl, cr, 0);
   if (!U) return;
   for (int i = 0; i < Np; ++i) {  // nodal initial condition (Element.cpp:124-179)
     const double xi = g.nodes_ref[2 * i], eta = g.nodes_ref[2 * i + 1], h0 = 1.0 - xi - eta;
@@ -255,8 +227,8 @@ __global__ void structured_mesh_kernel(const GridSpec g, int Np, long long Kpad,
     const double px = __dadd_rn(__dadd_rn(__dmul_rn(x0, h0), __dmul_rn(x1, xi)), __dmul_rn(x2, eta));
     const double py = __dadd_rn(__dadd_rn(__dmul_rn(y0, h0), __dmul_rn(y1, xi)), __dmul_rn(y2, eta));
     vortex_point(ic, px, py, 0.0, s4);
-    U[(2 * i) * Kpad + e] = make_double2(s4[0], s4[1]);
-    U[(2 * i + 1) * Kpad + e] = make_double2(s4[2], s4[3]);
+    U[state_index(Np, col, 2 * i)] = make_double2(s4[0], s4[1]);
+    U[state_index(Np, col, 2 * i + 1)] = make_double2(s4[2], s4[3]);
   }
 }
 
@@ -278,6 +250,25 @@ __global__ void totals_final_kernel(const double* __restrict__ partial, int nblo
 
 }  // namespace
 
+void pack_mesh(const vt_mesh_desc& d, const Numbering& num, double2* geo, int4* nbr, long long column) {
+  for (int n = 0; n < d.n_elements; ++n) {
+    const long long x = column + num.column(n);
+    const double* ji = d.inv_jacobian + 4 * static_cast<size_t>(n);
+    const double* nv = d.normals + 6 * static_cast<size_t>(n);
+    const double* ln = d.side_lengths + 3 * static_cast<size_t>(n);
+    const double det = d.det_jacobian[n];
+    geo[geo_index(x, 0)] = make_double2(ji[0], ji[1]);
+    geo[geo_index(x, 1)] = make_double2(ji[2], ji[3]);
+    geo[geo_index(x, 2)] = make_double2(ln[0] / det, ln[1] / det);
+    geo[geo_index(x, 3)] = make_double2(ln[2] / det, det);
+    for (int s = 0; s < 3; ++s) geo[geo_index(x, 4 + s)] = make_double2(nv[2 * s], nv[2 * s + 1]);
+    const int32_t* b = d.neighbours + 3 * static_cast<size_t>(n);
+    const int off = static_cast<int>(column);
+    const int right = off + num.column(b[0]), left = off + num.column(b[1]), vert = off + num.column(b[2]);
+    nbr[x] = d.element_type[n] == 0 ? make_int4(vert, right, left, 0) : make_int4(vert, left, right, 0);
+  }
+}
+
 std::string cuda_msg(const char* what, cudaError_t e) {
   return std::string(what) + ": " + cudaGetErrorString(e);
 }
@@ -298,9 +289,8 @@ void release(vt_ctx* c) {
   cudaSetDevice(c->device);
   vt::adjoint_release(c);
   if (c->rk4_graph) cudaGraphExecDestroy(c->rk4_graph);
-  void* bufs[] = {c->U,  c->A,     c->Sa,  c->Sb,         c->R,          c->geo,     c->nbr,
-                  c->err, c->aos,  c->W,   c->partial,    c->tot,        c->tiles,   c->tile_items,
-                  c->tile_count};
+  void* bufs[] = {c->U,   c->A,   c->Sa, c->Sb,      c->R,   c->geo,   c->nbr,
+                  c->err, c->aos, c->W,  c->partial, c->tot, c->elem,  c->lists};
   for (void* b : bufs)
     if (b) cudaFree(b);
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -320,13 +310,11 @@ vt::StageArgs stage_args(vt_ctx* c, const double2* in, const double2* base, doub
   a.out = out;
   a.geo = c->geo;
   a.nbr = c->nbr;
-  a.tiles = c->tiles;
-  a.tile_items = c->tile_items;
+  a.elem = c->elem;
+  a.lists = c->lists;
   a.tile_dt = c->tile_dt;
-  a.tile_count = c->tile_count;
   a.ntiles = c->ntiles;
   a.err = c->err;
-  a.Kpad = c->Kpad;
   a.K = c->K;
   a.stage = stage;
   a.c_acc = c_acc;
@@ -375,31 +363,31 @@ int ensure_aos(vt_ctx* c) {
   return e ? fail(VT_ERR_NO_MEMORY, vt::cuda_msg("staging buffer", e)) : VT_OK;
 }
 
-cudaError_t aos_to_soa(vt_ctx* c, const double* src, double2* dst) {
-  const int blocks = (c->K + vt::kTileE - 1) / vt::kTileE;
-  const size_t smem = sizeof(double2) * vt::kTileE * 2 * c->Np;
-  vt::aos_to_soa_kernel<<<blocks, 256, smem, c->stream>>>(reinterpret_cast<const double2*>(src), dst, c->K,
-                                                          c->Np, c->Kpad);
-  return cudaGetLastError();
+cudaError_t to_columns(vt_ctx* c, const double* src, double2* dst) {
+  if (c->parts.empty()) return launch_to_columns(src, dst, c->num, c->Np, c->stream);
+  cudaError_t e = cudaSuccess;
+  for (const auto& p : c->parts)
+    if (!e) e = launch_to_columns(src + 4ll * c->Np * p.element, dst + 2ll * c->Np * p.column, p.num, c->Np, c->stream);
+  return e;
 }
 
-cudaError_t soa_to_aos(vt_ctx* c, const double2* src, double* dst) {
-  const int blocks = (c->K + vt::kTileE - 1) / vt::kTileE;
-  const size_t smem = sizeof(double2) * vt::kTileE * 2 * c->Np;
-  vt::soa_to_aos_kernel<<<blocks, 256, smem, c->stream>>>(src, reinterpret_cast<double2*>(dst), c->K, c->Np,
-                                                          c->Kpad);
-  return cudaGetLastError();
+cudaError_t from_columns(vt_ctx* c, const double2* src, double* dst) {
+  if (c->parts.empty()) return launch_from_columns(src, dst, c->num, c->Np, c->stream);
+  cudaError_t e = cudaSuccess;
+  for (const auto& p : c->parts)
+    if (!e) e = launch_from_columns(src + 2ll * c->Np * p.column, dst + 4ll * c->Np * p.element, p.num, c->Np, c->stream);
+  return e;
 }
 
 }  // namespace vt
 
-using vt::aos_to_soa;
 using vt::enqueue_rk4_step;
 using vt::ensure_aos;
 using vt::finish;
 using vt::reset_error_words;
-using vt::soa_to_aos;
+using vt::from_columns;
 using vt::stage_args;
+using vt::to_columns;
 
 extern "C" {
 
@@ -442,13 +430,15 @@ vt_ctx* vt_create(const vt_mesh_desc* d, int device, int* status) {
   c->Np = vt::np_of(d->p);
   c->nfq = d->n_line_points;
   c->K = K;
-  c->Kpad = (static_cast<long long>(K) + 127) / 128 * 128;
-  c->ops = vt::fold_operators(c->p, c->nfq, d->inv_mass_ref, d->stiffness_ref, d->line_quadrature,
+  c->num = vt::number_mesh(K, d->element_type, d->neighbours);
+  c->ntiles = c->num.ntiles;
+  c->ncols = static_cast<long long>(vt::kTileElems) * c->ntiles;
+  c->ops = vt::host_operators(c->p, c->nfq, d->inv_mass_ref, d->stiffness_ref, d->line_quadrature,
                               d->phi_plus, d->phi_minus);
   const vt::StageKernel sk = vt::select_kernel(c->p, c->nfq, c->ops.data());
   c->launch = sk.launch;
   int per_sm = 0, sms = 0;
-  if ((e = vt::tensor_maps_available()) || (e = sk.configure(&per_sm)) ||
+  if ((e = sk.configure(&per_sm)) ||
       (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device))) {
     set(fail(VT_ERR_CUDA, vt::cuda_msg("stage kernel attributes", e)));
     delete c;
@@ -457,29 +447,18 @@ vt_ctx* vt_create(const vt_mesh_desc* d, int device, int* status) {
   c->max_blocks = sms * (per_sm > 0 ? per_sm : 1);
   c->minv_ref.assign(d->inv_mass_ref, d->inv_mass_ref + c->Np * c->Np);
 
-  // packed geometry and side-ordered neighbours (Evolve.cpp:167-202)
-  const long long KP = c->Kpad;
-  std::vector<double2> geo(7 * static_cast<size_t>(KP), make_double2(0.0, 0.0));
-  std::vector<int4> nbr(static_cast<size_t>(KP), make_int4(0, 0, 0, 0));
-  for (int n = 0; n < K; ++n) {
-    const double* ji = d->inv_jacobian + 4 * static_cast<size_t>(n);
-    const double* nv = d->normals + 6 * static_cast<size_t>(n);
-    const double* ln = d->side_lengths + 3 * static_cast<size_t>(n);
-    const double det = d->det_jacobian[n];
-    geo[0 * KP + n] = make_double2(ji[0], ji[1]);
-    geo[1 * KP + n] = make_double2(ji[2], ji[3]);
-    for (int s = 0; s < 3; ++s) geo[(2 + s) * KP + n] = make_double2(nv[2 * s], nv[2 * s + 1]);
-    geo[5 * KP + n] = make_double2(ln[0] / det, ln[1] / det);
-    geo[6 * KP + n] = make_double2(ln[2] / det, det);
-    const int right = d->neighbours[3 * n], left = d->neighbours[3 * n + 1], vert = d->neighbours[3 * n + 2];
-    nbr[n] = d->element_type[n] == 0 ? make_int4(vert, right, left, 0) : make_int4(vert, left, right, 0);
-  }
+  // packed geometry and side-ordered neighbours (Evolve.cpp:167-202), by column
+  const long long ncols = c->ncols;
+  std::vector<double2> geo(vt::kGeoRows * static_cast<size_t>(ncols), make_double2(0.0, 0.0));
+  std::vector<int4> nbr(static_cast<size_t>(ncols), make_int4(0, 0, 0, 0));
+  vt::pack_mesh(*d, c->num, geo.data(), nbr.data(), 0);
   // side s of an element faces side s of its neighbour (Evolve.cpp:167-202 on
   // the reference mesh); the adjoint's gather of neighbour face terms needs it
   c->side_pairing = true;
   for (int n = 0; n < K && c->side_pairing; ++n) {
-    const int4 b = nbr[n];
-    c->side_pairing = nbr[b.x].x == n && nbr[b.y].y == n && nbr[b.z].z == n;
+    const int x = c->num.column(n);
+    const int4 b = nbr[x];
+    c->side_pairing = nbr[b.x].x == x && nbr[b.y].y == x && nbr[b.z].z == x;
   }
   // W_i = integral of phi_i = sum_j M_ref[i][j] (the basis sums to one)
   std::vector<double> m(d->inv_mass_ref, d->inv_mass_ref + c->Np * c->Np), W(c->Np, 0.0);
@@ -487,13 +466,15 @@ vt_ctx* vt_create(const vt_mesh_desc* d, int device, int* status) {
   for (int i = 0; i < c->Np; ++i)
     for (int j = 0; j < c->Np; ++j) W[i] += m[i * c->Np + j];
 
-  const size_t state_bytes = sizeof(double2) * 2 * c->Np * static_cast<size_t>(KP);
-  const int tot_blocks = (K + 255) / 256;
+  const size_t state_bytes = sizeof(double2) * 2 * c->Np * static_cast<size_t>(ncols);
+  const int tot_blocks = static_cast<int>((ncols + 255) / 256);
   if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) || (e = alloc(&c->U, state_bytes)) ||
       (e = alloc(&c->A, state_bytes)) || (e = alloc(&c->Sa, state_bytes)) || (e = alloc(&c->Sb, state_bytes)) ||
       (e = alloc(&c->geo, geo.size() * sizeof(double2))) || (e = alloc(&c->nbr, nbr.size() * sizeof(int4))) ||
       (e = alloc(&c->err, 4 * sizeof(unsigned long long))) || (e = alloc(&c->W, sizeof(double) * c->Np)) ||
-      (e = alloc(&c->partial, sizeof(double) * 4 * tot_blocks)) || (e = alloc(&c->tot, sizeof(double) * 4))) {
+      (e = alloc(&c->partial, sizeof(double) * 4 * tot_blocks)) || (e = alloc(&c->tot, sizeof(double) * 4)) ||
+      (e = alloc(&c->elem, sizeof(int) * ncols)) ||
+      (e = alloc(&c->lists, vt::kTileListBytes * static_cast<size_t>(c->ntiles)))) {
     const bool oom = e == cudaErrorMemoryAllocation;
     set(fail(oom ? VT_ERR_NO_MEMORY : VT_ERR_CUDA, vt::cuda_msg("vt_create", e)));
     release(c);
@@ -508,29 +489,13 @@ vt_ctx* vt_create(const vt_mesh_desc* d, int device, int* status) {
     release(c);
     return nullptr;
   }
-  // tile schedule: two-row tiles on the reference's structured mesh, runs of
-  // consecutive elements otherwise; then each tile's face list
-  {
-    const std::vector<int4> runs = vt::structured_tile_runs(K, d->element_type, d->neighbours);
-    c->ntiles = runs.empty() ? (K + vt::kTileElems - 1) / vt::kTileElems : static_cast<int>(runs.size());
-    if ((e = alloc(&c->tiles, sizeof(int4) * c->ntiles)) ||
-        (e = alloc(&c->tile_items, sizeof(int) * vt::kMaxItems * static_cast<size_t>(c->ntiles))) ||
-        (e = alloc(&c->tile_count, sizeof(int) * c->ntiles))) {
-      set(fail(e == cudaErrorMemoryAllocation ? VT_ERR_NO_MEMORY : VT_ERR_CUDA, vt::cuda_msg("tiles", e)));
-      release(c);
-      return nullptr;
-    }
-    if (runs.empty())
-      e = vt::launch_contiguous_tiles(c->tiles, K, c->ntiles, c->stream);
-    else
-      e = cudaMemcpyAsync(c->tiles, runs.data(), sizeof(int4) * runs.size(), cudaMemcpyHostToDevice, c->stream);
-    if (!e) e = vt::launch_build_tile_items(c->tiles, c->nbr, c->tile_items, c->tile_count, c->ntiles, c->nfq, c->stream);
-    if (!e) e = cudaStreamSynchronize(c->stream);
-    if (e) {
-      set(fail(VT_ERR_CUDA, vt::cuda_msg("tile schedule", e)));
-      release(c);
-      return nullptr;
-    }
+  e = vt::launch_number_columns(c->num, c->elem, 0, 0, c->stream);
+  if (!e) e = vt::launch_build_tile_lists(c->nbr, c->elem, K, c->ntiles, c->nfq, c->lists, c->stream);
+  if (!e) e = cudaStreamSynchronize(c->stream);
+  if (e) {
+    set(fail(VT_ERR_CUDA, vt::cuda_msg("tile schedule", e)));
+    release(c);
+    return nullptr;
   }
   set(VT_OK);
   return c;
@@ -591,12 +556,14 @@ vt_ctx* vt_create_structured(const vt_params* prm, const vt_vortex* ic_in, int d
   c->Np = Np;
   c->nfq = nfq;
   c->K = 2 * nx * ny;
-  c->Kpad = (static_cast<long long>(c->K) + 127) / 128 * 128;
-  c->ops = vt::fold_operators(p, nfq, minv.data(), stiff.data(), line.data(), pp.data(), pm.data());
+  c->num = vt::number_grid(nx, ny);
+  c->ntiles = c->num.ntiles;
+  c->ncols = static_cast<long long>(vt::kTileElems) * c->ntiles;
+  c->ops = vt::host_operators(p, nfq, minv.data(), stiff.data(), line.data(), pp.data(), pm.data());
   const vt::StageKernel sk = vt::select_kernel(p, nfq, c->ops.data());
   c->launch = sk.launch;
   int per_sm = 0, sms = 0;
-  if ((e = vt::tensor_maps_available()) || (e = sk.configure(&per_sm)) ||
+  if ((e = sk.configure(&per_sm)) ||
       (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device))) {
     set(fail(VT_ERR_CUDA, vt::cuda_msg("stage kernel attributes", e)));
     delete c;
@@ -610,13 +577,15 @@ vt_ctx* vt_create_structured(const vt_params* prm, const vt_vortex* ic_in, int d
   for (int i = 0; i < Np; ++i)
     for (int j = 0; j < Np; ++j) W[i] += m[i * Np + j];
 
-  const long long KP = c->Kpad;
-  const size_t state_bytes = sizeof(double2) * 2 * Np * static_cast<size_t>(KP);
-  const int tot_blocks = (c->K + 255) / 256;
+  const long long ncols = c->ncols;
+  const size_t state_bytes = sizeof(double2) * 2 * Np * static_cast<size_t>(ncols);
+  const int tot_blocks = static_cast<int>((ncols + 255) / 256);
   double* verts = nullptr;
   if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) || (e = alloc(&c->U, state_bytes)) ||
       (e = alloc(&c->A, state_bytes)) || (e = alloc(&c->Sa, state_bytes)) || (e = alloc(&c->Sb, state_bytes)) ||
-      (e = alloc(&c->geo, sizeof(double2) * 7 * KP)) || (e = alloc(&c->nbr, sizeof(int4) * KP)) ||
+      (e = alloc(&c->geo, sizeof(double2) * vt::kGeoRows * ncols)) || (e = alloc(&c->nbr, sizeof(int4) * ncols)) ||
+      (e = alloc(&c->elem, sizeof(int) * ncols)) ||
+      (e = alloc(&c->lists, vt::kTileListBytes * static_cast<size_t>(c->ntiles))) ||
       (e = alloc(&c->err, 4 * sizeof(unsigned long long))) || (e = alloc(&c->W, sizeof(double) * Np)) ||
       (e = alloc(&c->partial, sizeof(double) * 4 * tot_blocks)) || (e = alloc(&c->tot, sizeof(double) * 4)) ||
       (e = alloc(&verts, sizeof(double) * 6 * static_cast<size_t>(c->K)))) {
@@ -652,36 +621,25 @@ vt_ctx* vt_create_structured(const vt_params* prm, const vt_vortex* ic_in, int d
   if (!e) e = cudaMemsetAsync(c->A, 0, state_bytes, c->stream);
   if (!e) e = cudaMemsetAsync(c->Sa, 0, state_bytes, c->stream);
   if (!e) e = cudaMemsetAsync(c->Sb, 0, state_bytes, c->stream);
-  if (!e) e = cudaMemsetAsync(c->geo, 0, sizeof(double2) * 7 * KP, c->stream);
-  if (!e) e = cudaMemsetAsync(c->nbr, 0, sizeof(int4) * KP, c->stream);
+  if (!e) e = cudaMemsetAsync(c->geo, 0, sizeof(double2) * vt::kGeoRows * ncols, c->stream);
+  if (!e) e = cudaMemsetAsync(c->nbr, 0, sizeof(int4) * ncols, c->stream);
   if (!e) e = cudaMemcpyAsync(c->W, W.data(), sizeof(double) * Np, cudaMemcpyHostToDevice, c->stream);
   if (!e) {
     vt::structured_mesh_kernel<<<(c->K + 127) / 128, 128, 0, c->stream>>>(
-        g, Np, KP, verts, c->geo, c->nbr, ic, prm->U_initialization_type == 0 ? c->U : nullptr);
+        g, c->num, Np, verts, c->geo, c->nbr, ic, prm->U_initialization_type == 0 ? c->U : nullptr);
     e = cudaGetLastError();
   }
+  if (!e) e = vt::launch_number_columns(c->num, c->elem, 0, 0, c->stream);
   if (!e && prm->U_initialization_type == 1) {
     e = alloc(&dtab, sizeof(double) * tab.size());
     if (!e) e = cudaMemcpyAsync(dtab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice, c->stream);
     if (!e) {
-      vt::project_vortex_kernel<<<(c->K + 127) / 128, 128, 0, c->stream>>>(verts, c->geo, dtab, nq, ic, 0.0, c->K, Np,
-                                                                          KP, c->U);
+      vt::project_vortex_kernel<<<static_cast<int>((ncols + 127) / 128), 128, 0, c->stream>>>(
+          verts, c->geo, dtab, nq, ic, 0.0, c->elem, static_cast<int>(ncols), Np, c->U);
       e = cudaGetLastError();
     }
   }
-  // tiles: two-row runs of the structured mesh, or runs of consecutive elements
-  const std::vector<int4> runs = vt::grid_tile_runs(nx, ny);
-  c->ntiles = runs.empty() ? (c->K + vt::kTileElems - 1) / vt::kTileElems : static_cast<int>(runs.size());
-  if (!e) e = alloc(&c->tiles, sizeof(int4) * c->ntiles);
-  if (!e) e = alloc(&c->tile_items, sizeof(int) * vt::kMaxItems * static_cast<size_t>(c->ntiles));
-  if (!e) e = alloc(&c->tile_count, sizeof(int) * c->ntiles);
-  if (!e) {
-    if (runs.empty())
-      e = vt::launch_contiguous_tiles(c->tiles, c->K, c->ntiles, c->stream);
-    else
-      e = cudaMemcpyAsync(c->tiles, runs.data(), sizeof(int4) * runs.size(), cudaMemcpyHostToDevice, c->stream);
-  }
-  if (!e) e = vt::launch_build_tile_items(c->tiles, c->nbr, c->tile_items, c->tile_count, c->ntiles, c->nfq, c->stream);
+  if (!e) e = vt::launch_build_tile_lists(c->nbr, c->elem, c->K, c->ntiles, c->nfq, c->lists, c->stream);
   if (!e) e = cudaStreamSynchronize(c->stream);
   cudaFree(verts);
   if (dtab) cudaFree(dtab);
@@ -701,7 +659,7 @@ int vt_upload_state_device(vt_ctx* c, const double* dU) {
   if (!vt::aligned_to(dU, 16)) return fail(VT_ERR_INVALID, "vt_upload_state_device: dU is not 16-byte aligned");
   std::lock_guard<std::mutex> lk(c->mu);
   cudaSetDevice(c->device);
-  cudaError_t e = aos_to_soa(c, dU, c->U);
+  cudaError_t e = to_columns(c, dU, c->U);
   if (!e) e = cudaStreamSynchronize(c->stream);
   return e ? fail(VT_ERR_CUDA, vt::cuda_msg("upload", e)) : VT_OK;
 }
@@ -714,7 +672,7 @@ int vt_upload_state(vt_ctx* c, const double* U) {
   if (st) return st;
   cudaError_t e = cudaMemcpyAsync(c->aos, U, sizeof(double) * 4 * static_cast<size_t>(c->K) * c->Np,
                                   cudaMemcpyHostToDevice, c->stream);
-  if (!e) e = aos_to_soa(c, reinterpret_cast<const double*>(c->aos), c->U);
+  if (!e) e = to_columns(c, reinterpret_cast<const double*>(c->aos), c->U);
   if (!e) e = cudaStreamSynchronize(c->stream);
   return e ? fail(VT_ERR_CUDA, vt::cuda_msg("upload", e)) : VT_OK;
 }
@@ -724,7 +682,7 @@ int vt_download_state_device(vt_ctx* c, double* dU) {
   if (!vt::aligned_to(dU, 16)) return fail(VT_ERR_INVALID, "vt_download_state_device: dU is not 16-byte aligned");
   std::lock_guard<std::mutex> lk(c->mu);
   cudaSetDevice(c->device);
-  cudaError_t e = soa_to_aos(c, c->U, dU);
+  cudaError_t e = from_columns(c, c->U, dU);
   if (!e) e = cudaStreamSynchronize(c->stream);
   return e ? fail(VT_ERR_CUDA, vt::cuda_msg("download", e)) : VT_OK;
 }
@@ -735,7 +693,7 @@ int vt_download_state(vt_ctx* c, double* U, double* F) {
   cudaSetDevice(c->device);
   int st = ensure_aos(c);
   if (st) return st;
-  cudaError_t e = soa_to_aos(c, c->U, reinterpret_cast<double*>(c->aos));
+  cudaError_t e = from_columns(c, c->U, reinterpret_cast<double*>(c->aos));
   if (!e)
     e = cudaMemcpyAsync(U, c->aos, sizeof(double) * 4 * static_cast<size_t>(c->K) * c->Np,
                         cudaMemcpyDeviceToHost, c->stream);
@@ -828,12 +786,12 @@ int vt_rhs(vt_ctx* c, double* Udot) {
   int st = ensure_aos(c);
   if (st) return st;
   cudaError_t e = cudaSuccess;
-  if (!c->R) e = alloc(&c->R, sizeof(double2) * 2 * c->Np * static_cast<size_t>(c->Kpad));
+  if (!c->R) e = alloc(&c->R, sizeof(double2) * 2 * c->Np * static_cast<size_t>(c->ncols));
   if (!e) e = reset_error_words(c);
   if (!e)
     e = c->launch(stage_args(c, c->U, c->U, c->A, c->R, vt::kStageRhs, 0.0, 0.0), c->ops.data(),
                   c->max_blocks, c->stream);
-  if (!e) e = soa_to_aos(c, c->R, reinterpret_cast<double*>(c->aos));
+  if (!e) e = from_columns(c, c->R, reinterpret_cast<double*>(c->aos));
   if (!e)
     e = cudaMemcpyAsync(Udot, c->aos, sizeof(double) * 4 * static_cast<size_t>(c->K) * c->Np,
                         cudaMemcpyDeviceToHost, c->stream);
@@ -859,8 +817,9 @@ int vt_totals(vt_ctx* c, double* out) {
   if (!c || !out) return fail(VT_ERR_INVALID, "null argument");
   std::lock_guard<std::mutex> lk(c->mu);
   cudaSetDevice(c->device);
-  const int blocks = (c->K + 255) / 256;
-  vt::totals_partial_kernel<<<blocks, 256, 0, c->stream>>>(c->U, c->geo, c->W, c->K, c->Np, c->Kpad, c->partial);
+  const int blocks = static_cast<int>((c->ncols + 255) / 256);
+  vt::totals_partial_kernel<<<blocks, 256, 0, c->stream>>>(c->U, c->geo, c->W, c->elem, static_cast<int>(c->ncols), c->Np,
+                                                           c->partial);
   vt::totals_final_kernel<<<1, 256, 0, c->stream>>>(c->partial, blocks, c->tot);
   cudaError_t e = cudaGetLastError();
   if (!e) e = cudaMemcpyAsync(out, c->tot, 4 * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
@@ -892,11 +851,11 @@ int vt_l2_error(vt_ctx* c, int nq, const double* area_quad, const double* U_ref,
     e = cudaMemcpyAsync(c->aos, U_ref, sizeof(double) * 4 * static_cast<size_t>(c->K) * Np, cudaMemcpyHostToDevice,
                         c->stream);
   }
-  if (!e) e = aos_to_soa(c, device_pointers ? U_ref : reinterpret_cast<const double*>(c->aos), c->Sa);
-  const int blocks = (c->K + 255) / 256;
+  if (!e) e = to_columns(c, device_pointers ? U_ref : reinterpret_cast<const double*>(c->aos), c->Sa);
+  const int blocks = static_cast<int>((c->ncols + 255) / 256);
   if (!e) {
     vt::l2_partial_kernel<<<blocks, 256, 0, c->stream>>>(c->U, c->Sa, c->geo, dtab, dtab + static_cast<size_t>(nq) * Np,
-                                                          nq, c->K, Np, c->Kpad, c->partial);
+                                                          c->elem, nq, static_cast<int>(c->ncols), Np, c->partial);
     vt::totals_final_kernel<<<1, 256, 0, c->stream>>>(c->partial, blocks, c->tot);
     e = cudaGetLastError();
   }
@@ -930,8 +889,8 @@ int vt_project_vortex(vt_ctx* c, const double* vertices, const vt_vortex* ic, do
   if (!e) e = cudaMemcpyAsync(dtab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice, c->stream);
   if (!e) e = cudaMemcpyAsync(dverts, vertices, vbytes, cudaMemcpyHostToDevice, c->stream);
   if (!e) {
-    vt::project_vortex_kernel<<<(c->K + 127) / 128, 128, 0, c->stream>>>(dverts, c->geo, dtab, nq, *ic, t, c->K, Np,
-                                                                        c->Kpad, c->U);
+    vt::project_vortex_kernel<<<static_cast<int>((c->ncols + 127) / 128), 128, 0, c->stream>>>(
+        dverts, c->geo, dtab, nq, *ic, t, c->elem, static_cast<int>(c->ncols), Np, c->U);
     e = cudaGetLastError();
   }
   if (!e) e = cudaStreamSynchronize(c->stream);
@@ -966,7 +925,7 @@ int vt_load_state(vt_ctx* c, const char* path) {
 void* vt_stream(vt_ctx* c) { return c ? static_cast<void*>(c->stream) : nullptr; }
 
 int vt_set_stage_mapping(vt_ctx* c, int mapping) {
-  if (!c || (mapping != vt::kMapComponent && mapping != vt::kMapPair))
+  if (!c || (mapping != vt::kMapComponent && mapping != vt::kMapDefault))
     return fail(VT_ERR_INVALID, "vt_set_stage_mapping: mapping must be 0 (component) or 1 (pair)");
   std::lock_guard<std::mutex> lk(c->mu);
   cudaSetDevice(c->device);
