@@ -74,8 +74,8 @@ cudaError_t launch_tile(const AdjArgs& a, const double* ops, int max_blocks, cud
   const int grid = a.ntiles < max_blocks ? a.ntiles : max_blocks;
   FoldedOps<P, NFQ> fo;
   fold_operators(o, &fo);
-  adjoint_tile_kernel<P, NFQ><<<grid, 4 * kTileElems, AdjTileLayout<P, NFQ>::kBytes, st>>>(a, o, fo);
-  return cudaGetLastError();
+  return launch_dependent(adjoint_tile_kernel<P, NFQ>, grid, 4 * kTileElems, AdjTileLayout<P, NFQ>::kBytes, st, a, o,
+                          fo);
 }
 
 template <int P, int NFQ>

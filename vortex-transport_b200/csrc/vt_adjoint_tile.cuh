@@ -11,7 +11,7 @@
 //
 //   1. load   the tile's stage state, stage adjoint, geometry and face list by
 //             bulk copies (issued during the previous tile); the side nodes of
-//             the neighbours outside the tile and the normals by cp.async;
+//             the neighbours outside the tile by cp.async;
 //   2. lift^T thread (element, component): the lifted face adjoint
 //             bF(s, q) = -(len_s/detJ) sa sum_i LIFT_s[i][q] a_i at every face
 //             point (the transpose of the lift and of the folded mass
@@ -39,7 +39,7 @@
 // are per-half named barriers and each half issues its own next copies; the
 // load phase has no block barrier (phase 2 reads only the thread's own column,
 // phase 3 comes after a barrier), and a tile ends with a per-half barrier (the
-// next tile's normals and phase 2 reuse rows that this tile's phase 6 reads).
+// next tile's phase 2 reuses rows that this tile's phase 6 reads).
 //
 // Every wait on the mbarrier is bounded; a wait that gives up sets bit 1 of
 // err[3] and the block stops taking tiles.
@@ -61,31 +61,38 @@ struct AdjTileLayout {
   static constexpr int NE = B::NE;
   static constexpr int kTP = B::kBytes;                        // double [3][NFQ][NE] own trace weights
   static constexpr int kLF = kTP + 3 * NFQ * NE * 8 + 8 * (3 * NFQ * NE % 2);  // double [3][NFQ][NP] LIFT by point
-  static constexpr int kOut = kLF + 3 * NP * NFQ * 8 + 8 * (3 * NP * NFQ % 2);  // uint32 [2][kSlots]
-  static constexpr int kA = (kOut + 2 * kSlots * 4 + 127) / 128 * 128;  // double2 [2][2NP][32] stage adjoint
+  static constexpr int kOut = kLF + 3 * NP * NFQ * 8 + 8 * (3 * NP * NFQ % 2);  // uint32 [kOuterWords]
+  static constexpr int kA = (kOut + kOuterWords * 4 + 127) / 128 * 128;  // double2 [2][2NP][32] stage adjoint
   static constexpr int kBytes = kA + 2 * NP * kTileElems * 16;
 };
 
-// One thread per half announces and issues the bulk copies of block `which` of
-// a tile: its stage state, stage adjoint and geometry rows 0..3 and, for block
-// 0, the face list with its slots.
+// One thread per half announces the bulk copies of block `which` of a tile and
+// issues those of the mesh's arrays (geometry and, for block 0, the face list
+// with its slots), then those of the stage state and stage adjoint.
 template <int P, int NFQ>
-__device__ __forceinline__ void issue_adj_copies(const AdjArgs& a, int tile, int which, unsigned char* smem) {
+__device__ __forceinline__ void issue_adj_mesh_copies(const AdjArgs& a, int tile, int which, unsigned char* smem) {
   using L = AdjTileLayout<P, NFQ>;
   using B = TileLayout<P, NFQ>;
-  constexpr unsigned kState = 2 * B::NP * kTileRun * 16, kGeo = 4 * kTileRun * 16, kOuter = 2 * kSlots * 4;
+  constexpr unsigned kState = 2 * B::NP * kTileRun * 16, kGeo = kGeoRows * kTileRun * 16, kOuter = kOuterWords * 4;
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem + B::kBar);
   fence_proxy_async_smem();
   mbar_arrive_expect_tx(bar, 2 * kState + kGeo + (which == 0 ? kListOuter + kOuter : 0u));
-  const long long blk = 2ll * tile + which;
-  bulk_g2s(smem + B::kS + which * kState, a.U + blk * (2 * B::NP * kTileRun), kState, bar);
-  bulk_g2s(smem + L::kA + which * kState, a.a + blk * (2 * B::NP * kTileRun), kState, bar);
-  bulk_g2s(smem + B::kGE + which * kGeo, a.geo + blk * (kGeoRows * kTileRun), kGeo, bar);
+  bulk_g2s(smem + B::kGE + which * kGeo, a.geo + (2ll * tile + which) * (kGeoRows * kTileRun), kGeo, bar);
   if (which == 0) {
     const unsigned char* list = a.lists + static_cast<long long>(tile) * kTileListBytes;
     bulk_g2s(smem + B::kItems, list, kListOuter, bar);
     bulk_g2s(smem + L::kOut, list + kListOuter, kOuter, bar);
   }
+}
+template <int P, int NFQ>
+__device__ __forceinline__ void issue_adj_state_copies(const AdjArgs& a, int tile, int which, unsigned char* smem) {
+  using L = AdjTileLayout<P, NFQ>;
+  using B = TileLayout<P, NFQ>;
+  constexpr unsigned kState = 2 * B::NP * kTileRun * 16;
+  unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem + B::kBar);
+  const long long at = (2ll * tile + which) * (2 * B::NP * kTileRun);
+  bulk_g2s(smem + B::kS + which * kState, a.U + at, kState, bar);
+  bulk_g2s(smem + L::kA + which * kState, a.a + at, kState, bar);
 }
 
 // Even and odd parts of one component of a column's stage adjoint (node pairs
@@ -126,12 +133,12 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
   double* FB = reinterpret_cast<double*>(smem + B::kFB);
   double2* FB2 = reinterpret_cast<double2*>(smem + B::kFB);
   double2* GE = reinterpret_cast<double2*>(smem + B::kGE);
-  double2* NR = FB2 + B::kNormalRow * E;  // normals, until the transposed volume operator
   double* TM = reinterpret_cast<double*>(smem + B::kTM);
   const unsigned short* items = reinterpret_cast<const unsigned short*>(smem + B::kItems);
-  const unsigned* counts = reinterpret_cast<const unsigned*>(smem + B::kItems + kListCount);
+  const FaceCounts* counts = reinterpret_cast<const FaceCounts*>(smem + B::kItems + kListCount);
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem + B::kBar);
   int* abort_flag = reinterpret_cast<int*>(smem + B::kBar + 8);
+  int* NEXT = reinterpret_cast<int*>(smem + B::kBar + 12);
   double* TP = reinterpret_cast<double*>(smem + L::kTP);
   double* LF = reinterpret_cast<double*>(smem + L::kLF);
   const unsigned* OUT = reinterpret_cast<const unsigned*>(smem + L::kOut);
@@ -144,6 +151,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
   const int col = t % E;           // load and transposed flux phases
   const int el = work_column(t), c = work_component(t);
   const int G = gridDim.x;
+  const bool hand_out = a.ntiles > kHandOut * G;
 
   {
     const double* tm = &ops.tm[0][0][0];
@@ -162,23 +170,25 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
     mbar_init(bar, 2);
     *abort_flag = 0;
   }
-  int tile = blockIdx.x;
-  if (tile >= a.ntiles) return;
+  let_next_start();
+  int tile = blockIdx.x;  // the grid has at most ntiles blocks
   unsigned code = neighbour_code(a.lists, tile, which, lane);
   __syncthreads();
-  if (grp == 0 && lane == 0) issue_adj_copies<P, NFQ>(a, tile, which, smem);
+  if (grp == 0 && lane == 0) issue_adj_mesh_copies<P, NFQ>(a, tile, which, smem);
+  wait_for_previous();
+  if (grp == 0 && lane == 0) issue_adj_state_copies<P, NFQ>(a, tile, which, smem);
   copy_neighbours<P>(H, a.U, code, which, grp, lane);
   cp_async_commit();
   unsigned parity = 0;
   Ad += sidx<NP>(c >> 1, el) * 2 + (c & 1);              // this thread's component and column
   double* FBt = FB + ((c >> 1) * E + el) * 2 + (c & 1);  // likewise in the face buffer
 
-  for (; tile < a.ntiles; tile += G) {
-    const bool has_next = tile + G < a.ntiles;
+  while (true) {
     const long long blk = 2ll * tile + which;
+    unsigned taken = 0;
+    if (t == 224 && hand_out) taken = take_tile(a.err + 6);
 
     // ---- 1. load ------------------------------------------------------------------
-    if (grp < 3) cp_async16(NR + grp * E + col, a.geo + (blk * kGeoRows + 4 + grp) * kTileRun + lane);
     const bool valid = __ldg(a.elem + blk * kTileRun + (el & 31)) >= 0;
     const double dtt = a.tile_dt ? __ldg(a.tile_dt + tile) : 1.0;
     const double sa = a.sa_dt ? a.sa * dtt : a.sa;
@@ -196,7 +206,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
     {
       double e[NS], o[NOA];
       folded_adjoint<P>(Ad, valid, e, o);
-      const double2* ge = GE + which * 4 * kTileRun + (el & 31);
+      const double2* ge = GE + which * kGeoRows * kTileRun + (el & 31);
       const double2 lsa = ge[2 * kTileRun], lsb = ge[3 * kTileRun];
       const double l0 = sa * lsa.x, l1 = sa * lsa.y, l2 = sa * lsb.x;
 #pragma unroll
@@ -222,22 +232,18 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
         FBt[(NFQ + q) * 4 * E] = l1 * (x + y);
       }
     }
-    cp_async_wait_all();  // this thread's copies of neighbour rows and normals
+    cp_async_wait_all();  // this thread's copies of neighbour rows
     __syncthreads();
     if (*abort_flag) break;
 
     // ---- 3. faces: transposed Roe Jacobian; the trace adjoints overwrite bF ----------
-    const int nfaces = counts[0], points = counts[1];
-    const unsigned factor = counts[2];
-    for (int w = t;; w += T) {
-      const int part = face_part(w, factor);
-      int q = part * points;
-      if (q >= NFQ || nfaces == 0) break;
-      const int it = items[w - part * nfaces];
+    const FaceCounts faces = *counts;
+    int entry, q, q1;
+    for (int w = t; face_work<NFQ>(faces, w, &entry, &q, &q1); w += T) {
+      const int it = items[entry];
       const int fl = it & 63, s = (it >> 6) & 3, x = it >> 9;
       const bool mirror = (it >> 8) & 1;
-      const double2 n = NR[s * E + fl];
-      const int q1 = min(q + points, NFQ);
+      const double2 n = GE[((fl >> 5) * kGeoRows + 4 + s) * kTileRun + (fl & 31)];
       // a neighbour outside the tile: its column and its lift's scale
       long long nb = 0;
       double sc = 0.0;
@@ -310,10 +316,13 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
         }
       }
     }
+    if (t == 224) *NEXT = hand_out ? static_cast<int>(taken) + G : tile + G;
     __syncthreads();
+    const int next = *NEXT;
+    const bool has_next = next < a.ntiles;
 
     // the next tile's neighbours: their codes now, their rows after the transposed flux
-    code = has_next ? neighbour_code(a.lists, tile + G, which, lane) : kNoNeighbour;
+    code = has_next ? neighbour_code(a.lists, next, which, lane) : kNoNeighbour;
 
     // ---- 4a. trace adjoints onto the side nodes, component c --------------------------
     double g[NP];
@@ -348,7 +357,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
 
     // ---- 5. transposed nodal flux Jacobian of every node, in place over the xi rows ----
     if (P > 0) {
-      const double2* ge = GE + which * 4 * kTileRun + lane;
+      const double2* ge = GE + which * kGeoRows * kTileRun + lane;
       const double2 j0 = ge[0], j1 = ge[kTileRun];
       for (int j = grp; j < NP; j += 4) {
         const double2 s0 = S[sidx<NP>(2 * j, col)], s1 = S[sidx<NP>(2 * j + 1, col)];
@@ -367,7 +376,10 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
     // this half's columns of the state and adjoint tiles are free: start its
     // next copies and the next tile's neighbour rows
     if (has_next) {
-      if (grp == 0 && lane == 0) issue_adj_copies<P, NFQ>(a, tile + G, which, smem);
+      if (grp == 0 && lane == 0) {
+        issue_adj_mesh_copies<P, NFQ>(a, next, which, smem);
+        issue_adj_state_copies<P, NFQ>(a, next, which, smem);
+      }
       copy_neighbours<P>(H, a.U, code, which, grp, lane);
     }
     cp_async_commit();
@@ -399,9 +411,11 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
       }
     }
     // the four warps of a half hold different components of the same columns:
-    // none may start the next tile's normals or phase 2 (which reuse rows of
-    // the face / flux buffer) before the others are done with this tile's
+    // none may start the next tile's phase 2 (which reuses rows of the face /
+    // flux buffer) before the others are done with this tile's
     run_sync(t);
+    if (!has_next) break;
+    tile = next;
   }
 
   cp_async_wait_all();  // none may land after the block has left
@@ -410,6 +424,13 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
     // them once more, with the same bound, before the block leaves
     for (unsigned n = 0; n < kMaxWaitTries; ++n)
       if (mbar_try_wait(bar, parity ^ 1u)) break;
+  }
+  if (t == 0 && hand_out) {
+    __threadfence();
+    if (atomicAdd(&a.err[5], 1ull) == gridDim.x - 1) {
+      a.err[5] = 0ull;
+      a.err[6] = 0ull;
+    }
   }
 }
 

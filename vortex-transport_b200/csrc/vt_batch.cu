@@ -195,7 +195,7 @@ cudaError_t reset_errors(vt_batch* b) {
   cudaError_t e = cudaSuccess;
   for (auto& g : b->groups) {
     if (!e) e = cudaMemsetAsync(g.err, 0xFF, sizeof(unsigned long long), b->stream);
-    if (!e) e = cudaMemsetAsync(g.err + 1, 0, 3 * sizeof(unsigned long long), b->stream);
+    if (!e) e = cudaMemsetAsync(g.err + 1, 0, (vt::kErrWords - 1) * sizeof(unsigned long long), b->stream);
   }
   return e;
 }
@@ -400,7 +400,7 @@ vt_batch* vt_batch_create(const vt_mesh_desc* descs, int n, int device, int* sta
         (e = vt::dalloc(&G.elem, sizeof(int) * G.ncols)) ||
         (e = vt::dalloc(&G.lists, vt::kTileListBytes * static_cast<size_t>(G.ntiles))) ||
         (e = vt::dalloc(&G.tile_dt, sizeof(double) * G.ntiles)) ||
-        (e = vt::dalloc(&G.err, 4 * sizeof(unsigned long long)))) {
+        (e = vt::dalloc(&G.err, vt::kErrWords * sizeof(unsigned long long)))) {
       set(fail(e == cudaErrorMemoryAllocation ? VT_ERR_NO_MEMORY : VT_ERR_CUDA, vt::cuda_msg("vt_batch_create", e)));
       release(b);
       return nullptr;

@@ -188,8 +188,7 @@ struct Numbering {
 //     read from global memory (no slot left). Bits 0-5 the column in the tile,
 //     6-7 the side, 8 both in the tile, 9-15 the neighbour's column in the tile
 //     or its slot (kNoSlot: none);
-//   uint32 [4]  their number n, the face points per work item and a factor
-//     that divides by n (face_part);
+//   uint32 [4]  the work items (FaceCounts);
 //   uint32 [2][kSlots]  per block, the neighbours to stage: 4 * column + side,
 //     kNoNeighbour where a slot is empty (the used slots come first).
 struct StageArgs {
@@ -202,7 +201,7 @@ struct StageArgs {
   const int* elem;      // element of each column (-1: empty), or null: Numbering with nx = 0
   const unsigned char* lists;
   const double* tile_dt;  // per-tile time step (batched problems), or null: c_* hold dt
-  unsigned long long* err;  // [0] first-error key, [1] steps done, [2] blocks done
+  unsigned long long* err;  // kErrWords words, below
   int K;
   int ntiles;
   int stage;     // 0..3 RK4 stages, 4 forward Euler, 5 right-hand side only
@@ -220,13 +219,21 @@ struct StageArgs {
 
 enum : int { kTestNoCopies = 1 };
 
+// The words behind `err`, cleared before every call (word 0 to all ones):
+// [0] first-error key, [1] steps done, [2] blocks of the running stage kernel
+// that are done, [3] flags (1 bad neighbour, 2 a wait gave up), [4] tiles its
+// blocks have taken beyond their first, [5], [6] likewise of the reverse stage.
+constexpr int kErrWords = 8;
+
 constexpr int kMaxItems = 3 * kTileElems;
-// A block of a W x H tile has W + H faces that leave the tile, one of 64
-// consecutive elements in a row of the reference's mesh 33.
-constexpr int kSlots = 32;
+// A block of a W x H tile has W + H faces that leave the tile (12 of 8 x 4
+// cells). 26 slots are what three blocks per SM have room for at p = 3; of 64
+// consecutive elements in a row of the reference's mesh, each half has 33.
+constexpr int kSlots = 26;
+constexpr int kOuterWords = (2 * kSlots + 3) / 4 * 4;
 constexpr int kListCount = 2 * kMaxItems;      // byte offset of the counts
 constexpr int kListOuter = kListCount + 16;    // byte offset of the slots
-constexpr int kTileListBytes = kListOuter + 2 * kSlots * 4;
+constexpr int kTileListBytes = kListOuter + kOuterWords * 4;
 static_assert(kListCount % 16 == 0 && kTileListBytes % 16 == 0, "16-byte copies");
 constexpr unsigned kNoNeighbour = 0xffffffffu;
 constexpr int kNoSlot = 127;
@@ -235,11 +242,31 @@ __host__ __device__ constexpr unsigned face_item(int col, int side, bool inside,
   return static_cast<unsigned>(col | (side << 6) | (inside ? 1 << 8 : 0) | (x << 9));
 }
 
-// The work items of a face list are its n faces times the parts of their nfq
-// points, part-major: item w is part w / n of face w % n. The factor 2^20 / n +
-// 1 makes w / n one multiplication, exact while w n < 2^20 (w < 10 n, n <= 192).
+// The work items of a face list: first the n0 faces inside the tile times the
+// parts of their nfq points (p0 points each), then the n1 others (p1 points
+// each), part-major: item w < first is part w / n0 of face w % n0. The factor
+// 2^20 / n + 1 makes w / n one multiplication, exact while w n < 2^20 (w < 10 n,
+// n <= 192).
+struct FaceCounts {
+  unsigned n;        // n0 | n1 << 16
+  unsigned points;   // p0 | p1 << 8 | first << 16 (the items of the faces inside the tile)
+  unsigned factor0, factor1;
+};
 __host__ __device__ constexpr unsigned face_factor(int n) { return n > 0 ? (1u << 20) / n + 1 : 0; }
-__device__ __forceinline__ int face_part(int w, unsigned factor) { return static_cast<int>((w * factor) >> 20); }
+
+// Work item w: its entry in the list and its points [q0, q1); false past the last one.
+template <int NFQ>
+__device__ __forceinline__ bool face_work(const FaceCounts& f, int w, int* entry, int* q0, int* q1) {
+  const int first = f.points >> 16, n0 = f.n & 0xffff;
+  const bool in = w < first;
+  const int v = in ? w : w - first, n = in ? n0 : f.n >> 16, pts = in ? f.points & 0xff : (f.points >> 8) & 0xff;
+  if (n == 0) return false;
+  const int part = static_cast<int>((v * (in ? f.factor0 : f.factor1)) >> 20);
+  *q0 = part * pts;
+  *q1 = min(*q0 + pts, NFQ);
+  *entry = (in ? 0 : n0) + v - part * n;
+  return *q0 < NFQ;
+}
 
 enum : int { kStageEuler = 4, kStageRhs = 5 };
 

@@ -8,6 +8,24 @@
 
 namespace vt {
 
+// Launches a kernel that may be scheduled while the stream's previous kernel is
+// still running (let_next_start and wait_for_previous, vt_tile.cuh).
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t st,
+                             Args&&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(static_cast<unsigned>(block));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 using LaunchFn = cudaError_t (*)(const StageArgs&, const double*, int, cudaStream_t);
 using ConfigFn = cudaError_t (*)(int*);
 

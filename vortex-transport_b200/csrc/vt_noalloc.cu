@@ -63,7 +63,7 @@ Carve carve(int p, int K) {
   const size_t cols = (static_cast<size_t>(K) + 127) / 128 * 128, tiles = static_cast<size_t>(c.num.ntiles);
   const size_t state = sizeof(double2) * 2 * np_of(p) * cols;
   c.err = 0;
-  c.geo = align256(c.err + 4 * sizeof(unsigned long long));
+  c.geo = align256(c.err + kErrWords * sizeof(unsigned long long));
   c.nbr = align256(c.geo + sizeof(double2) * kGeoRows * cols);
   c.lists = align256(c.nbr + sizeof(int4) * cols);
   c.U = align256(align256(align256(c.lists + 16 * tiles) + 768 * tiles) + 4 * tiles);
@@ -183,7 +183,7 @@ int vt_step_rk4_noalloc(const vt_device_mesh* m, const double* dU_in, double* dU
 
   // error key to "none", step and block counters and the neighbour flag to zero
   if ((e = cudaMemsetAsync(errw, 0xFF, sizeof(unsigned long long), st)) ||
-      (e = cudaMemsetAsync(errw + 1, 0, 3 * sizeof(unsigned long long), st)))
+      (e = cudaMemsetAsync(errw + 1, 0, (vt::kErrWords - 1) * sizeof(unsigned long long), st)))
     return fail(VT_ERR_CUDA, std::string("scratch reset: ") + cudaGetErrorString(e));
   vt::pack_geometry_kernel<<<(K + 255) / 256, 256, 0, st>>>(*m, cv.num, geo, nbr, errw);
   if ((e = vt::launch_build_tile_lists(nbr, nullptr, K, cv.num.ntiles, m->n_line_points, lists, st)))

@@ -79,21 +79,25 @@ __device__ __forceinline__ int side_of(const int4& n, int s) { return s == 0 ? n
 // warp, which take consecutive faces, follow one path and read consecutive
 // columns of the shared buffers.
 //
-// A work item is `points` face points of one face. The block's 256 threads
-// take ceil(n ceil(nfq / points) / 256) items each, so the points each
-// evaluates one after another are that times `points`: the list's `points` is
-// the one that makes this least (the largest among equals, since a list entry
-// and a normal are read per item): at nfq = 6, 3 for the 108 faces of 8 x 4
-// cells, 2 for up to 85, 1 for up to 42 faces.
+// A work item is p0 points of a face inside the tile, or p1 of another one,
+// whose outer trace the item forms itself (about 1.4 times the work of a
+// point). The block's 256 threads take ceil(items / 256) items each, and a
+// barrier waits for the longest, so p0 and p1 are those that make
+// rounds x max(p0, 1.4 p1) least (the largest among equals, since a list entry
+// and a normal are read per item): at nfq = 6, 3 and 2 for the 84 + 24 faces of
+// 8 x 4 cells (240 items), 1 and 1 for the 18 + 12 of 4 x 2. Against the same
+// number for both (3 and the normals copied apart from the other geometry), 5
+// RK4 steps at 768 x 768, p = 3 went from 7.98 to 7.94 ms, 20 at 384 x 384,
+// p = 1 from 4.10 to 4.06 ms.
 __global__ void build_tile_lists_kernel(const int4* __restrict__ nbr, const int* __restrict__ elem, int K, int nfq,
                                         unsigned char* __restrict__ lists) {
   __shared__ int warp_n[3][8], warp_out[2][8];
   const int tile = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
   unsigned char* list = lists + static_cast<long long>(tile) * kTileListBytes;
   unsigned short* items = reinterpret_cast<unsigned short*>(list);
-  unsigned* counts = reinterpret_cast<unsigned*>(list + kListCount);
+  FaceCounts* counts = reinterpret_cast<FaceCounts*>(list + kListCount);
   unsigned* outer = reinterpret_cast<unsigned*>(list + kListOuter);
-  if (t < 2 * kSlots) outer[t] = kNoNeighbour;
+  if (t < kOuterWords) outer[t] = kNoNeighbour;
   auto element = [&](int x) {
     if (elem) return elem[x];
     Numbering c;
@@ -127,10 +131,11 @@ __global__ void build_tile_lists_kernel(const int4* __restrict__ nbr, const int*
     if (lane == 0) warp_n[k][warp] = __popc(m[k]);
   }
   __syncthreads();
-  int n = 0, rank = 0;  // position within the (class 0, class 1, class 2) order
+  int n = 0, rank = 0, n_cls[3] = {0, 0, 0};  // position within the (class 0, class 1, class 2) order
   for (int k = 0; k < 3; ++k)
     for (int w = 0; w < 8; ++w) {
       n += warp_n[k][w];
+      n_cls[k] += warp_n[k][w];
       if (k < cls || (k == cls && w < warp)) rank += warp_n[k][w];
     }
   rank += __popc(m[cls] & ((1u << lane) - 1u));
@@ -140,18 +145,24 @@ __global__ void build_tile_lists_kernel(const int4* __restrict__ nbr, const int*
     if (cls == 1) outer[second * kSlots + slot] = 4u * static_cast<unsigned>(nb) + static_cast<unsigned>(s);
   }
   if (t == 0) {
-    int points = 1, least = 0;
-    for (int k = 1; k <= nfq; ++k) {
-      const int rounds = (n * ((nfq + k - 1) / k) + 4 * kTileElems - 1) / (4 * kTileElems);
-      if (k == 1 || rounds * k <= least) {
-        least = rounds * k;
-        points = k;
+    const int n0 = n_cls[0], n1 = n - n0;
+    int p0 = 1, p1 = 1, least = 0;  // in tenths of a point
+    for (int i = 1; i <= nfq; ++i)
+      for (int j = 1; j <= nfq; ++j) {
+        const int items = n0 * ((nfq + i - 1) / i) + n1 * ((nfq + j - 1) / j);
+        const int rounds = (items + 4 * kTileElems - 1) / (4 * kTileElems);
+        const int cost = rounds * max(n0 ? 10 * i : 0, n1 ? 14 * j : 0);
+        if ((i == 1 && j == 1) || cost <= least) {
+          least = cost;
+          p0 = i, p1 = j;
+        }
       }
-    }
-    counts[0] = n;
-    counts[1] = points;
-    counts[2] = face_factor(n);
-    counts[3] = 0;
+    FaceCounts f;
+    f.n = n0 | n1 << 16;
+    f.points = p0 | p1 << 8 | (n0 * ((nfq + p0 - 1) / p0)) << 16;
+    f.factor0 = face_factor(n0);
+    f.factor1 = face_factor(n1);
+    *counts = f;
   }
 }
 

@@ -336,7 +336,7 @@ cudaError_t enqueue_rk4_step(vt_ctx* c, double dt) {
 cudaError_t reset_error_words(vt_ctx* c) {
   cudaError_t e = cudaMemsetAsync(c->err, 0xFF, sizeof(unsigned long long), c->stream);
   if (e) return e;
-  return cudaMemsetAsync(c->err + 1, 0, 3 * sizeof(unsigned long long), c->stream);
+  return cudaMemsetAsync(c->err + 1, 0, (kErrWords - 1) * sizeof(unsigned long long), c->stream);
 }
 
 // Waits for the stream, decodes the first-error key and advances the clock.
@@ -471,7 +471,7 @@ vt_ctx* vt_create(const vt_mesh_desc* d, int device, int* status) {
   if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) || (e = alloc(&c->U, state_bytes)) ||
       (e = alloc(&c->A, state_bytes)) || (e = alloc(&c->Sa, state_bytes)) || (e = alloc(&c->Sb, state_bytes)) ||
       (e = alloc(&c->geo, geo.size() * sizeof(double2))) || (e = alloc(&c->nbr, nbr.size() * sizeof(int4))) ||
-      (e = alloc(&c->err, 4 * sizeof(unsigned long long))) || (e = alloc(&c->W, sizeof(double) * c->Np)) ||
+      (e = alloc(&c->err, vt::kErrWords * sizeof(unsigned long long))) || (e = alloc(&c->W, sizeof(double) * c->Np)) ||
       (e = alloc(&c->partial, sizeof(double) * 4 * tot_blocks)) || (e = alloc(&c->tot, sizeof(double) * 4)) ||
       (e = alloc(&c->elem, sizeof(int) * ncols)) ||
       (e = alloc(&c->lists, vt::kTileListBytes * static_cast<size_t>(c->ntiles)))) {
@@ -586,7 +586,7 @@ vt_ctx* vt_create_structured(const vt_params* prm, const vt_vortex* ic_in, int d
       (e = alloc(&c->geo, sizeof(double2) * vt::kGeoRows * ncols)) || (e = alloc(&c->nbr, sizeof(int4) * ncols)) ||
       (e = alloc(&c->elem, sizeof(int) * ncols)) ||
       (e = alloc(&c->lists, vt::kTileListBytes * static_cast<size_t>(c->ntiles))) ||
-      (e = alloc(&c->err, 4 * sizeof(unsigned long long))) || (e = alloc(&c->W, sizeof(double) * Np)) ||
+      (e = alloc(&c->err, vt::kErrWords * sizeof(unsigned long long))) || (e = alloc(&c->W, sizeof(double) * Np)) ||
       (e = alloc(&c->partial, sizeof(double) * 4 * tot_blocks)) || (e = alloc(&c->tot, sizeof(double) * 4)) ||
       (e = alloc(&verts, sizeof(double) * 6 * static_cast<size_t>(c->K)))) {
     set(fail(e == cudaErrorMemoryAllocation ? VT_ERR_NO_MEMORY : VT_ERR_CUDA, vt::cuda_msg("vt_create_structured", e)));

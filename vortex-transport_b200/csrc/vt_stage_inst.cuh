@@ -31,8 +31,7 @@ cudaError_t launch_stage(const StageArgs& a, const double* ops, int max_blocks, 
   if constexpr (MAP == kMapFolded) fold_operators(*reinterpret_cast<const StageOps<P, NFQ>*>(ops), &o);
   else std::memcpy(&o, ops, sizeof(o));
   const int grid = a.ntiles < max_blocks ? a.ntiles : max_blocks;
-  tile_stage_kernel<P, NFQ, MAP><<<grid, 4 * kTileElems, Lay::kBytes, st>>>(a, o);
-  return cudaGetLastError();
+  return launch_dependent(tile_stage_kernel<P, NFQ, MAP>, grid, 4 * kTileElems, Lay::kBytes, st, a, o);
 }
 
 template <int P, int NFQ, int MAP>

@@ -11,7 +11,7 @@
 //             an mbarrier), issued when that half finished the previous tile's
 //             flux phase; the side nodes of the neighbours outside the tile
 //             (one slot per face that leaves it) come by cp.async at the same
-//             time, and the normals when the previous tile ends;
+//             time;
 //   2. traces a thread evaluates its element's own trace of its component at
 //             every face point from the p+1 side nodes (coefficients are
 //             immediates);
@@ -36,9 +36,9 @@
 // its own next copies (the tile's mbarrier expects one arrival per half). The
 // load phase has no block barrier either: the traces read only columns of the
 // thread's own half of the state tile, which its own wait on the mbarrier
-// covers, and the face list, neighbour rows, normals and element numbers are
-// first read in phase 3, after the barrier that follows the traces. A tile ends
-// with a per-half barrier: the four warps of a half share its columns, and the
+// covers, and the other half's geometry and element numbers and the neighbour
+// rows are first read in phase 3, after the barrier that follows the traces. A
+// tile ends with a per-half barrier: the four warps of a half share its columns, and the
 // next tile's traces reuse rows of the buffer that this tile's volume phase
 // reads. So the two halves of a block run apart from phase 4 of one tile to the
 // end of the next tile's trace phase.
@@ -75,17 +75,16 @@ struct TileLayout {
   static constexpr int E = kTileElems;
   static constexpr int NP = np_of_p(P);
   static constexpr int NE = P + 1;
-  static constexpr int kNormalRow = 6 * NFQ;  // 3 rows of normals behind the face buffer's
-  static constexpr int kFBRows = kNormalRow + 3 > NP * 4 ? kNormalRow + 3 : NP * 4;
+  static constexpr int kFBRows = 6 * NFQ > NP * 4 ? 6 * NFQ : NP * 4;
   // byte offsets into dynamic shared memory, each 16-byte aligned
   static constexpr int kS = 0;                               // double2 [2][2NP][32]
   static constexpr int kH = kS + 2 * NP * E * 16;            // double2 [2NE][2 kSlots] neighbours' side nodes
-  static constexpr int kFB = kH + 2 * NE * 2 * kSlots * 16;  // double2 [3][NFQ][2][E] + [3][E] | [NP][4][E]
-  static constexpr int kGE = kFB + kFBRows * E * 16;         // double2 [2][4][32] geometry rows 0..3
-  static constexpr int kTM = kGE + 4 * E * 16;               // double [3][NFQ][NE]
+  static constexpr int kFB = kH + 2 * NE * 2 * kSlots * 16;  // double2 [3][NFQ][2][E] | [NP][4][E]
+  static constexpr int kGE = kFB + kFBRows * E * 16;         // double2 [2][kGeoRows][32] geometry
+  static constexpr int kTM = kGE + kGeoRows * E * 16;        // double [3][NFQ][NE]
   static constexpr int kEL = kTM + 3 * NFQ * NE * 8 + 8 * (3 * NFQ * NE % 2);  // int [E] element of each column
   static constexpr int kItems = kEL + E * 4;                 // uint16 [kMaxItems], uint32 [4] (face list)
-  static constexpr int kBar = kItems + kListOuter;           // mbarrier (8 B), abort flag
+  static constexpr int kBar = kItems + kListOuter;           // mbarrier (8 B), abort flag, next tile
   static constexpr int kBytes = kBar + 16;
 };
 
@@ -116,14 +115,10 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned 
 }
 
 // Global-to-shared copies that bypass the registers (cp.async, completed per
-// thread by cp.async.wait_all): 16 bytes (both addresses 16-byte aligned,
-// cached in L2 only) or 4 bytes.
+// thread by cp.async.wait_all): 16 bytes (both addresses 16-byte aligned),
+// cached in L2 only.
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(__cvta_generic_to_global(src))
-               : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(__cvta_generic_to_global(src))
                : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
@@ -145,6 +140,34 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* src, unsigned bytes
                : "memory");
 }
 
+// Programmatic dependent launch (launch_dependent, vt_launch.h): the next
+// kernel of the stream may be scheduled from now on, where this grid leaves
+// room, and does its set-up there until wait_for_previous, which returns when
+// the kernel before it has ended and its writes are visible. Every kernel
+// launched that way waits before it reads or writes anything that another
+// kernel writes or reads; only the mesh's own arrays, which no kernel of the
+// stream writes, are read before. With it 250 RK4 steps at 8 x 8 cells, p = 3
+// (two tiles) take 6.2 ms instead of 7.1, 20 at 150 x 90, p = 3 0.88 instead of
+// 0.95 ms, 50 at 64 x 64, p = 2 1.26 instead of 1.28 ms.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Which tile a block takes next. A block's first tile is blockIdx.x, the others
+// are handed out in order by an atomic counter, so that the blocks of SMs that
+// run ahead (their distance to the L2 slices differs) take more of them: with
+// tiles blockIdx.x + k gridDim.x the blocks ended up to 30 us apart at 768 x
+// 768, p = 3. The counter is read while the previous tile's faces are
+// evaluated; the last block to finish clears it. No result depends on the
+// assignment. A pass of 5 RK4 steps at 768 x 768, p = 3 (41 tiles a block)
+// takes 7.28 ms handed out, 7.54 ms otherwise; with few tiles a block there is
+// little to even out and the counter costs more: 384 x 384, p = 1 (10 tiles a
+// block) 4.22 against 4.18 ms, a gradient at 128 x 128, p = 3 (1 or 2 tiles)
+// 16.1 against 14.1 ms. So it is used from kHandOut tiles a block on.
+constexpr int kHandOut = 16;
+__device__ __forceinline__ unsigned take_tile(unsigned long long* taken) {
+  return atomicAdd(reinterpret_cast<unsigned*>(taken), 1u);
+}
+
 constexpr unsigned kMaxWaitTries = 1u << 22;
 
 // Shared-memory index of (row, column) of the state tile: the two blocks as they lie in HBM.
@@ -153,21 +176,30 @@ __device__ __forceinline__ int sidx(int row, int col) {
   return ((col >> 5) * 2 * NP + row) * kTileRun + (col & (kTileRun - 1));
 }
 
-// One thread per half announces and issues the bulk copies of block `which` of
-// a tile: its state, its geometry rows 0..3 and, for block 0, the face list.
+// One thread per half announces the bulk copies of block `which` of a tile and
+// issues those of the mesh's arrays (geometry, element numbers and, for block
+// 0, the face list), then the state's.
 template <int P, int NFQ>
-__device__ __forceinline__ void issue_tile_copies(const double2* in, const double2* geo, const unsigned char* lists,
-                                                  int tile, int which, unsigned char* smem, int test_flags) {
+__device__ __forceinline__ void issue_mesh_copies(const StageArgs& a, int tile, int which, unsigned char* smem) {
   using L = TileLayout<P, NFQ>;
-  constexpr unsigned kState = 2 * L::NP * kTileRun * 16, kGeo = 4 * kTileRun * 16;
+  constexpr unsigned kState = 2 * L::NP * kTileRun * 16, kGeo = kGeoRows * kTileRun * 16, kElem = kTileRun * 4;
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem + L::kBar);
-  if (test_flags & kTestNoCopies) return;  // test hook: nothing arrives, every wait gives up
+  if (a.test_flags & kTestNoCopies) return;  // test hook: nothing arrives, every wait gives up
   fence_proxy_async_smem();
-  mbar_arrive_expect_tx(bar, kState + kGeo + (which == 0 ? kListOuter : 0u));
+  mbar_arrive_expect_tx(bar, kState + kGeo + (a.elem ? kElem : 0u) + (which == 0 ? kListOuter : 0u));
   const long long blk = 2ll * tile + which;
-  bulk_g2s(smem + L::kS + which * kState, in + blk * (2 * L::NP * kTileRun), kState, bar);
-  bulk_g2s(smem + L::kGE + which * kGeo, geo + blk * (kGeoRows * kTileRun), kGeo, bar);
-  if (which == 0) bulk_g2s(smem + L::kItems, lists + static_cast<long long>(tile) * kTileListBytes, kListOuter, bar);
+  bulk_g2s(smem + L::kGE + which * kGeo, a.geo + blk * (kGeoRows * kTileRun), kGeo, bar);
+  if (a.elem) bulk_g2s(smem + L::kEL + which * kElem, a.elem + blk * kTileRun, kElem, bar);
+  if (which == 0) bulk_g2s(smem + L::kItems, a.lists + static_cast<long long>(tile) * kTileListBytes, kListOuter, bar);
+}
+template <int P, int NFQ>
+__device__ __forceinline__ void issue_state_copy(const double2* in, int tile, int which, unsigned char* smem,
+                                                 int test_flags) {
+  using L = TileLayout<P, NFQ>;
+  constexpr unsigned kState = 2 * L::NP * kTileRun * 16;
+  if (test_flags & kTestNoCopies) return;
+  bulk_g2s(smem + L::kS + which * kState, in + (2ll * tile + which) * (2 * L::NP * kTileRun), kState,
+           reinterpret_cast<unsigned long long*>(smem + L::kBar));
 }
 
 // Barrier of the four warps that hold one half's columns (warps of equal parity).
@@ -416,7 +448,7 @@ __device__ __forceinline__ const double2* first_operand(const StageArgs& a) {
 template <int P>
 __device__ __forceinline__ void copy_neighbours(double2* H, const double2* in, unsigned code, int which, int g, int lane) {
   static_assert(P + 1 <= 4, "a warp per side node");
-  if (g > P || code == kNoNeighbour) return;
+  if (g > P || code == kNoNeighbour) return;  // lanes past the slots hold no code
   const int base = g * (P + 1) - g * (g - 1) / 2;  // node_id(P, 0, g)
   const unsigned s = code & 3;
   const int node = s == 0 ? g : (s == 1 ? base + P - g : base);  // edge_node(P, s, g)
@@ -428,6 +460,7 @@ __device__ __forceinline__ void copy_neighbours(double2* H, const double2* in, u
 
 // The code of slot `lane` of half `which` of a tile.
 __device__ __forceinline__ unsigned neighbour_code(const unsigned char* lists, int tile, int which, int lane) {
+  if (lane >= kSlots) return kNoNeighbour;
   return __ldg(reinterpret_cast<const unsigned*>(lists + static_cast<long long>(tile) * kTileListBytes + kListOuter) +
                which * kSlots + lane);
 }
@@ -460,13 +493,13 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
   double* FB = reinterpret_cast<double*>(smem + L::kFB);
   double2* FB2 = reinterpret_cast<double2*>(smem + L::kFB);
   double2* GE = reinterpret_cast<double2*>(smem + L::kGE);
-  double2* NR = FB2 + L::kNormalRow * E;  // normals, until the nodal flux
   double* TM = reinterpret_cast<double*>(smem + L::kTM);
   int* EL = reinterpret_cast<int*>(smem + L::kEL);
   const unsigned short* items = reinterpret_cast<const unsigned short*>(smem + L::kItems);
-  const unsigned* counts = reinterpret_cast<const unsigned*>(smem + L::kItems + kListCount);
+  const FaceCounts* counts = reinterpret_cast<const FaceCounts*>(smem + L::kItems + kListCount);
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem + L::kBar);
   int* abort_flag = reinterpret_cast<int*>(smem + L::kBar + 8);
+  int* NEXT = reinterpret_cast<int*>(smem + L::kBar + 12);
 
   const int t = threadIdx.x;
   const int lane = t & 31;
@@ -475,6 +508,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
   const int col = t % E;                          // load and nodal flux phases
   const int el = work_column(t), c = work_component(t);
   const int G = gridDim.x;
+  const bool hand_out = a.ntiles > kHandOut * G;
   const unsigned max_tries = a.wait_tries ? a.wait_tries : kMaxWaitTries;
 
   {
@@ -485,27 +519,27 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
     mbar_init(bar, 2);
     *abort_flag = 0;
   }
-  int tile = blockIdx.x;
-  if (tile >= a.ntiles) return;
+  let_next_start();
+  int tile = blockIdx.x;  // the grid has at most ntiles blocks
   unsigned code = neighbour_code(a.lists, tile, which, lane);
   __syncthreads();
-  if (grp == 0 && lane == 0) issue_tile_copies<P, NFQ>(a.in, a.geo, a.lists, tile, which, smem, a.test_flags);
+  if (grp == 0 && lane == 0) issue_mesh_copies<P, NFQ>(a, tile, which, smem);
+  wait_for_previous();
+  if (grp == 0 && lane == 0) issue_state_copy<P, NFQ>(a.in, tile, which, smem, a.test_flags);
   copy_neighbours<P>(H, a.in, code, which, grp, lane);
   cp_async_commit();
   unsigned parity = 0;
 
-  for (; tile < a.ntiles; tile += G) {
-    const bool has_next = tile + G < a.ntiles;
+  while (true) {
     const long long blk = 2ll * tile + which;  // this half's block
+    unsigned taken = 0;
+    if (t == 224 && hand_out) taken = take_tile(a.err + 4);
 
     // ---- 1. load ------------------------------------------------------------------
-    // the normals go into rows that the previous tile's flux has left; this
-    // half's RK operand block (read in phase 6) into L2. The next tile's state
-    // is not prefetched: its bulk copies, issued in phase 5, read it from HBM
-    // themselves (prefetching it as well was 1.6% slower)
-    if (grp < 3) cp_async16(NR + grp * E + col, a.geo + (blk * kGeoRows + 4 + grp) * kTileRun + lane);
-    else if (a.elem) cp_async4(EL + col, a.elem + blk * kTileRun + lane);
-    else {
+    // this half's RK operand block (read in phase 6) into L2. The next tile's
+    // state is not prefetched: its bulk copies, issued in phase 5, read it from
+    // HBM themselves (prefetching it as well was 1.6% slower)
+    if (!a.elem && grp == 3) {
       Numbering n;
       n.K = a.K;
       EL[col] = n.element(tile * E + col);
@@ -524,22 +558,18 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
 
     // ---- 2. own traces at every face point -------------------------------------------
     own_traces<P, NFQ>(ops, S, FB, el, c);
-    cp_async_wait_all();  // this thread's copies of neighbour rows, normals and element numbers
+    cp_async_wait_all();  // this thread's copies of neighbour rows
     __syncthreads();
     if (*abort_flag) break;
 
     // ---- 3. faces: the (doubled) flux overwrites the traces it consumed ------------------
-    const int nfaces = counts[0], points = counts[1];
-    const unsigned factor = counts[2];
-    for (int w = t;; w += T) {
-      const int part = face_part(w, factor);
-      int q = part * points;
-      if (q >= NFQ || nfaces == 0) break;
-      const int it = items[w - part * nfaces];
+    const FaceCounts faces = *counts;
+    int entry, q, q1;
+    for (int w = t; face_work<NFQ>(faces, w, &entry, &q, &q1); w += T) {
+      const int it = items[entry];
       const int fl = it & 63, s = (it >> 6) & 3, x = it >> 9;
       const bool mirror = (it >> 8) & 1;
-      const double2 n = NR[s * E + fl];
-      const int q1 = min(q + points, NFQ);
+      const double2 n = GE[((fl >> 5) * kGeoRows + 4 + s) * kTileRun + (fl & 31)];
       double2* own = FB2 + (s * NFQ + q) * 2 * E + fl;
       double2* oth = FB2 + (s * NFQ + NFQ - 1 - q) * 2 * E + (mirror ? x : 0);
 #pragma unroll 1
@@ -582,17 +612,20 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
         }
       }
     }
+    if (t == 224) *NEXT = hand_out ? static_cast<int>(taken) + G : tile + G;
     __syncthreads();
+    const int next = *NEXT;
+    const bool has_next = next < a.ntiles;
 
     // the next tile's neighbours: their codes now, their rows after the nodal flux
-    code = has_next ? neighbour_code(a.lists, tile + G, which, lane) : kNoNeighbour;
+    code = has_next ? neighbour_code(a.lists, next, which, lane) : kNoNeighbour;
 
     // ---- 4. lift ---------------------------------------------------------------------------
     const bool valid = EL[el] >= 0;
     double* FBt = FB + ((c >> 1) * E + el) * 2 + (c & 1);  // this thread's component and column
     double r[NP];  // per node, or FOLD: the even parts, then the odd parts, of the node pairs
     {
-      const double2* ge = GE + which * 4 * kTileRun + (el & 31);
+      const double2* ge = GE + which * kGeoRows * kTileRun + (el & 31);
       lift_term<P, NFQ>(ops, FBt, ge[2 * kTileRun], ge[3 * kTileRun], r);
     }
     // stage 3: U3 / (3 c_out) into the accumulators while the state tile still
@@ -612,7 +645,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
 
     // ---- 5. nodal flux of every node, once, contracted with the inverse Jacobian --------
     if (P > 0) {
-      const double2* ge = GE + which * 4 * kTileRun + lane;
+      const double2* ge = GE + which * kGeoRows * kTileRun + lane;
       const double2 j0 = ge[0], j1 = ge[kTileRun];
       if constexpr (FOLD) {
         folded_nodal_flux<P>(S, FB2, col, grp, j0, j1);
@@ -634,7 +667,10 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
 
     // this half's state and geometry are free: start its next copies and neighbour rows
     if (has_next) {
-      if (grp == 0 && lane == 0) issue_tile_copies<P, NFQ>(a.in, a.geo, a.lists, tile + G, which, smem, a.test_flags);
+      if (grp == 0 && lane == 0) {
+        issue_mesh_copies<P, NFQ>(a, next, which, smem);
+        issue_state_copy<P, NFQ>(a.in, next, which, smem, a.test_flags);
+      }
       copy_neighbours<P>(H, a.in, code, which, grp, lane);
     }
     cp_async_commit();
@@ -688,9 +724,11 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
       }
     }
     // the four warps of a half work on the same columns: none may start the
-    // next tile's normals or traces (which reuse rows of the face / flux
-    // buffer) before the others are done with this tile's volume phase
+    // next tile's traces (which reuse rows of the face / flux buffer) before
+    // the others are done with this tile's volume phase
     run_sync(t);
+    if (!has_next) break;
+    tile = next;
   }
 
   cp_async_wait_all();  // none may land after the block has left
@@ -700,14 +738,14 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
     for (unsigned n = 0; n < max_tries; ++n)
       if (mbar_try_wait(bar, parity ^ 1u)) break;
   }
-  if (a.stage == 3 || a.stage == kStageEuler) {
-    if (t == 0) {
-      __threadfence();
-      const unsigned long long done = atomicAdd(&a.err[2], 1ull);
-      if (done == gridDim.x - 1) {
-        a.err[2] = 0ull;
-        atomicAdd(&a.err[1], 1ull);
-      }
+  const bool step_ends = a.stage == 3 || a.stage == kStageEuler;
+  if (t == 0 && (step_ends || hand_out)) {
+    __threadfence();
+    const unsigned long long done = atomicAdd(&a.err[2], 1ull);
+    if (done == gridDim.x - 1) {
+      a.err[2] = 0ull;
+      a.err[4] = 0ull;
+      if (step_ends) atomicAdd(&a.err[1], 1ull);
     }
   }
 }
