@@ -229,10 +229,11 @@ int vt_read_state_file(const char* path, double* U);
 /* The context's cudaStream_t, for callers that interleave their own work. */
 void* vt_stream(vt_ctx* ctx);
 
-/* Warp mapping of the context's stage kernel: 0 one thread per element and
- * conserved component, 1 (the default) one thread per element, component pair
- * and half of the nodes. Both compute the same arithmetic (results agree to
- * rounding); the choice only changes the speed. No reference counterpart. */
+/* Form of the context's stage kernel: 0 applies the operators as they are, 1
+ * (the default) their even and odd parts under the reference triangle's
+ * reflection, where they have that symmetry (else the same as 0). Both compute
+ * the same sums (results agree to rounding); the choice only changes the speed.
+ * No reference counterpart. */
 int vt_set_stage_mapping(vt_ctx* ctx, int mapping);
 int vt_get_stage_mapping(const vt_ctx* ctx);
 
@@ -248,7 +249,7 @@ int vt_get_stage_mapping(const vt_ctx* ctx);
 int vt_test_bulk_wait(vt_ctx* ctx, unsigned tries, int issue_no_copies);
 
 /* Device time of each kernel kind of one RK4 step, measured with CUDA events
- * around individual launches (no graph): ms[0..3] = stages 0..3, averaged over
+ * around individual launches: ms[0..3] = stages 0..3, averaged over
  * `reps` steps of size dt. Advances the state by `reps` steps. */
 int vt_profile_rk4_stages(vt_ctx* ctx, double dt, int reps, float* ms);
 
@@ -258,7 +259,7 @@ int vt_profile_rk4_stages(vt_ctx* ctx, double dt, int reps, float* ms);
  * `n` calls of rk4 (Timestepping.cpp:85-306) sharing each kernel launch.
  * Instances with the same p and reference tables form a group stored as one
  * ragged element array; one stage launch per group advances all its
- * instances, and one CUDA graph holds a whole RK4 step. Each instance keeps
+ * instances, and the groups' launches run side by side. Each instance keeps
  * its own time step, and its elements see exactly the arithmetic of a
  * vt_ctx built from the same descriptor. */
 typedef struct vt_batch vt_batch;
@@ -280,9 +281,8 @@ int vt_batch_set_dt(vt_batch* batch, const double* dt);
  * returns its code; vt_batch_last_error names the instance. */
 int vt_batch_step_rk4(vt_batch* batch, int nsteps);
 int vt_batch_last_error(const vt_batch* batch, int* instance, vt_error_info* out);
-/* Times each group's RK4 step for both warp mappings of the stage kernel
- * (0: one thread per element and component; 1: one thread per element,
- * component pair and half of the nodes) and 1..max resident blocks per SM
+/* Times each group's RK4 step for both forms of the stage kernel
+ * (vt_set_stage_mapping) and 1..max resident blocks per SM
  * (`trials` repetitions each), keeps the fastest and reports it per group in
  * blocks_per_sm[groups] and mapping[groups] (either may be NULL); the state is
  * left unchanged. No reference counterpart (the reference has one CPU loop). */

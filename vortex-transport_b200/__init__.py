@@ -652,7 +652,7 @@ class Solver:
 
     @property
     def stage_mapping(self) -> int:
-        """Warp mapping of the stage kernel: 0 component per thread, 1 pair per thread."""
+        """Form of the stage kernel: 0 the operators as they are, 1 (default) folded where they reflect."""
         return int(lib().vt_get_stage_mapping(self._h))
 
     @stage_mapping.setter

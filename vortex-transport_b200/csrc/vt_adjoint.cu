@@ -46,6 +46,7 @@ struct AdjKernels {
   JvpFn jvp = nullptr;
   TileFn tile = nullptr;
   TileConfigFn tile_config = nullptr;
+  std::vector<double> (*tile_pack)(const double*) = nullptr;
 };
 
 template <int P, int NFQ>
@@ -68,14 +69,21 @@ cudaError_t launch_element(const AdjArgs& a, const double* ops, cudaStream_t st)
 
 // One reverse stage as one persistent launch over the stage kernel's tiles.
 template <int P, int NFQ>
-cudaError_t launch_tile(const AdjArgs& a, const double* ops, int max_blocks, cudaStream_t st) {
-  StageOps<P, NFQ> o;
-  std::memcpy(&o, ops, sizeof(o));
+cudaError_t launch_tile(const AdjArgs& a, const double* block, int max_blocks, cudaStream_t st) {
   const int grid = a.ntiles < max_blocks ? a.ntiles : max_blocks;
-  FoldedOps<P, NFQ> fo;
-  fold_operators(o, &fo);
-  return launch_dependent(adjoint_tile_kernel<P, NFQ>, grid, 4 * kTileElems, AdjTileLayout<P, NFQ>::kBytes, st, a, o,
-                          fo);
+  return launch_dependent(adjoint_tile_kernel<P, NFQ>, grid, 4 * kTileElems, AdjTileLayout<P, NFQ>::kBytes, st, a,
+                          *reinterpret_cast<const AdjOps<P, NFQ>*>(block));
+}
+
+template <int P, int NFQ>
+std::vector<double> pack_tile(const double* ops) {
+  static_assert(sizeof(AdjOps<P, NFQ>) % sizeof(double) == 0, "a block of doubles");
+  const auto& o = *reinterpret_cast<const StageOps<P, NFQ>*>(ops);
+  AdjOps<P, NFQ> block;
+  fold_operators(o, &block.fo);
+  std::memcpy(block.lift, o.lift, sizeof(o.lift));
+  const double* b = reinterpret_cast<const double*>(&block);
+  return std::vector<double>(b, b + sizeof(block) / sizeof(double));
 }
 
 template <int P, int NFQ>
@@ -99,7 +107,7 @@ cudaError_t launch_jvp(const double2* U, const double2* V, double2* dR, const do
 template <int P, int NFQ>
 AdjKernels kernels_of() {
   return AdjKernels{launch_face<P, NFQ>, launch_element<P, NFQ>, launch_jvp<P, NFQ>, launch_tile<P, NFQ>,
-                    configure_tile<P, NFQ>};
+                    configure_tile<P, NFQ>, pack_tile<P, NFQ>};
 }
 
 template <int P>
@@ -131,18 +139,6 @@ AdjKernels select_adjoint(int p, int nfq) {
 
 }  // namespace
 
-// A sweep's launches depend only on its buffers, step count and time step, so
-// a repeated sweep replays a captured CUDA graph instead of relaunching.
-struct SweepGraph {
-  cudaGraphExec_t exec = nullptr;
-  std::vector<long long> key;
-  void reset() {
-    if (exec) cudaGraphExecDestroy(exec);
-    exec = nullptr;
-    key.clear();
-  }
-};
-
 // The overlapped reverse sweep (run_plan_overlapped) renames the checkpoint
 // slots onto the plan's slots, the work slot and kSpareSlots spare state
 // buffers, and orders its two streams through a ring of kRevRing events, one
@@ -152,7 +148,7 @@ constexpr int kRevRing = 8;
 
 struct AdjointState {
   AdjKernels k;
-  SweepGraph fwd_graph, bwd_graph;
+  std::vector<double> tile_ops;  // adjoint_tile_kernel's form of the operators
   size_t state_elems = 0;  // double2 entries of one state vector
   // work, stage states, adjoint, accumulator, two stage adjoints, second set
   // of stage states (contiguous)
@@ -268,6 +264,7 @@ int setup(vt_ctx* c) {
   }
   s->k = k;
   s->tile_blocks = tile_blocks;
+  if (tile_blocks > 0) s->tile_ops = k.tile_pack(c->ops.data());
   s->state_elems = state_elems;
   s->bufs = bufs;
   double2** named[kVectors] = {&s->work, &s->s1, &s->s2, &s->s3, &s->lam, &s->acc,
@@ -305,7 +302,7 @@ cudaError_t stage(vt_ctx* c, const double2* in, const double2* base, double2* ou
                   cudaStream_t stream, bool no_acc = false) {
   StageArgs a = stage_args(c, in, base, c->A, out, st, ca, co);
   a.no_acc = no_acc ? 1 : 0;
-  return c->launch(a, c->ops.data(), c->max_blocks, stream);
+  return c->launch(a, c->block.data(), c->max_blocks, stream);
 }
 
 // The step size the coefficients carry: dt, or 1 when the device scales them
@@ -367,7 +364,7 @@ AdjArgs adj_args(vt_ctx* c) {
 // on any mesh whose sides pair up).
 cudaError_t reverse_stage(vt_ctx* c, const AdjArgs& a) {
   AdjointState* s = c->adj;
-  if (s->tile_blocks > 0) return s->k.tile(a, c->ops.data(), s->tile_blocks, c->stream);
+  if (s->tile_blocks > 0) return s->k.tile(a, s->tile_ops.data(), s->tile_blocks, c->stream);
   const cudaError_t e = s->k.face(a, c->ops.data(), c->stream);
   return e ? e : s->k.element(a, c->ops.data(), c->stream);
 }
@@ -437,16 +434,16 @@ cudaError_t run_plan(vt_ctx* c, size_t begin, size_t end, double2* out_last) {
 // for; a ring entry recorded again by a later reverse step only makes a wait
 // stronger, since M runs in order.
 // Reads of the renamed slots (advances, stage steps, reverse steps) follow the
-// mapping at their place in the plan, which every replay of the captured graph
-// repeats from the same identity mapping (the forward part writes the
-// checkpoints to the plan's own slots). Must be called inside a stream capture
-// of the context's stream; set 0 (s1..s3) holds the stage states of the plan's
-// first reverse step on entry.
+// mapping at their place in the plan, which starts as the identity (the forward
+// part writes the checkpoints to the plan's own slots). Set 0 (s1..s3) holds
+// the stage states of the plan's first reverse step on entry. Nothing here can
+// wait for a launch that is yet to be made: every event a stream waits for was
+// recorded before, so a full launch queue only delays the host.
 cudaError_t run_plan_overlapped(vt_ctx* c, size_t begin, size_t end) {
   AdjointState* s = c->adj;
   cudaStream_t M = c->stream, R = s->side;
   double2* const sets[2][3] = {{s->s1, s->s2, s->s3}, {s->t1, s->t2, s->t3}};
-  bool ready_rec[2] = {false, false};  // ev_ready[k] recorded in this capture
+  bool ready_rec[2] = {false, false};  // ev_ready[k] recorded in this sweep
   // physical buffers: the plan's slots 0..nlog-1, the work slot (nlog), the spares
   const int nlog = s->plan_slots;
   std::vector<double2*> buf;
@@ -474,7 +471,7 @@ cudaError_t run_plan_overlapped(vt_ctx* c, size_t begin, size_t end) {
         break;
     }
   }
-  // the side stream rejoins the capture's origin stream
+  // the side stream rejoins the context's
   const cudaError_t j = cudaEventRecord(s->ev_join, R);
   const cudaError_t k = j ? j : cudaStreamWaitEvent(M, s->ev_join, 0);
   return e ? e : k;
@@ -504,36 +501,6 @@ cudaError_t lincomb(vt_ctx* c, double2* out, const double2* x, double cx, const 
   return cudaGetLastError();
 }
 
-template <typename F>
-cudaError_t run_captured(vt_ctx* c, SweepGraph& g, const std::vector<long long>& key, F&& enqueue) {
-  if (!g.exec || g.key != key) {
-    g.reset();
-    cudaGraph_t graph = nullptr;
-    cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
-    if (e) return e;
-    const cudaError_t le = enqueue();
-    e = cudaStreamEndCapture(c->stream, &graph);
-    if (le) e = le;
-    if (!e) e = cudaGraphInstantiate(&g.exec, graph, 0);
-    if (graph) cudaGraphDestroy(graph);
-    if (e) {
-      g.reset();
-      return e;
-    }
-    g.key = key;
-  }
-  return cudaGraphLaunch(g.exec, c->stream);
-}
-
-std::vector<long long> sweep_key(vt_ctx* c, int kind) {
-  const AdjointState* s = c->adj;
-  long long dt_bits = 0;
-  std::memcpy(&dt_bits, &s->dt, sizeof(dt_bits));
-  return {kind, s->nsteps, dt_bits, s->all_stages, reinterpret_cast<long long>(s->slots), s->nslots,
-          reinterpret_cast<long long>(c->U), reinterpret_cast<long long>(s->bufs),
-          static_cast<long long>(s->first_adjoint), static_cast<long long>(s->plan.size())};
-}
-
 int prepare(vt_ctx* c) {
   int st = setup(c);
   if (!st) st = ensure_aos(c);
@@ -542,16 +509,8 @@ int prepare(vt_ctx* c) {
 
 }  // namespace
 
-void adjoint_invalidate_graphs(vt_ctx* c) {
-  if (!c || !c->adj) return;
-  c->adj->fwd_graph.reset();
-  c->adj->bwd_graph.reset();
-}
-
 void adjoint_release(vt_ctx* c) {
   if (!c || !c->adj) return;
-  c->adj->fwd_graph.reset();
-  c->adj->bwd_graph.reset();
   if (c->adj->slots) cudaFree(c->adj->slots);
   if (c->adj->bufs) cudaFree(c->adj->bufs);
   release_streams(c->adj);
@@ -587,15 +546,10 @@ int vt_adjoint_forward(vt_ctx* c, double dt, int nsteps, int nsnapshots) {
     s->info.all_stages = 1;
     cudaError_t e = vt::reset_error_words(c);
     if (!e)
-      e = vt::run_captured(c, s->fwd_graph, vt::sweep_key(c, 0), [&]() {
-        cudaError_t x = cudaMemcpyAsync(vt::slot(c, 0), c->U, sizeof(double2) * s->state_elems,
-                                        cudaMemcpyDeviceToDevice, c->stream);
-        for (int i = 0; i < nsteps && !x; ++i)
-          x = vt::stage_step(c, vt::slot(c, 4ll * i), vt::slot(c, 4ll * i + 1), vt::slot(c, 4ll * i + 2),
-                             vt::slot(c, 4ll * i + 3), dt, i + 1 < nsteps ? vt::slot(c, 4ll * i + 4) : c->U,
-                             c->stream);
-        return x;
-      });
+      e = cudaMemcpyAsync(vt::slot(c, 0), c->U, sizeof(double2) * s->state_elems, cudaMemcpyDeviceToDevice, c->stream);
+    for (int i = 0; i < nsteps && !e; ++i)
+      e = vt::stage_step(c, vt::slot(c, 4ll * i), vt::slot(c, 4ll * i + 1), vt::slot(c, 4ll * i + 2),
+                         vt::slot(c, 4ll * i + 3), dt, i + 1 < nsteps ? vt::slot(c, 4ll * i + 4) : c->U, c->stream);
     if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("adjoint forward", e));
     st = vt::finish(c, nsteps, dt);
     if (st == VT_OK) s->have_forward = s->fresh = true;
@@ -614,11 +568,8 @@ int vt_adjoint_forward(vt_ctx* c, double dt, int nsteps, int nsnapshots) {
   if ((st = vt_checkpoint_plan(nsteps, S, &s->info))) return st;
   cudaError_t e = vt::reset_error_words(c);
   if (!e)
-    e = vt::run_captured(c, s->fwd_graph, vt::sweep_key(c, 1), [&]() {
-      cudaError_t x = cudaMemcpyAsync(vt::slot(c, 0), c->U, sizeof(double2) * s->state_elems,
-                                      cudaMemcpyDeviceToDevice, c->stream);
-      return x ? x : vt::run_plan(c, 0, s->first_adjoint, c->U);
-    });
+    e = cudaMemcpyAsync(vt::slot(c, 0), c->U, sizeof(double2) * s->state_elems, cudaMemcpyDeviceToDevice, c->stream);
+  if (!e) e = vt::run_plan(c, 0, s->first_adjoint, c->U);
   if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("adjoint forward", e));
   st = vt::finish(c, nsteps, dt);
   if (st == VT_OK) s->have_forward = s->fresh = true;
@@ -637,14 +588,9 @@ int vt_adjoint_backward(vt_ctx* c, const double* dJdU_T, double* dJdU_0, int dev
   cudaError_t e = vt::reset_error_words(c);
   if (s->all_stages) {  // nothing to recompute
     if (!e) e = vt::load_aos(c, dJdU_T, device_pointers, s->lam);
-    if (!e)
-      e = vt::run_captured(c, s->bwd_graph, vt::sweep_key(c, 2), [&]() {
-        cudaError_t x = cudaSuccess;
-        for (int i = s->nsteps - 1; i >= 0 && !x; --i)
-          x = vt::adjoint_step(c, vt::slot(c, 4ll * i), vt::slot(c, 4ll * i + 1), vt::slot(c, 4ll * i + 2),
-                               vt::slot(c, 4ll * i + 3), s->dt);
-        return x;
-      });
+    for (int i = s->nsteps - 1; i >= 0 && !e; --i)
+      e = vt::adjoint_step(c, vt::slot(c, 4ll * i), vt::slot(c, 4ll * i + 1), vt::slot(c, 4ll * i + 2),
+                           vt::slot(c, 4ll * i + 3), s->dt);
     if (!e) e = vt::store_aos(c, s->lam, dJdU_0, device_pointers);
     if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("adjoint backward", e));
     return vt::finish(c, 0, 0.0);
@@ -654,9 +600,7 @@ int vt_adjoint_backward(vt_ctx* c, const double* dJdU_T, double* dJdU_0, int dev
   if (!e && !s->fresh) e = vt::run_plan(c, 0, s->first_adjoint, nullptr);
   s->fresh = false;
   if (!e) e = vt::load_aos(c, dJdU_T, device_pointers, s->lam);
-  if (!e)
-    e = vt::run_captured(c, s->bwd_graph, vt::sweep_key(c, 3),
-                         [&]() { return vt::run_plan_overlapped(c, s->first_adjoint, s->plan.size()); });
+  if (!e) e = vt::run_plan_overlapped(c, s->first_adjoint, s->plan.size());
   if (!e) e = vt::store_aos(c, s->lam, dJdU_0, device_pointers);
   if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("adjoint backward", e));
   return vt::finish(c, 0, 0.0);

@@ -51,6 +51,13 @@
 
 namespace vt {
 
+// The operators: folded, and the lift as it is for the neighbours' adjoints.
+template <int P, int NFQ>
+struct AdjOps {
+  FoldedOps<P, NFQ> fo;
+  double lift[3][np_of_p(P)][NFQ];
+};
+
 // The stage kernel's buffers, the stage adjoint tile, and the operator tables
 // that the face phase indexes at run time (the face point and the side of a
 // work item are not known at compile time).
@@ -119,7 +126,8 @@ __device__ __forceinline__ void folded_adjoint(const double* Ad, bool valid, dou
 // adjoint tile.
 template <int P, int NFQ>
 __global__ void __launch_bounds__(4 * kTileElems, 2)
-    adjoint_tile_kernel(const __grid_constant__ AdjArgs a, const StageOps<P, NFQ> ops, const FoldedOps<P, NFQ> fo) {
+    adjoint_tile_kernel(const __grid_constant__ AdjArgs a, const AdjOps<P, NFQ> ops) {
+  const FoldedOps<P, NFQ>& fo = ops.fo;
   using B = TileLayout<P, NFQ>;
   using L = AdjTileLayout<P, NFQ>;
   constexpr int E = B::E;
@@ -154,8 +162,8 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
   const bool hand_out = a.ntiles > kHandOut * G;
 
   {
-    const double* tm = &ops.tm[0][0][0];
-    const double* tp = &ops.tp[0][0][0];
+    const double* tm = &fo.tm[0][0][0];
+    const double* tp = &fo.tp[0][0][0];
     const double* lf = &ops.lift[0][0][0];
     for (int l = t; l < 3 * NFQ * NE; l += T) {
       TM[l] = tm[l];
@@ -170,12 +178,13 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
     mbar_init(bar, 2);
     *abort_flag = 0;
   }
-  let_next_start();
+
   int tile = blockIdx.x;  // the grid has at most ntiles blocks
   unsigned code = neighbour_code(a.lists, tile, which, lane);
   __syncthreads();
   if (grp == 0 && lane == 0) issue_adj_mesh_copies<P, NFQ>(a, tile, which, smem);
   wait_for_previous();
+  let_next_start();
   if (grp == 0 && lane == 0) issue_adj_state_copies<P, NFQ>(a, tile, which, smem);
   copy_neighbours<P>(H, a.U, code, which, grp, lane);
   cp_async_commit();

@@ -8,8 +8,8 @@
 // shifted by the instance's offset, and their tiles (the same tiles a single
 // instance would get, so the arithmetic per element is identical) listed one
 // after another, each tile carrying its instance's time step. One launch of the
-// stage kernel per group and stage advances every instance of the group; one
-// CUDA graph holds a whole RK4 step of all groups.
+// stage kernel per group and stage advances every instance of the group; the
+// groups' launches run side by side on a stream each.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -62,8 +62,13 @@ struct Group {
   std::vector<long long> offset;  // element offset of each member
   std::vector<int> tile_begin;    // first tile of each member
   std::vector<Numbering> num;     // of each member's own elements and columns
-  std::vector<double> ops;
+  std::vector<double> ops, block;  // operator block, and the stage kernel's form of it
   StageKernel kern;
+  void use(const StageKernel& k) {
+    kern = k;
+    block.resize(ops.size() + kBlockExtra);
+    k.pack(ops.data(), block.data());
+  }
   int max_blocks = 0;
   double2 *U = nullptr, *A = nullptr, *Sa = nullptr, *Sb = nullptr, *geo = nullptr;
   int4* nbr = nullptr;
@@ -85,10 +90,8 @@ struct vt_batch {
   std::vector<int> group_of, index_in_group, K_of;
   double2* staging = nullptr;  // largest instance, AoS
   size_t staging_bytes = 0;
-  cudaGraphExec_t graph = nullptr;
-  // one stream per group: the groups' stage chains are independent and run as
-  // concurrent branches of the step graph, so one group's wave tail overlaps
-  // the next group's work
+  // one stream per group: the groups' stage chains are independent and run
+  // side by side, so one group's last tiles overlap another group's work
   std::vector<cudaStream_t> gstreams;
   cudaEvent_t fork = nullptr;
   std::vector<cudaEvent_t> join;
@@ -112,7 +115,6 @@ void release(vt_batch* b) {
     if (v->aos) cudaFree(v->aos);
     delete v;
   }
-  if (b->graph) cudaGraphExecDestroy(b->graph);
   for (cudaStream_t st : b->gstreams)
     if (st) cudaStreamDestroy(st);
   for (cudaEvent_t ev : b->join)
@@ -151,7 +153,7 @@ vt::StageArgs group_args(vt::Group& g, const double2* in, double2* out, int stag
 // The four stage launches of one RK4 step of group g on stream st; the
 // coefficients are fractions of each tile's dt.
 cudaError_t enqueue_group_step(vt::Group& g, cudaStream_t st) {
-  const double* ops = g.ops.data();
+  const double* ops = g.block.data();
   cudaError_t e = g.kern.launch(group_args(g, g.U, g.Sa, 0, 1.0 / 6, 0.5), ops, g.max_blocks, st);
   if (!e) e = g.kern.launch(group_args(g, g.Sa, g.Sb, 1, 1.0 / 3, 0.5), ops, g.max_blocks, st);
   if (!e) e = g.kern.launch(group_args(g, g.Sb, g.Sa, 2, 1.0 / 3, 1.0), ops, g.max_blocks, st);
@@ -159,20 +161,26 @@ cudaError_t enqueue_group_step(vt::Group& g, cudaStream_t st) {
   return e;
 }
 
-// One RK4 step of every group. The groups are independent problems: each
-// group's chain of four stages runs on its own stream, forked from and joined
-// back into the batch stream, so that in the captured graph they are parallel
-// branches and the GPU starts one group's blocks while another group's last
-// tiles finish.
-cudaError_t enqueue_step(vt_batch* b) {
-  if (b->groups.size() == 1) return enqueue_group_step(b->groups[0], b->stream);
-  cudaError_t e = cudaEventRecord(b->fork, b->stream);
-  for (size_t gi = 0; gi < b->groups.size() && !e; ++gi) {
-    e = cudaStreamWaitEvent(b->gstreams[gi], b->fork, 0);
-    if (!e) e = enqueue_group_step(b->groups[gi], b->gstreams[gi]);
-    if (!e) e = cudaEventRecord(b->join[gi], b->gstreams[gi]);
+// nsteps RK4 steps of every group. The groups are independent problems: each
+// group's chain of stages runs on its own stream, forked from and joined back
+// into the batch stream, so that the GPU starts one group's blocks while another
+// group's last tiles finish. The launches go round the groups step by step.
+cudaError_t enqueue_steps(vt_batch* b, int nsteps) {
+  cudaError_t e = cudaSuccess;
+  if (b->groups.size() == 1) {
+    for (int s = 0; s < nsteps && !e; ++s) e = enqueue_group_step(b->groups[0], b->stream);
+    return e;
   }
-  for (size_t gi = 0; gi < b->groups.size() && !e; ++gi) e = cudaStreamWaitEvent(b->stream, b->join[gi], 0);
+  e = cudaEventRecord(b->fork, b->stream);
+  for (size_t gi = 0; gi < b->groups.size() && !e; ++gi) e = cudaStreamWaitEvent(b->gstreams[gi], b->fork, 0);
+  for (int s = 0; s < nsteps && !e; ++s)
+    for (size_t gi = 0; gi < b->groups.size() && !e; ++gi) e = enqueue_group_step(b->groups[gi], b->gstreams[gi]);
+  // joined even after an error, so that what was launched is waited for
+  for (size_t gi = 0; gi < b->groups.size(); ++gi) {
+    cudaError_t j = cudaEventRecord(b->join[gi], b->gstreams[gi]);
+    if (!j) j = cudaStreamWaitEvent(b->stream, b->join[gi], 0);
+    if (!e) e = j;
+  }
   return e;
 }
 
@@ -198,23 +206,6 @@ cudaError_t reset_errors(vt_batch* b) {
     if (!e) e = cudaMemsetAsync(g.err + 1, 0, (vt::kErrWords - 1) * sizeof(unsigned long long), b->stream);
   }
   return e;
-}
-
-int capture(vt_batch* b) {
-  if (b->graph) {
-    cudaGraphExecDestroy(b->graph);
-    b->graph = nullptr;
-  }
-  cudaGraph_t gr = nullptr;
-  cudaError_t e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
-  if (!e) {
-    const cudaError_t le = enqueue_step(b);
-    e = cudaStreamEndCapture(b->stream, &gr);
-    if (le) e = le;
-  }
-  if (!e) e = cudaGraphInstantiate(&b->graph, gr, 0);
-  if (gr) cudaGraphDestroy(gr);
-  return e ? fail(VT_ERR_CUDA, vt::cuda_msg("batch graph", e)) : VT_OK;
 }
 
 int upload_dt(vt_batch* b) {
@@ -262,6 +253,7 @@ int ensure_views(vt_batch* b) {
     c->ntiles = G.ntiles;
     c->err = G.err;
     c->ops = G.ops;
+    c->block = G.block;
     c->launch = G.kern.launch;
     c->map = G.kern.map;
     c->tile_dt = G.tile_dt;
@@ -371,7 +363,7 @@ vt_batch* vt_batch_create(const vt_mesh_desc* descs, int n, int device, int* sta
   }
   size_t max_inst_bytes = 0;
   for (auto& G : b->groups) {
-    G.kern = vt::select_kernel(G.p, G.nfq, G.ops.data());
+    G.use(vt::select_kernel(G.p, G.nfq, G.ops.data()));
     int per_sm = 0;
     if ((e = G.kern.configure(&per_sm))) {
       set(fail(VT_ERR_CUDA, vt::cuda_msg("stage kernel attributes", e)));
@@ -391,7 +383,7 @@ vt_batch* vt_batch_create(const vt_mesh_desc* descs, int n, int device, int* sta
     std::vector<double2> geo(vt::kGeoRows * static_cast<size_t>(G.ncols), make_double2(0.0, 0.0));
     std::vector<int4> nbr(static_cast<size_t>(G.ncols), make_int4(0, 0, 0, 0));
     for (size_t m = 0; m < G.members.size(); ++m)
-      vt::pack_mesh(descs[G.members[m]], G.num[m], geo.data(), nbr.data(),
+      vt::pack_mesh(descs[G.members[m]], vt::element_columns(G.num[m]), geo.data(), nbr.data(),
                     static_cast<long long>(vt::kTileElems) * G.tile_begin[m]);
     const size_t state_bytes = sizeof(double2) * 2 * G.Np * static_cast<size_t>(G.ncols);
     if ((e = vt::dalloc(&G.U, state_bytes)) || (e = vt::dalloc(&G.A, state_bytes)) ||
@@ -500,12 +492,7 @@ int vt_batch_step_rk4(vt_batch* b, int nsteps) {
   cudaSetDevice(b->device);
   cudaError_t e = reset_errors(b);
   if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("batch reset", e));
-  if (!b->graph) {
-    const int st = capture(b);
-    if (st) return st;
-  }
-  for (int s = 0; s < nsteps; ++s)
-    if ((e = cudaGraphLaunch(b->graph, b->stream))) return fail(VT_ERR_CUDA, vt::cuda_msg("batch launch", e));
+  if ((e = enqueue_steps(b, nsteps))) return fail(VT_ERR_CUDA, vt::cuda_msg("batch launch", e));
   if ((e = cudaStreamSynchronize(b->stream))) return fail(VT_ERR_CUDA, vt::cuda_msg("batch step", e));
   // first failure over groups: earliest stage, then instance order
   b->last = vt_error_info{};
@@ -686,7 +673,7 @@ int vt_batch_autotune(vt_batch* b, int trials, int* blocks_per_sm_out, int* mapp
       const vt::StageKernel k = vt::select_kernel(G.p, G.nfq, G.ops.data(), map);
       int limit = 0;
       if (k.configure(&limit)) continue;
-      G.kern = k;
+      G.use(k);
       for (int bps = 1; bps <= std::max(1, limit); ++bps) {
         G.max_blocks = b->sms * bps;
         const float ms = time_group_steps(b, G, trials, e0, e1);
@@ -697,7 +684,7 @@ int vt_batch_autotune(vt_batch* b, int trials, int* blocks_per_sm_out, int* mapp
         }
       }
     }
-    G.kern = best_k;
+    G.use(best_k);
     G.max_blocks = b->sms * best_b;
     if (blocks_per_sm_out) blocks_per_sm_out[gi] = best_b;
     if (mapping_out) mapping_out[gi] = best_k.map;
@@ -712,11 +699,11 @@ int vt_batch_autotune(vt_batch* b, int trials, int* blocks_per_sm_out, int* mapp
   for (size_t gi = 0; gi < b->views.size(); ++gi) {  // the adjoint's group views step with the chosen kernels
     vt_ctx* v = b->views[gi];
     v->launch = b->groups[gi].kern.launch;
+    v->block = b->groups[gi].block;
     v->map = b->groups[gi].kern.map;
     v->max_blocks = b->groups[gi].max_blocks;
-    vt::adjoint_invalidate_graphs(v);
   }
-  return capture(b);
+  return VT_OK;
 }
 
 int vt_batch_set_mapping(vt_batch* b, const int* mapping) {
@@ -731,16 +718,16 @@ int vt_batch_set_mapping(vt_batch* b, const int* mapping) {
     int limit = 0;
     const cudaError_t e = k.configure(&limit);
     if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("vt_batch_set_mapping", e));
-    G.kern = k;
+    G.use(k);
     G.max_blocks = std::min(G.max_blocks, b->sms * std::max(1, limit));
     if (gi < b->views.size()) {
       b->views[gi]->launch = k.launch;
+      b->views[gi]->block = G.block;
       b->views[gi]->map = k.map;
       b->views[gi]->max_blocks = G.max_blocks;
-      vt::adjoint_invalidate_graphs(b->views[gi]);
     }
   }
-  return capture(b);
+  return VT_OK;
 }
 
 int vt_batch_time_groups(vt_batch* b, int reps, float* ms_per_step) {
@@ -782,7 +769,7 @@ int vt_batch_set_blocks_per_sm(vt_batch* b, const int* blocks_per_sm) {
     const int bps = std::max(1, std::min(blocks_per_sm[gi], std::max(1, limit)));
     b->groups[gi].max_blocks = b->sms * bps;
   }
-  return capture(b);
+  return VT_OK;
 }
 
 int vt_batch_group_info(const vt_batch* b, int g, int* p, int* n_instances, int64_t* n_elements) {

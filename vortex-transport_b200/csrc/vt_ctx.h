@@ -31,13 +31,12 @@ struct vt_ctx {
   unsigned long long* err = nullptr;
   double2* aos = nullptr;
   double *W = nullptr, *partial = nullptr, *tot = nullptr;
-  std::vector<double> ops;
+  std::vector<double> ops;    // operator block (StageOps)
+  std::vector<double> block;  // the stage kernel's form of it
   std::vector<double> minv_ref;  // Np x Np, for the projected initial condition
   vt::LaunchFn launch = nullptr;
   int map = vt::kDefaultMap;  // warp mapping of the stage kernel
   double time = 0.0;
-  cudaGraphExec_t rk4_graph = nullptr;
-  double rk4_graph_dt = 0.0;
   vt_error_info last{};
   int pending_steps = 0;
   double pending_dt = 0.0;
@@ -62,9 +61,11 @@ namespace vt {
 
 std::string cuda_msg(const char* what, cudaError_t e);
 
+// The column of every element of a numbering.
+std::vector<int> element_columns(const Numbering& num);
 // A mesh's geometry rows and side-ordered neighbour columns (StageArgs), its
 // columns starting at `column` of the arrays.
-void pack_mesh(const vt_mesh_desc& d, const Numbering& num, double2* geo, int4* nbr, long long column);
+void pack_mesh(const vt_mesh_desc& d, const std::vector<int>& col, double2* geo, int4* nbr, long long column);
 
 // Arguments of one stage launch on this context's mesh and schedule.
 StageArgs stage_args(vt_ctx* c, const double2* in, const double2* base, double2* acc, double2* out, int stage,
@@ -84,7 +85,5 @@ cudaError_t from_columns(vt_ctx* c, const double2* src, double* dst);
 
 // Frees the adjoint's buffers (no-op without them).
 void adjoint_release(vt_ctx* c);
-// Drops the adjoint's captured sweep graphs (after the stage kernel changed).
-void adjoint_invalidate_graphs(vt_ctx* c);
 
 }  // namespace vt

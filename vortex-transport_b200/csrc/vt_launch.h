@@ -27,11 +27,18 @@ cudaError_t launch_dependent(void (*kernel)(Params...), int grid, int block, siz
 }
 
 using LaunchFn = cudaError_t (*)(const StageArgs&, const double*, int, cudaStream_t);
+using PackFn = void (*)(const double*, double*);
 using ConfigFn = cudaError_t (*)(int*);
 
+constexpr int kBlockExtra = 2;
+
 struct StageKernel {
-  // Launches one stage with at most `max_blocks` persistent blocks.
+  // Launches one stage with at most `max_blocks` persistent blocks; its second
+  // argument is the kernel's own form of the operators, written by `pack`.
   LaunchFn launch = nullptr;
+  // Writes that form (at most stage_ops_doubles(p, nfq) + kBlockExtra doubles)
+  // from the operator block.
+  PackFn pack = nullptr;
   // Sets the dynamic shared-memory attribute on the current device and
   // reports resident blocks per SM. Call before any launch or capture.
   ConfigFn configure = nullptr;

@@ -144,6 +144,8 @@ int vt_step_rk4_noalloc(const vt_device_mesh* m, const double* dU_in, double* dU
   vt::fold_stage_operators(m->p, m->n_line_points, m->inv_mass_ref, m->stiffness_ref, m->line_quadrature,
                            m->phi_plus, m->phi_minus, ops);
   const vt::StageKernel pk = vt::select_kernel(m->p, m->n_line_points, ops);
+  double block[vt::kMaxOps];
+  pk.pack(ops, block);
 
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -210,10 +212,10 @@ int vt_step_rk4_noalloc(const vt_device_mesh* m, const double* dU_in, double* dU
     return a;
   };
   for (int s = 0; s < nsteps && !e; ++s) {
-    if (!e) e = pk.launch(args(U, Sa, 0, (1.0 / 6) * dt, 0.5 * dt), ops, max_blocks, st);
-    if (!e) e = pk.launch(args(Sa, Sb, 1, (1.0 / 3) * dt, 0.5 * dt), ops, max_blocks, st);
-    if (!e) e = pk.launch(args(Sb, Sa, 2, (1.0 / 3) * dt, dt), ops, max_blocks, st);
-    if (!e) e = pk.launch(args(Sa, U, 3, 0.0, (1.0 / 6) * dt), ops, max_blocks, st);
+    if (!e) e = pk.launch(args(U, Sa, 0, (1.0 / 6) * dt, 0.5 * dt), block, max_blocks, st);
+    if (!e) e = pk.launch(args(Sa, Sb, 1, (1.0 / 3) * dt, 0.5 * dt), block, max_blocks, st);
+    if (!e) e = pk.launch(args(Sb, Sa, 2, (1.0 / 3) * dt, dt), block, max_blocks, st);
+    if (!e) e = pk.launch(args(Sa, U, 3, 0.0, (1.0 / 6) * dt), block, max_blocks, st);
   }
   if (!e) e = vt::launch_from_columns(U, dU_out, cv.num, Np, st);
   unsigned long long words[4] = {~0ull, 0, 0, 0};

@@ -46,9 +46,9 @@ inline Numbering mesh_numbering(int K, const int32_t* type, const int32_t* conn)
   const int nx = (conn[1] + 1) / 2;  // element 0's left neighbour is 2 nx - 1
   if (nx < 1 || K % (2 * nx)) return other;
   const int ny = K / (2 * nx);
-  for (int i = 0; i < K; ++i) {
-    const int left = i % (2 * nx) == 0 ? i - 1 + 2 * nx : i - 1;
-    const int right = (i + 1) % (2 * nx) == 0 ? i + 1 - 2 * nx : i + 1;
+  for (int i = 0, in_row = 0; i < K; ++i, in_row = in_row + 1 == 2 * nx ? 0 : in_row + 1) {
+    const int left = in_row == 0 ? i - 1 + 2 * nx : i - 1;
+    const int right = in_row + 1 == 2 * nx ? i + 1 - 2 * nx : i + 1;
     // the reference's three loops, later ones overwriting earlier ones
     int vert;
     if (i >= 2 * nx * (ny - 1)) vert = i % 2 == 0 ? i + 1 - 2 * nx : i - 1 - 2 * nx * (ny - 1);

@@ -1,10 +1,18 @@
 // C ABI of the device solver (include/vortex_b200.h, "drop-in boundary").
 //
 // vt_create folds the reference-space operators into the per-stage kernel
-// parameter block and uploads packed per-element geometry; vt_step_rk4 replays
-// a captured CUDA graph of the four fused stage kernels once per step.
+// parameter block and uploads packed per-element geometry; vt_step_rk4 launches
+// the four fused stage kernels of each step, every launch overlapping the one
+// before it (launch_dependent). Without a graph: the host needs about 2.5 us a
+// launch, less than the shortest stage takes, a graph of one step had an
+// ordinary dependency between two steps, and a new problem or time step waited
+// for a capture. 50 steps at 64 x 64 cells, p = 2 take 1.12 ms launched and
+// 1.28 as graphs of a step, 250 at 8 x 8, p = 3 6.18 and 6.24; the first
+// gradient of a new 128 x 128, p = 3 problem 15 to 18 ms against 27 with
+// its sweeps captured (later ones 14.7 against 14.2).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -250,9 +258,28 @@ __global__ void totals_final_kernel(const double* __restrict__ partial, int nblo
 
 }  // namespace
 
-void pack_mesh(const vt_mesh_desc& d, const Numbering& num, double2* geo, int4* nbr, long long column) {
+std::vector<int> element_columns(const Numbering& num) {
+  std::vector<int> col(static_cast<size_t>(num.K));
+  if (num.nx == 0) {
+    for (int e = 0; e < num.K; ++e) col[e] = num.column(e);
+    return col;
+  }
+  for (int r = 0; r < num.ny; ++r)  // row by row, tile by tile: no divisions per element
+    for (int ti = 0, j0 = 0; j0 < num.nx; ++ti, j0 += num.W) {
+      const int w = std::min(num.W, num.nx - j0), tj = r / num.H;
+      const int x = (tj * num.ntx + ti) * kTileElems + (r - tj * num.H) * w;
+      int* out = col.data() + 2 * (static_cast<size_t>(r) * num.nx + j0);
+      for (int k = 0; k < w; ++k) {
+        out[2 * k] = x + k;
+        out[2 * k + 1] = x + k + kTileRun;
+      }
+    }
+  return col;
+}
+
+void pack_mesh(const vt_mesh_desc& d, const std::vector<int>& col, double2* geo, int4* nbr, long long column) {
   for (int n = 0; n < d.n_elements; ++n) {
-    const long long x = column + num.column(n);
+    const long long x = column + col[n];
     const double* ji = d.inv_jacobian + 4 * static_cast<size_t>(n);
     const double* nv = d.normals + 6 * static_cast<size_t>(n);
     const double* ln = d.side_lengths + 3 * static_cast<size_t>(n);
@@ -264,7 +291,7 @@ void pack_mesh(const vt_mesh_desc& d, const Numbering& num, double2* geo, int4* 
     for (int s = 0; s < 3; ++s) geo[geo_index(x, 4 + s)] = make_double2(nv[2 * s], nv[2 * s + 1]);
     const int32_t* b = d.neighbours + 3 * static_cast<size_t>(n);
     const int off = static_cast<int>(column);
-    const int right = off + num.column(b[0]), left = off + num.column(b[1]), vert = off + num.column(b[2]);
+    const int right = off + col[b[0]], left = off + col[b[1]], vert = off + col[b[2]];
     nbr[x] = d.element_type[n] == 0 ? make_int4(vert, right, left, 0) : make_int4(vert, left, right, 0);
   }
 }
@@ -288,7 +315,6 @@ void release(vt_ctx* c) {
   if (!c) return;
   cudaSetDevice(c->device);
   vt::adjoint_release(c);
-  if (c->rk4_graph) cudaGraphExecDestroy(c->rk4_graph);
   void* bufs[] = {c->U,   c->A,   c->Sa, c->Sb,      c->R,   c->geo,   c->nbr,
                   c->err, c->aos, c->W,  c->partial, c->tot, c->elem,  c->lists};
   for (void* b : bufs)
@@ -326,7 +352,7 @@ vt::StageArgs stage_args(vt_ctx* c, const double2* in, const double2* base, doub
 
 cudaError_t enqueue_rk4_step(vt_ctx* c, double dt) {
   cudaError_t e;
-  const double* ops = c->ops.data();
+  const double* ops = c->block.data();
   if ((e = c->launch(stage_args(c, c->U, c->U, c->A, c->Sa, 0, (1.0 / 6) * dt, 0.5 * dt), ops, c->max_blocks, c->stream))) return e;
   if ((e = c->launch(stage_args(c, c->Sa, c->U, c->A, c->Sb, 1, (1.0 / 3) * dt, 0.5 * dt), ops, c->max_blocks, c->stream))) return e;
   if ((e = c->launch(stage_args(c, c->Sb, c->U, c->A, c->Sa, 2, (1.0 / 3) * dt, dt), ops, c->max_blocks, c->stream))) return e;
@@ -437,6 +463,8 @@ vt_ctx* vt_create(const vt_mesh_desc* d, int device, int* status) {
                               d->phi_plus, d->phi_minus);
   const vt::StageKernel sk = vt::select_kernel(c->p, c->nfq, c->ops.data());
   c->launch = sk.launch;
+  c->block.resize(c->ops.size() + vt::kBlockExtra);
+  sk.pack(c->ops.data(), c->block.data());
   int per_sm = 0, sms = 0;
   if ((e = sk.configure(&per_sm)) ||
       (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device))) {
@@ -451,12 +479,13 @@ vt_ctx* vt_create(const vt_mesh_desc* d, int device, int* status) {
   const long long ncols = c->ncols;
   std::vector<double2> geo(vt::kGeoRows * static_cast<size_t>(ncols), make_double2(0.0, 0.0));
   std::vector<int4> nbr(static_cast<size_t>(ncols), make_int4(0, 0, 0, 0));
-  vt::pack_mesh(*d, c->num, geo.data(), nbr.data(), 0);
+  const std::vector<int> columns = vt::element_columns(c->num);
+  vt::pack_mesh(*d, columns, geo.data(), nbr.data(), 0);
   // side s of an element faces side s of its neighbour (Evolve.cpp:167-202 on
   // the reference mesh); the adjoint's gather of neighbour face terms needs it
   c->side_pairing = true;
   for (int n = 0; n < K && c->side_pairing; ++n) {
-    const int x = c->num.column(n);
+    const int x = columns[n];
     const int4 b = nbr[x];
     c->side_pairing = nbr[b.x].x == x && nbr[b.y].y == x && nbr[b.z].z == x;
   }
@@ -562,6 +591,8 @@ vt_ctx* vt_create_structured(const vt_params* prm, const vt_vortex* ic_in, int d
   c->ops = vt::host_operators(p, nfq, minv.data(), stiff.data(), line.data(), pp.data(), pm.data());
   const vt::StageKernel sk = vt::select_kernel(p, nfq, c->ops.data());
   c->launch = sk.launch;
+  c->block.resize(c->ops.size() + vt::kBlockExtra);
+  sk.pack(c->ops.data(), c->block.data());
   int per_sm = 0, sms = 0;
   if ((e = sk.configure(&per_sm)) ||
       (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device))) {
@@ -706,25 +737,8 @@ int vt_download_state(vt_ctx* c, double* U, double* F) {
 static int rk4_enqueue(vt_ctx* c, double dt, int nsteps) {
   cudaError_t e = reset_error_words(c);
   if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("reset", e));
-  if (!c->rk4_graph || c->rk4_graph_dt != dt) {
-    if (c->rk4_graph) {
-      cudaGraphExecDestroy(c->rk4_graph);
-      c->rk4_graph = nullptr;
-    }
-    cudaGraph_t g = nullptr;
-    e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
-    if (!e) {
-      const cudaError_t le = enqueue_rk4_step(c, dt);
-      e = cudaStreamEndCapture(c->stream, &g);
-      if (le) e = le;
-    }
-    if (!e) e = cudaGraphInstantiate(&c->rk4_graph, g, 0);
-    if (g) cudaGraphDestroy(g);
-    if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("graph capture", e));
-    c->rk4_graph_dt = dt;
-  }
   for (int s = 0; s < nsteps; ++s)
-    if ((e = cudaGraphLaunch(c->rk4_graph, c->stream))) return fail(VT_ERR_CUDA, vt::cuda_msg("graph launch", e));
+    if ((e = enqueue_rk4_step(c, dt))) return fail(VT_ERR_CUDA, vt::cuda_msg("rk4 launch", e));
   c->pending_steps += nsteps;
   c->pending_dt = dt;
   return VT_OK;
@@ -766,16 +780,11 @@ int vt_step_euler(vt_ctx* c, double dt, int nsteps) {
   cudaError_t e = reset_error_words(c);
   for (int s = 0; s < nsteps && !e; ++s) {
     // double buffer: the neighbours of an element read the old state
-    e = c->launch(stage_args(c, c->U, c->U, c->A, c->Sa, vt::kStageEuler, 0.0, dt), c->ops.data(),
+    e = c->launch(stage_args(c, c->U, c->U, c->A, c->Sa, vt::kStageEuler, 0.0, dt), c->block.data(),
                   c->max_blocks, c->stream);
     std::swap(c->U, c->Sa);
   }
   if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("euler", e));
-  // the RK4 graph captured the old buffer roles
-  if (nsteps % 2 && c->rk4_graph) {
-    cudaGraphExecDestroy(c->rk4_graph);
-    c->rk4_graph = nullptr;
-  }
   return finish(c, nsteps, dt);
 }
 
@@ -789,7 +798,7 @@ int vt_rhs(vt_ctx* c, double* Udot) {
   if (!c->R) e = alloc(&c->R, sizeof(double2) * 2 * c->Np * static_cast<size_t>(c->ncols));
   if (!e) e = reset_error_words(c);
   if (!e)
-    e = c->launch(stage_args(c, c->U, c->U, c->A, c->R, vt::kStageRhs, 0.0, 0.0), c->ops.data(),
+    e = c->launch(stage_args(c, c->U, c->U, c->A, c->R, vt::kStageRhs, 0.0, 0.0), c->block.data(),
                   c->max_blocks, c->stream);
   if (!e) e = from_columns(c, c->R, reinterpret_cast<double*>(c->aos));
   if (!e)
@@ -935,13 +944,9 @@ int vt_set_stage_mapping(vt_ctx* c, int mapping) {
   if (!e) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
   if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("vt_set_stage_mapping", e));
   c->launch = sk.launch;
+  sk.pack(c->ops.data(), c->block.data());
   c->map = mapping;
   c->max_blocks = sms * (per_sm > 0 ? per_sm : 1);
-  if (c->rk4_graph) {  // the captured step holds the old kernel
-    cudaGraphExecDestroy(c->rk4_graph);
-    c->rk4_graph = nullptr;
-  }
-  vt::adjoint_invalidate_graphs(c);
   return VT_OK;
 }
 
@@ -953,10 +958,6 @@ int vt_test_bulk_wait(vt_ctx* c, unsigned tries, int issue_no_copies) {
   cudaSetDevice(c->device);
   c->test_wait_tries = tries;
   c->test_flags = issue_no_copies ? vt::kTestNoCopies : 0;
-  if (c->rk4_graph) {  // the captured step holds the old kernel arguments
-    cudaGraphExecDestroy(c->rk4_graph);
-    c->rk4_graph = nullptr;
-  }
   return VT_OK;
 }
 
@@ -968,7 +969,7 @@ int vt_profile_rk4_stages(vt_ctx* c, double dt, int reps, float* ms) {
   for (auto& x : ev) cudaEventCreate(&x);
   double acc[4] = {0, 0, 0, 0};
   cudaError_t e = reset_error_words(c);
-  const double* ops = c->ops.data();
+  const double* ops = c->block.data();
   for (int r = 0; r < reps && !e; ++r) {
     const vt::StageArgs args[4] = {stage_args(c, c->U, c->U, c->A, c->Sa, 0, (1.0 / 6) * dt, 0.5 * dt),
                                    stage_args(c, c->Sa, c->U, c->A, c->Sb, 1, (1.0 / 3) * dt, 0.5 * dt),

@@ -21,22 +21,33 @@ cudaError_t configure_stage(int* blocks_per_sm) {
                                                        4 * kTileElems, Lay::kBytes);
 }
 
+template <int P, int NFQ, int MAP>
+void pack_operators(const double* ops, double* block) {
+  using Ops = OpsOf<P, NFQ, MAP>;
+  static_assert(sizeof(Ops) % sizeof(double) == 0 && sizeof(Ops) <= sizeof(StageOps<P, NFQ>) + kBlockExtra * sizeof(double),
+                "a block of doubles");
+  if constexpr (MAP == kMapFolded) {
+    Ops o;
+    fold_operators(*reinterpret_cast<const StageOps<P, NFQ>*>(ops), &o);
+    std::memcpy(block, &o, sizeof(o));
+  } else {
+    std::memcpy(block, ops, sizeof(Ops));
+  }
+}
+
 // Persistent launch: at most `max_blocks` blocks (SMs x resident blocks), each
 // walking tiles blockIdx.x, blockIdx.x + gridDim.x, ...
 template <int P, int NFQ, int MAP>
-cudaError_t launch_stage(const StageArgs& a, const double* ops, int max_blocks, cudaStream_t st) {
+cudaError_t launch_stage(const StageArgs& a, const double* block, int max_blocks, cudaStream_t st) {
   using Lay = TileLayout<P, NFQ>;
-  static_assert(sizeof(StageOps<P, NFQ>) % sizeof(double) == 0, "operator block is doubles");
-  OpsOf<P, NFQ, MAP> o;
-  if constexpr (MAP == kMapFolded) fold_operators(*reinterpret_cast<const StageOps<P, NFQ>*>(ops), &o);
-  else std::memcpy(&o, ops, sizeof(o));
   const int grid = a.ntiles < max_blocks ? a.ntiles : max_blocks;
-  return launch_dependent(tile_stage_kernel<P, NFQ, MAP>, grid, 4 * kTileElems, Lay::kBytes, st, a, o);
+  return launch_dependent(tile_stage_kernel<P, NFQ, MAP>, grid, 4 * kTileElems, Lay::kBytes, st, a,
+                          *reinterpret_cast<const OpsOf<P, NFQ, MAP>*>(block));
 }
 
 template <int P, int NFQ, int MAP>
 StageKernel kernel_of() {
-  return StageKernel{launch_stage<P, NFQ, MAP>, configure_stage<P, NFQ, MAP>};
+  return StageKernel{launch_stage<P, NFQ, MAP>, pack_operators<P, NFQ, MAP>, configure_stage<P, NFQ, MAP>};
 }
 
 template <int P, int MAP>

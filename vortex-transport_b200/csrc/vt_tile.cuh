@@ -140,15 +140,18 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* src, unsigned bytes
                : "memory");
 }
 
-// Programmatic dependent launch (launch_dependent, vt_launch.h): the next
-// kernel of the stream may be scheduled from now on, where this grid leaves
-// room, and does its set-up there until wait_for_previous, which returns when
-// the kernel before it has ended and its writes are visible. Every kernel
+// Programmatic dependent launch (launch_dependent, vt_launch.h): after
+// let_next_start the next kernel of the stream may be scheduled where this grid
+// leaves room, and does its set-up there until wait_for_previous, which returns
+// when the kernel before it has ended and its writes are visible. Every kernel
 // launched that way waits before it reads or writes anything that another
 // kernel writes or reads; only the mesh's own arrays, which no kernel of the
-// stream writes, are read before. With it 250 RK4 steps at 8 x 8 cells, p = 3
-// (two tiles) take 6.2 ms instead of 7.1, 20 at 150 x 90, p = 3 0.88 instead of
-// 0.95 ms, 50 at 64 x 64, p = 2 1.26 instead of 1.28 ms.
+// stream writes, are read before. let_next_start comes after the own wait, so
+// that at most one later kernel is resident: when it came first, several were,
+// and blocks of one kernel shared an SM while other SMs had none. 50 RK4 steps
+// at 64 x 64 cells, p = 2 (128 tiles) take 1.23 ms without it, 1.79 with
+// let_next_start first and 1.12 as it is; 250 at 8 x 8, p = 3 6.35, 6.42 and
+// 6.18; 20 at 150 x 90, p = 3 0.91, 0.88 and 0.87; large meshes the same.
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -519,12 +522,13 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
     mbar_init(bar, 2);
     *abort_flag = 0;
   }
-  let_next_start();
+
   int tile = blockIdx.x;  // the grid has at most ntiles blocks
   unsigned code = neighbour_code(a.lists, tile, which, lane);
   __syncthreads();
   if (grp == 0 && lane == 0) issue_mesh_copies<P, NFQ>(a, tile, which, smem);
   wait_for_previous();
+  let_next_start();
   if (grp == 0 && lane == 0) issue_state_copy<P, NFQ>(a.in, tile, which, smem, a.test_flags);
   copy_neighbours<P>(H, a.in, code, which, grp, lane);
   cp_async_commit();
