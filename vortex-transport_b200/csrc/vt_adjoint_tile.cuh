@@ -22,8 +22,8 @@
 //             bF_e(q) - bF_nb(nfq-1-q) gives the adjoints of both traces, each
 //             written over its element's bF slot. A face leaving the tile is
 //             taken by each side, with the neighbour's bF recomputed from its
-//             stage adjoint, and gives the own trace's adjoint only (the
-//             neighbour's tile takes the other);
+//             stage adjoint in phase 2, and gives the own trace's adjoint only
+//             (the neighbour's tile takes the other);
 //   4. traces^T  thread (element, component): the trace adjoints onto the
 //             side nodes (transposed trace weights) into Np accumulators; then
 //             the transposed volume operator sa sum_i D[d][i][j] a_i per node;
@@ -68,28 +68,74 @@ struct AdjTileLayout {
   static constexpr int NE = B::NE;
   static constexpr int kTP = B::kBytes;                        // double [3][NFQ][NE] own trace weights
   static constexpr int kLF = kTP + 3 * NFQ * NE * 8 + 8 * (3 * NFQ * NE % 2);  // double [3][NFQ][NP] LIFT by point
-  static constexpr int kOut = kLF + 3 * NP * NFQ * 8 + 8 * (3 * NP * NFQ % 2);  // uint32 [kOuterWords]
-  static constexpr int kA = (kOut + kOuterWords * 4 + 127) / 128 * 128;  // double2 [2][2NP][32] stage adjoint
-  static constexpr int kBytes = kA + 2 * NP * kTileElems * 16;
+  static constexpr int kA = (kLF + 3 * NP * NFQ * 8 + 127) / 128 * 128;  // double2 [2][2NP][32] stage adjoint
+  // double2 [kHARows][2 kSlots]: the slots' stage adjoints, then their lifted face adjoints
+  static constexpr int kHARows = 2 * NP > 2 * NFQ ? 2 * NP : 2 * NFQ;
+  static constexpr int kHA = kA + 2 * NP * kTileElems * 16;
+  static constexpr int kBytes = kHA + kHARows * 2 * kSlots * 16;
 };
 
+// The stage adjoint of the neighbour in slot `lane` of half `which`, component
+// pair g, by the one thread that lifts it (lift_neighbour).
+template <int P>
+__device__ __forceinline__ void copy_neighbour_adjoint(double2* HA, const double2* a, unsigned code, int which, int g,
+                                                       int lane) {
+  constexpr int NP = np_of_p(P);
+  if (g > 1 || code == kNoNeighbour) return;
+  const double2* src = a + state_index(NP, code >> 2, g);
+  double2* dst = HA + g * 2 * kSlots + which * kSlots + lane;
+#pragma unroll
+  for (int i = 0; i < NP; ++i) cp_async16(dst + i * 4 * kSlots, src + i * 2 * kTileRun);
+}
+
+// Its lifted face adjoint at this side's face points (the neighbour's point
+// nfq-1-q for point q), in place: row 2 q + h for component pair h = g. Taken
+// once per face, from shared memory; formed per face point from the
+// neighbour's rows in global memory it was most of the reverse stage's waiting
+// (3.4 of 11 cycles per instruction on L2, 2.2 at the barrier behind the face
+// phase; 128 x 128 cells, p = 3).
+template <int P, int NFQ>
+__device__ __forceinline__ void lift_neighbour(double2* HA, const double* LF, unsigned code, double scale, int which,
+                                               int g, int lane) {
+  constexpr int NP = np_of_p(P);
+  if (g > 1 || code == kNoNeighbour) return;
+  double2* own = HA + g * 2 * kSlots + which * kSlots + lane;
+  double2 v[NP];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) v[i] = own[i * 4 * kSlots];
+  const double* lf = LF + (code & 3) * NFQ * NP;
+#pragma unroll
+  for (int q = 0; q < NFQ; ++q) {
+    double x = 0.0, y = 0.0;
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      const double l = lf[(NFQ - 1 - q) * NP + i];
+      x = fma(l, v[i].x, x);
+      y = fma(l, v[i].y, y);
+    }
+    own[q * 4 * kSlots] = make_double2(scale * x, scale * y);
+  }
+}
+
+// The neighbour's side length over det J.
+__device__ __forceinline__ double neighbour_scale(const double2* geo, unsigned code, int g) {
+  if (g > 1 || code == kNoNeighbour) return 0.0;
+  const unsigned s = code & 3;
+  return __ldg(reinterpret_cast<const double*>(geo + geo_index(code >> 2, s < 2 ? 2 : 3)) + (s == 1 ? 1 : 0));
+}
+
 // One thread per half announces the bulk copies of block `which` of a tile and
-// issues those of the mesh's arrays (geometry and, for block 0, the face list
-// with its slots), then those of the stage state and stage adjoint.
+// issues those of the mesh's arrays (geometry and, for block 0, the face list),
+// then those of the stage state and stage adjoint.
 template <int P, int NFQ>
 __device__ __forceinline__ void issue_adj_mesh_copies(const AdjArgs& a, int tile, int which, unsigned char* smem) {
-  using L = AdjTileLayout<P, NFQ>;
   using B = TileLayout<P, NFQ>;
-  constexpr unsigned kState = 2 * B::NP * kTileRun * 16, kGeo = kGeoRows * kTileRun * 16, kOuter = kOuterWords * 4;
+  constexpr unsigned kState = 2 * B::NP * kTileRun * 16, kGeo = kGeoRows * kTileRun * 16;
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem + B::kBar);
   fence_proxy_async_smem();
-  mbar_arrive_expect_tx(bar, 2 * kState + kGeo + (which == 0 ? kListOuter + kOuter : 0u));
+  mbar_arrive_expect_tx(bar, 2 * kState + kGeo + (which == 0 ? kListOuter : 0u));
   bulk_g2s(smem + B::kGE + which * kGeo, a.geo + (2ll * tile + which) * (kGeoRows * kTileRun), kGeo, bar);
-  if (which == 0) {
-    const unsigned char* list = a.lists + static_cast<long long>(tile) * kTileListBytes;
-    bulk_g2s(smem + B::kItems, list, kListOuter, bar);
-    bulk_g2s(smem + L::kOut, list + kListOuter, kOuter, bar);
-  }
+  if (which == 0) bulk_g2s(smem + B::kItems, a.lists + static_cast<long long>(tile) * kTileListBytes, kListOuter, bar);
 }
 template <int P, int NFQ>
 __device__ __forceinline__ void issue_adj_state_copies(const AdjArgs& a, int tile, int which, unsigned char* smem) {
@@ -103,16 +149,17 @@ __device__ __forceinline__ void issue_adj_state_copies(const AdjArgs& a, int til
 }
 
 // Even and odd parts of one component of a column's stage adjoint (node pairs
-// as sums and differences, the fixed nodes in the even part).
+// as sums and differences, the fixed nodes in the even part). Of an empty
+// column they are whatever lies there; nothing that is read comes from them.
 template <int P>
-__device__ __forceinline__ void folded_adjoint(const double* Ad, bool valid, double* e, double* o) {
+__device__ __forceinline__ void folded_adjoint(const double* Ad, double* e, double* o) {
   constexpr int NS = fold_nodes(P), NO = fold_pairs(P);
 #pragma unroll
   for (int k = 0; k < NS; ++k) {
     const int i = fold_node(P, k);
-    const double u = valid ? Ad[i * 4 * kTileRun] : 0.0;
+    const double u = Ad[i * 4 * kTileRun];
     if (k < NO) {
-      const double v = valid ? Ad[mirror_node(P, i) * 4 * kTileRun] : 0.0;
+      const double v = Ad[mirror_node(P, i) * 4 * kTileRun];
       e[k] = u + v;
       o[k] = u - v;
     } else {
@@ -149,7 +196,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
   int* NEXT = reinterpret_cast<int*>(smem + B::kBar + 12);
   double* TP = reinterpret_cast<double*>(smem + L::kTP);
   double* LF = reinterpret_cast<double*>(smem + L::kLF);
-  const unsigned* OUT = reinterpret_cast<const unsigned*>(smem + L::kOut);
+  double2* HA = reinterpret_cast<double2*>(smem + L::kHA);
   const double* Ad = reinterpret_cast<const double*>(smem + L::kA);  // stage adjoint tile
 
   const int t = threadIdx.x;
@@ -187,7 +234,9 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
   let_next_start();
   if (grp == 0 && lane == 0) issue_adj_state_copies<P, NFQ>(a, tile, which, smem);
   copy_neighbours<P>(H, a.U, code, which, grp, lane);
+  copy_neighbour_adjoint<P>(HA, a.a, code, which, grp, lane);
   cp_async_commit();
+  double scale = neighbour_scale(a.geo, code, grp);
   unsigned parity = 0;
   Ad += sidx<NP>(c >> 1, el) * 2 + (c & 1);              // this thread's component and column
   double* FBt = FB + ((c >> 1) * E + el) * 2 + (c & 1);  // likewise in the face buffer
@@ -214,7 +263,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
     // ---- 2. lifted face adjoints (half of them), component c of column el --------------
     {
       double e[NS], o[NOA];
-      folded_adjoint<P>(Ad, valid, e, o);
+      folded_adjoint<P>(Ad, e, o);
       const double2* ge = GE + which * kGeoRows * kTileRun + (el & 31);
       const double2 lsa = ge[2 * kTileRun], lsb = ge[3 * kTileRun];
       const double l0 = sa * lsa.x, l1 = sa * lsa.y, l2 = sa * lsb.x;
@@ -242,6 +291,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
       }
     }
     cp_async_wait_all();  // this thread's copies of neighbour rows
+    lift_neighbour<P, NFQ>(HA, LF, code, -0.5 * sa * scale, which, grp, lane);
     __syncthreads();
     if (*abort_flag) break;
 
@@ -253,12 +303,12 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
       const int fl = it & 63, s = (it >> 6) & 3, x = it >> 9;
       const bool mirror = (it >> 8) & 1;
       const double2 n = GE[((fl >> 5) * kGeoRows + 4 + s) * kTileRun + (fl & 31)];
-      // a neighbour outside the tile: its column and its lift's scale
+      // a neighbour without a slot: its column and its lift's scale
+      const bool far = !mirror && x == kNoSlot;
       long long nb = 0;
       double sc = 0.0;
-      if (!mirror) {
-        nb = x != kNoSlot ? OUT[x] >> 2
-                          : __ldg(reinterpret_cast<const int*>(a.nbr + (static_cast<long long>(tile) * E + fl)) + s);
+      if (far) {
+        nb = __ldg(reinterpret_cast<const int*>(a.nbr + (static_cast<long long>(tile) * E + fl)) + s);
         const double* gn = reinterpret_cast<const double*>(a.geo + geo_index(nb, s < 2 ? 2 : 3));
         sc = -0.5 * sa * __ldg(gn + (s == 1 ? 1 : 0));
       }
@@ -283,7 +333,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
           if (mirror) {  // the partner's own trace at its point nfq-1-q, as the stage kernel reads it
             y0 = S[sidx<NP>(2 * node, x)];
             y1 = S[sidx<NP>(2 * node + 1, x)];
-          } else if (x != kNoSlot) {
+          } else if (!far) {
             y0 = H[2 * k * 2 * kSlots + x];
             y1 = H[(2 * k + 1) * 2 * kSlots + x];
           } else {
@@ -296,8 +346,9 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
           um[2] = fma(cm[k], y1.x, um[2]);
           um[3] = fma(cm[k], y1.y, um[3]);
         }
-        if (mirror) {
-          const double2 m0 = oth[0], m1 = oth[E];
+        if (!far) {
+          const double2* m = mirror ? oth : HA + 4 * q * kSlots + x;
+          const double2 m0 = m[0], m1 = m[mirror ? E : 2 * kSlots];
           bf[0] = b0.x - m0.x, bf[1] = b0.y - m0.y, bf[2] = b1.x - m1.x, bf[3] = b1.y - m1.y;
         } else {
           // the neighbour's lifted adjoint at its point nfq-1-q
@@ -350,7 +401,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
     // ---- 4b. transposed volume operator: rows j*4 + h (xi), j*4 + 2 + h (eta) ----------
     if (P > 0) {
       double e[NS], o[NOA];
-      folded_adjoint<P>(Ad, valid, e, o);
+      folded_adjoint<P>(Ad, e, o);
 #pragma unroll
       for (int j = 0; j < NP; ++j) {
         double x = 0.0, y = 0.0;
@@ -360,6 +411,23 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
         for (int k = 0; k < NO; ++k) y = fma(fo.Do[k][j], o[k], y);
         FBt[j * 8 * E] = sa * (x + y);
         FBt[(mirror_node(P, j) * 8 + 4) * E] = sa * (x - y);
+      }
+    }
+    // the combine's operands, requested now so that they are in flight during
+    // the transposed flux (every load before the first store: acc_in and
+    // acc_out are the same array in three of the four reverse stages)
+    constexpr int kStep = 4 * kTileRun;  // doubles between node rows of the same pair
+    const long long off0 = blk * (4 * NP * kTileRun) + (c >> 1) * (2 * kTileRun) + (el & 31) * 2 + (c & 1);
+    double lv[NP], av[NP];
+    {
+      const bool need_lam = valid && (a.lam_coef != 0.0 || a.a_out);
+      const bool need_acc = valid && a.acc_in;
+      const double* lam = reinterpret_cast<const double*>(a.lam) + off0;
+      const double* acc_in = reinterpret_cast<const double*>(a.acc_in) + off0;
+#pragma unroll
+      for (int i = 0; i < NP; ++i) {
+        lv[i] = need_lam ? ld_early_rw(lam + i * kStep) : 0.0;
+        av[i] = need_acc ? ld_early_rw(acc_in + i * kStep) : 0.0;
       }
     }
     run_sync(t);
@@ -390,28 +458,16 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
         issue_adj_state_copies<P, NFQ>(a, next, which, smem);
       }
       copy_neighbours<P>(H, a.U, code, which, grp, lane);
+      copy_neighbour_adjoint<P>(HA, a.a, code, which, grp, lane);
+      scale = neighbour_scale(a.geo, code, grp);
     }
     cp_async_commit();
 
     // ---- 6. reverse RK combine -------------------------------------------------------------
-    // every load before the first store: acc_in and acc_out are the same array
-    // in three of the four reverse stages, so loads that follow a store could
-    // not be moved above it and each would wait on its own round trip to L2
     if (valid) {
-      constexpr int kStep = 4 * kTileRun;  // doubles between node rows of the same pair
-      const long long off0 = blk * (4 * NP * kTileRun) + (c >> 1) * (2 * kTileRun) + (el & 31) * 2 + (c & 1);
       const double cl = a.tile_dt ? a.cl * dtt : a.cl, cg = a.tile_dt ? a.cg * dtt : a.cg;
-      const bool need_lam = a.lam_coef != 0.0 || a.a_out;
-      const double* lam = reinterpret_cast<const double*>(a.lam) + off0;
-      const double* acc_in = reinterpret_cast<const double*>(a.acc_in) + off0;
       double* acc_out = reinterpret_cast<double*>(a.acc_out) + off0;
       double* a_out = reinterpret_cast<double*>(a.a_out) + off0;
-      double lv[NP], av[NP];
-#pragma unroll
-      for (int i = 0; i < NP; ++i) {
-        lv[i] = need_lam ? lam[i * kStep] : 0.0;
-        av[i] = a.acc_in ? acc_in[i * kStep] : 0.0;
-      }
 #pragma unroll
       for (int i = 0; i < NP; ++i) {
         const double gi = P > 0 ? g[i] + FBt[i * 8 * E] : g[i];

@@ -227,9 +227,10 @@ constexpr int kErrWords = 8;
 
 constexpr int kMaxItems = 3 * kTileElems;
 // A block of a W x H tile has W + H faces that leave the tile (12 of 8 x 4
-// cells). 26 slots are what three blocks per SM have room for at p = 3; of 64
-// consecutive elements in a row of the reference's mesh, each half has 33.
-constexpr int kSlots = 26;
+// cells). 24 slots are what the stage kernel's three blocks per SM and the
+// reverse stage's two have room for at p = 3; of 64 consecutive elements in a
+// row of the reference's mesh, each half has 33.
+constexpr int kSlots = 24;
 constexpr int kOuterWords = (2 * kSlots + 3) / 4 * 4;
 constexpr int kListCount = 2 * kMaxItems;      // byte offset of the counts
 constexpr int kListOuter = kListCount + 16;    // byte offset of the slots

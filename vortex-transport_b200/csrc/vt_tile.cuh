@@ -422,6 +422,14 @@ __device__ __forceinline__ double ld_early(const double* p) {
   return v;
 }
 
+// The same for an array that this kernel writes elsewhere (no other thread
+// writes the loaded element).
+__device__ __forceinline__ double ld_early_rw(const double* p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+  return v;
+}
+
 // The RK4 step in 12 state-vector passes. Classical RK4 (Timestepping.cpp:85-306)
 // with k_i the right-hand side at stage i's input has the stage states
 // U1 = U + dt/2 k1, U2 = U + dt/2 k2, U3 = U + dt k3, and since
