@@ -35,6 +35,12 @@ struct vt_ctx {
   std::vector<double> block;  // the stage kernel's form of it
   std::vector<double> minv_ref;  // Np x Np, for the projected initial condition
   vt::LaunchFn launch = nullptr;
+  // many steps in one launch, for a problem of few tiles (null otherwise): the
+  // kernel, the tiles' flags and what they hold (unknown after an error)
+  decltype(vt::StageKernel::resident) resident = nullptr;
+  unsigned* flags = nullptr;
+  unsigned flag_base = 0;
+  bool flags_known = false, flag_launches = false;
   int map = vt::kDefaultMap;  // warp mapping of the stage kernel
   double time = 0.0;
   vt_error_info last{};

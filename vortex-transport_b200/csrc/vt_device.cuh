@@ -281,14 +281,17 @@ enum : int { kMapComponent = 0, kMapDefault = 1, kMapFolded = 2 };
 // First-error key: (stage epoch << 40) | (((e * nfq + q) * 3 + s) * 4 + code).
 // The minimum over all failures is the failure the reference's serial loop
 // meets first: earliest stage, then element, face point, side, check.
+__device__ __forceinline__ void record_error_at(unsigned long long* err, unsigned long long epoch, int nfq, int e, int q,
+                                                int s, int code) {
+  const unsigned long long local =
+      ((static_cast<unsigned long long>(e) * nfq + q) * 3ull + s) * 4ull + code;
+  atomicMin(&err[0], (epoch << 40) | local);
+}
 __device__ __forceinline__ void record_error(const StageArgs& a, int nfq, int e, int q, int s,
                                              int code) {
   const unsigned long long steps = *(volatile unsigned long long*)&a.err[1];
   const int slot = a.stage < 4 ? a.stage : 0;
-  const unsigned long long epoch = steps * 4ull + static_cast<unsigned long long>(slot);
-  const unsigned long long local =
-      ((static_cast<unsigned long long>(e) * nfq + q) * 3ull + s) * 4ull + code;
-  atomicMin(&a.err[0], (epoch << 40) | local);
+  record_error_at(a.err, steps * 4ull + static_cast<unsigned long long>(slot), nfq, e, q, s, code);
 }
 
 // 1/x for the positive, normal x of the flux formulas (densities, Roe-average
@@ -358,9 +361,14 @@ __device__ __forceinline__ int flux_error_code(const double* uL, const double* u
 // eigenvalue test. Equal to the reference's expression up to rounding.
 // on_error is called with the reference's error code (1 left state, 2 right
 // state, 3 c2 <= 0).
-template <typename OnError>
-__device__ __forceinline__ void roe_flux2(const double* uL, const double* uR, double nx, double ny, double* f,
-                                          OnError&& on_error) {
+// In three parts, so that several points can be evaluated side by side
+// (face_points, vt_resident.cuh): the first two need no branch.
+struct RoeAverages {
+  double mn, unL, unR, pLR, rHL, rHR, du0, du1, du2, du3;  // mn: both sides' normal momentum
+  double ui, vi, Hi, q2, ucp, c2, ci, ci1, l3, s1l3, s2;
+  int usual;  // positive where |t| < 7/8 and the checked values are positive
+};
+__device__ __forceinline__ void roe_averages(const double* uL, const double* uR, double nx, double ny, RoeAverages& r) {
   const double rL = uL[0], rR = uR[0];
   const double rLR = rL * rR;
   const double y = rsqrt_nr(rLR);
@@ -368,50 +376,64 @@ __device__ __forceinline__ void roe_flux2(const double* uL, const double* uR, do
   const double irL = rR * irLR, irR = rL * irLR;
 
   const double mnL = fma(uL[1], nx, uL[2] * ny);
-  const double unL = mnL * irL;
+  r.unL = mnL * irL;
   const double pL = kGm1 * fma(-0.5, fma(uL[1], uL[1], uL[2] * uL[2]) * irL, uL[3]);
-  const double rHL = uL[3] + pL;
+  r.rHL = uL[3] + pL;
   const double mnR = fma(uR[1], nx, uR[2] * ny);
-  const double unR = mnR * irR;
+  r.unR = mnR * irR;
   const double pR = kGm1 * fma(-0.5, fma(uR[1], uR[1], uR[2] * uR[2]) * irR, uR[3]);
-  const double rHR = uR[3] + pR;
-  const double du0 = rR - rL, du1 = uR[1] - uL[1], du2 = uR[2] - uL[2], du3 = uR[3] - uL[3];
+  r.rHR = uR[3] + pR;
+  r.mn = mnL + mnR;
+  r.pLR = pL + pR;
+  r.du0 = rR - rL, r.du1 = uR[1] - uL[1], r.du2 = uR[2] - uL[2], r.du3 = uR[3] - uL[3];
 
   const double g = w * irR;  // sqrt(rhoL / rhoR)
   const double d1 = recip_nr(rL + w);
-  const double ui = fma(g, uR[1], uL[1]) * d1;
-  const double vi = fma(g, uR[2], uL[2]) * d1;
-  const double Hi = fma(g, rHR, rHL) * d1;
-  const double q2 = fma(ui, ui, vi * vi);
-  const double ucp = fma(ui, nx, vi * ny);
-  const double c2 = kGm1 * fma(-0.5, q2, Hi);
-  const double ci = c2 * c2;
-  const double ci1 = recip_nr(ci);
+  r.ui = fma(g, uR[1], uL[1]) * d1;
+  r.vi = fma(g, uR[2], uL[2]) * d1;
+  r.Hi = fma(g, r.rHR, r.rHL) * d1;
+  r.q2 = fma(r.ui, r.ui, r.vi * r.vi);
+  r.ucp = fma(r.ui, nx, r.vi * ny);
+  r.c2 = kGm1 * fma(-0.5, r.q2, r.Hi);
+  r.ci = r.c2 * r.c2;
+  r.ci1 = recip_nr(r.ci);
 
-  const double t = ucp * ci1;
-  const double l3 = fabs(t) < 0.1 ? fma(5.0 * ucp, t, 0.05 * ci) : fabs(ucp);
-  double s1l3 = ci - l3, s2 = ucp;  // (|l0| + |l1|)/2 - l3 and (|l0| - |l1|)/2
-  // positive where |t| < 7/8 and the checked values are positive
-  const int usual = min(min(min(__double2hiint(rL), __double2hiint(rR)), min(__double2hiint(pL), __double2hiint(pR))),
-                        min(__double2hiint(c2), 0x3fec0000 - (__double2hiint(t) & 0x7fffffff)));
-  if (__builtin_expect(usual <= 0, 0)) {
-    const int code = flux_error_code(uL, uR, c2);
-    if (code) on_error(code);
-    const double l0r = ucp + ci, l1r = ucp - ci, eps = 0.1 * ci;
-    const double l0 = fabs(l0r) < eps ? fma(l0r * l0r, 5.0 * ci1, 0.05 * ci) : fabs(l0r);
-    const double l1 = fabs(l1r) < eps ? fma(l1r * l1r, 5.0 * ci1, 0.05 * ci) : fabs(l1r);
-    s1l3 = fma(0.5, l0 + l1, -l3);
-    s2 = 0.5 * (l0 - l1);
-  }
-  const double G1 = (kGm1 * ci1) * fma(0.5 * q2, du0, fma(-ui, du1, fma(-vi, du2, du3)));  // over ci
-  const double G2 = fma(-ucp, du0, fma(du1, nx, du2 * ny));
-  const double C1 = fma(G1, s1l3, G2 * s2) * ci1;
-  const double C2 = fma(G1, s2, G2 * s1l3);
-  const double pC = (pL + pR) - C2;
-  f[0] = (mnL + mnR) - fma(l3, du0, C1);
-  f[1] = fma(uL[1], unL, fma(uR[1], unR, fma(pC, nx, -fma(l3, du1, C1 * ui))));
-  f[2] = fma(uL[2], unL, fma(uR[2], unR, fma(pC, ny, -fma(l3, du2, C1 * vi))));
-  f[3] = fma(rHL, unL, fma(rHR, unR, -fma(l3, du3, fma(C1, Hi, C2 * ucp))));
+  const double t = r.ucp * r.ci1;
+  r.l3 = fabs(t) < 0.1 ? fma(5.0 * r.ucp, t, 0.05 * r.ci) : fabs(r.ucp);
+  r.s1l3 = r.ci - r.l3;  // (|l0| + |l1|)/2 - l3
+  r.s2 = r.ucp;          // (|l0| - |l1|)/2
+  r.usual = min(min(min(__double2hiint(rL), __double2hiint(rR)), min(__double2hiint(pL), __double2hiint(pR))),
+                min(__double2hiint(r.c2), 0x3fec0000 - (__double2hiint(t) & 0x7fffffff)));
+}
+template <typename OnError>
+__device__ __forceinline__ void roe_unusual(const double* uL, const double* uR, RoeAverages& r, OnError&& on_error) {
+  const int code = flux_error_code(uL, uR, r.c2);
+  if (code) on_error(code);
+  const double l0r = r.ucp + r.ci, l1r = r.ucp - r.ci, eps = 0.1 * r.ci;
+  const double l0 = fabs(l0r) < eps ? fma(l0r * l0r, 5.0 * r.ci1, 0.05 * r.ci) : fabs(l0r);
+  const double l1 = fabs(l1r) < eps ? fma(l1r * l1r, 5.0 * r.ci1, 0.05 * r.ci) : fabs(l1r);
+  r.s1l3 = fma(0.5, l0 + l1, -r.l3);
+  r.s2 = 0.5 * (l0 - l1);
+}
+__device__ __forceinline__ void roe_sum(const double* uL, const double* uR, double nx, double ny, const RoeAverages& r,
+                                        double* f) {
+  const double G1 = (kGm1 * r.ci1) * fma(0.5 * r.q2, r.du0, fma(-r.ui, r.du1, fma(-r.vi, r.du2, r.du3)));  // over ci
+  const double G2 = fma(-r.ucp, r.du0, fma(r.du1, nx, r.du2 * ny));
+  const double C1 = fma(G1, r.s1l3, G2 * r.s2) * r.ci1;
+  const double C2 = fma(G1, r.s2, G2 * r.s1l3);
+  const double pC = r.pLR - C2;
+  f[0] = r.mn - fma(r.l3, r.du0, C1);
+  f[1] = fma(uL[1], r.unL, fma(uR[1], r.unR, fma(pC, nx, -fma(r.l3, r.du1, C1 * r.ui))));
+  f[2] = fma(uL[2], r.unL, fma(uR[2], r.unR, fma(pC, ny, -fma(r.l3, r.du2, C1 * r.vi))));
+  f[3] = fma(r.rHL, r.unL, fma(r.rHR, r.unR, -fma(r.l3, r.du3, fma(C1, r.Hi, C2 * r.ucp))));
+}
+template <typename OnError>
+__device__ __forceinline__ void roe_flux2(const double* uL, const double* uR, double nx, double ny, double* f,
+                                          OnError&& on_error) {
+  RoeAverages r;
+  roe_averages(uL, uR, nx, ny, r);
+  if (__builtin_expect(r.usual <= 0, 0)) roe_unusual(uL, uR, r, on_error);
+  roe_sum(uL, uR, nx, ny, r, f);
 }
 
 // Nodal Euler flux of one node's state (the formula of Timestepping.cpp:141-158)

@@ -8,6 +8,8 @@
 
 namespace vt {
 
+struct ResidentArgs;  // vt_resident.cuh
+
 // Launches a kernel that may be scheduled while the stream's previous kernel is
 // still running (let_next_start and wait_for_previous, vt_tile.cuh).
 template <typename... Params, typename... Args>
@@ -42,6 +44,11 @@ struct StageKernel {
   // Sets the dynamic shared-memory attribute on the current device and
   // reports resident blocks per SM. Call before any launch or capture.
   ConfigFn configure = nullptr;
+  // The kernel of many steps of a small problem (vt_resident.cuh): launches it
+  // for a.ntiles tiles, all resident at once; its configure reports how many
+  // fit an SM (0: it cannot run). Same form of the operators.
+  cudaError_t (*resident)(const StageArgs&, const ResidentArgs&, const double*, cudaStream_t) = nullptr;
+  ConfigFn configure_resident = nullptr;
   // The mapping it was selected for (kMapComponent or kMapDefault).
   int map = 0;
 };

@@ -24,6 +24,7 @@
 #include "vt_ctx.h"
 #include "vt_precompute.h"
 #include "vt_launch.h"
+#include "vt_resident.cuh"
 
 namespace vt {
 namespace {
@@ -316,7 +317,7 @@ void release(vt_ctx* c) {
   cudaSetDevice(c->device);
   vt::adjoint_release(c);
   void* bufs[] = {c->U,   c->A,   c->Sa, c->Sb,      c->R,   c->geo,   c->nbr,
-                  c->err, c->aos, c->W,  c->partial, c->tot, c->elem,  c->lists};
+                  c->err, c->aos, c->W,  c->partial, c->tot, c->elem,  c->lists, c->flags};
   for (void* b : bufs)
     if (b) cudaFree(b);
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -359,6 +360,49 @@ cudaError_t enqueue_rk4_step(vt_ctx* c, double dt) {
   return c->launch(stage_args(c, c->Sa, c->U, c->A, c->U, 3, 0.0, (1.0 / 6) * dt), ops, c->max_blocks, c->stream);
 }
 
+// Takes the resident kernel (vt_resident.cuh) into use where the problem has at
+// most one tile per SM. With more tiles than SMs its blocks would share an SM,
+// for which it has neither the shared memory (p = 3) nor the warps: the stage
+// kernel's three blocks per SM then hide what it saves.
+cudaError_t use_resident(vt_ctx* c, const StageKernel& k, int sms) {
+  c->resident = nullptr;
+  if (c->ntiles > sms) return cudaSuccess;
+  int per_sm = 0, coop = 0;
+  cudaError_t e = k.configure_resident(&per_sm);
+  if (!e) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device);
+  if (e || per_sm < 1 || !coop) return e;
+  if (!c->flags) e = alloc(&c->flags, sizeof(unsigned) * kFlagStride * c->ntiles);
+  if (!e) c->resident = k.resident;
+  return e;
+}
+
+// nsteps steps by the resident kernel, at most kResidentSteps a launch.
+constexpr int kResidentSteps = 1024;
+cudaError_t enqueue_resident(vt_ctx* c, double dt, int nsteps, bool euler) {
+  cudaError_t e = cudaSuccess;
+  if (!c->flags_known) {
+    e = cudaMemsetAsync(c->flags, 0, sizeof(unsigned) * kFlagStride * c->ntiles, c->stream);
+    c->flag_base = 0;
+  }
+  c->flags_known = false;  // until finish() has seen the launches end without an error
+  c->flag_launches = true;
+  for (int done = 0; done < nsteps && !e;) {
+    ResidentArgs r;
+    r.U = c->U, r.Sa = c->Sa, r.Sb = c->Sb;
+    r.flags = c->flags;
+    r.flag0 = c->flag_base;
+    r.nsteps = std::min(nsteps - done, kResidentSteps);
+    r.step0 = static_cast<unsigned long long>(done);
+    r.dt = dt;
+    r.euler = euler ? 1 : 0;
+    e = c->resident(stage_args(c, c->U, c->U, c->A, c->U, 0, 0.0, 0.0), r, c->block.data(), c->stream);
+    done += r.nsteps;
+    c->flag_base += static_cast<unsigned>(euler ? r.nsteps : 4 * r.nsteps);
+    if (euler && r.nsteps % 2) std::swap(c->U, c->Sa);
+  }
+  return e;
+}
+
 cudaError_t reset_error_words(vt_ctx* c) {
   cudaError_t e = cudaMemsetAsync(c->err, 0xFF, sizeof(unsigned long long), c->stream);
   if (e) return e;
@@ -375,6 +419,8 @@ int finish(vt_ctx* c, int nsteps, double dt) {
   c->last = vt_error_info{};
   if (words[3] & 2ull)
     return fail(VT_ERR_CUDA, "stage kernel: a bulk-copy wait gave up (the state is not valid)");
+  if (c->flag_launches) c->flags_known = true;
+  c->flag_launches = false;
   const unsigned long long key = words[0];
   if (key == ~0ull) return VT_OK;
   c->last = vt::decode_error_key(key, c->nfq);
@@ -407,6 +453,7 @@ cudaError_t from_columns(vt_ctx* c, const double2* src, double* dst) {
 
 }  // namespace vt
 
+using vt::enqueue_resident;
 using vt::enqueue_rk4_step;
 using vt::ensure_aos;
 using vt::finish;
@@ -473,6 +520,11 @@ vt_ctx* vt_create(const vt_mesh_desc* d, int device, int* status) {
     return nullptr;
   }
   c->max_blocks = sms * (per_sm > 0 ? per_sm : 1);
+  if ((e = vt::use_resident(c, sk, sms))) {
+    set(fail(VT_ERR_CUDA, vt::cuda_msg("resident kernel attributes", e)));
+    release(c);
+    return nullptr;
+  }
   c->minv_ref.assign(d->inv_mass_ref, d->inv_mass_ref + c->Np * c->Np);
 
   // packed geometry and side-ordered neighbours (Evolve.cpp:167-202), by column
@@ -601,6 +653,11 @@ vt_ctx* vt_create_structured(const vt_params* prm, const vt_vortex* ic_in, int d
     return nullptr;
   }
   c->max_blocks = sms * (per_sm > 0 ? per_sm : 1);
+  if ((e = vt::use_resident(c, sk, sms))) {
+    set(fail(VT_ERR_CUDA, vt::cuda_msg("resident kernel attributes", e)));
+    release(c);
+    return nullptr;
+  }
   c->minv_ref = minv;
   c->side_pairing = true;
   std::vector<double> m(minv), W(Np, 0.0);
@@ -737,8 +794,11 @@ int vt_download_state(vt_ctx* c, double* U, double* F) {
 static int rk4_enqueue(vt_ctx* c, double dt, int nsteps) {
   cudaError_t e = reset_error_words(c);
   if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("reset", e));
-  for (int s = 0; s < nsteps; ++s)
-    if ((e = enqueue_rk4_step(c, dt))) return fail(VT_ERR_CUDA, vt::cuda_msg("rk4 launch", e));
+  if (c->resident)
+    e = enqueue_resident(c, dt, nsteps, false);
+  else
+    for (int s = 0; s < nsteps && !e; ++s) e = enqueue_rk4_step(c, dt);
+  if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("rk4 launch", e));
   c->pending_steps += nsteps;
   c->pending_dt = dt;
   return VT_OK;
@@ -778,7 +838,8 @@ int vt_step_euler(vt_ctx* c, double dt, int nsteps) {
   cudaSetDevice(c->device);
   if (c->pending_steps) return fail(VT_ERR_INVALID, "a previous async step is not synchronised");
   cudaError_t e = reset_error_words(c);
-  for (int s = 0; s < nsteps && !e; ++s) {
+  if (c->resident && !e) e = enqueue_resident(c, dt, nsteps, true);
+  for (int s = 0; s < nsteps && !e && !c->resident; ++s) {
     // double buffer: the neighbours of an element read the old state
     e = c->launch(stage_args(c, c->U, c->U, c->A, c->Sa, vt::kStageEuler, 0.0, dt), c->block.data(),
                   c->max_blocks, c->stream);
@@ -942,6 +1003,7 @@ int vt_set_stage_mapping(vt_ctx* c, int mapping) {
   int per_sm = 0, sms = 0;
   cudaError_t e = sk.configure(&per_sm);
   if (!e) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+  if (!e) e = vt::use_resident(c, sk, sms);
   if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("vt_set_stage_mapping", e));
   c->launch = sk.launch;
   sk.pack(c->ops.data(), c->block.data());

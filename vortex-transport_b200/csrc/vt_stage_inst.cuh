@@ -6,6 +6,7 @@
 #include <cstring>
 
 #include "vt_launch.h"
+#include "vt_resident.cuh"
 #include "vt_tile.cuh"
 
 namespace vt {
@@ -46,8 +47,37 @@ cudaError_t launch_stage(const StageArgs& a, const double* block, int max_blocks
 }
 
 template <int P, int NFQ, int MAP>
+cudaError_t configure_resident(int* blocks_per_sm) {
+  constexpr int bytes = ResidentLayout<P, NFQ>::kBytes;
+  *blocks_per_sm = 0;
+  if (bytes > 227 * 1024) return cudaSuccess;  // more than a block may have
+  const cudaError_t e = cudaFuncSetAttribute(resident_steps_kernel<P, NFQ, MAP>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e) return e;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, resident_steps_kernel<P, NFQ, MAP>,
+                                                       4 * kTileElems, bytes);
+}
+
+template <int P, int NFQ, int MAP>
+cudaError_t launch_resident(const StageArgs& a, const ResidentArgs& r, const double* block, cudaStream_t st) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeCooperative;
+  attr.val.cooperative = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(a.ntiles));
+  cfg.blockDim = dim3(4 * kTileElems);
+  cfg.dynamicSmemBytes = ResidentLayout<P, NFQ>::kBytes;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, resident_steps_kernel<P, NFQ, MAP>, a, r,
+                            *reinterpret_cast<const OpsOf<P, NFQ, MAP>*>(block));
+}
+
+template <int P, int NFQ, int MAP>
 StageKernel kernel_of() {
-  return StageKernel{launch_stage<P, NFQ, MAP>, pack_operators<P, NFQ, MAP>, configure_stage<P, NFQ, MAP>};
+  return StageKernel{launch_stage<P, NFQ, MAP>, pack_operators<P, NFQ, MAP>, configure_stage<P, NFQ, MAP>,
+                     launch_resident<P, NFQ, MAP>, configure_resident<P, NFQ, MAP>};
 }
 
 template <int P, int MAP>

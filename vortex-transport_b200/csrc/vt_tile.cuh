@@ -408,6 +408,25 @@ __device__ __forceinline__ void unfold(double* r) {
   for (int i = 0; i < NP; ++i) r[i] = v[i];
 }
 
+// The nodal flux as the unfolded volume operator reads it: rows j*4 + h xi,
+// j*4 + 2 + h eta (component pair h). A thread takes every fourth node.
+template <int P>
+__device__ __forceinline__ void plain_nodal_flux(const double2* S, double2* G2, int el, int grp, double2 j0,
+                                                 double2 j1) {
+  constexpr int NP = np_of_p(P), ES = kTileElems;
+  for (int j = grp; j < NP; j += 4) {
+    const double2 s0 = S[sidx<NP>(2 * j, el)], s1 = S[sidx<NP>(2 * j + 1, el)];
+    const double sv[4] = {s0.x, s0.y, s1.x, s1.y};
+    double gxi[4], geta[4];
+    contravariant_flux(sv, j0.x, j0.y, j1.x, j1.y, gxi, geta);
+    double2* g = G2 + j * 4 * ES + el;
+    g[0] = make_double2(gxi[0], gxi[1]);
+    g[ES] = make_double2(gxi[2], gxi[3]);
+    g[2 * ES] = make_double2(geta[0], geta[1]);
+    g[3 * ES] = make_double2(geta[2], geta[3]);
+  }
+}
+
 // Non-coherent loads issued where they are written, so that the stage
 // update's first operand is in flight during the volume phase (the compiler
 // would otherwise sink them to their use), and so that stage 1's re-read of
@@ -659,21 +678,8 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
     if (P > 0) {
       const double2* ge = GE + which * kGeoRows * kTileRun + lane;
       const double2 j0 = ge[0], j1 = ge[kTileRun];
-      if constexpr (FOLD) {
-        folded_nodal_flux<P>(S, FB2, col, grp, j0, j1);
-      } else {
-        for (int j = grp; j < NP; j += 4) {  // rows j*4 + 0..1 xi pairs, 2..3 eta pairs
-          const double2 s0 = S[sidx<NP>(2 * j, col)], s1 = S[sidx<NP>(2 * j + 1, col)];
-          const double sv[4] = {s0.x, s0.y, s1.x, s1.y};
-          double gxi[4], geta[4];
-          contravariant_flux(sv, j0.x, j0.y, j1.x, j1.y, gxi, geta);
-          double2* g = FB2 + j * 4 * E + col;
-          g[0] = make_double2(gxi[0], gxi[1]);
-          g[E] = make_double2(gxi[2], gxi[3]);
-          g[2 * E] = make_double2(geta[0], geta[1]);
-          g[3 * E] = make_double2(geta[2], geta[3]);
-        }
-      }
+      if constexpr (FOLD) folded_nodal_flux<P>(S, FB2, col, grp, j0, j1);
+      else plain_nodal_flux<P>(S, FB2, col, grp, j0, j1);
     }
     run_sync(t);
 
