@@ -30,6 +30,7 @@
 #include "vt_checkpoint.h"
 #include "vt_common.h"
 #include "vt_ctx.h"
+#include "vt_jvp_tile.cuh"
 
 namespace vt {
 namespace {
@@ -37,13 +38,10 @@ namespace {
 using FaceFn = cudaError_t (*)(const AdjArgs&, const double*, cudaStream_t);
 using TileFn = cudaError_t (*)(const AdjArgs&, const double*, int, cudaStream_t);
 using TileConfigFn = cudaError_t (*)(int*);
-using JvpFn = cudaError_t (*)(const double2*, const double2*, double2*, const double2*, const int4*, const int*,
-                              long long, const double*, cudaStream_t);
 
 struct AdjKernels {
   FaceFn face = nullptr;
   FaceFn element = nullptr;
-  JvpFn jvp = nullptr;
   TileFn tile = nullptr;
   TileConfigFn tile_config = nullptr;
   std::vector<double> (*tile_pack)(const double*) = nullptr;
@@ -96,17 +94,8 @@ cudaError_t configure_tile(int* blocks_per_sm) {
 }
 
 template <int P, int NFQ>
-cudaError_t launch_jvp(const double2* U, const double2* V, double2* dR, const double2* geo, const int4* nbr,
-                       const int* elem, long long ncols, const double* ops, cudaStream_t st) {
-  StageOps<P, NFQ> o;
-  std::memcpy(&o, ops, sizeof(o));
-  rhs_jvp_kernel<P, NFQ><<<static_cast<unsigned>((ncols + 127) / 128), 128, 0, st>>>(U, V, dR, geo, nbr, elem, ncols, o);
-  return cudaGetLastError();
-}
-
-template <int P, int NFQ>
 AdjKernels kernels_of() {
-  return AdjKernels{launch_face<P, NFQ>, launch_element<P, NFQ>, launch_jvp<P, NFQ>, launch_tile<P, NFQ>,
+  return AdjKernels{launch_face<P, NFQ>, launch_element<P, NFQ>, launch_tile<P, NFQ>,
                     configure_tile<P, NFQ>, pack_tile<P, NFQ>};
 }
 
@@ -494,11 +483,22 @@ cudaError_t store_aos(vt_ctx* c, const double2* src, double* dst, int device_poi
   return e;
 }
 
-cudaError_t lincomb(vt_ctx* c, double2* out, const double2* x, double cx, const double2* y, double cy,
-                    const double2* z = nullptr, double cz = 0.0) {
-  const long long n = static_cast<long long>(c->adj->state_elems);
-  lincomb_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, c->stream>>>(out, x, cx, y, cy, z, cz, n);
-  return cudaGetLastError();
+// out1 = x1 + c1 dk, out2 = x2 + c2 dk with dk = R'(U) V (JvpArgs).
+cudaError_t jvp(vt_ctx* c, const double2* U, const double2* V, double2* out1, const double2* x1 = nullptr, double c1 = 0.0,
+                double2* out2 = nullptr, const double2* x2 = nullptr, double c2 = 0.0) {
+  const StageKernel k = select_kernel(c->p, c->nfq, c->ops.data(), c->map);
+  int per_sm = 0, sms = 0;
+  cudaError_t e = k.configure_jvp(&per_sm);
+  if (!e) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+  if (e) return e;
+  JvpArgs j;
+  j.U = U, j.V = V;
+  j.x1 = x1, j.x2 = x2;
+  j.out1 = out1, j.out2 = out2;
+  j.c1 = c1, j.c2 = c2;
+  StageArgs a = stage_args(c, U, U, c->A, out1, kStageRhs, 0.0, 0.0);
+  a.test_flags = 0;  // the test hook is the stage kernel's
+  return k.jvp(a, j, c->block.data(), sms * std::max(1, per_sm), c->stream);
 }
 
 int prepare(vt_ctx* c) {
@@ -631,10 +631,11 @@ int vt_rhs_jvp(vt_ctx* c, const double* U, const double* V, double* dR, int devi
   s->fresh = false;
   cudaError_t e = vt::load_aos(c, U, device_pointers, s->s1);
   if (!e) e = vt::load_aos(c, V, device_pointers, s->s2);
-  if (!e) e = s->k.jvp(s->s1, s->s2, s->s3, c->geo, c->nbr, c->elem, c->ncols, c->ops.data(), c->stream);
+  if (!e) e = vt::reset_error_words(c);
+  if (!e) e = vt::jvp(c, s->s1, s->s2, s->s3);
   if (!e) e = vt::store_aos(c, s->s3, dR, device_pointers);
-  if (!e) e = cudaStreamSynchronize(c->stream);
-  return e ? fail(VT_ERR_CUDA, vt::cuda_msg("rhs jvp", e)) : VT_OK;
+  if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("rhs jvp", e));
+  return vt::finish(c, 0, 0.0);
 }
 
 int vt_rhs_vjp(vt_ctx* c, const double* U, const double* W, double* G, int device_pointers) {
@@ -671,25 +672,18 @@ int vt_tangent_rk4(vt_ctx* c, double dt, int nsteps, const double* dU_0, double*
   if (st) return st;
   vt::AdjointState* s = c->adj;
   s->fresh = false;
-  double2 *dX = s->a0, *dS = s->a1, *dacc = s->acc, *dk = s->lam;
+  double2 *dX = s->a0, *dS = s->a1, *dacc = s->acc, *dT = s->lam;
   const double2* X = c->U;
-  auto jvp = [&](const double2* at, const double2* v) {
-    return s->k.jvp(at, v, dk, c->geo, c->nbr, c->elem, c->ncols, c->ops.data(), c->stream);
-  };
   cudaError_t e = vt::load_aos(c, dU_0, device_pointers, dX);
   if (!e) e = vt::reset_error_words(c);
   for (int n = 0; n < nsteps && !e; ++n) {
+    // the stage directions alternate between dS and dT: a launch must not
+    // overwrite the direction whose neighbours its own tiles still read
     if ((e = vt::stage_step(c, X, dt, nullptr))) break;
-    if ((e = jvp(X, dX)) || (e = vt::lincomb(c, dacc, dX, 1.0, dk, (1.0 / 6) * dt)) ||
-        (e = vt::lincomb(c, dS, dX, 1.0, dk, 0.5 * dt)))
-      break;
-    if ((e = jvp(s->s1, dS)) || (e = vt::lincomb(c, dacc, dacc, 1.0, dk, (1.0 / 3) * dt)) ||
-        (e = vt::lincomb(c, dS, dX, 1.0, dk, 0.5 * dt)))
-      break;
-    if ((e = jvp(s->s2, dS)) || (e = vt::lincomb(c, dacc, dacc, 1.0, dk, (1.0 / 3) * dt)) ||
-        (e = vt::lincomb(c, dS, dX, 1.0, dk, dt)))
-      break;
-    if ((e = jvp(s->s3, dS)) || (e = vt::lincomb(c, dX, dacc, 1.0, dk, (1.0 / 6) * dt))) break;
+    if ((e = vt::jvp(c, X, dX, dacc, dX, (1.0 / 6) * dt, dS, dX, 0.5 * dt))) break;
+    if ((e = vt::jvp(c, s->s1, dS, dacc, dacc, (1.0 / 3) * dt, dT, dX, 0.5 * dt))) break;
+    if ((e = vt::jvp(c, s->s2, dT, dacc, dacc, (1.0 / 3) * dt, dS, dX, dt))) break;
+    if ((e = vt::jvp(c, s->s3, dS, dX, dacc, (1.0 / 6) * dt))) break;
     e = vt::stage(c, s->s3, X, c->U, 3, 0.0, (1.0 / 6) * dt, c->stream);
   }
   if (!e) e = vt::store_aos(c, dX, dU_T, device_pointers);

@@ -7,10 +7,11 @@
 //                        speed" and the entropy fix (Numericalflux.cpp:99-156);
 //   contravariant_vjp    reverse sweep of contravariant_flux (the nodal Euler
 //                        flux of Timestepping.cpp:141-158 contracted with J^-1);
-//   Dual<N>, roe_flux_t,
-//   contravariant_flux_t forward-mode versions of the same formulas on dual
-//                        numbers, for the tangent-linear model and as the
-//                        independent check of the reverse sweeps.
+//   roe_flux2_jvp,
+//   contravariant_jvp    their derivatives along a direction, for the
+//                        tangent-linear model;
+//   Dual<N>, roe_flux_t  the flux on dual numbers, the independent check of
+//                        both (on the host).
 //
 // All functions are __host__ __device__ so the reverse sweeps can be checked
 // against the dual-number Jacobians on the CPU.
@@ -170,21 +171,6 @@ __host__ __device__ inline int roe_flux_t(const T* uL, const T* uR, double nx, d
   return code;
 }
 
-template <typename T>
-__host__ __device__ inline void contravariant_flux_t(const T* s, double j00, double j01, double j10,
-                                                     double j11, T* gxi, T* geta) {
-  const T ir = 1.0 / s[0];
-  const T vx = s[1] * ir, vy = s[2] * ir;
-  const T p = kGm1 * (s[3] - 0.5 * (s[1] * vx + s[2] * vy));
-  const T rH = s[3] + p;
-  const T fx[4] = {s[1], s[1] * vx + p, s[2] * vx, rH * vx};
-  const T fy[4] = {s[2], s[1] * vy, s[2] * vy + p, rH * vy};
-  for (int c = 0; c < 4; ++c) {
-    gxi[c] = j00 * fx[c] + j01 * fy[c];
-    geta[c] = j10 * fx[c] + j11 * fy[c];
-  }
-}
-
 // ---- reverse sweeps ------------------------------------------------------------------
 // b: adjoint of roe_flux2's doubled flux (4); writes the adjoints of uL and uR
 // to buL, buR. The reverse sweep of roe_flux2's own arrangement: about 190 FP64
@@ -302,6 +288,93 @@ __host__ __device__ inline void roe_flux2_vjp(const double* uL, const double* uR
   buR[1] = cR * nx + b[1] * unR + g * ai - mR * uR[1] + b_du1;
   buR[2] = cR * ny + b[2] * unR + g * av - mR * uR[2] + b_du2;
   buR[3] = rhR + tR + b_du3;
+}
+
+// Derivative of roe_flux2's doubled flux along (dL, dR), in the same
+// arrangement (names as in roe_flux2_vjp; d... are derivatives).
+__host__ __device__ inline void roe_flux2_jvp(const double* uL, const double* uR, double nx, double ny, const double* dL,
+                                              const double* dR, double* df) {
+  const double rL = uL[0], rR = uR[0];
+  const double rLR = rL * rR;
+  const double y = rsq(rLR);
+  const double irLR = y * y, w = rLR * y;
+  const double irL = rR * irLR, irR = rL * irLR;
+  const double unL = (uL[1] * nx + uL[2] * ny) * irL, unR = (uR[1] * nx + uR[2] * ny) * irR;
+  const double kinL = (uL[1] * uL[1] + uL[2] * uL[2]) * irL, kinR = (uR[1] * uR[1] + uR[2] * uR[2]) * irR;
+  const double rHL = uL[3] + kGm1 * (uL[3] - 0.5 * kinL), rHR = uR[3] + kGm1 * (uR[3] - 0.5 * kinR);
+  const double dmL = dL[1] * nx + dL[2] * ny, dmR = dR[1] * nx + dR[2] * ny;
+  const double dunL = (dmL - unL * dL[0]) * irL, dunR = (dmR - unR * dR[0]) * irR;
+  const double dpL = kGm1 * (dL[3] - (uL[1] * dL[1] + uL[2] * dL[2] - 0.5 * kinL * dL[0]) * irL);
+  const double dpR = kGm1 * (dR[3] - (uR[1] * dR[1] + uR[2] * dR[2] - 0.5 * kinR * dR[0]) * irR);
+  const double drHL = dL[3] + dpL, drHR = dR[3] + dpR;
+  const double du0 = rR - rL, du1 = uR[1] - uL[1], du2 = uR[2] - uL[2], du3 = uR[3] - uL[3];
+  const double e0 = dR[0] - dL[0], e1 = dR[1] - dL[1], e2 = dR[2] - dL[2], e3 = dR[3] - dL[3];
+  // averages
+  const double g = w * irR, d1 = rcp(rL + w);
+  const double lL = 0.5 * dL[0] * irL, lR = 0.5 * dR[0] * irR;  // halved logarithmic derivatives of the densities
+  const double dg = g * (lL - lR), ds = dL[0] + w * (lL + lR);
+  const double ui = (g * uR[1] + uL[1]) * d1, vi = (g * uR[2] + uL[2]) * d1, Hi = (g * rHR + rHL) * d1;
+  const double dui = (dg * uR[1] + g * dR[1] + dL[1] - ui * ds) * d1;
+  const double dvi = (dg * uR[2] + g * dR[2] + dL[2] - vi * ds) * d1;
+  const double dHi = (dg * rHR + g * drHR + drHL - Hi * ds) * d1;
+  const double h = 0.5 * (ui * ui + vi * vi), dh = ui * dui + vi * dvi;
+  const double ucp = ui * nx + vi * ny, ducp = dui * nx + dvi * ny;
+  const double c2 = kGm1 * (Hi - h), ci = c2 * c2, dci = 2.0 * c2 * kGm1 * (dHi - dh);
+  const double ci1 = rcp(ci);
+  const double t = ucp * ci1;
+  const bool fix = fabs(t) < 0.1;
+  const double l3 = fix ? 5.0 * ucp * t + 0.05 * ci : fabs(ucp);
+  const double dl3 = fix ? 10.0 * t * ducp + (0.05 - 5.0 * t * t) * dci : (ucp < 0 ? -ducp : ducp);
+  double s1 = ci, s2 = ucp, ds1 = dci, ds2 = ducp;
+  if (!(fabs(t) < 0.875)) {
+    const double l0r = ucp + ci, l1r = ucp - ci, eps = 0.1 * ci;
+    double l0 = fabs(l0r), l1 = fabs(l1r);
+    double dl0 = l0r < 0 ? -(ducp + dci) : ducp + dci, dl1 = l1r < 0 ? dci - ducp : ducp - dci;
+    if (l0 < eps) {
+      const double z = l0r * ci1;
+      l0 = 5.0 * l0r * z + 0.05 * ci, dl0 = 10.0 * z * (ducp + dci) + (0.05 - 5.0 * z * z) * dci;
+    }
+    if (l1 < eps) {
+      const double z = l1r * ci1;
+      l1 = 5.0 * l1r * z + 0.05 * ci, dl1 = 10.0 * z * (ducp - dci) + (0.05 - 5.0 * z * z) * dci;
+    }
+    s1 = 0.5 * (l0 + l1), s2 = 0.5 * (l0 - l1);
+    ds1 = 0.5 * (dl0 + dl1), ds2 = 0.5 * (dl0 - dl1);
+  }
+  const double S = s1 - l3, dS = ds1 - dl3, k1 = kGm1 * ci1;
+  const double G1 = k1 * (h * du0 - ui * du1 - vi * du2 + du3);
+  const double dG1 = k1 * (dh * du0 + h * e0 - dui * du1 - ui * e1 - dvi * du2 - vi * e2 + e3) - G1 * ci1 * dci;
+  const double G2 = du1 * nx + du2 * ny - ucp * du0, dG2 = e1 * nx + e2 * ny - ducp * du0 - ucp * e0;
+  const double C1 = (G1 * S + G2 * s2) * ci1;
+  const double dC1 = (dG1 * S + G1 * dS + dG2 * s2 + G2 * ds2 - C1 * dci) * ci1;
+  const double C2 = G1 * s2 + G2 * S, dC2 = dG1 * s2 + G1 * ds2 + dG2 * S + G2 * dS;
+  const double dp = dpL + dpR - dC2;
+  df[0] = dmL + dmR - dl3 * du0 - l3 * e0 - dC1;
+  df[1] = dL[1] * unL + uL[1] * dunL + dR[1] * unR + uR[1] * dunR + dp * nx - dl3 * du1 - l3 * e1 - dC1 * ui - C1 * dui;
+  df[2] = dL[2] * unL + uL[2] * dunL + dR[2] * unR + uR[2] * dunR + dp * ny - dl3 * du2 - l3 * e2 - dC1 * vi - C1 * dvi;
+  df[3] = drHL * unL + rHL * dunL + drHR * unR + rHR * dunR - dl3 * du3 - l3 * e3 - dC1 * Hi - C1 * dHi - dC2 * ucp -
+          C2 * ducp;
+}
+
+// Derivative of the contravariant flux of a node's state s along d.
+__host__ __device__ inline void contravariant_jvp(const double* s, const double* d, double j00, double j01, double j10,
+                                                  double j11, double* dgxi, double* dgeta) {
+  const double ir = rcp(s[0]);
+  const double vx = s[1] * ir, vy = s[2] * ir;
+  const double dvx = (d[1] - vx * d[0]) * ir, dvy = (d[2] - vy * d[0]) * ir;
+  const double rH = s[3] + kGm1 * (s[3] - 0.5 * (s[1] * vx + s[2] * vy));
+  const double dp = kGm1 * (d[3] - 0.5 * (d[1] * vx + d[2] * vy + s[1] * dvx + s[2] * dvy));
+  const double drH = d[3] + dp;
+  const double vxi = j00 * vx + j01 * vy, veta = j10 * vx + j11 * vy;
+  const double dvxi = j00 * dvx + j01 * dvy, dveta = j10 * dvx + j11 * dvy;
+  dgxi[0] = j00 * d[1] + j01 * d[2];
+  dgxi[1] = d[1] * vxi + s[1] * dvxi + j00 * dp;
+  dgxi[2] = d[2] * vxi + s[2] * dvxi + j01 * dp;
+  dgxi[3] = drH * vxi + rH * dvxi;
+  dgeta[0] = j10 * d[1] + j11 * d[2];
+  dgeta[1] = d[1] * veta + s[1] * dveta + j10 * dp;
+  dgeta[2] = d[2] * veta + s[2] * dveta + j11 * dp;
+  dgeta[3] = drH * veta + rH * dveta;
 }
 
 // bf: adjoint of the flux itself (4). Adds the adjoints of uL and uR to buL, buR.

@@ -1,4 +1,4 @@
-// Kernels of the discrete adjoint and the tangent-linear model.
+// Kernels of the discrete adjoint on meshes or operators without the fused form.
 //
 // One reverse RK4 stage (the transpose of one stage's right-hand side at the
 // stage state U, applied to the stage adjoint a) is two launches:
@@ -210,99 +210,6 @@ __global__ void __launch_bounds__(kAdjRun * np_of_p(P), 3)
   }
   a.acc_out[r0] = make_double2(acc[0], acc[1]);
   a.acc_out[r1] = make_double2(acc[2], acc[3]);
-}
-
-// dR = R'(U) V for all elements, one thread per element, on dual numbers:
-// the right-hand side restated element by element (volume, traces, Roe flux,
-// lift) with every quantity carrying its derivative along V.
-template <int P, int NFQ>
-__global__ void __launch_bounds__(128)
-    rhs_jvp_kernel(const double2* __restrict__ U, const double2* __restrict__ V, double2* __restrict__ dR,
-                   const double2* __restrict__ geo, const int4* __restrict__ nbr, const int* __restrict__ elem,
-                   long long ncols, const StageOps<P, NFQ> o) {
-  constexpr int NP = np_of_p(P), NE = P + 1;
-  using D1 = Dual<1>;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ncols || elem[e] < 0) return;
-  D1 u[NP][4], r[NP][4];
-  for (int i = 0; i < NP; ++i) {
-    const long long r0 = state_index(NP, e, 2 * i), r1 = r0 + kTileRun;
-    const double2 x0 = U[r0], x1 = U[r1], v0 = V[r0], v1 = V[r1];
-    const double xs[4] = {x0.x, x0.y, x1.x, x1.y}, vs[4] = {v0.x, v0.y, v1.x, v1.y};
-    for (int c = 0; c < 4; ++c) {
-      u[i][c] = D1(xs[c]);
-      u[i][c].d[0] = vs[c];
-      r[i][c] = D1(0.0);
-    }
-  }
-  if (P > 0) {
-    const double2 j0 = geo[geo_index(e, 0)], j1 = geo[geo_index(e, 1)];
-    for (int j = 0; j < NP; ++j) {
-      D1 gxi[4], geta[4];
-      contravariant_flux_t(u[j], j0.x, j0.y, j1.x, j1.y, gxi, geta);
-      for (int i = 0; i < NP; ++i)
-        for (int c = 0; c < 4; ++c) r[i][c] = r[i][c] + (o.D[0][i][j] * gxi[c] + o.D[1][i][j] * geta[c]);
-    }
-  }
-  const int4 nb4 = nbr[e];
-  const double2 lsa = geo[geo_index(e, 2)], lsb = geo[geo_index(e, 3)];
-  for (int s = 0; s < 3; ++s) {
-    const int nb = s == 0 ? nb4.x : (s == 1 ? nb4.y : nb4.z);
-    const double ls = s == 0 ? lsa.x : (s == 1 ? lsa.y : lsb.x);
-    const double2 n = geo[geo_index(e, 4 + s)];
-    D1 un[NE][4];
-    for (int k = 0; k < NE; ++k) {
-      const int node = edge_node(P, s, k);
-      const long long r0 = state_index(NP, nb, 2 * node), r1 = r0 + kTileRun;
-      const double2 x0 = U[r0], x1 = U[r1], v0 = V[r0], v1 = V[r1];
-      const double xs[4] = {x0.x, x0.y, x1.x, x1.y}, vs[4] = {v0.x, v0.y, v1.x, v1.y};
-      for (int c = 0; c < 4; ++c) {
-        un[k][c] = D1(xs[c]);
-        un[k][c].d[0] = vs[c];
-      }
-    }
-    for (int q = 0; q < NFQ; ++q) {
-      D1 up[4], um[4], f[4];
-      for (int k = 0; k < NE; ++k) {
-        const int node = edge_node(P, s, k);
-        for (int c = 0; c < 4; ++c) {
-          up[c] = up[c] + o.tp[s][q][k] * u[node][c];
-          um[c] = um[c] + o.tm[s][q][k] * un[k][c];
-        }
-      }
-      roe_flux_t(up, um, n.x, n.y, f);
-      for (int i = 0; i < NP; ++i)
-        for (int c = 0; c < 4; ++c) r[i][c] = r[i][c] - o.lift[s][i][q] * (ls * f[c]);
-    }
-  }
-  for (int i = 0; i < NP; ++i) {
-    dR[state_index(NP, e, 2 * i)] = make_double2(r[i][0].d[0], r[i][1].d[0]);
-    dR[state_index(NP, e, 2 * i + 1)] = make_double2(r[i][2].d[0], r[i][3].d[0]);
-  }
-}
-
-// out = cx x + cy y + cz z over n double2 entries (null operands are skipped).
-__global__ void lincomb_kernel(double2* out, const double2* x, double cx, const double2* y, double cy,
-                               const double2* z, double cz, long long n) {
-  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double2 r = make_double2(0.0, 0.0);
-  if (x) {
-    const double2 v = x[i];
-    r.x = cx * v.x;
-    r.y = cx * v.y;
-  }
-  if (y) {
-    const double2 v = y[i];
-    r.x = fma(cy, v.x, r.x);
-    r.y = fma(cy, v.y, r.y);
-  }
-  if (z) {
-    const double2 v = z[i];
-    r.x = fma(cz, v.x, r.x);
-    r.y = fma(cz, v.y, r.y);
-  }
-  out[i] = r;
 }
 
 }  // namespace vt

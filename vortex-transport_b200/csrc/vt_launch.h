@@ -9,6 +9,7 @@
 namespace vt {
 
 struct ResidentArgs;  // vt_resident.cuh
+struct JvpArgs;       // vt_jvp_tile.cuh
 
 // Launches a kernel that may be scheduled while the stream's previous kernel is
 // still running (let_next_start and wait_for_previous, vt_tile.cuh).
@@ -49,6 +50,10 @@ struct StageKernel {
   // fit an SM (0: it cannot run). Same form of the operators.
   cudaError_t (*resident)(const StageArgs&, const ResidentArgs&, const double*, cudaStream_t) = nullptr;
   ConfigFn configure_resident = nullptr;
+  // The derivative of a stage along a direction (vt_jvp_tile.cuh), at most
+  // `max_blocks` blocks. Same form of the operators.
+  cudaError_t (*jvp)(const StageArgs&, const JvpArgs&, const double*, int, cudaStream_t) = nullptr;
+  ConfigFn configure_jvp = nullptr;
   // The mapping it was selected for (kMapComponent or kMapDefault).
   int map = 0;
 };

@@ -5,6 +5,7 @@
 
 #include <cstring>
 
+#include "vt_jvp_tile.cuh"
 #include "vt_launch.h"
 #include "vt_resident.cuh"
 #include "vt_tile.cuh"
@@ -75,9 +76,28 @@ cudaError_t launch_resident(const StageArgs& a, const ResidentArgs& r, const dou
 }
 
 template <int P, int NFQ, int MAP>
+cudaError_t configure_jvp(int* blocks_per_sm) {
+  constexpr int bytes = JvpLayout<P, NFQ>::kBytes;
+  static_assert(bytes <= 227 * 1024, "one block per SM");
+  const cudaError_t e = cudaFuncSetAttribute(jvp_tile_kernel<P, NFQ, MAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             bytes);
+  if (e) return e;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, jvp_tile_kernel<P, NFQ, MAP>, 4 * kTileElems,
+                                                       bytes);
+}
+
+template <int P, int NFQ, int MAP>
+cudaError_t launch_jvp(const StageArgs& a, const JvpArgs& j, const double* block, int max_blocks, cudaStream_t st) {
+  const int grid = a.ntiles < max_blocks ? a.ntiles : max_blocks;
+  return launch_dependent(jvp_tile_kernel<P, NFQ, MAP>, grid, 4 * kTileElems, JvpLayout<P, NFQ>::kBytes, st, a, j,
+                          *reinterpret_cast<const OpsOf<P, NFQ, MAP>*>(block));
+}
+
+template <int P, int NFQ, int MAP>
 StageKernel kernel_of() {
   return StageKernel{launch_stage<P, NFQ, MAP>, pack_operators<P, NFQ, MAP>, configure_stage<P, NFQ, MAP>,
-                     launch_resident<P, NFQ, MAP>, configure_resident<P, NFQ, MAP>};
+                     launch_resident<P, NFQ, MAP>, configure_resident<P, NFQ, MAP>,
+                     launch_jvp<P, NFQ, MAP>, configure_jvp<P, NFQ, MAP>};
 }
 
 template <int P, int MAP>

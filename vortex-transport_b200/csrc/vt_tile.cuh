@@ -331,19 +331,13 @@ __device__ __forceinline__ void folded_state(const double2* S, int el, int c, do
   }
 }
 
-// The nodal flux in the form that the folded volume operator reads: for node j
+// Nodal fluxes in the form that the folded volume operator reads: for node j
 // with mirror image Pj, rows j*4 + h hold Gxi_j + Geta_Pj and rows j*4 + 2 + h
 // Gxi_j - Geta_Pj (component pair h). A thread takes both nodes of a pair, or
-// one fixed node, of element el.
-template <int P>
-__device__ __forceinline__ void folded_nodal_flux(const double2* S, double2* G2, int el, int grp, double2 j0,
-                                                  double2 j1) {
-  constexpr int NP = np_of_p(P), ES = kTileElems, NS = fold_nodes(P), NO = fold_pairs(P);
-  auto flux = [&](int j, double* gxi, double* geta) {
-    const double2 s0 = S[sidx<NP>(2 * j, el)], s1 = S[sidx<NP>(2 * j + 1, el)];
-    const double sv[4] = {s0.x, s0.y, s1.x, s1.y};
-    contravariant_flux(sv, j0.x, j0.y, j1.x, j1.y, gxi, geta);
-  };
+// one fixed node, of column el; flux(j, gxi, geta) is node j's.
+template <int P, typename Flux>
+__device__ __forceinline__ void folded_flux_rows(double2* G2, int el, int grp, Flux&& flux) {
+  constexpr int ES = kTileElems, NS = fold_nodes(P), NO = fold_pairs(P);
   auto store = [&](int j, const double* gxi, const double* geta) {
     double2* g = G2 + j * 4 * ES + el;
     g[0] = make_double2(gxi[0] + geta[0], gxi[1] + geta[1]);
@@ -374,6 +368,17 @@ __device__ __forceinline__ void folded_nodal_flux(const double2* S, double2* G2,
       store(j, gxi, geta);
     }
   }
+}
+
+template <int P>
+__device__ __forceinline__ void folded_nodal_flux(const double2* S, double2* G2, int el, int grp, double2 j0,
+                                                  double2 j1) {
+  constexpr int NP = np_of_p(P);
+  folded_flux_rows<P>(G2, el, grp, [&](int j, double* gxi, double* geta) {
+    const double2 s0 = S[sidx<NP>(2 * j, el)], s1 = S[sidx<NP>(2 * j + 1, el)];
+    const double sv[4] = {s0.x, s0.y, s1.x, s1.y};
+    contravariant_flux(sv, j0.x, j0.y, j1.x, j1.y, gxi, geta);
+  });
 }
 
 template <int P, int NFQ>
