@@ -223,6 +223,12 @@ int upload_dt(vt_batch* b) {
   return VT_OK;
 }
 
+size_t instance_offset(const vt_batch* b, int i) {  // in an array of all instances in order (doubles)
+  size_t off = 0;
+  for (int k = 0; k < i; ++k) off += 4 * static_cast<size_t>(b->K_of[k]) * b->groups[b->group_of[k]].Np;
+  return off;
+}
+
 // A vt_ctx over a group's buffers (not owning them), so the single-problem
 // adjoint runs on the group's ragged element array: one launch per stage for
 // all its instances. The group's tiles and face lists are the ones the batch
@@ -239,7 +245,8 @@ int ensure_views(vt_batch* b) {
     c->K = static_cast<int>(G.K);
     c->ncols = G.ncols;
     for (size_t m = 0; m < G.members.size(); ++m)
-      c->parts.push_back({G.num[m], static_cast<long long>(vt::kTileElems) * G.tile_begin[m], G.offset[m]});
+      c->parts.push_back({G.num[m], static_cast<long long>(vt::kTileElems) * G.tile_begin[m], 4ll * G.Np * G.offset[m],
+                          static_cast<long long>(instance_offset(b, G.members[m]))});
     c->max_blocks = G.max_blocks;
     c->stream = b->stream;
     c->U = G.U;
@@ -576,7 +583,18 @@ static int batch_backward(vt_batch* b, const double* dJdU_T, double* dJdU_0, int
   for (size_t gi = 0; gi < b->groups.size(); ++gi) {
     vt::Group& G = b->groups[gi];
     const size_t per = 4 * static_cast<size_t>(G.Np);
-    if (device_pointers) {
+    if (device_pointers && vt::aligned_to(dJdU_T, 16) && vt::aligned_to(dJdU_0, 16)) {
+      // Every instance straight from and to its place in the caller's arrays.
+      // Twelve instances of 64 x 64 cells at p = 2, 20 steps forward and back:
+      // 9.7 ms, where gathering the group into an array allocated for the call,
+      // and scattering from it, gave 10.7 to 14.7 ms with the allocator's mood.
+      b->views[gi]->all_instances = true;
+      const int st = vt_adjoint_backward(b->views[gi], dJdU_T, dJdU_0, 1);
+      b->views[gi]->all_instances = false;
+      if (st) return st;
+      continue;
+    }
+    if (device_pointers) {  // arrays of 8-byte alignment, which the kernels cannot read as pairs
       // group-order device buffers: the view's staging array and a scratch copy
       double *din = nullptr, *dout = nullptr;
       cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&din), 2 * sizeof(double) * per * G.K);

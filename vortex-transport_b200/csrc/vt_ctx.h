@@ -50,13 +50,17 @@ struct vt_ctx {
   // Per-tile time steps (a batch group's view; null otherwise): stage and
   // adjoint coefficients are then fractions scaled on the device.
   const double* tile_dt = nullptr;
-  // A batch group's view: the numbering of each instance, at its first column
-  // and its first element (else empty: num numbers everything).
+  // A batch group's view: the numbering of each instance, at its first column,
+  // and where its block starts in a caller's array (doubles), when that holds
+  // the group's instances in order (`at`) or all instances of the batch in
+  // order (`at_all`, used while `all_instances` is set). Else empty: num numbers
+  // everything.
   struct Part {
     vt::Numbering num;
-    long long column, element;
+    long long column, at, at_all;
   };
   std::vector<Part> parts;
+  bool all_instances = false;
   vt::AdjointState* adj = nullptr;
   // vt_test_bulk_wait: the stage kernels' wait bound and test flags
   unsigned test_wait_tries = 0;

@@ -439,7 +439,9 @@ cudaError_t to_columns(vt_ctx* c, const double* src, double2* dst) {
   if (c->parts.empty()) return launch_to_columns(src, dst, c->num, c->Np, c->stream);
   cudaError_t e = cudaSuccess;
   for (const auto& p : c->parts)
-    if (!e) e = launch_to_columns(src + 4ll * c->Np * p.element, dst + 2ll * c->Np * p.column, p.num, c->Np, c->stream);
+    if (!e)
+      e = launch_to_columns(src + (c->all_instances ? p.at_all : p.at), dst + 2ll * c->Np * p.column, p.num, c->Np,
+                            c->stream);
   return e;
 }
 
@@ -447,7 +449,9 @@ cudaError_t from_columns(vt_ctx* c, const double2* src, double* dst) {
   if (c->parts.empty()) return launch_from_columns(src, dst, c->num, c->Np, c->stream);
   cudaError_t e = cudaSuccess;
   for (const auto& p : c->parts)
-    if (!e) e = launch_from_columns(src + 2ll * c->Np * p.column, dst + 4ll * c->Np * p.element, p.num, c->Np, c->stream);
+    if (!e)
+      e = launch_from_columns(src + 2ll * c->Np * p.column, dst + (c->all_instances ? p.at_all : p.at), p.num, c->Np,
+                              c->stream);
   return e;
 }
 
