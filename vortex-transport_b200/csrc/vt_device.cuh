@@ -255,6 +255,17 @@ struct FaceCounts {
 };
 __host__ __device__ constexpr unsigned face_factor(int n) { return n > 0 ? (1u << 20) / n + 1 : 0; }
 
+__host__ __device__ constexpr FaceCounts face_counts(int n0, int n1, int nfq, int p0, int p1) {
+  return {static_cast<unsigned>(n0 | n1 << 16), static_cast<unsigned>(p0 | p1 << 8 | (n0 * ((nfq + p0 - 1) / p0)) << 16),
+          face_factor(n0), face_factor(n1)};
+}
+// What the face phase costs a thread with i and j points per item, in tenths of
+// a point inside the tile (the other ones take the neighbour's trace as well).
+__device__ __forceinline__ int face_cost(int n0, int n1, int nfq, int i, int j, int threads) {
+  const int items = n0 * ((nfq + i - 1) / i) + n1 * ((nfq + j - 1) / j);
+  return (items + threads - 1) / threads * max(n0 ? 10 * i : 0, n1 ? 14 * j : 0);
+}
+
 // Work item w: its entry in the list and its points [q0, q1); false past the last one.
 template <int NFQ>
 __device__ __forceinline__ bool face_work(const FaceCounts& f, int w, int* entry, int* q0, int* q1) {
@@ -440,7 +451,9 @@ __device__ __forceinline__ void roe_flux2(const double* uL, const double* uR, do
 // contracted with the inverse Jacobian rows: gxi = Jinv00 Fx + Jinv01 Fy,
 // geta = Jinv10 Fx + Jinv11 Fy, formed through the contravariant velocities
 // (25 FP64 instructions and a reciprocal estimate against 34 when Fx and Fy
-// are formed first).
+// are formed first). With FACTORED the energy flux stays a product: gxi[3] and
+// geta[3] are the contravariant velocities and gxi[4] = geta[4] = rH.
+template <bool FACTORED = false>
 __device__ __forceinline__ void contravariant_flux(const double* s, double j00, double j01,
                                                    double j10, double j11, double* gxi,
                                                    double* geta) {
@@ -452,10 +465,15 @@ __device__ __forceinline__ void contravariant_flux(const double* s, double j00, 
   const double vxi = gxi[0] * ir, veta = geta[0] * ir;
   gxi[1] = fma(s[1], vxi, j00 * p);
   gxi[2] = fma(s[2], vxi, j01 * p);
-  gxi[3] = rH * vxi;
   geta[1] = fma(s[1], veta, j10 * p);
   geta[2] = fma(s[2], veta, j11 * p);
-  geta[3] = rH * veta;
+  if constexpr (FACTORED) {
+    gxi[3] = vxi, geta[3] = veta;
+    gxi[4] = geta[4] = rH;
+  } else {
+    gxi[3] = rH * vxi;
+    geta[3] = rH * veta;
+  }
 }
 
 }  // namespace vt

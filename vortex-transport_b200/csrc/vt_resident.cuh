@@ -6,21 +6,27 @@
 // next and the tile's way to HBM and back. Here every block keeps its tile for
 // all the steps of a call: state, geometry and face list stay in shared memory,
 // U_n and the RK accumulator in registers, and a tile waits only for the tiles
-// it shares a face with. A stage takes 4.8 us there, 250 RK4 steps 4.8 instead
-// of 6.2 ms; 50 steps at 64 x 64, p = 2 (128 tiles) 0.97 instead of 1.12 ms, 100
-// Euler steps at 27 x 18, p = 1 0.42 instead of 0.51 ms. What is left at 128
-// tiles, in cycles of about 9000: faces 2700, waiting for the neighbours 2700,
-// lift and the barrier before it 1500, the rest 2100. The numbers are the stage
-// kernel's, bit for bit: the same functions in the same order (vt_tile.cuh).
+// it shares a face with. Alone on its SM a tile is bound by latency, so with
+// the folded operators it has two threads per element and component, one for
+// the even and one for the odd parts, and twice the threads for the faces:
+//
+//                                    stage kernel  256 threads  512 threads
+//   250 RK4 steps,  8 x 8,   p = 3       6.2 ms       4.7 ms      4.15 ms
+//   50 RK4 steps,   64 x 64, p = 2       1.12         0.97        0.86
+//   100 Euler steps, 27 x 18, p = 1      0.51         0.42        0.37
+//
+// (768 threads, which leave 80 registers each: 4.43, 0.93 and 0.40 ms.) What is
+// left of a stage at 8 x 8, p = 3, in cycles of 7900: lift and volume, with the
+// wait for the slowest faces, 2300, faces 2000, waiting for the neighbours and
+// copying their nodes 1300, the rest 2300. The numbers are the stage kernel's,
+// bit for bit: the same functions in the same order (vt_tile.cuh).
 //
 // Stage s of a launch (counted over its steps):
 //   1. one warp of each half waits until the neighbours' tiles have published s
 //      stages (flags, below);
 //   2. meanwhile the nodal flux into a buffer of its own; then the neighbours'
 //      side nodes are requested (cp.async) and the own traces formed;
-//   3. barrier; faces, with all points of a work item side by side (one block
-//      per SM has the registers: three independent fluxes hide each other's
-//      latency); barrier;
+//   3. barrier; faces; barrier;
 //   4. lift, volume, update: the new stage state goes to shared memory and to
 //      the stage's vector in HBM, where the neighbours find it;
 //   5. barrier; one thread makes the block's writes visible and publishes.
@@ -32,6 +38,8 @@
 // one that gives up sets bit 1 of err[3], the block leaves, and the others give
 // up in turn.
 #pragma once
+
+#include <type_traits>
 
 #include "vt_tile.cuh"
 
@@ -120,15 +128,42 @@ __device__ __forceinline__ void face_points(double2* own, double2* oth, bool mir
   }
 }
 
+// Threads of a block: with the folded operators two per element and component,
+// one for the even and one for the odd parts.
+constexpr int resident_threads(int map) { return (map == kMapFolded ? 8 : 4) * kTileElems; }
+
+// The even (ODD = 0), the odd (1) or all (-1) parts of the update, and the nodes
+// whose new values this thread forms from them: the first ones of the mirrored
+// pairs and the fixed nodes, the second ones, or all.
+template <int P, int PART>
+struct ResidentPart {
+  static constexpr int kParts = PART < 0 ? np_of_p(P) : (PART == 0 ? fold_nodes(P) : fold_pairs(P));
+  static constexpr int kArray = PART < 0 ? np_of_p(P) : fold_nodes(P);
+  __device__ static constexpr int node(int a) {
+    return PART < 0 ? a : (PART == 0 ? fold_node(P, a) : mirror_node(P, fold_node(P, a)));
+  }
+};
+
+// Barrier of the THREADS threads that hold one half's columns.
+template <int THREADS>
+__device__ __forceinline__ void half_sync(int which) {
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + which), "n"(THREADS) : "memory");
+}
+// Barrier of the two warps with the same elements and components.
+__device__ __forceinline__ void pair_sync(int t) {
+  asm volatile("bar.sync %0, 64;" ::"r"(3 + ((t >> 5) & 7)) : "memory");
+}
+
 template <int P, int NFQ, int MAP>
-__global__ void __launch_bounds__(4 * kTileElems, 1)
+__global__ void __launch_bounds__(resident_threads(MAP), 1)
     resident_steps_kernel(const __grid_constant__ StageArgs a, const __grid_constant__ ResidentArgs ra,
                           const OpsOf<P, NFQ, MAP> ops) {
   using L = TileLayout<P, NFQ>;
   constexpr int E = L::E;
   constexpr int NP = L::NP;
   constexpr int NE = L::NE;
-  constexpr int T = 4 * E;
+  constexpr int T = resident_threads(MAP);
+  constexpr int G = T / E;  // groups of a thread per column
   constexpr bool FOLD = MAP == kMapFolded;
   extern __shared__ __align__(128) unsigned char smem[];
   double2* S = reinterpret_cast<double2*>(smem + L::kS);
@@ -141,7 +176,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 1)
   double* TM = reinterpret_cast<double*>(smem + L::kTM);
   const int* EL = reinterpret_cast<const int*>(smem + L::kEL);
   const unsigned short* items = reinterpret_cast<const unsigned short*>(smem + L::kItems);
-  const FaceCounts* counts = reinterpret_cast<const FaceCounts*>(smem + L::kItems + kListCount);
+  FaceCounts* counts = reinterpret_cast<FaceCounts*>(smem + L::kItems + kListCount);
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem + L::kBar);
   // abort_flag is set only between a stage's start and its first barrier, and
   // read by all behind that barrier, so that all leave together; late_flag is
@@ -152,9 +187,9 @@ __global__ void __launch_bounds__(4 * kTileElems, 1)
   const int t = threadIdx.x;
   const int lane = t & 31;
   const int which = (t >> 5) & 1;  // this warp's half of the tile
-  const int grp = t >> 6;          // and its number among the half's four
+  const int grp = t >> 6;          // and its number among the half's G
   const int col = t % E;           // nodal flux phase
-  const int el = work_column(t), c = work_component(t);
+  const int el = work_column(t % (4 * E)), c = work_component(t % (4 * E));
   const int tile = blockIdx.x;
   const long long blk = 2ll * tile + which;
   const unsigned max_tries = a.wait_tries ? a.wait_tries : kMaxWaitTries;
@@ -164,9 +199,11 @@ __global__ void __launch_bounds__(4 * kTileElems, 1)
     const double* tm = &ops.tm[0][0][0];
     for (int l = t; l < 3 * NFQ * NE; l += T) TM[l] = tm[l];
   }
+  __shared__ unsigned least;
   if (t == 0) {
     mbar_init(bar, 2);
     *abort_flag = *late_flag = 0;
+    least = ~0u;
   }
   const unsigned code = neighbour_code(a.lists, tile, which, lane);
   __syncthreads();
@@ -182,11 +219,20 @@ __global__ void __launch_bounds__(4 * kTileElems, 1)
       *abort_flag = 1;
     }
   }
+  if constexpr (T != 4 * E) {  // points per work item for this number of threads
+    const int n0 = counts->n & 0xffff, n1 = counts->n >> 16, i = 1 + t / NFQ, j = 1 + t % NFQ;
+    if (t < NFQ * NFQ) atomicMin(&least, static_cast<unsigned>(face_cost(n0, n1, NFQ, i, j, T) << 8 | (NFQ * NFQ - 1 - t)));
+    __syncthreads();
+    if (t == 0) {
+      const int best = NFQ * NFQ - 1 - (least & 0xff);
+      *counts = face_counts(n0, n1, NFQ, 1 + best / NFQ, 1 + best % NFQ);
+    }
+  }
   __syncthreads();
 
   // a lane polls for its slot's tile unless the slot before it has the same one
   const unsigned before = __shfl_up_sync(0xffffffffu, code, 1);
-  const bool polls = grp == 0 && code != kNoNeighbour &&
+  const bool polls = grp == G - 1 && code != kNoNeighbour &&
                      (lane == 0 || (before >> 2) / kTileElems != (code >> 2) / kTileElems);
 
   constexpr int kStep = 4 * kTileRun;  // doubles between node rows of the same pair
@@ -194,10 +240,10 @@ __global__ void __launch_bounds__(4 * kTileElems, 1)
   double* Sd = reinterpret_cast<double*>(S) + sidx<NP>(c >> 1, el) * 2 + (c & 1);  // this thread's cells of the state
   const int at = ((c >> 1) * E + el) * 2 + (c & 1);  // its component and column in the face and flux buffers
   const int nstages = ra.euler ? ra.nsteps : 4 * ra.nsteps;
-  bool valid = false;
-  double base[NP], X[NP];
+  constexpr int kOwn = FOLD ? fold_nodes(P) : NP;
+  double base[kOwn], X[kOwn];
 #pragma unroll
-  for (int i = 0; i < NP; ++i) base[i] = X[i] = 0.0;
+  for (int i = 0; i < kOwn; ++i) base[i] = X[i] = 0.0;
 
   for (int s = 0; s < nstages; ++s) {
     const int stage = ra.euler ? static_cast<int>(kStageEuler) : s & 3;
@@ -217,17 +263,25 @@ __global__ void __launch_bounds__(4 * kTileElems, 1)
     if (P > 0) {
       const double2* ge = GE + which * kGeoRows * kTileRun + lane;
       const double2 j0 = ge[0], j1 = ge[kTileRun];
-      if constexpr (FOLD) folded_nodal_flux<P>(S, GB2, col, grp, j0, j1);
+      if constexpr (FOLD) folded_nodal_flux<P, G>(S, GB2, col, grp, j0, j1);
       else plain_nodal_flux<P>(S, GB2, col, grp, j0, j1);
     }
-    run_sync(t);  // the half's neighbours have published
-    copy_neighbours<P>(H, in, code, which, grp, lane);
-    own_traces<P, NFQ>(ops, S, FB, el, c);
+    half_sync<T / 2>(which);  // the half's neighbours have published
+    copy_neighbours<P>(H, in, code, which, G - 1 - grp, lane);
+    if constexpr (FOLD) {
+      if (t < 4 * E) own_traces<P, NFQ, 0, 3 * NFQ / 2>(ops, S, FB, el, c);
+      else own_traces<P, NFQ, 3 * NFQ / 2, 3 * NFQ>(ops, S, FB, el, c);
+    } else {
+      own_traces<P, NFQ>(ops, S, FB, el, c);
+    }
     cp_async_wait_all();
     __syncthreads();
     if (*abort_flag) break;
 
     // ---- 3. faces ------------------------------------------------------------------
+    // Points side by side, to hide each other's latency where there are the
+    // registers: 512 threads have them for one (two: 5.2 ms at 8 x 8, spilling).
+    constexpr int kSide = FOLD || NFQ < 3 ? 1 : 3;
     const FaceCounts faces = *counts;
     int entry, q, q1;
     for (int w = t; face_work<NFQ>(faces, w, &entry, &q, &q1); w += T) {
@@ -273,15 +327,9 @@ __global__ void __launch_bounds__(4 * kTileElems, 1)
       };
       auto on_error = [&](int point, int err) { record_error_at(a.err, epoch, NFQ, EL[fl], point, sd, err); };
       while (q < q1) {
-        const int left = q1 - q;
-        if (left >= 3) {
-          if constexpr (NFQ >= 3) face_points<P, NFQ, 3>(own, oth, mirror, n, q, outer, on_error);
-        } else if (left == 2) {
-          if constexpr (NFQ >= 2) face_points<P, NFQ, 2>(own, oth, mirror, n, q, outer, on_error);
-        } else {
-          face_points<P, NFQ, 1>(own, oth, mirror, n, q, outer, on_error);
-        }
-        const int done = left >= 3 ? 3 : left;
+        const int done = q1 - q >= kSide ? kSide : 1;
+        if (done == kSide) face_points<P, NFQ, kSide>(own, oth, mirror, n, q, outer, on_error);
+        else face_points<P, NFQ, 1>(own, oth, mirror, n, q, outer, on_error);
         q += done;
         own += done * 2 * E;
         oth -= done * 2 * E;
@@ -290,43 +338,67 @@ __global__ void __launch_bounds__(4 * kTileElems, 1)
     __syncthreads();
 
     // ---- 4. lift, volume, update ---------------------------------------------------
-    valid = EL[el] >= 0;
-    double r[NP], u[NP];
-    {
-      const double2* ge = GE + which * kGeoRows * kTileRun + (el & 31);
-      lift_term<P, NFQ>(ops, FB + at, ge[2 * kTileRun], ge[3 * kTileRun], r);
-    }
+    auto update = [&](auto part) {
+      constexpr int PART = decltype(part)::value;
+      using R = ResidentPart<P, PART>;
+      double r[R::kArray], u[R::kArray];
+      {
+        const double2* ge = GE + which * kGeoRows * kTileRun + (el & 31);
+        if constexpr (PART < 0) lift_term<P, NFQ>(ops, FB + at, ge[2 * kTileRun], ge[3 * kTileRun], r);
+        else lift_term<P, NFQ, PART == 0, PART == 1>(ops, FB + at, ge[2 * kTileRun], ge[3 * kTileRun], r);
+      }
 #pragma unroll
-    for (int i = 0; i < NP; ++i) u[i] = Sd[i * kStep];  // the stage's input
-    const double c_out = (stage == 0 || stage == 1 ? 0.5 : (stage == 3 ? 1.0 / 6 : 1.0)) * ra.dt;
-    if (stage == 3) {
-      const double f = kThird / c_out;
-      if constexpr (FOLD) {
-        folded_state<P>(S, el, c, f, r);
+      for (int i = 0; i < R::kParts; ++i) u[i] = Sd[R::node(i) * kStep];  // the stage's input
+      const double c_out = (stage == 0 || stage == 1 ? 0.5 : (stage == 3 ? 1.0 / 6 : 1.0)) * ra.dt;
+      if (stage == 3) {
+        const double f = kThird / c_out;
+        if constexpr (PART < 0) {
+#pragma unroll
+          for (int i = 0; i < NP; ++i) r[i] = fma(f, u[i], r[i]);
+        } else {
+          folded_state<P, PART == 0, PART == 1>(S, el, c, f, r);
+        }
+      }
+      if constexpr (PART < 0) {
+        if (P > 0) volume_term<P, NFQ>(ops, GB + at, r);
       } else {
+        if (P > 0) volume_term<P, NFQ, PART == 0, PART == 1>(ops, GB + at, r);
+        // the other thread's parts, through the flux rows that only this thread has read
+        double* G = GB + at;
+        constexpr int NO = fold_pairs(P);
 #pragma unroll
-        for (int i = 0; i < NP; ++i) r[i] = fma(f, u[i], r[i]);
+        for (int a = 0; a < NO; ++a) G[(a * 8 + 4 * PART) * E] = r[a];
+        pair_sync(t);
+#pragma unroll
+        for (int a = 0; a < NO; ++a) {
+          const double o = G[(a * 8 + 4 - 4 * PART) * E];
+          r[a] = PART == 0 ? r[a] + o : o - r[a];
+        }
       }
-    }
-    if (P > 0) volume_term<P, NFQ>(ops, GB + at, r);
-    if constexpr (FOLD) unfold<P>(r);
-    if (stage == 0 || stage == kStageEuler) {
+      if (stage == 0 || stage == kStageEuler) {
 #pragma unroll
-      for (int i = 0; i < NP; ++i) base[i] = u[i];
-    }
-    if (stage == 1) {
-      const double c_acc = (1.0 / 3) * ra.dt;
-#pragma unroll
-      for (int i = 0; i < NP; ++i) X[i] = fma(c_acc, r[i], (base[i] + u[i]) * kThird);
-    }
-    if (valid) {
-      double* out = reinterpret_cast<double*>(out2) + off0;
-#pragma unroll
-      for (int i = 0; i < NP; ++i) {
-        const double v = fma(c_out, r[i], stage == 3 ? X[i] : base[i]);
-        Sd[i * kStep] = v;
-        out[i * kStep] = v;
+        for (int i = 0; i < R::kParts; ++i) base[i] = u[i];
       }
+      if (stage == 1) {
+        const double c_acc = (1.0 / 3) * ra.dt;
+#pragma unroll
+        for (int i = 0; i < R::kParts; ++i) X[i] = fma(c_acc, r[i], (base[i] + u[i]) * kThird);
+      }
+      if (EL[el] >= 0) {
+        double* out = reinterpret_cast<double*>(out2) + off0;
+#pragma unroll
+        for (int i = 0; i < R::kParts; ++i) {
+          const double v = fma(c_out, r[i], stage == 3 ? X[i] : base[i]);
+          Sd[R::node(i) * kStep] = v;
+          out[R::node(i) * kStep] = v;
+        }
+      }
+    };
+    if constexpr (FOLD) {
+      if (t < 4 * E) update(std::integral_constant<int, 0>{});
+      else update(std::integral_constant<int, 1>{});
+    } else {
+      update(std::integral_constant<int, -1>{});
     }
 
     // ---- 5. publish ----------------------------------------------------------------

@@ -149,20 +149,13 @@ __global__ void build_tile_lists_kernel(const int4* __restrict__ nbr, const int*
     int p0 = 1, p1 = 1, least = 0;  // in tenths of a point
     for (int i = 1; i <= nfq; ++i)
       for (int j = 1; j <= nfq; ++j) {
-        const int items = n0 * ((nfq + i - 1) / i) + n1 * ((nfq + j - 1) / j);
-        const int rounds = (items + 4 * kTileElems - 1) / (4 * kTileElems);
-        const int cost = rounds * max(n0 ? 10 * i : 0, n1 ? 14 * j : 0);
+        const int cost = face_cost(n0, n1, nfq, i, j, 4 * kTileElems);
         if ((i == 1 && j == 1) || cost <= least) {
           least = cost;
           p0 = i, p1 = j;
         }
       }
-    FaceCounts f;
-    f.n = n0 | n1 << 16;
-    f.points = p0 | p1 << 8 | (n0 * ((nfq + p0 - 1) / p0)) << 16;
-    f.factor0 = face_factor(n0);
-    f.factor1 = face_factor(n1);
-    *counts = f;
+    *counts = face_counts(n0, n1, nfq, p0, p1);
   }
 }
 

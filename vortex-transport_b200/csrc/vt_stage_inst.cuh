@@ -56,7 +56,7 @@ cudaError_t configure_resident(int* blocks_per_sm) {
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, resident_steps_kernel<P, NFQ, MAP>,
-                                                       4 * kTileElems, bytes);
+                                                       resident_threads(MAP), bytes);
 }
 
 template <int P, int NFQ, int MAP>
@@ -66,7 +66,7 @@ cudaError_t launch_resident(const StageArgs& a, const ResidentArgs& r, const dou
   attr.val.cooperative = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(a.ntiles));
-  cfg.blockDim = dim3(4 * kTileElems);
+  cfg.blockDim = dim3(resident_threads(MAP));
   cfg.dynamicSmemBytes = ResidentLayout<P, NFQ>::kBytes;
   cfg.stream = st;
   cfg.attrs = &attr;

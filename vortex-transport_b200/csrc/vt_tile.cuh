@@ -229,8 +229,9 @@ __device__ __forceinline__ int work_column(int t) {
 }
 __device__ __forceinline__ int work_component(int t) { return ((t >> 6) & 1) * 2 + (t & 1); }
 
-// Traces of component c of column el at every face point.
-template <int P, int NFQ, typename Ops>
+// Traces of component c of column el at every face point (or at the points
+// FIRST ... END - 1 of the three sides').
+template <int P, int NFQ, int FIRST = 0, int END = 3 * NFQ, typename Ops>
 __device__ __forceinline__ void own_traces(const Ops& ops, const double2* S, double* FB, int el, int c) {
   constexpr int NP = np_of_p(P), NE = P + 1, ES = kTileElems;
   const double* Sd = reinterpret_cast<const double*>(S) + sidx<NP>(c >> 1, el) * 2 + (c & 1);
@@ -242,6 +243,7 @@ __device__ __forceinline__ void own_traces(const Ops& ops, const double2* S, dou
   for (int s = 0; s < 3; ++s)
 #pragma unroll
     for (int q = 0; q < NFQ; ++q) {
+      if (s * NFQ + q < FIRST || s * NFQ + q >= END) continue;
       double v = 0.0;
 #pragma unroll
       for (int k = 0; k < NE; ++k) v = fma(ops.tp[s][q][k], u[edge_node(P, s, k)], v);
@@ -280,10 +282,11 @@ __device__ __forceinline__ void volume_term(const StageOps<P, NFQ>& ops, const d
   }
 }
 
-template <int P, int NFQ>
+// The folded terms give the even parts, the odd parts, or both in this order.
+template <int P, int NFQ, bool EVEN = true, bool ODD = true>
 __device__ __forceinline__ void lift_term(const FoldedOps<P, NFQ>& ops, const double* F, double2 lsa, double2 lsb,
                                           double* r) {
-  constexpr int ES = kTileElems, NS = FoldedOps<P, NFQ>::NS, NO = FoldedOps<P, NFQ>::NO;
+  constexpr int ES = kTileElems, NS = EVEN ? FoldedOps<P, NFQ>::NS : 0, NO = ODD ? FoldedOps<P, NFQ>::NO : 0;
 #pragma unroll
   for (int a = 0; a < NS + NO; ++a) r[a] = 0.0;
 #pragma unroll
@@ -314,17 +317,17 @@ __device__ __forceinline__ void lift_term(const FoldedOps<P, NFQ>& ops, const do
 }
 
 // Stage 3's U3 / (3 c_out) (f = 1 / (3 c_out)) added to the even and odd parts.
-template <int P>
+template <int P, bool EVEN = true, bool ODD = true>
 __device__ __forceinline__ void folded_state(const double2* S, int el, int c, double f, double* r) {
   constexpr int NP = np_of_p(P), NS = fold_nodes(P), NO = fold_pairs(P);
   const double* Sd = reinterpret_cast<const double*>(S) + sidx<NP>(c >> 1, el) * 2 + (c & 1);
 #pragma unroll
-  for (int a = 0; a < NS; ++a) {
+  for (int a = 0; a < (EVEN ? NS : NO); ++a) {
     const double u = Sd[fold_node(P, a) * 4 * kTileRun];
     if (a < NO) {
       const double v = Sd[mirror_node(P, fold_node(P, a)) * 4 * kTileRun];
-      r[a] = fma(0.5 * f, u + v, r[a]);
-      r[NS + a] = fma(0.5 * f, u - v, r[NS + a]);
+      if (EVEN) r[a] = fma(0.5 * f, u + v, r[a]);
+      if (ODD) r[(EVEN ? NS : 0) + a] = fma(0.5 * f, u - v, r[(EVEN ? NS : 0) + a]);
     } else {
       r[a] = fma(f, u, r[a]);
     }
@@ -334,56 +337,69 @@ __device__ __forceinline__ void folded_state(const double2* S, int el, int c, do
 // Nodal fluxes in the form that the folded volume operator reads: for node j
 // with mirror image Pj, rows j*4 + h hold Gxi_j + Geta_Pj and rows j*4 + 2 + h
 // Gxi_j - Geta_Pj (component pair h). A thread takes both nodes of a pair, or
-// one fixed node, of column el; flux(j, gxi, geta) is node j's.
-template <int P, typename Flux>
+// one fixed node, of column el (group grp of G); flux(j, gxi, geta) is node j's.
+// With FACTORED it gives the energy flux as contravariant_flux<true> does: the
+// roundings of the sums are then spelled out (the first node's products are
+// rounded, the second's go into multiply-adds), since the kernels that share
+// this function must agree bit for bit and the compiler's choice varies. Both
+// nodes' products in multiply-adds, which need more registers, took 0.888 ms
+// at 150 x 90, p = 3, 20 steps, against 0.869.
+template <int P, int G = 4, bool FACTORED = false, typename Flux>
 __device__ __forceinline__ void folded_flux_rows(double2* G2, int el, int grp, Flux&& flux) {
   constexpr int ES = kTileElems, NS = fold_nodes(P), NO = fold_pairs(P);
-  auto store = [&](int j, const double* gxi, const double* geta) {
+  auto store = [&](int j, const double* gxi, const double* geta, double even, double odd) {
     double2* g = G2 + j * 4 * ES + el;
     g[0] = make_double2(gxi[0] + geta[0], gxi[1] + geta[1]);
-    g[ES] = make_double2(gxi[2] + geta[2], gxi[3] + geta[3]);
+    g[ES] = make_double2(gxi[2] + geta[2], even);
     g[2 * ES] = make_double2(gxi[0] - geta[0], gxi[1] - geta[1]);
-    g[3 * ES] = make_double2(gxi[2] - geta[2], gxi[3] - geta[3]);
+    g[3 * ES] = make_double2(gxi[2] - geta[2], odd);
   };
 #pragma unroll
-  for (int u0 = 0; u0 < NS; u0 += 4) {
+  for (int u0 = 0; u0 < NS; u0 += G) {
     const int u = u0 + grp;  // uniform per warp
     if (u >= NS) break;
     int j = 0;
 #pragma unroll
-    for (int k = u0; k < u0 + 4 && k < NS; ++k)
+    for (int k = u0; k < u0 + G && k < NS; ++k)
       if (u == k) j = fold_node(P, k);
-    double gxi[4], geta[4];
+    double gxi[5], geta[5];
     flux(j, gxi, geta);
+    if constexpr (FACTORED) gxi[3] = __dmul_rn(gxi[4], gxi[3]), geta[3] = __dmul_rn(geta[4], geta[3]);
     if (u < NO) {
       int m = 0;
 #pragma unroll
-      for (int k = u0; k < u0 + 4 && k < NO; ++k)
+      for (int k = u0; k < u0 + G && k < NO; ++k)
         if (u == k) m = mirror_node(P, fold_node(P, k));
-      double hxi[4], heta[4];
+      double hxi[5], heta[5];
       flux(m, hxi, heta);
-      store(j, gxi, heta);
-      store(m, hxi, geta);
+      if constexpr (FACTORED) {
+        store(j, gxi, heta, fma(heta[4], heta[3], gxi[3]), fma(-heta[4], heta[3], gxi[3]));
+        store(m, hxi, geta, fma(hxi[4], hxi[3], geta[3]), fma(hxi[4], hxi[3], -geta[3]));
+      } else {
+        store(j, gxi, heta, gxi[3] + heta[3], gxi[3] - heta[3]);
+        store(m, hxi, geta, hxi[3] + geta[3], hxi[3] - geta[3]);
+      }
     } else {
-      store(j, gxi, geta);
+      store(j, gxi, geta, gxi[3] + geta[3], gxi[3] - geta[3]);
     }
   }
 }
 
-template <int P>
+template <int P, int G = 4>
 __device__ __forceinline__ void folded_nodal_flux(const double2* S, double2* G2, int el, int grp, double2 j0,
                                                   double2 j1) {
   constexpr int NP = np_of_p(P);
-  folded_flux_rows<P>(G2, el, grp, [&](int j, double* gxi, double* geta) {
+  folded_flux_rows<P, G, true>(G2, el, grp, [&](int j, double* gxi, double* geta) {
     const double2 s0 = S[sidx<NP>(2 * j, el)], s1 = S[sidx<NP>(2 * j + 1, el)];
     const double sv[4] = {s0.x, s0.y, s1.x, s1.y};
-    contravariant_flux(sv, j0.x, j0.y, j1.x, j1.y, gxi, geta);
+    contravariant_flux<true>(sv, j0.x, j0.y, j1.x, j1.y, gxi, geta);
   });
 }
 
-template <int P, int NFQ>
+template <int P, int NFQ, bool EVEN = true, bool ODD = true>
 __device__ __forceinline__ void volume_term(const FoldedOps<P, NFQ>& ops, const double* G, double* r) {
-  constexpr int NP = np_of_p(P), ES = kTileElems, NS = FoldedOps<P, NFQ>::NS, NO = FoldedOps<P, NFQ>::NO;
+  constexpr int NP = np_of_p(P), ES = kTileElems;
+  constexpr int NS = EVEN ? FoldedOps<P, NFQ>::NS : 0, NO = ODD ? FoldedOps<P, NFQ>::NO : 0;
 #pragma unroll
   for (int j = 0; j < NP; ++j) {
     const double ge = G[j * 8 * ES], go = G[(j * 8 + 4) * ES];
