@@ -198,10 +198,10 @@ def import_package():
 def ensemble(vt, steps: int, n: int = 512, device: int = 0, rank: int = 0, world: int = 1, pg=None):
     """The batched forward ensemble: n seeded vortex problems of uneven size and
     order (workloads.ensemble_instances, seed 1) advanced `steps` RK4 steps as
-    one ragged batch (one persistent launch per stage and order group, the step
-    in a CUDA graph, grid autotuned), against the same n problems run one at a
-    time through the plain solver. Set-up (host precompute, device upload, graph
-    capture, tuning) is outside both timed regions; both are host wall-clock
+    one ragged batch (one persistent launch per stage and order group, grid
+    autotuned), against the same n problems run one at a
+    time through the plain solver. Set-up (host precompute, device upload,
+    tuning) is outside both timed regions; both are host wall-clock
     around synchronous calls, the device idle at the start of each.
 
     With several ranks the instances are split by DOF-stages
@@ -269,9 +269,9 @@ def ensemble(vt, steps: int, n: int = 512, device: int = 0, rank: int = 0, world
         "instances_per_rank": [len(q) for q in parts],
         "groups": [list(g) for g in groups],
         "per_group": per_group,
-        "tuning": {"per_group": [{"p": g[0], "blocks_per_sm": b, "mapping": "pair" if m == 1 else "component"}
+        "tuning": {"per_group": [{"p": g[0], "blocks_per_sm": b, "mapping": "folded" if m == 1 else "component"}
                                  for g, (b, m) in zip(groups, tuned)],
-                   "note": "autotuned per group over both warp mappings and 1..3 resident blocks per SM"},
+                   "note": "autotuned per group over both forms of the operators and 1..3 resident blocks per SM"},
         "batched_solves_per_s": n / batched_s,
         "sequential_solves_per_s": n / seq_s,
         "speedup": seq_s / batched_s,
@@ -305,7 +305,7 @@ def adjoint(vt, steps: int = 2000, snapshots=None, device: int = 0):
     lamT = torch.tensor(np.random.default_rng(3).standard_normal(U0.shape), device=torch.device("cuda", device))
 
     def timed(fn):
-        fn()  # untimed: graph capture, buffers
+        fn()  # untimed: buffers
         s.upload(U0)
         torch.cuda.synchronize()
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -482,7 +482,7 @@ def b200_arm(args):
         if pg:
             pg.barrier()
 
-    # warm-up (also captures the step graph)
+    # warm-up
     solver.rk4(DT, max(args.warmup, 1))
 
     # ---- timed region: K steps, state resident in HBM -----------------------

@@ -797,7 +797,7 @@ class Batch:
         return info.as_dict()
 
     def autotune(self, trials: int = 3, cache: str | None = None) -> list[tuple[int, int]]:
-        """(resident blocks per SM, warp mapping) for each group, tuned on the
+        """(resident blocks per SM, stage mapping) for each group, tuned on the
         device and cached in `cache` (a JSON file keyed by the batch's makeup
         and the GPU)."""
         import hashlib

@@ -668,9 +668,9 @@ int vt_batch_autotune(vt_batch* b, int trials, int* blocks_per_sm_out, int* mapp
   if (!b || trials < 1) return fail(VT_ERR_INVALID, "vt_batch_autotune: bad argument");
   std::lock_guard<std::mutex> lk(b->mu);
   cudaSetDevice(b->device);
-  // candidates per group: both warp mappings of the stage kernel (one thread
-  // per component, or per component pair and node half) x persistent grids of
-  // SMs x {1 .. resident limit} blocks; the state is restored afterwards so
+  // candidates per group: both forms of the stage kernel (the operators as they
+  // are, or folded where they reflect) x persistent grids of SMs x {1 ..
+  // resident limit} blocks; the state is restored afterwards so
   // tuning does not advance the solution
   std::vector<std::vector<double2>> saved;
   for (auto& G : b->groups) {

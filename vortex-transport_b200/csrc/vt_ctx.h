@@ -41,7 +41,7 @@ struct vt_ctx {
   unsigned* flags = nullptr;
   unsigned flag_base = 0;
   bool flags_known = false, flag_launches = false;
-  int map = vt::kDefaultMap;  // warp mapping of the stage kernel
+  int map = vt::kDefaultMap;  // form of the stage kernel
   double time = 0.0;
   vt_error_info last{};
   int pending_steps = 0;

@@ -1,4 +1,4 @@
-// Kernel selection by (p, nfq, warp mapping) -- the instantiations are in
+// Kernel selection by (p, nfq, form of the operators) -- the instantiations are in
 // vt_stage_component.cu and vt_stage_folded.cu -- and the tile schedule kernels
 // (vt_launch.h).
 #include <algorithm>

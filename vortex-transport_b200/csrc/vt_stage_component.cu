@@ -1,4 +1,4 @@
-// The stage kernel instantiations of the component warp mapping (vt_tile.cuh).
+// The stage kernel instantiations with the operators as they are (vt_tile.cuh).
 #include "vt_stage_inst.cuh"
 
 namespace vt {

@@ -1,4 +1,4 @@
-// Launch and configuration of the tiled stage kernel for one warp mapping,
+// Launch and configuration of the tiled stage kernel for one form of the operators,
 // instantiated for p = 0..3 and nfq = 1..10 by vt_stage_component.cu and
 // vt_stage_folded.cu (one translation unit per mapping, compiled in parallel).
 #pragma once
