@@ -430,7 +430,7 @@ def reference_arm(args):
         return 0
     threads = os.cpu_count() or 1
     if not os.path.exists(HARNESS):
-        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/vt_ref_harness was not built "
+        print(json.dumps({"impl": "reference", "n_gpus": world, "unavailable": "oracle/_ref/vt_ref_harness was not built "
                           "(needs the reference sources at build time)"}))
         return 0
     r = run_reference_harness(NX, args.steps, threads, warmup=args.warmup)
