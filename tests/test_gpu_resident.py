@@ -107,3 +107,20 @@ def test_a_wait_that_gives_up(vt):
     np.testing.assert_array_equal(s.download(), b.download(0))
     s.close()
     b.close()
+
+
+@pytest.mark.parametrize("nx,ny,p,io", [(5, 7, 3, 10), (8, 8, 1, 3), (27, 18, 1, 4), (9, 6, 0, 2)])
+def test_operators_as_they_are(vt, nx, ny, p, io):
+    """The form without folded operators has half the threads and more points
+    of a face side by side (2, 3 and more of them per item here)."""
+    import ctypes
+    s, b, pb = pair(vt, nx, ny, p, io)
+    dt = small_dt(nx, ny, p)
+    s.stage_mapping = 0
+    assert vt.lib().vt_batch_set_mapping(b._h, (ctypes.c_int * 1)(0)) == 0
+    b.set_dt([dt])
+    s.rk4(dt, 5)
+    b.rk4(5)
+    np.testing.assert_array_equal(s.download(), b.download(0))
+    s.close()
+    b.close()
