@@ -199,6 +199,9 @@ double2* member_columns(const vt_batch* b, int i, double2* group) {
   return group + 2ll * G.Np * vt::kTileElems * G.tile_begin[b->index_in_group[i]];
 }
 
+// Clears the groups' error words. Every call that launches a stage kernel does
+// so first: they hold the counter that hands out tiles (take_tile, vt_tile.cuh),
+// and what an allocation leaves there is not a number of tiles.
 cudaError_t reset_errors(vt_batch* b) {
   cudaError_t e = cudaSuccess;
   for (auto& g : b->groups) {
@@ -422,6 +425,11 @@ vt_batch* vt_batch_create(const vt_mesh_desc* descs, int n, int device, int* sta
     return nullptr;
   }
   b->staging_bytes = max_inst_bytes;
+  if ((e = reset_errors(b)) || (e = cudaStreamSynchronize(b->stream))) {
+    set(fail(VT_ERR_CUDA, vt::cuda_msg("vt_batch_create", e)));
+    release(b);
+    return nullptr;
+  }
   set(VT_OK);
   return b;
 }
@@ -650,18 +658,27 @@ int vt_batch_last_error(const vt_batch* b, int* instance, vt_error_info* out) {
 
 // Times `trials` RK4 steps (after one untimed) of group G alone with its
 // current kernel and grid; the group's state must be saved by the caller.
-static float time_group_steps(vt_batch* b, vt::Group& G, int trials, cudaEvent_t e0, cudaEvent_t e1) {
-  float tot = 0;
-  for (int r = 0; r < trials + 1; ++r) {
-    cudaEventRecord(e0, b->stream);
-    enqueue_group_step(G, b->stream);
-    cudaEventRecord(e1, b->stream);
-    cudaEventSynchronize(e1);
+static cudaError_t time_group_steps(vt_batch* b, vt::Group& G, int trials, cudaEvent_t e0, cudaEvent_t e1, float* tot) {
+  cudaError_t e = cudaSuccess;
+  *tot = 0;
+  for (int r = 0; r < trials + 1 && !e; ++r) {
+    e = cudaEventRecord(e0, b->stream);
+    if (!e) e = enqueue_group_step(G, b->stream);
+    if (!e) e = cudaEventRecord(e1, b->stream);
+    if (!e) e = cudaEventSynchronize(e1);
     float ms = 0;
-    cudaEventElapsedTime(&ms, e0, e1);
-    if (r) tot += ms;  // the first repetition warms up
+    if (!e) e = cudaEventElapsedTime(&ms, e0, e1);
+    if (r) *tot += ms;  // the first repetition warms up
   }
-  return tot;
+  return e;
+}
+
+// VT_ERR_CUDA when a wait of group G's stage kernels gave up since reset_errors.
+static int check_waits(const vt::Group& G, const char* what) {
+  unsigned long long flags = 0;
+  const cudaError_t e = cudaMemcpy(&flags, G.err + 3, sizeof(flags), cudaMemcpyDeviceToHost);
+  if (e) return fail(VT_ERR_CUDA, vt::cuda_msg(what, e));
+  return flags & 2ull ? fail(VT_ERR_CUDA, std::string(what) + ": a bulk-copy wait gave up") : VT_OK;
 }
 
 int vt_batch_autotune(vt_batch* b, int trials, int* blocks_per_sm_out, int* mapping_out) {
@@ -680,9 +697,10 @@ int vt_batch_autotune(vt_batch* b, int trials, int* blocks_per_sm_out, int* mapp
       return fail(VT_ERR_CUDA, "autotune save");
   }
   cudaEvent_t e0, e1;
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
-  for (size_t gi = 0; gi < b->groups.size(); ++gi) {
+  if (cudaEventCreate(&e0) || cudaEventCreate(&e1)) return fail(VT_ERR_CUDA, "vt_batch_autotune: events");
+  int st = VT_OK;
+  cudaError_t err = reset_errors(b);
+  for (size_t gi = 0; gi < b->groups.size() && !err; ++gi) {
     vt::Group& G = b->groups[gi];
     vt::StageKernel best_k = G.kern;
     int best_b = 1;
@@ -692,10 +710,11 @@ int vt_batch_autotune(vt_batch* b, int trials, int* blocks_per_sm_out, int* mapp
       int limit = 0;
       if (k.configure(&limit)) continue;
       G.use(k);
-      for (int bps = 1; bps <= std::max(1, limit); ++bps) {
+      for (int bps = 1; bps <= std::max(1, limit) && !err; ++bps) {
         G.max_blocks = b->sms * bps;
-        const float ms = time_group_steps(b, G, trials, e0, e1);
-        if (ms < best_ms) {
+        float ms = 0;
+        err = time_group_steps(b, G, trials, e0, e1, &ms);
+        if (!err && ms < best_ms) {
           best_ms = ms;
           best_b = bps;
           best_k = k;
@@ -706,9 +725,11 @@ int vt_batch_autotune(vt_batch* b, int trials, int* blocks_per_sm_out, int* mapp
     G.max_blocks = b->sms * best_b;
     if (blocks_per_sm_out) blocks_per_sm_out[gi] = best_b;
     if (mapping_out) mapping_out[gi] = best_k.map;
+    if (!err && !st) st = check_waits(G, "vt_batch_autotune");
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  if (err) return fail(VT_ERR_CUDA, vt::cuda_msg("vt_batch_autotune", err));
   for (size_t gi = 0; gi < b->groups.size(); ++gi) {
     vt::Group& G = b->groups[gi];
     if (cudaMemcpy(G.U, saved[gi].data(), saved[gi].size() * sizeof(double2), cudaMemcpyHostToDevice))
@@ -721,7 +742,7 @@ int vt_batch_autotune(vt_batch* b, int trials, int* blocks_per_sm_out, int* mapp
     v->map = b->groups[gi].kern.map;
     v->max_blocks = b->groups[gi].max_blocks;
   }
-  return VT_OK;
+  return st;
 }
 
 int vt_batch_set_mapping(vt_batch* b, const int* mapping) {
@@ -755,6 +776,7 @@ int vt_batch_time_groups(vt_batch* b, int reps, float* ms_per_step) {
   cudaEvent_t e0, e1;
   if (cudaEventCreate(&e0) || cudaEventCreate(&e1)) return fail(VT_ERR_CUDA, "vt_batch_time_groups: events");
   int st = VT_OK;
+  if (const cudaError_t e = reset_errors(b)) st = fail(VT_ERR_CUDA, vt::cuda_msg("vt_batch_time_groups", e));
   for (size_t gi = 0; gi < b->groups.size() && !st; ++gi) {
     vt::Group& G = b->groups[gi];
     // the group's state is saved and restored, so timing does not advance the solution
@@ -769,7 +791,7 @@ int vt_batch_time_groups(vt_batch* b, int reps, float* ms_per_step) {
     float ms = 0;
     if (!e) e = cudaEventElapsedTime(&ms, e0, e1);
     if (!e) e = cudaMemcpy(G.U, saved.data(), state * sizeof(double2), cudaMemcpyHostToDevice);
-    if (e) st = fail(VT_ERR_CUDA, vt::cuda_msg("vt_batch_time_groups", e));
+    st = e ? fail(VT_ERR_CUDA, vt::cuda_msg("vt_batch_time_groups", e)) : check_waits(G, "vt_batch_time_groups");
     ms_per_step[gi] = ms / reps;
   }
   cudaEventDestroy(e0);
