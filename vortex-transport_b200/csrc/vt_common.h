@@ -4,6 +4,7 @@
 
 #include <cstdint>
 #include <string>
+#include <vector>
 
 #include "../../include/vortex_b200.h"
 
@@ -31,6 +32,22 @@ inline vt_error_info decode_error_key(unsigned long long key, int nfq) {
   info.step = static_cast<int64_t>(epoch / 4);
   info.stage = static_cast<int>(epoch % 4);
   return info;
+}
+
+// Whether every tile that reads another tile's elements is read by it in turn.
+// Elements lie in tiles of `per_tile` columns (column[e] of element e) and read
+// their three neighbours; an arbitrary neighbour table need not be mutual.
+inline bool tiles_read_mutually(int K, const int32_t* neighbours, const int* column, int per_tile, int ntiles) {
+  std::vector<char> reads(static_cast<size_t>(ntiles) * ntiles, 0);
+  for (int e = 0; e < K; ++e)
+    for (int s = 0; s < 3; ++s) {
+      const int tile = column[e] / per_tile, other = column[neighbours[3 * static_cast<size_t>(e) + s]] / per_tile;
+      reads[static_cast<size_t>(tile) * ntiles + other] = 1;
+    }
+  for (int i = 0; i < ntiles; ++i)
+    for (int j = 0; j < i; ++j)
+      if (reads[static_cast<size_t>(i) * ntiles + j] != reads[static_cast<size_t>(j) * ntiles + i]) return false;
+  return true;
 }
 
 // Records the message returned by vt_last_message() on this thread and passes

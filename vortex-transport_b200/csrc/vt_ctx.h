@@ -47,6 +47,7 @@ struct vt_ctx {
   int pending_steps = 0;
   double pending_dt = 0.0;
   bool side_pairing = false;  // nbr(nbr(e, s), s) == e for every element and side
+  bool mutual_tiles = false;  // a tile that reads another is read by it (implied by side_pairing)
   // Per-tile time steps (a batch group's view; null otherwise): stage and
   // adjoint coefficients are then fractions scaled on the device.
   const double* tile_dt = nullptr;

@@ -32,7 +32,9 @@
 //   5. barrier; one thread makes the block's writes visible and publishes.
 // A vector that a tile overwrites in stage s was last read by its neighbours in
 // a stage before s, and they have published that stage before this tile passes
-// its own wait of stage s; so two stage vectors and U are enough.
+// its own wait of stage s; so two stage vectors and U are enough. That needs
+// every tile that reads this one to be one that it waits for, that is, reads
+// itself: use_resident (vt_solver.cu) takes the kernel for such meshes only.
 //
 // All blocks are resident at once (a cooperative launch). Every wait is bounded;
 // one that gives up sets bit 1 of err[3], the block leaves, and the others give

@@ -361,12 +361,14 @@ cudaError_t enqueue_rk4_step(vt_ctx* c, double dt) {
 }
 
 // Takes the resident kernel (vt_resident.cuh) into use where the problem has at
-// most one tile per SM. With more tiles than SMs its blocks would share an SM,
+// most one tile per SM and its tiles read each other mutually, which the order
+// of the resident steps rests on (a caller's neighbours need not be mutual; a
+// launch per stage is right for any). With more tiles than SMs its blocks would share an SM,
 // for which it has neither the shared memory (p = 3) nor the warps: the stage
 // kernel's three blocks per SM then hide what it saves.
 cudaError_t use_resident(vt_ctx* c, const StageKernel& k, int sms) {
   c->resident = nullptr;
-  if (c->ntiles > sms) return cudaSuccess;
+  if (c->ntiles > sms || !c->mutual_tiles) return cudaSuccess;
   int per_sm = 0, coop = 0;
   cudaError_t e = k.configure_resident(&per_sm);
   if (!e) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device);
@@ -524,11 +526,6 @@ vt_ctx* vt_create(const vt_mesh_desc* d, int device, int* status) {
     return nullptr;
   }
   c->max_blocks = sms * (per_sm > 0 ? per_sm : 1);
-  if ((e = vt::use_resident(c, sk, sms))) {
-    set(fail(VT_ERR_CUDA, vt::cuda_msg("resident kernel attributes", e)));
-    release(c);
-    return nullptr;
-  }
   c->minv_ref.assign(d->inv_mass_ref, d->inv_mass_ref + c->Np * c->Np);
 
   // packed geometry and side-ordered neighbours (Evolve.cpp:167-202), by column
@@ -544,6 +541,13 @@ vt_ctx* vt_create(const vt_mesh_desc* d, int device, int* status) {
     const int x = columns[n];
     const int4 b = nbr[x];
     c->side_pairing = nbr[b.x].x == x && nbr[b.y].y == x && nbr[b.z].z == x;
+  }
+  c->mutual_tiles = c->side_pairing || (c->ntiles <= sms && vt::tiles_read_mutually(K, d->neighbours, columns.data(),
+                                                                                     vt::kTileElems, c->ntiles));
+  if ((e = vt::use_resident(c, sk, sms))) {
+    set(fail(VT_ERR_CUDA, vt::cuda_msg("resident kernel attributes", e)));
+    release(c);
+    return nullptr;
   }
   // W_i = integral of phi_i = sum_j M_ref[i][j] (the basis sums to one)
   std::vector<double> m(d->inv_mass_ref, d->inv_mass_ref + c->Np * c->Np), W(c->Np, 0.0);
@@ -657,6 +661,7 @@ vt_ctx* vt_create_structured(const vt_params* prm, const vt_vortex* ic_in, int d
     return nullptr;
   }
   c->max_blocks = sms * (per_sm > 0 ? per_sm : 1);
+  c->mutual_tiles = true;
   if ((e = vt::use_resident(c, sk, sms))) {
     set(fail(VT_ERR_CUDA, vt::cuda_msg("resident kernel attributes", e)));
     release(c);
