@@ -36,7 +36,8 @@ struct vt_ctx {
   std::vector<double> minv_ref;  // Np x Np, for the projected initial condition
   vt::LaunchFn launch = nullptr;
   // many steps in one launch, for a problem of few tiles (null otherwise): the
-  // kernel, the tiles' flags and what they hold (unknown after an error)
+  // kernel, the tiles' flags and what they hold (unknown after an error);
+  // flag_launches: steps whose outcome finish() has still to see
   decltype(vt::StageKernel::resident) resident = nullptr;
   unsigned* flags = nullptr;
   unsigned flag_base = 0;

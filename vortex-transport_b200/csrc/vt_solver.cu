@@ -406,6 +406,9 @@ cudaError_t enqueue_resident(vt_ctx* c, double dt, int nsteps, bool euler) {
 }
 
 cudaError_t reset_error_words(vt_ctx* c) {
+  // a wait of earlier resident steps that gave up is not seen from here on, so
+  // nothing may be concluded about their flags
+  c->flag_launches = false;
   cudaError_t e = cudaMemsetAsync(c->err, 0xFF, sizeof(unsigned long long), c->stream);
   if (e) return e;
   return cudaMemsetAsync(c->err + 1, 0, (kErrWords - 1) * sizeof(unsigned long long), c->stream);
@@ -413,6 +416,8 @@ cudaError_t reset_error_words(vt_ctx* c) {
 
 // Waits for the stream, decodes the first-error key and advances the clock.
 int finish(vt_ctx* c, int nsteps, double dt) {
+  const bool flag_launches = c->flag_launches;
+  c->flag_launches = false;
   unsigned long long words[4] = {~0ull, 0, 0, 0};
   cudaError_t e = cudaMemcpyAsync(words, c->err, sizeof(words), cudaMemcpyDeviceToHost, c->stream);
   if (!e) e = cudaStreamSynchronize(c->stream);
@@ -421,8 +426,7 @@ int finish(vt_ctx* c, int nsteps, double dt) {
   c->last = vt_error_info{};
   if (words[3] & 2ull)
     return fail(VT_ERR_CUDA, "stage kernel: a bulk-copy wait gave up (the state is not valid)");
-  if (c->flag_launches) c->flags_known = true;
-  c->flag_launches = false;
+  if (flag_launches) c->flags_known = true;
   const unsigned long long key = words[0];
   if (key == ~0ull) return VT_OK;
   c->last = vt::decode_error_key(key, c->nfq);
