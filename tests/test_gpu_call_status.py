@@ -1,4 +1,7 @@
-"""What one call leaves for the next: a wait that gave up does not fail later calls."""
+"""What one call leaves for the next: failures of asynchronous steps survive a
+derivative call in between, and a wait that gave up does not fail later calls."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -59,5 +62,26 @@ def test_steps_after_an_unseen_wait_that_gave_up(vt):
     s.rk4(dt, 3)
     b.rk4(3)
     np.testing.assert_array_equal(s.download(), b.download(0))
+    s.close()
+    b.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(8, 8), (72, 70)])
+def test_jvp_keeps_the_failure_of_asynchronous_steps(vt, nx, ny):
+    s, b, pb, dt = make(vt, nx, ny)
+    good = pb.array("U0")
+    V = np.random.default_rng(0).standard_normal(good.shape)
+    want = s.rhs_jvp(good, V)
+    U = good.copy()
+    U[17, :, 0] = -1.0
+    s.upload(U)
+    s.rk4_async(dt, 2)
+    np.testing.assert_array_equal(s.rhs_jvp(good, V), want)
+    with pytest.raises(vt.NonPhysicalState) as e:
+        s.synchronize()
+    info = vt.vt_error_info()
+    s.rhs_jvp(good, V)  # and the record of it
+    assert vt.lib().vt_last_error(s._h, ctypes.byref(info)) == 0
+    assert info.code == e.value.code != 0 and info.element == e.value.element
     s.close()
     b.close()

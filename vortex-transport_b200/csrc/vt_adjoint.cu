@@ -483,8 +483,9 @@ cudaError_t store_aos(vt_ctx* c, const double2* src, double* dst, int device_poi
   return e;
 }
 
-// out1 = x1 + c1 dk, out2 = x2 + c2 dk with dk = R'(U) V (JvpArgs).
-cudaError_t jvp(vt_ctx* c, const double2* U, const double2* V, double2* out1, const double2* x1 = nullptr, double c1 = 0.0,
+// out1 = x1 + c1 dk, out2 = x2 + c2 dk with dk = R'(U) V (JvpArgs); a wait that
+// gives up shows in `flags`.
+cudaError_t jvp(vt_ctx* c, unsigned long long* flags, const double2* U, const double2* V, double2* out1, const double2* x1 = nullptr, double c1 = 0.0,
                 double2* out2 = nullptr, const double2* x2 = nullptr, double c2 = 0.0) {
   const StageKernel k = select_kernel(c->p, c->nfq, c->ops.data(), c->map);
   int per_sm = 0, sms = 0;
@@ -496,6 +497,7 @@ cudaError_t jvp(vt_ctx* c, const double2* U, const double2* V, double2* out1, co
   j.x1 = x1, j.x2 = x2;
   j.out1 = out1, j.out2 = out2;
   j.c1 = c1, j.c2 = c2;
+  j.flags = flags;
   StageArgs a = stage_args(c, U, U, c->A, out1, kStageRhs, 0.0, 0.0);
   a.test_flags = 0;  // the test hook is the stage kernel's
   return k.jvp(a, j, c->block.data(), sms * std::max(1, per_sm), c->stream);
@@ -631,11 +633,16 @@ int vt_rhs_jvp(vt_ctx* c, const double* U, const double* V, double* dR, int devi
   s->fresh = false;
   cudaError_t e = vt::load_aos(c, U, device_pointers, s->s1);
   if (!e) e = vt::load_aos(c, V, device_pointers, s->s2);
-  if (!e) e = vt::reset_error_words(c);
-  if (!e) e = vt::jvp(c, s->s1, s->s2, s->s3);
+  // a flag word of its own: steps that are still under way (vt_step_rk4_async)
+  // keep their outcome for vt_synchronize, and vt_last_error its record
+  unsigned long long flags = 0, *word = c->err + 7;
+  if (!e) e = cudaMemsetAsync(word, 0, sizeof(flags), c->stream);
+  if (!e) e = vt::jvp(c, word, s->s1, s->s2, s->s3);
   if (!e) e = vt::store_aos(c, s->s3, dR, device_pointers);
+  if (!e) e = cudaMemcpyAsync(&flags, word, sizeof(flags), cudaMemcpyDeviceToHost, c->stream);
+  if (!e) e = cudaStreamSynchronize(c->stream);
   if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("rhs jvp", e));
-  return vt::finish(c, 0, 0.0);
+  return flags ? fail(VT_ERR_CUDA, "vt_rhs_jvp: a bulk-copy wait gave up") : VT_OK;
 }
 
 int vt_rhs_vjp(vt_ctx* c, const double* U, const double* W, double* G, int device_pointers) {
@@ -680,10 +687,10 @@ int vt_tangent_rk4(vt_ctx* c, double dt, int nsteps, const double* dU_0, double*
     // the stage directions alternate between dS and dT: a launch must not
     // overwrite the direction whose neighbours its own tiles still read
     if ((e = vt::stage_step(c, X, dt, nullptr))) break;
-    if ((e = vt::jvp(c, X, dX, dacc, dX, (1.0 / 6) * dt, dS, dX, 0.5 * dt))) break;
-    if ((e = vt::jvp(c, s->s1, dS, dacc, dacc, (1.0 / 3) * dt, dT, dX, 0.5 * dt))) break;
-    if ((e = vt::jvp(c, s->s2, dT, dacc, dacc, (1.0 / 3) * dt, dS, dX, dt))) break;
-    if ((e = vt::jvp(c, s->s3, dS, dX, dacc, (1.0 / 6) * dt))) break;
+    if ((e = vt::jvp(c, c->err + 3, X, dX, dacc, dX, (1.0 / 6) * dt, dS, dX, 0.5 * dt))) break;
+    if ((e = vt::jvp(c, c->err + 3, s->s1, dS, dacc, dacc, (1.0 / 3) * dt, dT, dX, 0.5 * dt))) break;
+    if ((e = vt::jvp(c, c->err + 3, s->s2, dT, dacc, dacc, (1.0 / 3) * dt, dS, dX, dt))) break;
+    if ((e = vt::jvp(c, c->err + 3, s->s3, dS, dX, dacc, (1.0 / 6) * dt))) break;
     e = vt::stage(c, s->s3, X, c->U, 3, 0.0, (1.0 / 6) * dt, c->stream);
   }
   if (!e) e = vt::store_aos(c, dX, dU_T, device_pointers);

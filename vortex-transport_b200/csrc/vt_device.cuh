@@ -222,7 +222,8 @@ enum : int { kTestNoCopies = 1 };
 // The words behind `err`, cleared before every call (word 0 to all ones):
 // [0] first-error key, [1] steps done, [2] blocks of the running stage kernel
 // that are done, [3] flags (1 bad neighbour, 2 a wait gave up), [4] tiles its
-// blocks have taken beyond their first, [5], [6] likewise of the reverse stage.
+// blocks have taken beyond their first, [5], [6] likewise of the reverse stage,
+// [7] the flags of vt_rhs_jvp, which leaves the other words as they are.
 constexpr int kErrWords = 8;
 
 constexpr int kMaxItems = 3 * kTileElems;

@@ -22,6 +22,7 @@ struct JvpArgs {
   const double2 *x1, *x2;  // out1 = x1 + c1 dk, out2 = x2 + c2 dk; x1 null: out1 = dk; out2 may be null
   double2 *out1, *out2;
   double c1, c2;
+  unsigned long long* flags;  // the error word whose bit 1 says that a wait gave up
 };
 
 template <int P, int NFQ>
@@ -103,7 +104,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 1)
       bool ok = false;
       for (unsigned n = 0; n < kMaxWaitTries && !ok; ++n) ok = mbar_try_wait(bar, parity);
       if (!ok) {
-        atomicOr(&a.err[3], 2ull);
+        atomicOr(ja.flags, 2ull);
         *abort_flag = 1;
       }
     }
