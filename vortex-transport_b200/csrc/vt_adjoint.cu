@@ -66,10 +66,10 @@ cudaError_t launch_element(const AdjArgs& a, const double* ops, cudaStream_t st)
 }
 
 // One reverse stage as one persistent launch over the stage kernel's tiles.
-template <int P, int NFQ>
+template <int P, int NFQ, bool FAR>
 cudaError_t launch_tile(const AdjArgs& a, const double* block, int max_blocks, cudaStream_t st) {
   const int grid = a.ntiles < max_blocks ? a.ntiles : max_blocks;
-  return launch_dependent(adjoint_tile_kernel<P, NFQ>, grid, 4 * kTileElems, AdjTileLayout<P, NFQ>::kBytes, st, a,
+  return launch_dependent(adjoint_tile_kernel<P, NFQ, FAR>, grid, 4 * kTileElems, AdjTileLayout<P, NFQ>::kBytes, st, a,
                           *reinterpret_cast<const AdjOps<P, NFQ>*>(block));
 }
 
@@ -84,44 +84,45 @@ std::vector<double> pack_tile(const double* ops) {
   return std::vector<double>(b, b + sizeof(block) / sizeof(double));
 }
 
-template <int P, int NFQ>
+template <int P, int NFQ, bool FAR>
 cudaError_t configure_tile(int* blocks_per_sm) {
   constexpr int bytes = AdjTileLayout<P, NFQ>::kBytes;
-  cudaError_t e = cudaFuncSetAttribute(adjoint_tile_kernel<P, NFQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  cudaError_t e = cudaFuncSetAttribute(adjoint_tile_kernel<P, NFQ, FAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, adjoint_tile_kernel<P, NFQ>, 4 * kTileElems,
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, adjoint_tile_kernel<P, NFQ, FAR>, 4 * kTileElems,
                                                        bytes);
 }
 
 template <int P, int NFQ>
-AdjKernels kernels_of() {
-  return AdjKernels{launch_face<P, NFQ>, launch_element<P, NFQ>, launch_tile<P, NFQ>,
-                    configure_tile<P, NFQ>, pack_tile<P, NFQ>};
+AdjKernels kernels_of(bool far) {
+  return AdjKernels{launch_face<P, NFQ>, launch_element<P, NFQ>,
+                    far ? launch_tile<P, NFQ, true> : launch_tile<P, NFQ, false>,
+                    far ? configure_tile<P, NFQ, true> : configure_tile<P, NFQ, false>, pack_tile<P, NFQ>};
 }
 
 template <int P>
-AdjKernels kernels_for_nfq(int nfq) {
+AdjKernels kernels_for_nfq(int nfq, bool far) {
   switch (nfq) {
-    case 1: return kernels_of<P, 1>();
-    case 2: return kernels_of<P, 2>();
-    case 3: return kernels_of<P, 3>();
-    case 4: return kernels_of<P, 4>();
-    case 5: return kernels_of<P, 5>();
-    case 6: return kernels_of<P, 6>();
-    case 7: return kernels_of<P, 7>();
-    case 8: return kernels_of<P, 8>();
-    case 9: return kernels_of<P, 9>();
-    case 10: return kernels_of<P, 10>();
+    case 1: return kernels_of<P, 1>(far);
+    case 2: return kernels_of<P, 2>(far);
+    case 3: return kernels_of<P, 3>(far);
+    case 4: return kernels_of<P, 4>(far);
+    case 5: return kernels_of<P, 5>(far);
+    case 6: return kernels_of<P, 6>(far);
+    case 7: return kernels_of<P, 7>(far);
+    case 8: return kernels_of<P, 8>(far);
+    case 9: return kernels_of<P, 9>(far);
+    case 10: return kernels_of<P, 10>(far);
     default: return AdjKernels{};
   }
 }
 
-AdjKernels select_adjoint(int p, int nfq) {
+AdjKernels select_adjoint(int p, int nfq, bool far) {
   switch (p) {
-    case 0: return kernels_for_nfq<0>(nfq);
-    case 1: return kernels_for_nfq<1>(nfq);
-    case 2: return kernels_for_nfq<2>(nfq);
-    case 3: return kernels_for_nfq<3>(nfq);
+    case 0: return kernels_for_nfq<0>(nfq, far);
+    case 1: return kernels_for_nfq<1>(nfq, far);
+    case 2: return kernels_for_nfq<2>(nfq, far);
+    case 3: return kernels_for_nfq<3>(nfq, far);
     default: return AdjKernels{};
   }
 }
@@ -185,7 +186,7 @@ int setup(vt_ctx* c) {
   if (c->adj) return VT_OK;
   if (!c->side_pairing)
     return fail(VT_ERR_UNSUPPORTED, "adjoint: side s of some element does not face side s of its neighbour");
-  const AdjKernels k = select_adjoint(c->p, c->nfq);
+  const AdjKernels k = select_adjoint(c->p, c->nfq, c->far);
   if (!k.face) return fail(VT_ERR_UNSUPPORTED, "adjoint: unsupported (p, nfq)");
   // The edge-once form needs every edge to join elements whose sides face each
   // other with opposite normals; a 2-colouring of the element adjacency
@@ -219,10 +220,8 @@ int setup(vt_ctx* c) {
   // the fused reverse stage runs on the stage kernel's tiles, with the folded operators
   int tile_blocks = 0;
   if (ok && operators_reflect(c->p, c->nfq, c->ops.data())) {
-    int per_sm = 0, sms = 0;
-    if (c->ntiles > 0 && !k.tile_config(&per_sm) &&
-        !cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) && per_sm > 0)
-      tile_blocks = sms * per_sm;
+    int per_sm = 0;
+    if (c->ntiles > 0 && !k.tile_config(&per_sm) && per_sm > 0) tile_blocks = c->sms * per_sm;
     cudaGetLastError();
   }
   // eleven state vectors, plus the face adjoints of the two-launch form when
@@ -487,10 +486,9 @@ cudaError_t store_aos(vt_ctx* c, const double2* src, double* dst, int device_poi
 // gives up shows in `flags`.
 cudaError_t jvp(vt_ctx* c, unsigned long long* flags, const double2* U, const double2* V, double2* out1, const double2* x1 = nullptr, double c1 = 0.0,
                 double2* out2 = nullptr, const double2* x2 = nullptr, double c2 = 0.0) {
-  const StageKernel k = select_kernel(c->p, c->nfq, c->ops.data(), c->map);
-  int per_sm = 0, sms = 0;
-  cudaError_t e = k.configure_jvp(&per_sm);
-  if (!e) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+  const StageKernel k = select_kernel(c->p, c->nfq, c->ops.data(), c->far, c->map);
+  int per_sm = 0;
+  const cudaError_t e = k.configure_jvp(&per_sm);
   if (e) return e;
   JvpArgs j;
   j.U = U, j.V = V;
@@ -500,7 +498,7 @@ cudaError_t jvp(vt_ctx* c, unsigned long long* flags, const double2* U, const do
   j.flags = flags;
   StageArgs a = stage_args(c, U, U, c->A, out1, kStageRhs, 0.0, 0.0);
   a.test_flags = 0;  // the test hook is the stage kernel's
-  return k.jvp(a, j, c->block.data(), sms * std::max(1, per_sm), c->stream);
+  return k.jvp(a, j, c->block.data(), c->sms * std::max(1, per_sm), c->stream);
 }
 
 int prepare(vt_ctx* c) {

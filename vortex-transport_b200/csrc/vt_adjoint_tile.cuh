@@ -171,7 +171,7 @@ __device__ __forceinline__ void folded_adjoint(const double* Ad, double* e, doub
 // Two 256-thread blocks per SM: the transposed Roe Jacobian needs more than the
 // 80 registers of three blocks, and two leave shared memory for the stage
 // adjoint tile.
-template <int P, int NFQ>
+template <int P, int NFQ, bool FAR>
 __global__ void __launch_bounds__(4 * kTileElems, 2)
     adjoint_tile_kernel(const __grid_constant__ AdjArgs a, const AdjOps<P, NFQ> ops) {
   const FoldedOps<P, NFQ>& fo = ops.fo;
@@ -303,15 +303,6 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
       const int fl = it & 63, s = (it >> 6) & 3, x = it >> 9;
       const bool mirror = (it >> 8) & 1;
       const double2 n = GE[((fl >> 5) * kGeoRows + 4 + s) * kTileRun + (fl & 31)];
-      // a neighbour without a slot: its column and its lift's scale
-      const bool far = !mirror && x == kNoSlot;
-      long long nb = 0;
-      double sc = 0.0;
-      if (far) {
-        nb = __ldg(reinterpret_cast<const int*>(a.nbr + (static_cast<long long>(tile) * E + fl)) + s);
-        const double* gn = reinterpret_cast<const double*>(a.geo + geo_index(nb, s < 2 ? 2 : 3));
-        sc = -0.5 * sa * __ldg(gn + (s == 1 ? 1 : 0));
-      }
 #pragma unroll 1
       for (; q < q1; ++q) {
         const int qm = NFQ - 1 - q;
@@ -333,39 +324,19 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
           if (mirror) {  // the partner's own trace at its point nfq-1-q, as the stage kernel reads it
             y0 = S[sidx<NP>(2 * node, x)];
             y1 = S[sidx<NP>(2 * node + 1, x)];
-          } else if (!far) {
+          } else {
             y0 = H[2 * k * 2 * kSlots + x];
             y1 = H[(2 * k + 1) * 2 * kSlots + x];
-          } else {
-            const double2* src = a.U + state_index(NP, nb, 2 * node);
-            y0 = __ldg(src);
-            y1 = __ldg(src + kTileRun);
           }
           um[0] = fma(cm[k], y0.x, um[0]);
           um[1] = fma(cm[k], y0.y, um[1]);
           um[2] = fma(cm[k], y1.x, um[2]);
           um[3] = fma(cm[k], y1.y, um[3]);
         }
-        if (!far) {
-          const double2* m = mirror ? oth : HA + 4 * q * kSlots + x;
-          const double2 m0 = m[0], m1 = m[mirror ? E : 2 * kSlots];
-          bf[0] = b0.x - m0.x, bf[1] = b0.y - m0.y, bf[2] = b1.x - m1.x, bf[3] = b1.y - m1.y;
-        } else {
-          // the neighbour's lifted adjoint at its point nfq-1-q
-          double v[4] = {0.0, 0.0, 0.0, 0.0};
-          const double* lf = LF + (s * NFQ + qm) * NP;
-          const double2* src = a.a + state_index(NP, nb, 0);
-#pragma unroll
-          for (int i = 0; i < NP; ++i) {
-            const double2 a0 = __ldg(src + 2 * i * kTileRun), a1 = __ldg(src + (2 * i + 1) * kTileRun);
-            v[0] = fma(lf[i], a0.x, v[0]);
-            v[1] = fma(lf[i], a0.y, v[1]);
-            v[2] = fma(lf[i], a1.x, v[2]);
-            v[3] = fma(lf[i], a1.y, v[3]);
-          }
-          bf[0] = fma(-sc, v[0], b0.x), bf[1] = fma(-sc, v[1], b0.y);
-          bf[2] = fma(-sc, v[2], b1.x), bf[3] = fma(-sc, v[3], b1.y);
-        }
+        // the partner's or the neighbour's lifted adjoint at its point nfq-1-q
+        const double2* m = mirror ? oth : HA + 4 * q * kSlots + x;
+        const double2 m0 = m[0], m1 = m[mirror ? E : 2 * kSlots];
+        bf[0] = b0.x - m0.x, bf[1] = b0.y - m0.y, bf[2] = b1.x - m1.x, bf[3] = b1.y - m1.y;
         double bu[4], bv[4];
         roe_flux2_vjp(up, um, n.x, n.y, bf, bu, bv);
         own[0] = make_double2(bu[0], bu[1]);
@@ -374,6 +345,45 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
           oth[0] = make_double2(bv[0], bv[1]);
           oth[E] = make_double2(bv[2], bv[3]);
         }
+      }
+    }
+    if constexpr (FAR) {
+      FarFace x;
+      for (int w = t; far_face<NFQ>(faces, items, a.nbr, tile, w, &x); w += T) {
+        const double2 n = GE[((x.col >> 5) * kGeoRows + 4 + x.s) * kTileRun + (x.col & 31)];
+        double2* own = FB2 + (x.s * NFQ + x.q) * 2 * E + x.col;
+        const double2 b0 = own[0], b1 = own[E];
+        double up[4] = {0.0, 0.0, 0.0, 0.0}, um[4];
+        const double* cp = TP + (x.s * NFQ + x.q) * NE;
+#pragma unroll
+        for (int k = 0; k < NE; ++k) {
+          const int node = x.s == 0 ? edge_node(P, 0, k) : (x.s == 1 ? edge_node(P, 1, k) : edge_node(P, 2, k));
+          const double2 x0 = S[sidx<NP>(2 * node, x.col)], x1 = S[sidx<NP>(2 * node + 1, x.col)];
+          up[0] = fma(cp[k], x0.x, up[0]);
+          up[1] = fma(cp[k], x0.y, up[1]);
+          up[2] = fma(cp[k], x1.x, up[2]);
+          up[3] = fma(cp[k], x1.y, up[3]);
+        }
+        far_trace<P>(a.U, x, TM + (x.s * NFQ + x.q) * NE, um, [](const double2* p) { return __ldg(p); });
+        // the neighbour's lifted adjoint at its point nfq-1-q
+        const double* gn = reinterpret_cast<const double*>(a.geo + geo_index(x.nb, x.s < 2 ? 2 : 3));
+        const double sc = -0.5 * sa * __ldg(gn + (x.s == 1 ? 1 : 0));
+        double v[4] = {0.0, 0.0, 0.0, 0.0};
+        const double* lf = LF + (x.s * NFQ + NFQ - 1 - x.q) * NP;
+        const double2* src = a.a + state_index(NP, x.nb, 0);
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+          const double2 a0 = __ldg(src + 2 * i * kTileRun), a1 = __ldg(src + (2 * i + 1) * kTileRun);
+          v[0] = fma(lf[i], a0.x, v[0]);
+          v[1] = fma(lf[i], a0.y, v[1]);
+          v[2] = fma(lf[i], a1.x, v[2]);
+          v[3] = fma(lf[i], a1.y, v[3]);
+        }
+        const double bf[4] = {fma(-sc, v[0], b0.x), fma(-sc, v[1], b0.y), fma(-sc, v[2], b1.x), fma(-sc, v[3], b1.y)};
+        double bu[4], bv[4];
+        roe_flux2_vjp(up, um, n.x, n.y, bf, bu, bv);
+        own[0] = make_double2(bu[0], bu[1]);
+        own[E] = make_double2(bu[2], bu[3]);
       }
     }
     if (t == 224) *NEXT = hand_out ? static_cast<int>(taken) + G : tile + G;

@@ -70,6 +70,7 @@ struct Group {
     k.pack(ops.data(), block.data());
   }
   int max_blocks = 0;
+  bool far = false;  // a tile has more leaving faces than slots
   double2 *U = nullptr, *A = nullptr, *Sa = nullptr, *Sb = nullptr, *geo = nullptr;
   int4* nbr = nullptr;
   int* elem = nullptr;
@@ -250,6 +251,7 @@ int ensure_views(vt_batch* b) {
     for (size_t m = 0; m < G.members.size(); ++m)
       c->parts.push_back({G.num[m], static_cast<long long>(vt::kTileElems) * G.tile_begin[m], 4ll * G.Np * G.offset[m],
                           static_cast<long long>(instance_offset(b, G.members[m]))});
+    c->sms = b->sms;
     c->max_blocks = G.max_blocks;
     c->stream = b->stream;
     c->U = G.U;
@@ -260,6 +262,7 @@ int ensure_views(vt_batch* b) {
     c->nbr = G.nbr;
     c->elem = G.elem;
     c->lists = G.lists;
+    c->far = G.far;
     c->ntiles = G.ntiles;
     c->err = G.err;
     c->ops = G.ops;
@@ -373,14 +376,6 @@ vt_batch* vt_batch_create(const vt_mesh_desc* descs, int n, int device, int* sta
   }
   size_t max_inst_bytes = 0;
   for (auto& G : b->groups) {
-    G.use(vt::select_kernel(G.p, G.nfq, G.ops.data()));
-    int per_sm = 0;
-    if ((e = G.kern.configure(&per_sm))) {
-      set(fail(VT_ERR_CUDA, vt::cuda_msg("stage kernel attributes", e)));
-      release(b);
-      return nullptr;
-    }
-    G.max_blocks = b->sms * (per_sm > 0 ? per_sm : 1);
     // each member's columns, and so its tiles, follow the previous member's
     for (size_t m = 0; m < G.members.size(); ++m) {
       const vt_mesh_desc& d = descs[G.members[m]];
@@ -396,6 +391,7 @@ vt_batch* vt_batch_create(const vt_mesh_desc* descs, int n, int device, int* sta
       vt::pack_mesh(descs[G.members[m]], vt::element_columns(G.num[m]), geo.data(), nbr.data(),
                     static_cast<long long>(vt::kTileElems) * G.tile_begin[m]);
     const size_t state_bytes = sizeof(double2) * 2 * G.Np * static_cast<size_t>(G.ncols);
+    unsigned long long far = 0;
     if ((e = vt::dalloc(&G.U, state_bytes)) || (e = vt::dalloc(&G.A, state_bytes)) ||
         (e = vt::dalloc(&G.Sa, state_bytes)) || (e = vt::dalloc(&G.Sb, state_bytes)) ||
         (e = vt::dalloc(&G.geo, geo.size() * sizeof(double2))) || (e = vt::dalloc(&G.nbr, nbr.size() * sizeof(int4))) ||
@@ -412,12 +408,24 @@ vt_batch* vt_batch_create(const vt_mesh_desc* descs, int n, int device, int* sta
         (e = cudaMemset(G.U, 0, state_bytes)) || (e = cudaMemset(G.A, 0, state_bytes)) ||
         (e = cudaMemset(G.Sa, 0, state_bytes)) || (e = cudaMemset(G.Sb, 0, state_bytes)) ||
         (e = cudaMemset(G.tile_dt, 0, sizeof(double) * G.ntiles)) || (e = number_members(b, G)) ||
-        (e = vt::launch_build_tile_lists(G.nbr, G.elem, static_cast<int>(G.K), G.ntiles, G.nfq, G.lists, b->stream)) ||
+        (e = cudaMemset(G.err, 0, sizeof(far))) ||
+        (e = vt::launch_build_tile_lists(G.nbr, G.elem, static_cast<int>(G.K), G.ntiles, G.nfq, G.lists, G.err,
+                                         b->stream)) ||
+        (e = cudaMemcpyAsync(&far, G.err, sizeof(far), cudaMemcpyDeviceToHost, b->stream)) ||
         (e = cudaStreamSynchronize(b->stream))) {
       set(fail(VT_ERR_CUDA, vt::cuda_msg("vt_batch_create upload", e)));
       release(b);
       return nullptr;
     }
+    G.far = far & 1ull;
+    G.use(vt::select_kernel(G.p, G.nfq, G.ops.data(), G.far));
+    int per_sm = 0;
+    if ((e = G.kern.configure(&per_sm))) {
+      set(fail(VT_ERR_CUDA, vt::cuda_msg("stage kernel attributes", e)));
+      release(b);
+      return nullptr;
+    }
+    G.max_blocks = b->sms * (per_sm > 0 ? per_sm : 1);
   }
   if ((e = vt::dalloc(&b->staging, max_inst_bytes))) {
     set(fail(VT_ERR_NO_MEMORY, vt::cuda_msg("vt_batch_create staging", e)));
@@ -706,7 +714,7 @@ int vt_batch_autotune(vt_batch* b, int trials, int* blocks_per_sm_out, int* mapp
     int best_b = 1;
     float best_ms = 1e30f;
     for (int map : {vt::kMapComponent, vt::kMapDefault}) {
-      const vt::StageKernel k = vt::select_kernel(G.p, G.nfq, G.ops.data(), map);
+      const vt::StageKernel k = vt::select_kernel(G.p, G.nfq, G.ops.data(), G.far, map);
       int limit = 0;
       if (k.configure(&limit)) continue;
       G.use(k);
@@ -753,7 +761,7 @@ int vt_batch_set_mapping(vt_batch* b, const int* mapping) {
     if (mapping[gi] != vt::kMapComponent && mapping[gi] != vt::kMapDefault)
       return fail(VT_ERR_INVALID, "vt_batch_set_mapping: mapping must be 0 (component) or 1 (pair)");
     vt::Group& G = b->groups[gi];
-    const vt::StageKernel k = vt::select_kernel(G.p, G.nfq, G.ops.data(), mapping[gi]);
+    const vt::StageKernel k = vt::select_kernel(G.p, G.nfq, G.ops.data(), G.far, mapping[gi]);
     int limit = 0;
     const cudaError_t e = k.configure(&limit);
     if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("vt_batch_set_mapping", e));

@@ -20,13 +20,14 @@ struct vt_ctx {
   int device = 0, p = 0, Np = 0, nfq = 0, K = 0;
   vt::Numbering num;
   long long ncols = 0;  // columns: 64 per tile
-  int max_blocks = 0;  // persistent grid: SMs x resident blocks per SM
+  int sms = 0, max_blocks = 0;  // persistent grid: SMs x resident blocks per SM
   cudaStream_t stream = nullptr;
   double2 *U = nullptr, *A = nullptr, *Sa = nullptr, *Sb = nullptr, *R = nullptr;
   double2* geo = nullptr;
   int4* nbr = nullptr;
   int* elem = nullptr;              // element of each column
   unsigned char* lists = nullptr;   // per-tile face lists
+  bool far = false;                 // a tile has more leaving faces than slots (launch_build_tile_lists)
   int ntiles = 0;
   unsigned long long* err = nullptr;
   double2* aos = nullptr;
@@ -86,6 +87,11 @@ StageArgs stage_args(vt_ctx* c, const double2* in, const double2* base, double2*
 cudaError_t enqueue_rk4_step(vt_ctx* c, double dt);
 // Clears the first-error key and the step counters.
 cudaError_t reset_error_words(vt_ctx* c);
+// Builds the tiles' face lists, waits for them and sets c->far.
+cudaError_t build_lists(vt_ctx* c);
+// Takes the context's stage kernel of form `map` (and, where it may, the
+// resident one) into use.
+cudaError_t use_kernel(vt_ctx* c, int map);
 // Waits for the stream, decodes the first-error key, advances the clock by
 // nsteps * dt and returns the status.
 int finish(vt_ctx* c, int nsteps, double dt);

@@ -185,9 +185,9 @@ struct Numbering {
 // lists holds kTileListBytes per tile, built once per mesh (vt_schedule.cuh):
 //   uint16 [kMaxItems]  the (column, side) faces the tile evaluates, by class:
 //     both columns in the tile, the neighbour staged in a slot, the neighbour
-//     read from global memory (no slot left). Bits 0-5 the column in the tile,
-//     6-7 the side, 8 both in the tile, 9-15 the neighbour's column in the tile
-//     or its slot (kNoSlot: none);
+//     read from global memory (no slot left: FarFace, vt_tile.cuh). Bits 0-5 the
+//     column in the tile, 6-7 the side, 8 both in the tile, 9-15 the neighbour's
+//     column in the tile or its slot;
 //   uint32 [4]  the work items (FaceCounts);
 //   uint32 [2][kSlots]  per block, the neighbours to stage: 4 * column + side,
 //     kNoNeighbour where a slot is empty (the used slots come first).
@@ -238,26 +238,26 @@ constexpr int kListOuter = kListCount + 16;    // byte offset of the slots
 constexpr int kTileListBytes = kListOuter + kOuterWords * 4;
 static_assert(kListCount % 16 == 0 && kTileListBytes % 16 == 0, "16-byte copies");
 constexpr unsigned kNoNeighbour = 0xffffffffu;
-constexpr int kNoSlot = 127;
 
 __host__ __device__ constexpr unsigned face_item(int col, int side, bool inside, int x) {
   return static_cast<unsigned>(col | (side << 6) | (inside ? 1 << 8 : 0) | (x << 9));
 }
 
 // The work items of a face list: first the n0 faces inside the tile times the
-// parts of their nfq points (p0 points each), then the n1 others (p1 points
+// parts of their nfq points (p0 points each), then the n1 with a slot (p1 points
 // each), part-major: item w < first is part w / n0 of face w % n0. The factor
 // 2^20 / n + 1 makes w / n one multiplication, exact while w n < 2^20 (w < 10 n,
-// n <= 192).
+// n <= 192). The n2 faces without a slot are the end of the list (FarFace,
+// vt_tile.cuh).
 struct FaceCounts {
-  unsigned n;        // n0 | n1 << 16
+  unsigned n;        // n0 | n1 << 8 | n2 << 16
   unsigned points;   // p0 | p1 << 8 | first << 16 (the items of the faces inside the tile)
   unsigned factor0, factor1;
 };
 __host__ __device__ constexpr unsigned face_factor(int n) { return n > 0 ? (1u << 20) / n + 1 : 0; }
 
-__host__ __device__ constexpr FaceCounts face_counts(int n0, int n1, int nfq, int p0, int p1) {
-  return {static_cast<unsigned>(n0 | n1 << 16), static_cast<unsigned>(p0 | p1 << 8 | (n0 * ((nfq + p0 - 1) / p0)) << 16),
+__host__ __device__ constexpr FaceCounts face_counts(int n0, int n1, int n2, int nfq, int p0, int p1) {
+  return {static_cast<unsigned>(n0 | n1 << 8 | n2 << 16), static_cast<unsigned>(p0 | p1 << 8 | (n0 * ((nfq + p0 - 1) / p0)) << 16),
           face_factor(n0), face_factor(n1)};
 }
 // What the face phase costs a thread with i and j points per item, in tenths of
@@ -270,9 +270,9 @@ __device__ __forceinline__ int face_cost(int n0, int n1, int nfq, int i, int j, 
 // Work item w: its entry in the list and its points [q0, q1); false past the last one.
 template <int NFQ>
 __device__ __forceinline__ bool face_work(const FaceCounts& f, int w, int* entry, int* q0, int* q1) {
-  const int first = f.points >> 16, n0 = f.n & 0xffff;
+  const int first = f.points >> 16, n0 = f.n & 0xff;
   const bool in = w < first;
-  const int v = in ? w : w - first, n = in ? n0 : f.n >> 16, pts = in ? f.points & 0xff : (f.points >> 8) & 0xff;
+  const int v = in ? w : w - first, n = in ? n0 : (f.n >> 8) & 0xff, pts = in ? f.points & 0xff : (f.points >> 8) & 0xff;
   if (n == 0) return false;
   const int part = static_cast<int>((v * (in ? f.factor0 : f.factor1)) >> 20);
   *q0 = part * pts;

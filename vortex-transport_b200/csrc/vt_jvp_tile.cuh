@@ -34,7 +34,7 @@ struct JvpLayout {
   static constexpr int kBytes = kFV + 6 * NFQ * kTileElems * 16;
 };
 
-template <int P, int NFQ, int MAP>
+template <int P, int NFQ, int MAP, bool FAR>
 __global__ void __launch_bounds__(4 * kTileElems, 1)
     jvp_tile_kernel(const __grid_constant__ StageArgs a, const __grid_constant__ JvpArgs ja,
                     const OpsOf<P, NFQ, MAP> ops) {
@@ -125,9 +125,6 @@ __global__ void __launch_bounds__(4 * kTileElems, 1)
       const int fl = it & 63, s = (it >> 6) & 3, x = it >> 9;
       const bool mirror = (it >> 8) & 1;
       const double2 n = GE[((fl >> 5) * kGeoRows + 4 + s) * kTileRun + (fl & 31)];
-      const int nb = !mirror && x == kNoSlot
-                         ? __ldg(reinterpret_cast<const int*>(a.nbr + (static_cast<long long>(tile) * E + fl)) + s)
-                         : 0;
       int own = (s * NFQ + q) * 2 * E + fl, oth = (s * NFQ + NFQ - 1 - q) * 2 * E + (mirror ? x : 0);
 #pragma unroll 1
       for (; q < q1; ++q, own += 2 * E, oth -= 2 * E) {
@@ -142,16 +139,8 @@ __global__ void __launch_bounds__(4 * kTileElems, 1)
           const double* cm = TM + (s * NFQ + q) * NE;
 #pragma unroll
           for (int k = 0; k < NE; ++k) {
-            double2 n0, n1, m0, m1;
-            if (x != kNoSlot) {
-              n0 = H[2 * k * 2 * kSlots + x], n1 = H[(2 * k + 1) * 2 * kSlots + x];
-              m0 = HV[2 * k * 2 * kSlots + x], m1 = HV[(2 * k + 1) * 2 * kSlots + x];
-            } else {
-              const int node = s == 0 ? edge_node(P, 0, k) : (s == 1 ? edge_node(P, 1, k) : edge_node(P, 2, k));
-              const long long at = state_index(NP, nb, 2 * node);
-              n0 = __ldg(ja.U + at), n1 = __ldg(ja.U + at + kTileRun);
-              m0 = __ldg(ja.V + at), m1 = __ldg(ja.V + at + kTileRun);
-            }
+            const double2 n0 = H[2 * k * 2 * kSlots + x], n1 = H[(2 * k + 1) * 2 * kSlots + x];
+            const double2 m0 = HV[2 * k * 2 * kSlots + x], m1 = HV[(2 * k + 1) * 2 * kSlots + x];
             um[0] = fma(cm[k], n0.x, um[0]), um[1] = fma(cm[k], n0.y, um[1]);
             um[2] = fma(cm[k], n1.x, um[2]), um[3] = fma(cm[k], n1.y, um[3]);
             dm[0] = fma(cm[k], m0.x, dm[0]), dm[1] = fma(cm[k], m0.y, dm[1]);
@@ -166,6 +155,22 @@ __global__ void __launch_bounds__(4 * kTileElems, 1)
           FV2[oth] = make_double2(-f[0], -f[1]);
           FV2[oth + E] = make_double2(-f[2], -f[3]);
         }
+      }
+    }
+    if constexpr (FAR) {
+      FarFace x;
+      for (int w = t; far_face<NFQ>(faces, items, a.nbr, tile, w, &x); w += T) {
+        const double2 n = GE[((x.col >> 5) * kGeoRows + 4 + x.s) * kTileRun + (x.col & 31)];
+        const int own = (x.s * NFQ + x.q) * 2 * E + x.col;
+        const double2 u0 = FU2[own], u1 = FU2[own + E], v0 = FV2[own], v1 = FV2[own + E];
+        const double up[4] = {u0.x, u0.y, u1.x, u1.y}, dp[4] = {v0.x, v0.y, v1.x, v1.y};
+        double um[4], dm[4], f[4];
+        const double* cm = TM + (x.s * NFQ + x.q) * NE;
+        far_trace<P>(ja.U, x, cm, um, [](const double2* p) { return __ldg(p); });
+        far_trace<P>(ja.V, x, cm, dm, [](const double2* p) { return __ldg(p); });
+        roe_flux2_jvp(up, um, n.x, n.y, dp, dm, f);
+        FV2[own] = make_double2(f[0], f[1]);
+        FV2[own + E] = make_double2(f[2], f[3]);
       }
     }
     __syncthreads();

@@ -1,5 +1,5 @@
 // Kernel selection by (p, nfq, form of the operators) -- the instantiations are in
-// vt_stage_component.cu and vt_stage_folded.cu -- and the tile schedule kernels
+// vt_stage_component.cu, vt_stage_folded.cu and their _far forms -- and the tile schedule kernels
 // (vt_launch.h).
 #include <algorithm>
 #include <cmath>
@@ -10,9 +10,10 @@
 
 namespace vt {
 
-StageKernel select_kernel(int p, int nfq, const double* ops, int map) {
+StageKernel select_kernel(int p, int nfq, const double* ops, bool far, int map) {
   const bool fold = map == kMapDefault && operators_reflect(p, nfq, ops);
-  StageKernel k = fold ? select_kernel_folded(p, nfq) : select_kernel_component(p, nfq);
+  StageKernel k = far ? (fold ? select_kernel_folded_far(p, nfq) : select_kernel_component_far(p, nfq))
+                      : (fold ? select_kernel_folded(p, nfq) : select_kernel_component(p, nfq));
   k.map = map;
   return k;
 }
@@ -81,8 +82,8 @@ cudaError_t launch_number_columns(const Numbering& num, int* elem, int x0, int e
 }
 
 cudaError_t launch_build_tile_lists(const int4* nbr, const int* elem, int K, int ntiles, int nfq, unsigned char* lists,
-                                    cudaStream_t st) {
-  build_tile_lists_kernel<<<ntiles, 256, 0, st>>>(nbr, elem, K, nfq, lists);
+                                    unsigned long long* far, cudaStream_t st) {
+  build_tile_lists_kernel<<<ntiles, 256, 0, st>>>(nbr, elem, K, nfq, lists, far);
   return cudaGetLastError();
 }
 

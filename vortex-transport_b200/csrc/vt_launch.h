@@ -64,10 +64,14 @@ constexpr int kDefaultMap = kMapDefault;
 // The kernel for the operator block `ops` (stage_ops_doubles(p, nfq) doubles):
 // kMapDefault takes the folded form where operators_reflect says so, else the
 // same kernel as kMapComponent.
+// `far`: a tile of the mesh may have a face without a slot (launch_build_tile_lists
+// tells; the kernels for such meshes are right for any, and a little slower).
 // Empty (null members) for p outside 0..3, nfq outside 1..10.
-StageKernel select_kernel(int p, int nfq, const double* ops, int map = kDefaultMap);
+StageKernel select_kernel(int p, int nfq, const double* ops, bool far, int map = kDefaultMap);
 StageKernel select_kernel_component(int p, int nfq);
 StageKernel select_kernel_folded(int p, int nfq);
+StageKernel select_kernel_component_far(int p, int nfq);
+StageKernel select_kernel_folded_far(int p, int nfq);
 
 // Whether the operator block has the reference triangle's reflection symmetry
 // (vt_device.cuh) to 1e-13 of each operator's largest entry, a few roundings
@@ -98,9 +102,10 @@ Numbering number_contiguous(int K);
 // elem[x0 + x] = e0 + element of the numbering's column x (-1: empty).
 cudaError_t launch_number_columns(const Numbering& num, int* elem, int x0, int e0, cudaStream_t st);
 // The tiles' face lists (kTileListBytes each, 16-byte aligned) from the columns'
-// neighbours and elements (elem null: contiguous numbering of K elements).
+// neighbours and elements (elem null: contiguous numbering of K elements). Bit 0
+// of `far` (when given) is set if a tile has more leaving faces than slots.
 cudaError_t launch_build_tile_lists(const int4* nbr, const int* elem, int K, int ntiles, int nfq, unsigned char* lists,
-                                    cudaStream_t st);
+                                    unsigned long long* far, cudaStream_t st);
 // The callers' layout (K x Np x 4 doubles, 16-byte aligned) <-> a state vector's columns.
 cudaError_t launch_to_columns(const double* aos, double2* columns, const Numbering& num, int Np, cudaStream_t st);
 cudaError_t launch_from_columns(const double2* columns, double* aos, const Numbering& num, int Np, cudaStream_t st);

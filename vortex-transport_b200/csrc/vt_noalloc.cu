@@ -143,7 +143,9 @@ int vt_step_rk4_noalloc(const vt_device_mesh* m, const double* dU_in, double* dU
   double ops[vt::kMaxOps];
   vt::fold_stage_operators(m->p, m->n_line_points, m->inv_mass_ref, m->stiffness_ref, m->line_quadrature,
                            m->phi_plus, m->phi_minus, ops);
-  const vt::StageKernel pk = vt::select_kernel(m->p, m->n_line_points, ops);
+  // the contiguous numbering leaves more faces of a tile than slots from 23 cells
+  // a row on, and nothing here waits to see whether it does
+  const vt::StageKernel pk = vt::select_kernel(m->p, m->n_line_points, ops, true);
   double block[vt::kMaxOps];
   pk.pack(ops, block);
 
@@ -188,7 +190,7 @@ int vt_step_rk4_noalloc(const vt_device_mesh* m, const double* dU_in, double* dU
       (e = cudaMemsetAsync(errw + 1, 0, (vt::kErrWords - 1) * sizeof(unsigned long long), st)))
     return fail(VT_ERR_CUDA, std::string("scratch reset: ") + cudaGetErrorString(e));
   vt::pack_geometry_kernel<<<(K + 255) / 256, 256, 0, st>>>(*m, cv.num, geo, nbr, errw);
-  if ((e = vt::launch_build_tile_lists(nbr, nullptr, K, cv.num.ntiles, m->n_line_points, lists, st)))
+  if ((e = vt::launch_build_tile_lists(nbr, nullptr, K, cv.num.ntiles, m->n_line_points, lists, nullptr, st)))
     return fail(VT_ERR_CUDA, std::string("tile schedule: ") + cudaGetErrorString(e));
   if ((e = vt::launch_to_columns(dU_in, U, cv.num, Np, st))) return fail(VT_ERR_CUDA, std::string("pack: ") + cudaGetErrorString(e));
 

@@ -156,7 +156,7 @@ __device__ __forceinline__ void pair_sync(int t) {
   asm volatile("bar.sync %0, 64;" ::"r"(3 + ((t >> 5) & 7)) : "memory");
 }
 
-template <int P, int NFQ, int MAP>
+template <int P, int NFQ, int MAP, bool FAR>
 __global__ void __launch_bounds__(resident_threads(MAP), 1)
     resident_steps_kernel(const __grid_constant__ StageArgs a, const __grid_constant__ ResidentArgs ra,
                           const OpsOf<P, NFQ, MAP> ops) {
@@ -222,12 +222,12 @@ __global__ void __launch_bounds__(resident_threads(MAP), 1)
     }
   }
   if constexpr (T != 4 * E) {  // points per work item for this number of threads
-    const int n0 = counts->n & 0xffff, n1 = counts->n >> 16, i = 1 + t / NFQ, j = 1 + t % NFQ;
+    const int n0 = counts->n & 0xff, n1 = (counts->n >> 8) & 0xff, i = 1 + t / NFQ, j = 1 + t % NFQ;
     if (t < NFQ * NFQ) atomicMin(&least, static_cast<unsigned>(face_cost(n0, n1, NFQ, i, j, T) << 8 | (NFQ * NFQ - 1 - t)));
     __syncthreads();
     if (t == 0) {
       const int best = NFQ * NFQ - 1 - (least & 0xff);
-      *counts = face_counts(n0, n1, NFQ, 1 + best / NFQ, 1 + best % NFQ);
+      *counts = face_counts(n0, n1, counts->n >> 16, NFQ, 1 + best / NFQ, 1 + best % NFQ);
     }
   }
   __syncthreads();
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(resident_threads(MAP), 1)
       atomicOr(&a.err[3], 2ull);
       *abort_flag = 1;
     }
-    if (t == 0 && *late_flag) *abort_flag = 1;
+    if (FAR && t == 0 && *late_flag) *abort_flag = 1;
 
     // ---- 2. nodal flux; the neighbours' side nodes; own traces ----------------------
     if (P > 0) {
@@ -293,14 +293,6 @@ __global__ void __launch_bounds__(resident_threads(MAP), 1)
       const double2 n = GE[((fl >> 5) * kGeoRows + 4 + sd) * kTileRun + (fl & 31)];
       double2* own = FB2 + (sd * NFQ + q) * 2 * E + fl;
       double2* oth = FB2 + (sd * NFQ + NFQ - 1 - q) * 2 * E + (mirror ? x : 0);
-      int nb = 0;
-      if (!mirror && x == kNoSlot) {
-        nb = __ldg(reinterpret_cast<const int*>(a.nbr + (static_cast<long long>(tile) * E + fl)) + sd);
-        if (!wait_for_tile(ra.flags, nb / kTileElems, ra.flag0 + s, flag_tries)) {
-          atomicOr(&a.err[3], 2ull);
-          *late_flag = 1;
-        }
-      }
       auto outer = [&](int q0, auto& um) {
         constexpr int N = sizeof(um) / sizeof(um[0]);
 #pragma unroll
@@ -308,16 +300,7 @@ __global__ void __launch_bounds__(resident_threads(MAP), 1)
         const double* cm = TM + (sd * NFQ + q0) * NE;
 #pragma unroll
         for (int j = 0; j < NE; ++j) {
-          double2 n0, n1;
-          if (x != kNoSlot) {
-            n0 = H[2 * j * 2 * kSlots + x];
-            n1 = H[(2 * j + 1) * 2 * kSlots + x];
-          } else {
-            const int node = sd == 0 ? edge_node(P, 0, j) : (sd == 1 ? edge_node(P, 1, j) : edge_node(P, 2, j));
-            const double2* src = in + state_index(NP, nb, 2 * node);
-            n0 = __ldcg(src);
-            n1 = __ldcg(src + kTileRun);
-          }
+          const double2 n0 = H[2 * j * 2 * kSlots + x], n1 = H[(2 * j + 1) * 2 * kSlots + x];
 #pragma unroll
           for (int k = 0; k < N; ++k) {
             um[k][0] = fma(cm[k * NE + j], n0.x, um[k][0]);
@@ -335,6 +318,24 @@ __global__ void __launch_bounds__(resident_threads(MAP), 1)
         q += done;
         own += done * 2 * E;
         oth -= done * 2 * E;
+      }
+    }
+    if constexpr (FAR) {
+      FarFace x;
+      for (int w = t; far_face<NFQ>(faces, items, a.nbr, tile, w, &x); w += T) {
+        if (!wait_for_tile(ra.flags, x.nb / kTileElems, ra.flag0 + s, flag_tries)) {
+          atomicOr(&a.err[3], 2ull);
+          *late_flag = 1;
+        }
+        const double2 n = GE[((x.col >> 5) * kGeoRows + 4 + x.s) * kTileRun + (x.col & 31)];
+        face_points<P, NFQ, 1>(FB2 + (x.s * NFQ + x.q) * 2 * E + x.col, nullptr, false, n, x.q,
+                               [&](int q0, auto& um) {
+                                 far_trace<P>(in, x, TM + (x.s * NFQ + q0) * NE, um[0],
+                                              [](const double2* p) { return __ldcg(p); });
+                               },
+                               [&](int point, int err) {
+                                 record_error_at(a.err, epoch, NFQ, EL[x.col], point, x.s, err);
+                               });
       }
     }
     __syncthreads();

@@ -89,8 +89,9 @@ __device__ __forceinline__ int side_of(const int4& n, int s) { return s == 0 ? n
 // number for both (3 and the normals copied apart from the other geometry), 5
 // RK4 steps at 768 x 768, p = 3 went from 7.98 to 7.94 ms, 20 at 384 x 384,
 // p = 1 from 4.10 to 4.06 ms.
+// Bit 0 of `far` (when given) is set if any tile has a face without a slot.
 __global__ void build_tile_lists_kernel(const int4* __restrict__ nbr, const int* __restrict__ elem, int K, int nfq,
-                                        unsigned char* __restrict__ lists) {
+                                        unsigned char* __restrict__ lists, unsigned long long* __restrict__ far) {
   __shared__ int warp_n[3][8], warp_out[2][8];
   const int tile = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
   unsigned char* list = lists + static_cast<long long>(tile) * kTileListBytes;
@@ -131,21 +132,21 @@ __global__ void build_tile_lists_kernel(const int4* __restrict__ nbr, const int*
     if (lane == 0) warp_n[k][warp] = __popc(m[k]);
   }
   __syncthreads();
-  int n = 0, rank = 0, n_cls[3] = {0, 0, 0};  // position within the (class 0, class 1, class 2) order
+  int rank = 0, n_cls[3] = {0, 0, 0};  // position within the (class 0, class 1, class 2) order
   for (int k = 0; k < 3; ++k)
     for (int w = 0; w < 8; ++w) {
-      n += warp_n[k][w];
       n_cls[k] += warp_n[k][w];
       if (k < cls || (k == cls && w < warp)) rank += warp_n[k][w];
     }
   rank += __popc(m[cls] & ((1u << lane) - 1u));
   if (take) {
-    const int y = inside ? nb % kTileElems : (cls == 1 ? second * kSlots + slot : kNoSlot);
+    const int y = inside ? nb % kTileElems : (cls == 1 ? second * kSlots + slot : 0);
     items[rank] = static_cast<unsigned short>(face_item(col, s, inside, y));
     if (cls == 1) outer[second * kSlots + slot] = 4u * static_cast<unsigned>(nb) + static_cast<unsigned>(s);
   }
   if (t == 0) {
-    const int n0 = n_cls[0], n1 = n - n0;
+    const int n0 = n_cls[0], n1 = n_cls[1];
+    if (far && n_cls[2]) atomicOr(far, 1ull);
     int p0 = 1, p1 = 1, least = 0;  // in tenths of a point
     for (int i = 1; i <= nfq; ++i)
       for (int j = 1; j <= nfq; ++j) {
@@ -155,7 +156,7 @@ __global__ void build_tile_lists_kernel(const int4* __restrict__ nbr, const int*
           p0 = i, p1 = j;
         }
       }
-    *counts = face_counts(n0, n1, nfq, p0, p1);
+    *counts = face_counts(n0, n1, n_cls[2], nfq, p0, p1);
   }
 }
 

@@ -366,9 +366,9 @@ cudaError_t enqueue_rk4_step(vt_ctx* c, double dt) {
 // launch per stage is right for any). With more tiles than SMs its blocks would share an SM,
 // for which it has neither the shared memory (p = 3) nor the warps: the stage
 // kernel's three blocks per SM then hide what it saves.
-cudaError_t use_resident(vt_ctx* c, const StageKernel& k, int sms) {
+cudaError_t use_resident(vt_ctx* c, const StageKernel& k) {
   c->resident = nullptr;
-  if (c->ntiles > sms || !c->mutual_tiles) return cudaSuccess;
+  if (c->ntiles > c->sms || !c->mutual_tiles) return cudaSuccess;
   int per_sm = 0, coop = 0;
   cudaError_t e = k.configure_resident(&per_sm);
   if (!e) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device);
@@ -376,6 +376,31 @@ cudaError_t use_resident(vt_ctx* c, const StageKernel& k, int sms) {
   if (!c->flags) e = alloc(&c->flags, sizeof(unsigned) * kFlagStride * c->ntiles);
   if (!e) c->resident = k.resident;
   return e;
+}
+
+cudaError_t build_lists(vt_ctx* c) {
+  // the flag goes through the first error word, which every call clears
+  unsigned long long far = 0;
+  cudaError_t e = cudaMemsetAsync(c->err, 0, sizeof(far), c->stream);
+  if (!e) e = launch_build_tile_lists(c->nbr, c->elem, c->K, c->ntiles, c->nfq, c->lists, c->err, c->stream);
+  if (!e) e = cudaMemcpyAsync(&far, c->err, sizeof(far), cudaMemcpyDeviceToHost, c->stream);
+  if (!e) e = cudaStreamSynchronize(c->stream);
+  c->far = far & 1ull;
+  return e;
+}
+
+cudaError_t use_kernel(vt_ctx* c, int map) {
+  const StageKernel k = select_kernel(c->p, c->nfq, c->ops.data(), c->far, map);
+  int per_sm = 0;
+  cudaError_t e = k.configure(&per_sm);
+  if (!e) e = use_resident(c, k);
+  if (e) return e;
+  c->launch = k.launch;
+  c->block.resize(c->ops.size() + kBlockExtra);
+  k.pack(c->ops.data(), c->block.data());
+  c->map = map;
+  c->max_blocks = c->sms * (per_sm > 0 ? per_sm : 1);
+  return cudaSuccess;
 }
 
 // nsteps steps by the resident kernel, at most kResidentSteps a launch.
@@ -518,18 +543,11 @@ vt_ctx* vt_create(const vt_mesh_desc* d, int device, int* status) {
   c->ncols = static_cast<long long>(vt::kTileElems) * c->ntiles;
   c->ops = vt::host_operators(c->p, c->nfq, d->inv_mass_ref, d->stiffness_ref, d->line_quadrature,
                               d->phi_plus, d->phi_minus);
-  const vt::StageKernel sk = vt::select_kernel(c->p, c->nfq, c->ops.data());
-  c->launch = sk.launch;
-  c->block.resize(c->ops.size() + vt::kBlockExtra);
-  sk.pack(c->ops.data(), c->block.data());
-  int per_sm = 0, sms = 0;
-  if ((e = sk.configure(&per_sm)) ||
-      (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device))) {
-    set(fail(VT_ERR_CUDA, vt::cuda_msg("stage kernel attributes", e)));
+  if ((e = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device))) {
+    set(fail(VT_ERR_CUDA, vt::cuda_msg("device attributes", e)));
     delete c;
     return nullptr;
   }
-  c->max_blocks = sms * (per_sm > 0 ? per_sm : 1);
   c->minv_ref.assign(d->inv_mass_ref, d->inv_mass_ref + c->Np * c->Np);
 
   // packed geometry and side-ordered neighbours (Evolve.cpp:167-202), by column
@@ -546,13 +564,8 @@ vt_ctx* vt_create(const vt_mesh_desc* d, int device, int* status) {
     const int4 b = nbr[x];
     c->side_pairing = nbr[b.x].x == x && nbr[b.y].y == x && nbr[b.z].z == x;
   }
-  c->mutual_tiles = c->side_pairing || (c->ntiles <= sms && vt::tiles_read_mutually(K, d->neighbours, columns.data(),
-                                                                                     vt::kTileElems, c->ntiles));
-  if ((e = vt::use_resident(c, sk, sms))) {
-    set(fail(VT_ERR_CUDA, vt::cuda_msg("resident kernel attributes", e)));
-    release(c);
-    return nullptr;
-  }
+  c->mutual_tiles = c->side_pairing || (c->ntiles <= c->sms && vt::tiles_read_mutually(K, d->neighbours, columns.data(),
+                                                                                       vt::kTileElems, c->ntiles));
   // W_i = integral of phi_i = sum_j M_ref[i][j] (the basis sums to one)
   std::vector<double> m(d->inv_mass_ref, d->inv_mass_ref + c->Np * c->Np), W(c->Np, 0.0);
   vt::invert_gauss_jordan(c->Np, &m);
@@ -583,8 +596,8 @@ vt_ctx* vt_create(const vt_mesh_desc* d, int device, int* status) {
     return nullptr;
   }
   e = vt::launch_number_columns(c->num, c->elem, 0, 0, c->stream);
-  if (!e) e = vt::launch_build_tile_lists(c->nbr, c->elem, K, c->ntiles, c->nfq, c->lists, c->stream);
-  if (!e) e = cudaStreamSynchronize(c->stream);
+  if (!e) e = vt::build_lists(c);
+  if (!e) e = vt::use_kernel(c, vt::kDefaultMap);
   if (e) {
     set(fail(VT_ERR_CUDA, vt::cuda_msg("tile schedule", e)));
     release(c);
@@ -653,24 +666,12 @@ vt_ctx* vt_create_structured(const vt_params* prm, const vt_vortex* ic_in, int d
   c->ntiles = c->num.ntiles;
   c->ncols = static_cast<long long>(vt::kTileElems) * c->ntiles;
   c->ops = vt::host_operators(p, nfq, minv.data(), stiff.data(), line.data(), pp.data(), pm.data());
-  const vt::StageKernel sk = vt::select_kernel(p, nfq, c->ops.data());
-  c->launch = sk.launch;
-  c->block.resize(c->ops.size() + vt::kBlockExtra);
-  sk.pack(c->ops.data(), c->block.data());
-  int per_sm = 0, sms = 0;
-  if ((e = sk.configure(&per_sm)) ||
-      (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device))) {
-    set(fail(VT_ERR_CUDA, vt::cuda_msg("stage kernel attributes", e)));
+  if ((e = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device))) {
+    set(fail(VT_ERR_CUDA, vt::cuda_msg("device attributes", e)));
     delete c;
     return nullptr;
   }
-  c->max_blocks = sms * (per_sm > 0 ? per_sm : 1);
   c->mutual_tiles = true;
-  if ((e = vt::use_resident(c, sk, sms))) {
-    set(fail(VT_ERR_CUDA, vt::cuda_msg("resident kernel attributes", e)));
-    release(c);
-    return nullptr;
-  }
   c->minv_ref = minv;
   c->side_pairing = true;
   std::vector<double> m(minv), W(Np, 0.0);
@@ -740,8 +741,8 @@ vt_ctx* vt_create_structured(const vt_params* prm, const vt_vortex* ic_in, int d
       e = cudaGetLastError();
     }
   }
-  if (!e) e = vt::launch_build_tile_lists(c->nbr, c->elem, c->K, c->ntiles, c->nfq, c->lists, c->stream);
-  if (!e) e = cudaStreamSynchronize(c->stream);
+  if (!e) e = vt::build_lists(c);
+  if (!e) e = vt::use_kernel(c, vt::kDefaultMap);
   cudaFree(verts);
   if (dtab) cudaFree(dtab);
   if (e) {
@@ -1012,17 +1013,8 @@ int vt_set_stage_mapping(vt_ctx* c, int mapping) {
     return fail(VT_ERR_INVALID, "vt_set_stage_mapping: mapping must be 0 (component) or 1 (pair)");
   std::lock_guard<std::mutex> lk(c->mu);
   cudaSetDevice(c->device);
-  const vt::StageKernel sk = vt::select_kernel(c->p, c->nfq, c->ops.data(), mapping);
-  int per_sm = 0, sms = 0;
-  cudaError_t e = sk.configure(&per_sm);
-  if (!e) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-  if (!e) e = vt::use_resident(c, sk, sms);
-  if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("vt_set_stage_mapping", e));
-  c->launch = sk.launch;
-  sk.pack(c->ops.data(), c->block.data());
-  c->map = mapping;
-  c->max_blocks = sms * (per_sm > 0 ? per_sm : 1);
-  return VT_OK;
+  const cudaError_t e = vt::use_kernel(c, mapping);
+  return e ? fail(VT_ERR_CUDA, vt::cuda_msg("vt_set_stage_mapping", e)) : VT_OK;
 }
 
 int vt_get_stage_mapping(const vt_ctx* c) { return c ? c->map : -1; }

@@ -2,5 +2,5 @@
 #include "vt_stage_inst.cuh"
 
 namespace vt {
-StageKernel select_kernel_folded(int p, int nfq) { return stage_inst::select_for_map<kMapFolded>(p, nfq); }
+StageKernel select_kernel_folded(int p, int nfq) { return stage_inst::select_for_map<kMapFolded, false>(p, nfq); }
 }  // namespace vt

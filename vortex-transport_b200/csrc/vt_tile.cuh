@@ -516,6 +516,45 @@ __device__ __forceinline__ unsigned neighbour_code(const unsigned char* lists, i
                which * kSlots + lane);
 }
 
+// Face points of faces whose neighbour has no slot: a tile has up to 192 leaving
+// faces where the elements' order does not follow the mesh (33 per half where it
+// follows its rows, from 23 cells a row on). Only the kernels with FAR take them,
+// and a mesh without such faces takes the others: the loop costs registers. Point
+// w is point w % nfq of far face w / nfq, so that the lanes of a warp read the
+// same few neighbours' nodes; when each lane had a face of its own, as in the
+// list's other classes, and read it again for each of its points, 4 RK4 steps at
+// 200 x 200 cells in random order, p = 3 took 1.55 ms (now 0.80) and a gradient
+// of 10 steps 20.8 (now 8.8).
+struct FarFace {
+  int col, s, q;  // column in the tile, side, point
+  int nb;         // the neighbour's column
+};
+template <int NFQ>
+__device__ __forceinline__ bool far_face(const FaceCounts& f, const unsigned short* items, const int4* nbr, int tile, int w,
+                                         FarFace* x) {
+  const int k = w / NFQ;
+  if (k >= static_cast<int>(f.n >> 16)) return false;
+  const int it = items[(f.n & 0xff) + ((f.n >> 8) & 0xff) + k];
+  x->col = it & 63, x->s = (it >> 6) & 3, x->q = w - k * NFQ;
+  x->nb = __ldg(reinterpret_cast<const int*>(nbr + (static_cast<long long>(tile) * kTileElems + x->col)) + x->s);
+  return true;
+}
+// The neighbour's trace there: weights cm of its side nodes, loaded by ld.
+template <int P, typename Load>
+__device__ __forceinline__ void far_trace(const double2* v, const FarFace& x, const double* cm, double* um, Load&& ld) {
+  um[0] = um[1] = um[2] = um[3] = 0.0;
+#pragma unroll
+  for (int k = 0; k <= P; ++k) {
+    const int node = x.s == 0 ? edge_node(P, 0, k) : (x.s == 1 ? edge_node(P, 1, k) : edge_node(P, 2, k));
+    const double2* src = v + state_index(np_of_p(P), x.nb, 2 * node);
+    const double2 n0 = ld(src), n1 = ld(src + kTileRun);
+    um[0] = fma(cm[k], n0.x, um[0]);
+    um[1] = fma(cm[k], n0.y, um[1]);
+    um[2] = fma(cm[k], n1.x, um[2]);
+    um[3] = fma(cm[k], n1.y, um[3]);
+  }
+}
+
 template <int P, int NFQ, int MAP>
 struct OpsOfMap {
   using type = StageOps<P, NFQ>;
@@ -527,7 +566,7 @@ struct OpsOfMap<P, NFQ, kMapFolded> {
 template <int P, int NFQ, int MAP>
 using OpsOf = typename OpsOfMap<P, NFQ, MAP>::type;
 
-template <int P, int NFQ, int MAP>
+template <int P, int NFQ, int MAP, bool FAR>
 // Three 256-thread blocks per SM (<= 80 registers per thread) keep 24 warps
 // resident alongside 3 x ~75 KB of shared memory.
 __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __grid_constant__ StageArgs a,
@@ -635,19 +674,12 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
         } else {
           um[0] = um[1] = um[2] = um[3] = 0.0;
           const double* cm = TM + (s * NFQ + q) * NE;
-#pragma unroll
+          // all 2 NE loads in flight would take the registers of the flux: 5 RK4
+          // steps at 768 x 768, p = 3 took 6.78 ms (two nodes at a time 6.61,
+          // one 6.67), 20 at 384 x 384, p = 1 4.12 (one 4.06)
+#pragma unroll(P == 3 ? 2 : 1)
           for (int k = 0; k < NE; ++k) {
-            double2 n0, n1;
-            if (x != kNoSlot) {
-              n0 = H[2 * k * 2 * kSlots + x];
-              n1 = H[(2 * k + 1) * 2 * kSlots + x];
-            } else {
-              const int node = s == 0 ? edge_node(P, 0, k) : (s == 1 ? edge_node(P, 1, k) : edge_node(P, 2, k));
-              const int nb = __ldg(reinterpret_cast<const int*>(a.nbr + (static_cast<long long>(tile) * E + fl)) + s);
-              const double2* src = a.in + state_index(NP, nb, 2 * node);
-              n0 = __ldg(src);
-              n1 = __ldg(src + kTileRun);
-            }
+            const double2 n0 = H[2 * k * 2 * kSlots + x], n1 = H[(2 * k + 1) * 2 * kSlots + x];
             um[0] = fma(cm[k], n0.x, um[0]);
             um[1] = fma(cm[k], n0.y, um[1]);
             um[2] = fma(cm[k], n1.x, um[2]);
@@ -662,6 +694,20 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
           oth[0] = make_double2(-f[0], -f[1]);
           oth[E] = make_double2(-f[2], -f[3]);
         }
+      }
+    }
+    if constexpr (FAR) {
+      FarFace x;
+      for (int w = t; far_face<NFQ>(faces, items, a.nbr, tile, w, &x); w += T) {
+        const double2 n = GE[((x.col >> 5) * kGeoRows + 4 + x.s) * kTileRun + (x.col & 31)];
+        double2* own = FB2 + (x.s * NFQ + x.q) * 2 * E + x.col;
+        const double2 x0 = own[0], x1 = own[E];
+        const double up[4] = {x0.x, x0.y, x1.x, x1.y};
+        double um[4], f[4];
+        far_trace<P>(a.in, x, TM + (x.s * NFQ + x.q) * NE, um, [](const double2* p) { return __ldg(p); });
+        roe_flux2(up, um, n.x, n.y, f, [&](int err) { record_error(a, NFQ, EL[x.col], x.q, x.s, err); });
+        own[0] = make_double2(f[0], f[1]);
+        own[E] = make_double2(f[2], f[3]);
       }
     }
     if (t == 224) *NEXT = hand_out ? static_cast<int>(taken) + G : tile + G;
