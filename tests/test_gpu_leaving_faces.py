@@ -128,3 +128,25 @@ def test_gradient(vt):
     np.testing.assert_allclose(got, want, rtol=0, atol=1e-11 * np.abs(want).max())
     r.close()
     s.close()
+
+
+def test_batches_made_in_a_row(vt):
+    """A batch's set-up is ordered on its own stream: what it learns about its
+    lists does not depend on when the default stream's work is done."""
+    import torch
+    pb = problem(vt, 80, 70, 1, 4)
+    m = Reordered(vt, pb, orders(pb.K)["random"])
+    dt = small_dt(80, 70, 1)
+    r = vt.Solver((m.desc, m.keep))
+    r.upload(m.U)
+    r.rk4(dt, 3)
+    want = r.download()
+    busy = torch.zeros(1 << 26, dtype=torch.float64, device="cuda")
+    for _ in range(12):
+        busy.add_(1.0)  # work under way on the default stream
+        b = vt.Batch([m])
+        b.set_dt([dt])
+        b.rk4(3)
+        np.testing.assert_array_equal(b.download(0), want)
+        b.close()
+    r.close()

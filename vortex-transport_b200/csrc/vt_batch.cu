@@ -403,12 +403,14 @@ vt_batch* vt_batch_create(const vt_mesh_desc* descs, int n, int device, int* sta
       release(b);
       return nullptr;
     }
-    if ((e = cudaMemcpy(G.geo, geo.data(), geo.size() * sizeof(double2), cudaMemcpyHostToDevice)) ||
-        (e = cudaMemcpy(G.nbr, nbr.data(), nbr.size() * sizeof(int4), cudaMemcpyHostToDevice)) ||
-        (e = cudaMemset(G.U, 0, state_bytes)) || (e = cudaMemset(G.A, 0, state_bytes)) ||
-        (e = cudaMemset(G.Sa, 0, state_bytes)) || (e = cudaMemset(G.Sb, 0, state_bytes)) ||
-        (e = cudaMemset(G.tile_dt, 0, sizeof(double) * G.ntiles)) || (e = number_members(b, G)) ||
-        (e = cudaMemset(G.err, 0, sizeof(far))) ||
+    // everything in the order of the batch's own stream, which does not wait for the default one
+    const cudaStream_t st = b->stream;
+    if ((e = cudaMemcpyAsync(G.geo, geo.data(), geo.size() * sizeof(double2), cudaMemcpyHostToDevice, st)) ||
+        (e = cudaMemcpyAsync(G.nbr, nbr.data(), nbr.size() * sizeof(int4), cudaMemcpyHostToDevice, st)) ||
+        (e = cudaMemsetAsync(G.U, 0, state_bytes, st)) || (e = cudaMemsetAsync(G.A, 0, state_bytes, st)) ||
+        (e = cudaMemsetAsync(G.Sa, 0, state_bytes, st)) || (e = cudaMemsetAsync(G.Sb, 0, state_bytes, st)) ||
+        (e = cudaMemsetAsync(G.tile_dt, 0, sizeof(double) * G.ntiles, st)) || (e = number_members(b, G)) ||
+        (e = cudaMemsetAsync(G.err, 0, sizeof(far), st)) ||
         (e = vt::launch_build_tile_lists(G.nbr, G.elem, static_cast<int>(G.K), G.ntiles, G.nfq, G.lists, G.err,
                                          b->stream)) ||
         (e = cudaMemcpyAsync(&far, G.err, sizeof(far), cudaMemcpyDeviceToHost, b->stream)) ||
@@ -740,7 +742,8 @@ int vt_batch_autotune(vt_batch* b, int trials, int* blocks_per_sm_out, int* mapp
   if (err) return fail(VT_ERR_CUDA, vt::cuda_msg("vt_batch_autotune", err));
   for (size_t gi = 0; gi < b->groups.size(); ++gi) {
     vt::Group& G = b->groups[gi];
-    if (cudaMemcpy(G.U, saved[gi].data(), saved[gi].size() * sizeof(double2), cudaMemcpyHostToDevice))
+    if (cudaMemcpyAsync(G.U, saved[gi].data(), saved[gi].size() * sizeof(double2), cudaMemcpyHostToDevice, b->stream) ||
+        cudaStreamSynchronize(b->stream))
       return fail(VT_ERR_CUDA, "autotune restore");
   }
   for (size_t gi = 0; gi < b->views.size(); ++gi) {  // the adjoint's group views step with the chosen kernels
@@ -798,7 +801,8 @@ int vt_batch_time_groups(vt_batch* b, int reps, float* ms_per_step) {
     if (!e) e = cudaEventSynchronize(e1);
     float ms = 0;
     if (!e) e = cudaEventElapsedTime(&ms, e0, e1);
-    if (!e) e = cudaMemcpy(G.U, saved.data(), state * sizeof(double2), cudaMemcpyHostToDevice);
+    if (!e) e = cudaMemcpyAsync(G.U, saved.data(), state * sizeof(double2), cudaMemcpyHostToDevice, b->stream);
+    if (!e) e = cudaStreamSynchronize(b->stream);
     st = e ? fail(VT_ERR_CUDA, vt::cuda_msg("vt_batch_time_groups", e)) : check_waits(G, "vt_batch_time_groups");
     ms_per_step[gi] = ms / reps;
   }

@@ -586,11 +586,13 @@ vt_ctx* vt_create(const vt_mesh_desc* d, int device, int* status) {
     release(c);
     return nullptr;
   }
-  if ((e = cudaMemcpy(c->geo, geo.data(), geo.size() * sizeof(double2), cudaMemcpyHostToDevice)) ||
-      (e = cudaMemcpy(c->nbr, nbr.data(), nbr.size() * sizeof(int4), cudaMemcpyHostToDevice)) ||
-      (e = cudaMemcpy(c->W, W.data(), sizeof(double) * c->Np, cudaMemcpyHostToDevice)) ||
-      (e = cudaMemset(c->U, 0, state_bytes)) || (e = cudaMemset(c->A, 0, state_bytes)) ||
-      (e = cudaMemset(c->Sa, 0, state_bytes)) || (e = cudaMemset(c->Sb, 0, state_bytes))) {
+  // everything in the order of the context's own stream, which does not wait for the default one
+  const cudaStream_t st = c->stream;
+  if ((e = cudaMemcpyAsync(c->geo, geo.data(), geo.size() * sizeof(double2), cudaMemcpyHostToDevice, st)) ||
+      (e = cudaMemcpyAsync(c->nbr, nbr.data(), nbr.size() * sizeof(int4), cudaMemcpyHostToDevice, st)) ||
+      (e = cudaMemcpyAsync(c->W, W.data(), sizeof(double) * c->Np, cudaMemcpyHostToDevice, st)) ||
+      (e = cudaMemsetAsync(c->U, 0, state_bytes, st)) || (e = cudaMemsetAsync(c->A, 0, state_bytes, st)) ||
+      (e = cudaMemsetAsync(c->Sa, 0, state_bytes, st)) || (e = cudaMemsetAsync(c->Sb, 0, state_bytes, st))) {
     set(fail(VT_ERR_CUDA, vt::cuda_msg("vt_create upload", e)));
     release(c);
     return nullptr;
