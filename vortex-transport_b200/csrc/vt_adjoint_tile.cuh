@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
           up[2] = fma(cp[k], x1.x, up[2]);
           up[3] = fma(cp[k], x1.y, up[3]);
         }
-        far_trace<P>(a.U, x, TM + (x.s * NFQ + x.q) * NE, um, [](const double2* p) { return __ldg(p); });
+        far_trace<P>(a.U, x, TM + (x.s * NFQ + x.q) * NE, um, [](const double2* p) { return *p; });
         // the neighbour's lifted adjoint at its point nfq-1-q
         const double* gn = reinterpret_cast<const double*>(a.geo + geo_index(x.nb, x.s < 2 ? 2 : 3));
         const double sc = -0.5 * sa * __ldg(gn + (x.s == 1 ? 1 : 0));
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
         const double2* src = a.a + state_index(NP, x.nb, 0);
 #pragma unroll
         for (int i = 0; i < NP; ++i) {
-          const double2 a0 = __ldg(src + 2 * i * kTileRun), a1 = __ldg(src + (2 * i + 1) * kTileRun);
+          const double2 a0 = src[2 * i * kTileRun], a1 = src[(2 * i + 1) * kTileRun];
           v[0] = fma(lf[i], a0.x, v[0]);
           v[1] = fma(lf[i], a0.y, v[1]);
           v[2] = fma(lf[i], a1.x, v[2]);

@@ -166,8 +166,8 @@ __global__ void __launch_bounds__(4 * kTileElems, 1)
         const double up[4] = {u0.x, u0.y, u1.x, u1.y}, dp[4] = {v0.x, v0.y, v1.x, v1.y};
         double um[4], dm[4], f[4];
         const double* cm = TM + (x.s * NFQ + x.q) * NE;
-        far_trace<P>(ja.U, x, cm, um, [](const double2* p) { return __ldg(p); });
-        far_trace<P>(ja.V, x, cm, dm, [](const double2* p) { return __ldg(p); });
+        far_trace<P>(ja.U, x, cm, um, [](const double2* p) { return *p; });
+        far_trace<P>(ja.V, x, cm, dm, [](const double2* p) { return *p; });
         roe_flux2_jvp(up, um, n.x, n.y, dp, dm, f);
         FV2[own] = make_double2(f[0], f[1]);
         FV2[own + E] = make_double2(f[2], f[3]);

@@ -146,7 +146,9 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* src, unsigned bytes
 // when the kernel before it has ended and its writes are visible. Every kernel
 // launched that way waits before it reads or writes anything that another
 // kernel writes or reads; only the mesh's own arrays, which no kernel of the
-// stream writes, are read before. let_next_start comes after the own wait, so
+// stream writes, are read before. Only those are read by non-coherent loads
+// (__ldg), too: a vector that the kernel before writes changes while this grid
+// exists, which such loads do not allow for. let_next_start comes after the own wait, so
 // that at most one later kernel is resident: when it came first, several were,
 // and blocks of one kernel shared an SM while other SMs had none. 50 RK4 steps
 // at 64 x 64 cells, p = 2 (128 tiles) take 1.23 ms without it, 1.79 with
@@ -448,17 +450,15 @@ __device__ __forceinline__ void plain_nodal_flux(const double2* S, double2* G2, 
   }
 }
 
-// Non-coherent loads issued where they are written, so that the stage
-// update's first operand is in flight during the volume phase (the compiler
-// would otherwise sink them to their use), and so that stage 1's re-read of
-// its input stays in the update (plain loads were hoisted and spilled). They
-// do not allocate in L1: three
-// 73 KB blocks leave about 30 KB of it, which the tile's geometry rows and the
-// face phase's neighbour rows use, and each operand row is read once (0.2%
-// faster at 768 x 768, p = 3).
+// Loads issued where they are written, so that the stage update's first operand
+// is in flight during the volume phase (the compiler would otherwise sink them
+// to their use), and so that stage 1's re-read of its input stays in the update
+// (plain loads were hoisted and spilled). They do not allocate in L1: three
+// 73 KB blocks leave about 30 KB of it, which the tile's geometry rows use, and
+// each operand row is read once (0.2% faster at 768 x 768, p = 3).
 __device__ __forceinline__ double ld_early(const double* p) {
   double v;
-  asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
   return v;
 }
 
@@ -674,10 +674,10 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
         } else {
           um[0] = um[1] = um[2] = um[3] = 0.0;
           const double* cm = TM + (s * NFQ + q) * NE;
-          // all 2 NE loads in flight would take the registers of the flux: 5 RK4
-          // steps at 768 x 768, p = 3 took 6.78 ms (two nodes at a time 6.61,
-          // one 6.67), 20 at 384 x 384, p = 1 4.12 (one 4.06)
-#pragma unroll(P == 3 ? 2 : 1)
+          // one node at a time: with all 2 NE loads in flight, which take the
+          // flux's registers, 5 RK4 steps at 768 x 768, p = 3 took 6.78 ms (6.68),
+          // 20 at 384 x 384, p = 1 4.12 (4.04)
+#pragma unroll 1
           for (int k = 0; k < NE; ++k) {
             const double2 n0 = H[2 * k * 2 * kSlots + x], n1 = H[(2 * k + 1) * 2 * kSlots + x];
             um[0] = fma(cm[k], n0.x, um[0]);
@@ -704,7 +704,7 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
         const double2 x0 = own[0], x1 = own[E];
         const double up[4] = {x0.x, x0.y, x1.x, x1.y};
         double um[4], f[4];
-        far_trace<P>(a.in, x, TM + (x.s * NFQ + x.q) * NE, um, [](const double2* p) { return __ldg(p); });
+        far_trace<P>(a.in, x, TM + (x.s * NFQ + x.q) * NE, um, [](const double2* p) { return *p; });
         roe_flux2(up, um, n.x, n.y, f, [&](int err) { record_error(a, NFQ, EL[x.col], x.q, x.s, err); });
         own[0] = make_double2(f[0], f[1]);
         own[E] = make_double2(f[2], f[3]);
@@ -787,18 +787,23 @@ __global__ void __launch_bounds__(4 * kTileElems, 3) tile_stage_kernel(const __g
       double* out = reinterpret_cast<double*>(a.out) + off0;
       if (a.stage == 1 && !a.no_acc) {
         // X = (U_n + U1) / 3 + c_acc k2, U1 being this stage's input, re-read
-        // here (its tile was copied one tile ago and is still in L2) by
-        // loads that stay where they are written (plain loads of the
-        // read-only input were hoisted and spilled); every row is read
-        // before the first store, since a load that follows a store to
-        // another array cannot be moved above it
+        // here (its tile was copied one tile ago and is still in L2) by loads
+        // that stay where they are written (plain loads were hoisted and
+        // spilled). Half of the rows at a time: a load that follows a store to
+        // another array cannot be moved above it, and all of them before the
+        // first store took 0.3% longer at 150 x 90, p = 3
         const double* in = reinterpret_cast<const double*>(a.in) + off0;
         double* acc = reinterpret_cast<double*>(a.acc) + off0;
-        double iv[NP];
+        constexpr int kHalf = (NP + 1) / 2;
 #pragma unroll
-        for (int i = 0; i < NP; ++i) iv[i] = ld_early(in + i * kStep);
+        for (int h = 0; h < NP; h += kHalf) {
+          double iv[kHalf];
 #pragma unroll
-        for (int i = 0; i < NP; ++i) __stcs(acc + i * kStep, fma(c_acc, r[i], (pre[i] + iv[i]) * kThird));
+          for (int i = h; i < h + kHalf && i < NP; ++i) iv[i - h] = ld_early(in + i * kStep);
+#pragma unroll
+          for (int i = h; i < h + kHalf && i < NP; ++i)
+            __stcs(acc + i * kStep, fma(c_acc, r[i], (pre[i] + iv[i - h]) * kThird));
+        }
       }
       if (a.stage != kStageRhs) {
 #pragma unroll
