@@ -66,63 +66,73 @@ cudaError_t launch_element(const AdjArgs& a, const double* ops, cudaStream_t st)
 }
 
 // One reverse stage as one persistent launch over the stage kernel's tiles.
-template <int P, int NFQ, bool FAR>
+template <int P, int NFQ, int MAP, bool FAR>
 cudaError_t launch_tile(const AdjArgs& a, const double* block, int max_blocks, cudaStream_t st) {
   const int grid = a.ntiles < max_blocks ? a.ntiles : max_blocks;
-  return launch_dependent(adjoint_tile_kernel<P, NFQ, FAR>, grid, 4 * kTileElems, AdjTileLayout<P, NFQ>::kBytes, st, a,
-                          *reinterpret_cast<const AdjOps<P, NFQ>*>(block));
+  return launch_dependent(adjoint_tile_kernel<P, NFQ, MAP, FAR>, grid, 4 * kTileElems, AdjTileLayout<P, NFQ>::kBytes, st, a,
+                          *reinterpret_cast<const AdjOps<P, NFQ, MAP>*>(block));
 }
 
-template <int P, int NFQ>
+template <int P, int NFQ, int MAP>
 std::vector<double> pack_tile(const double* ops) {
-  static_assert(sizeof(AdjOps<P, NFQ>) % sizeof(double) == 0, "a block of doubles");
+  using Ops = AdjOps<P, NFQ, MAP>;
+  static_assert(sizeof(Ops) % sizeof(double) == 0, "a block of doubles");
   const auto& o = *reinterpret_cast<const StageOps<P, NFQ>*>(ops);
-  AdjOps<P, NFQ> block;
-  fold_operators(o, &block.fo);
-  std::memcpy(block.lift, o.lift, sizeof(o.lift));
+  Ops block;
+  if constexpr (MAP == kMapFolded) {
+    fold_operators(o, &block.o);
+    std::memcpy(block.full_lift, o.lift, sizeof(o.lift));
+  } else {
+    block.o = o;
+  }
   const double* b = reinterpret_cast<const double*>(&block);
   return std::vector<double>(b, b + sizeof(block) / sizeof(double));
 }
 
-template <int P, int NFQ, bool FAR>
+template <int P, int NFQ, int MAP, bool FAR>
 cudaError_t configure_tile(int* blocks_per_sm) {
   constexpr int bytes = AdjTileLayout<P, NFQ>::kBytes;
-  cudaError_t e = cudaFuncSetAttribute(adjoint_tile_kernel<P, NFQ, FAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  cudaError_t e = cudaFuncSetAttribute(adjoint_tile_kernel<P, NFQ, MAP, FAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, adjoint_tile_kernel<P, NFQ, FAR>, 4 * kTileElems,
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, adjoint_tile_kernel<P, NFQ, MAP, FAR>, 4 * kTileElems,
                                                        bytes);
 }
 
+template <int P, int NFQ, int MAP, bool FAR>
+AdjKernels kernels_of() {
+  return AdjKernels{launch_face<P, NFQ>, launch_element<P, NFQ>, launch_tile<P, NFQ, MAP, FAR>,
+                    configure_tile<P, NFQ, MAP, FAR>, pack_tile<P, NFQ, MAP>};
+}
+
 template <int P, int NFQ>
-AdjKernels kernels_of(bool far) {
-  return AdjKernels{launch_face<P, NFQ>, launch_element<P, NFQ>,
-                    far ? launch_tile<P, NFQ, true> : launch_tile<P, NFQ, false>,
-                    far ? configure_tile<P, NFQ, true> : configure_tile<P, NFQ, false>, pack_tile<P, NFQ>};
+AdjKernels kernels_of(bool fold, bool far) {
+  return fold ? (far ? kernels_of<P, NFQ, kMapFolded, true>() : kernels_of<P, NFQ, kMapFolded, false>())
+              : (far ? kernels_of<P, NFQ, kMapComponent, true>() : kernels_of<P, NFQ, kMapComponent, false>());
 }
 
 template <int P>
-AdjKernels kernels_for_nfq(int nfq, bool far) {
+AdjKernels kernels_for_nfq(int nfq, bool fold, bool far) {
   switch (nfq) {
-    case 1: return kernels_of<P, 1>(far);
-    case 2: return kernels_of<P, 2>(far);
-    case 3: return kernels_of<P, 3>(far);
-    case 4: return kernels_of<P, 4>(far);
-    case 5: return kernels_of<P, 5>(far);
-    case 6: return kernels_of<P, 6>(far);
-    case 7: return kernels_of<P, 7>(far);
-    case 8: return kernels_of<P, 8>(far);
-    case 9: return kernels_of<P, 9>(far);
-    case 10: return kernels_of<P, 10>(far);
+    case 1: return kernels_of<P, 1>(fold, far);
+    case 2: return kernels_of<P, 2>(fold, far);
+    case 3: return kernels_of<P, 3>(fold, far);
+    case 4: return kernels_of<P, 4>(fold, far);
+    case 5: return kernels_of<P, 5>(fold, far);
+    case 6: return kernels_of<P, 6>(fold, far);
+    case 7: return kernels_of<P, 7>(fold, far);
+    case 8: return kernels_of<P, 8>(fold, far);
+    case 9: return kernels_of<P, 9>(fold, far);
+    case 10: return kernels_of<P, 10>(fold, far);
     default: return AdjKernels{};
   }
 }
 
-AdjKernels select_adjoint(int p, int nfq, bool far) {
+AdjKernels select_adjoint(int p, int nfq, bool fold, bool far) {
   switch (p) {
-    case 0: return kernels_for_nfq<0>(nfq, far);
-    case 1: return kernels_for_nfq<1>(nfq, far);
-    case 2: return kernels_for_nfq<2>(nfq, far);
-    case 3: return kernels_for_nfq<3>(nfq, far);
+    case 0: return kernels_for_nfq<0>(nfq, fold, far);
+    case 1: return kernels_for_nfq<1>(nfq, fold, far);
+    case 2: return kernels_for_nfq<2>(nfq, fold, far);
+    case 3: return kernels_for_nfq<3>(nfq, fold, far);
     default: return AdjKernels{};
   }
 }
@@ -186,7 +196,7 @@ int setup(vt_ctx* c) {
   if (c->adj) return VT_OK;
   if (!c->side_pairing)
     return fail(VT_ERR_UNSUPPORTED, "adjoint: side s of some element does not face side s of its neighbour");
-  const AdjKernels k = select_adjoint(c->p, c->nfq, c->far);
+  const AdjKernels k = select_adjoint(c->p, c->nfq, operators_reflect(c->p, c->nfq, c->ops.data()), c->far);
   if (!k.face) return fail(VT_ERR_UNSUPPORTED, "adjoint: unsupported (p, nfq)");
   // The edge-once form needs every edge to join elements whose sides face each
   // other with opposite normals; a 2-colouring of the element adjacency
@@ -217,9 +227,9 @@ int setup(vt_ctx* c) {
       }
     }
   }
-  // the fused reverse stage runs on the stage kernel's tiles, with the folded operators
+  // the fused reverse stage runs on the stage kernel's tiles
   int tile_blocks = 0;
-  if (ok && operators_reflect(c->p, c->nfq, c->ops.data())) {
+  if (ok) {
     int per_sm = 0;
     if (c->ntiles > 0 && !k.tile_config(&per_sm) && per_sm > 0) tile_blocks = c->sms * per_sm;
     cudaGetLastError();

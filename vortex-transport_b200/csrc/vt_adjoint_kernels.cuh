@@ -1,4 +1,4 @@
-// Kernels of the discrete adjoint on meshes or operators without the fused form.
+// Kernels of the discrete adjoint on meshes without the fused form.
 //
 // One reverse RK4 stage (the transpose of one stage's right-hand side at the
 // stage state U, applied to the stage adjoint a) is two launches:

@@ -4,10 +4,12 @@
 // the stage adjoint a (times sa), g = R'(U)^T (sa a), followed by the reverse
 // RK4 combine of adjoint_element_kernel, for meshes on which the face phase
 // may take the edge-once form (a face's flux is evaluated once for both
-// sides: F(u-, u+, -n) = -F(u+, u-, n)) and operators that reflect
-// (FoldedOps). A persistent block walks the forward stage kernel's tiles (64
-// columns, Numbering in vt_device.cuh) and keeps every intermediate in shared
-// memory, so nothing but the state, the adjoints and the geometry crosses HBM:
+// sides: F(u-, u+, -n) = -F(u+, u-, n)). The operators come folded (FoldedOps)
+// where they reflect, else as they are (kMapComponent; 10 steps' gradient at
+// 128 x 128, p = 2: 1.73 ms, with the two-launch form 2.59). A persistent block
+// walks the forward stage kernel's tiles (64 columns, Numbering in
+// vt_device.cuh) and keeps every intermediate in shared memory, so nothing but
+// the state, the adjoints and the geometry crosses HBM:
 //
 //   1. load   the tile's stage state, stage adjoint, geometry and face list by
 //             bulk copies (issued during the previous tile); the side nodes of
@@ -51,11 +53,18 @@
 
 namespace vt {
 
-// The operators: folded, and the lift as it is for the neighbours' adjoints.
-template <int P, int NFQ>
+// The operators: as they are, or folded, with the lift as it is for the
+// neighbours' adjoints.
+template <int P, int NFQ, int MAP>
 struct AdjOps {
-  FoldedOps<P, NFQ> fo;
-  double lift[3][np_of_p(P)][NFQ];
+  StageOps<P, NFQ> o;
+  __host__ __device__ static const double* lift(const AdjOps& a) { return &a.o.lift[0][0][0]; }
+};
+template <int P, int NFQ>
+struct AdjOps<P, NFQ, kMapFolded> {
+  FoldedOps<P, NFQ> o;
+  double full_lift[3][np_of_p(P)][NFQ];
+  __host__ __device__ static const double* lift(const AdjOps& a) { return &a.full_lift[0][0][0]; }
 };
 
 // The stage kernel's buffers, the stage adjoint tile, and the operator tables
@@ -171,10 +180,11 @@ __device__ __forceinline__ void folded_adjoint(const double* Ad, double* e, doub
 // Two 256-thread blocks per SM: the transposed Roe Jacobian needs more than the
 // 80 registers of three blocks, and two leave shared memory for the stage
 // adjoint tile.
-template <int P, int NFQ, bool FAR>
+template <int P, int NFQ, int MAP, bool FAR>
 __global__ void __launch_bounds__(4 * kTileElems, 2)
-    adjoint_tile_kernel(const __grid_constant__ AdjArgs a, const AdjOps<P, NFQ> ops) {
-  const FoldedOps<P, NFQ>& fo = ops.fo;
+    adjoint_tile_kernel(const __grid_constant__ AdjArgs a, const AdjOps<P, NFQ, MAP> ops) {
+  constexpr bool FOLD = MAP == kMapFolded;
+  const auto& o = ops.o;
   using B = TileLayout<P, NFQ>;
   using L = AdjTileLayout<P, NFQ>;
   constexpr int E = B::E;
@@ -209,9 +219,9 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
   const bool hand_out = a.ntiles > kHandOut * G;
 
   {
-    const double* tm = &fo.tm[0][0][0];
-    const double* tp = &fo.tp[0][0][0];
-    const double* lf = &ops.lift[0][0][0];
+    const double* tm = &o.tm[0][0][0];
+    const double* tp = &o.tp[0][0][0];
+    const double* lf = AdjOps<P, NFQ, MAP>::lift(ops);
     for (int l = t; l < 3 * NFQ * NE; l += T) {
       TM[l] = tm[l];
       TP[l] = tp[l];
@@ -261,19 +271,18 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
     parity ^= 1u;
 
     // ---- 2. lifted face adjoints (half of them), component c of column el --------------
-    {
-      double e[NS], o[NOA];
-      folded_adjoint<P>(Ad, e, o);
-      const double2* ge = GE + which * kGeoRows * kTileRun + (el & 31);
-      const double2 lsa = ge[2 * kTileRun], lsb = ge[3 * kTileRun];
-      const double l0 = sa * lsa.x, l1 = sa * lsa.y, l2 = sa * lsb.x;
+    const double2* ge = GE + which * kGeoRows * kTileRun + (el & 31);
+    const double l0 = sa * ge[2 * kTileRun].x, l1 = sa * ge[2 * kTileRun].y, l2 = sa * ge[3 * kTileRun].x;
+    if constexpr (FOLD) {
+      double ev[NS], od[NOA];
+      folded_adjoint<P>(Ad, ev, od);
 #pragma unroll
       for (int q = 0; q < NFQ; ++q) {
         double x = 0.0, y = 0.0;
 #pragma unroll
-        for (int k = 0; k < NS; ++k) x = fma(fo.Le[k][q], e[k], x);
+        for (int k = 0; k < NS; ++k) x = fma(o.Le[k][q], ev[k], x);
 #pragma unroll
-        for (int k = 0; k < NO; ++k) y = fma(fo.Lo[k][q], o[k], y);
+        for (int k = 0; k < NO; ++k) y = fma(o.Lo[k][q], od[k], y);
         FBt[q * 4 * E] = l0 * (x + y);
         FBt[(2 * NFQ + NFQ - 1 - q) * 4 * E] = l2 * (x - y);
       }
@@ -281,13 +290,28 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
       for (int q = 0; q < (NFQ + 1) / 2; ++q) {
         double x = 0.0, y = 0.0;
 #pragma unroll
-        for (int k = 0; k < NS; ++k) x = fma(fo.L1e[k][q], e[k], x);
+        for (int k = 0; k < NS; ++k) x = fma(o.L1e[k][q], ev[k], x);
         if (q < NFQ / 2) {
 #pragma unroll
-          for (int k = 0; k < NO; ++k) y = fma(fo.L1o[k][q], o[k], y);
+          for (int k = 0; k < NO; ++k) y = fma(o.L1o[k][q], od[k], y);
           FBt[(NFQ + NFQ - 1 - q) * 4 * E] = l1 * (x - y);
         }
         FBt[(NFQ + q) * 4 * E] = l1 * (x + y);
+      }
+    } else {
+      double u[NP];
+#pragma unroll
+      for (int i = 0; i < NP; ++i) u[i] = Ad[i * 4 * kTileRun];
+#pragma unroll
+      for (int s = 0; s < 3; ++s) {
+        const double ls = -0.5 * (s == 0 ? l0 : (s == 1 ? l1 : l2));
+#pragma unroll
+        for (int q = 0; q < NFQ; ++q) {
+          double x = 0.0;
+#pragma unroll
+          for (int i = 0; i < NP; ++i) x = fma(o.lift[s][i][q], u[i], x);
+          FBt[(s * NFQ + q) * 4 * E] = ls * x;
+        }
       }
     }
     cp_async_wait_all();  // this thread's copies of neighbour rows
@@ -404,23 +428,38 @@ __global__ void __launch_bounds__(4 * kTileElems, 2)
       for (int q = 0; q < NFQ; ++q) {
         const double b = FBt[(s * NFQ + q) * 4 * E];
 #pragma unroll
-        for (int k = 0; k < NE; ++k) g[edge_node(P, s, k)] = fma(fo.tp[s][q][k], b, g[edge_node(P, s, k)]);
+        for (int k = 0; k < NE; ++k) g[edge_node(P, s, k)] = fma(o.tp[s][q][k], b, g[edge_node(P, s, k)]);
       }
     run_sync(t);
 
     // ---- 4b. transposed volume operator: rows j*4 + h (xi), j*4 + 2 + h (eta) ----------
-    if (P > 0) {
-      double e[NS], o[NOA];
-      folded_adjoint<P>(Ad, e, o);
+    if constexpr (P > 0 && FOLD) {
+      double ev[NS], od[NOA];
+      folded_adjoint<P>(Ad, ev, od);
 #pragma unroll
       for (int j = 0; j < NP; ++j) {
         double x = 0.0, y = 0.0;
 #pragma unroll
-        for (int k = 0; k < NS; ++k) x = fma(fo.De[k][j], e[k], x);
+        for (int k = 0; k < NS; ++k) x = fma(o.De[k][j], ev[k], x);
 #pragma unroll
-        for (int k = 0; k < NO; ++k) y = fma(fo.Do[k][j], o[k], y);
+        for (int k = 0; k < NO; ++k) y = fma(o.Do[k][j], od[k], y);
         FBt[j * 8 * E] = sa * (x + y);
         FBt[(mirror_node(P, j) * 8 + 4) * E] = sa * (x - y);
+      }
+    } else if constexpr (P > 0) {
+      double u[NP];
+#pragma unroll
+      for (int i = 0; i < NP; ++i) u[i] = Ad[i * 4 * kTileRun];
+#pragma unroll
+      for (int j = 0; j < NP; ++j) {
+        double x = 0.0, y = 0.0;
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+          x = fma(o.D[0][i][j], u[i], x);
+          y = fma(o.D[1][i][j], u[i], y);
+        }
+        FBt[j * 8 * E] = sa * x;
+        FBt[(j * 8 + 4) * E] = sa * y;
       }
     }
     // the combine's operands, requested now so that they are in flight during
