@@ -808,9 +808,14 @@ int vt_download_state(vt_ctx* c, double* U, double* F) {
 }
 
 static int rk4_enqueue(vt_ctx* c, double dt, int nsteps) {
-  cudaError_t e = reset_error_words(c);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(c->stream, &capture);
+  if (!e) e = reset_error_words(c);
   if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("reset", e));
-  if (c->resident)
+  // A caller that captures the context's stream may replay the steps. A
+  // resident launch waits for the flags' numbers of its first time, which a
+  // replay finds passed already, so captured steps are a launch per stage.
+  if (c->resident && capture == cudaStreamCaptureStatusNone)
     e = enqueue_resident(c, dt, nsteps, false);
   else
     for (int s = 0; s < nsteps && !e; ++s) e = enqueue_rk4_step(c, dt);
