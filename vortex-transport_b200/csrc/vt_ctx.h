@@ -48,6 +48,15 @@ struct vt_ctx {
   vt_error_info last{};
   int pending_steps = 0;
   double pending_dt = 0.0;
+  // asynchronous steps by launches of a graph (enqueue_graphs, vt_solver.cu):
+  // the graph, and what its launches were made with
+  struct StepsGraph {
+    cudaGraphExec_t exec = nullptr;
+    double dt = 0.0;
+    const double2* U = nullptr;
+    int map = 0, flags = 0;
+    unsigned tries = 0;
+  } steps;
   bool side_pairing = false;  // nbr(nbr(e, s), s) == e for every element and side
   bool mutual_tiles = false;  // a tile that reads another is read by it (implied by side_pairing)
   // Per-tile time steps (a batch group's view; null otherwise): stage and

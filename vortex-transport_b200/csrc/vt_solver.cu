@@ -9,7 +9,8 @@
 // for a capture. 50 steps at 64 x 64 cells, p = 2 take 1.12 ms launched and
 // 1.28 as graphs of a step, 250 at 8 x 8, p = 3 6.18 and 6.24; the first
 // gradient of a new 128 x 128, p = 3 problem 15 to 18 ms against 27 with
-// its sweeps captured (later ones 14.7 against 14.2).
+// its sweeps captured (later ones 14.7 against 14.2). Only vt_step_rk4_async,
+// whose caller does not wait for the steps, launches graphs (enqueue_graphs).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -316,6 +317,7 @@ void release(vt_ctx* c) {
   if (!c) return;
   cudaSetDevice(c->device);
   vt::adjoint_release(c);
+  if (c->steps.exec) cudaGraphExecDestroy(c->steps.exec);
   void* bufs[] = {c->U,   c->A,   c->Sa, c->Sb,      c->R,   c->geo,   c->nbr,
                   c->err, c->aos, c->W,  c->partial, c->tot, c->elem,  c->lists, c->flags};
   for (void* b : bufs)
@@ -807,16 +809,51 @@ int vt_download_state(vt_ctx* c, double* U, double* F) {
   return VT_OK;
 }
 
-static int rk4_enqueue(vt_ctx* c, double dt, int nsteps) {
+// nsteps steps by launches of a graph of kGraphSteps (and plain launches for the
+// rest), for vt_step_rk4_async, which is to return early: 4 launches a step take
+// the host 10 us, and once about 1000 are under way it waits for the GPU. 500 and
+// 1000 steps at 384 x 384, p = 1 held the caller for 44 and 135 ms, now for 0.16
+// and 0.32 (0.5 and 0.7 where the graph has to be made); the steps take 90.5 and
+// 91.0, 181.1 and 182.0 ms. With a graph of one step 64 at 100 x 100, p = 2 take
+// 1.98 ms, of 4 1.83, of 16 1.79 (launched 1.88), and instantiating 16 takes 0.5 ms.
+constexpr int kGraphSteps = 4;
+static cudaError_t enqueue_graphs(vt_ctx* c, double dt, int nsteps) {
+  vt_ctx::StepsGraph& g = c->steps;
+  cudaError_t e = cudaSuccess;
+  if (!g.exec || g.dt != dt || g.U != c->U || g.map != c->map || g.tries != c->test_wait_tries || g.flags != c->test_flags) {
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    g = vt_ctx::StepsGraph{};
+    cudaGraph_t graph = nullptr;
+    e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
+    if (!e) {
+      cudaError_t l = cudaSuccess;
+      for (int s = 0; s < kGraphSteps && !l; ++s) l = enqueue_rk4_step(c, dt);
+      e = cudaStreamEndCapture(c->stream, &graph);
+      if (l) e = l;
+    }
+    if (!e) e = cudaGraphInstantiate(&g.exec, graph, 0);
+    if (graph) cudaGraphDestroy(graph);
+    if (e) return e;
+    g.dt = dt, g.U = c->U, g.map = c->map, g.tries = c->test_wait_tries, g.flags = c->test_flags;
+  }
+  for (; nsteps >= kGraphSteps && !e; nsteps -= kGraphSteps) e = cudaGraphLaunch(g.exec, c->stream);
+  for (; nsteps > 0 && !e; --nsteps) e = enqueue_rk4_step(c, dt);
+  return e;
+}
+
+static int rk4_enqueue(vt_ctx* c, double dt, int nsteps, bool async) {
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   cudaError_t e = cudaStreamIsCapturing(c->stream, &capture);
   if (!e) e = reset_error_words(c);
   if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("reset", e));
+  const bool captured = capture != cudaStreamCaptureStatusNone;
   // A caller that captures the context's stream may replay the steps. A
   // resident launch waits for the flags' numbers of its first time, which a
   // replay finds passed already, so captured steps are a launch per stage.
-  if (c->resident && capture == cudaStreamCaptureStatusNone)
+  if (c->resident && !captured)
     e = enqueue_resident(c, dt, nsteps, false);
+  else if (async && !captured && nsteps >= 2 * kGraphSteps)
+    e = enqueue_graphs(c, dt, nsteps);
   else
     for (int s = 0; s < nsteps && !e; ++s) e = enqueue_rk4_step(c, dt);
   if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("rk4 launch", e));
@@ -830,7 +867,7 @@ int vt_step_rk4_async(vt_ctx* c, double dt, int nsteps) {
   std::lock_guard<std::mutex> lk(c->mu);
   cudaSetDevice(c->device);
   if (c->pending_steps) return fail(VT_ERR_INVALID, "a previous async step is not synchronised");
-  return rk4_enqueue(c, dt, nsteps);
+  return rk4_enqueue(c, dt, nsteps, true);
 }
 
 int vt_synchronize(vt_ctx* c) {
@@ -847,7 +884,7 @@ int vt_step_rk4(vt_ctx* c, double dt, int nsteps) {
   std::lock_guard<std::mutex> lk(c->mu);
   cudaSetDevice(c->device);
   if (c->pending_steps) return fail(VT_ERR_INVALID, "a previous async step is not synchronised");
-  int st = rk4_enqueue(c, dt, nsteps);
+  int st = rk4_enqueue(c, dt, nsteps, false);
   if (st) return st;
   c->pending_steps = 0;
   return finish(c, nsteps, dt);
