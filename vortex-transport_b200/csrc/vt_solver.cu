@@ -686,15 +686,12 @@ vt_ctx* vt_create_structured(const vt_params* prm, const vt_vortex* ic_in, int d
   const long long ncols = c->ncols;
   const size_t state_bytes = sizeof(double2) * 2 * Np * static_cast<size_t>(ncols);
   const int tot_blocks = static_cast<int>((ncols + 255) / 256);
+  // What the mesh kernel writes comes first: the GPU works while the host makes
+  // the other allocations, which take most of a set-up.
   double* verts = nullptr;
   if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) || (e = alloc(&c->U, state_bytes)) ||
-      (e = alloc(&c->A, state_bytes)) || (e = alloc(&c->Sa, state_bytes)) || (e = alloc(&c->Sb, state_bytes)) ||
       (e = alloc(&c->geo, sizeof(double2) * vt::kGeoRows * ncols)) || (e = alloc(&c->nbr, sizeof(int4) * ncols)) ||
-      (e = alloc(&c->elem, sizeof(int) * ncols)) ||
-      (e = alloc(&c->lists, vt::kTileListBytes * static_cast<size_t>(c->ntiles))) ||
-      (e = alloc(&c->err, vt::kErrWords * sizeof(unsigned long long))) || (e = alloc(&c->W, sizeof(double) * Np)) ||
-      (e = alloc(&c->partial, sizeof(double) * 4 * tot_blocks)) || (e = alloc(&c->tot, sizeof(double) * 4)) ||
-      (e = alloc(&verts, sizeof(double) * 6 * static_cast<size_t>(c->K)))) {
+      (e = alloc(&c->elem, sizeof(int) * ncols)) || (e = alloc(&verts, sizeof(double) * 6 * static_cast<size_t>(c->K)))) {
     set(fail(e == cudaErrorMemoryAllocation ? VT_ERR_NO_MEMORY : VT_ERR_CUDA, vt::cuda_msg("vt_create_structured", e)));
     if (verts) cudaFree(verts);
     release(c);
@@ -724,18 +721,24 @@ vt_ctx* vt_create_structured(const vt_params* prm, const vt_vortex* ic_in, int d
   std::copy(minv.begin(), minv.end(), tab.begin() + static_cast<size_t>(nq) * (Np + 3));
   double* dtab = nullptr;
   if (!e) e = cudaMemsetAsync(c->U, 0, state_bytes, c->stream);
-  if (!e) e = cudaMemsetAsync(c->A, 0, state_bytes, c->stream);
-  if (!e) e = cudaMemsetAsync(c->Sa, 0, state_bytes, c->stream);
-  if (!e) e = cudaMemsetAsync(c->Sb, 0, state_bytes, c->stream);
   if (!e) e = cudaMemsetAsync(c->geo, 0, sizeof(double2) * vt::kGeoRows * ncols, c->stream);
   if (!e) e = cudaMemsetAsync(c->nbr, 0, sizeof(int4) * ncols, c->stream);
-  if (!e) e = cudaMemcpyAsync(c->W, W.data(), sizeof(double) * Np, cudaMemcpyHostToDevice, c->stream);
   if (!e) {
     vt::structured_mesh_kernel<<<(c->K + 127) / 128, 128, 0, c->stream>>>(
         g, c->num, Np, verts, c->geo, c->nbr, ic, prm->U_initialization_type == 0 ? c->U : nullptr);
     e = cudaGetLastError();
   }
   if (!e) e = vt::launch_number_columns(c->num, c->elem, 0, 0, c->stream);
+  if (!e) e = alloc(&c->err, vt::kErrWords * sizeof(unsigned long long));
+  if (!e) e = alloc(&c->lists, vt::kTileListBytes * static_cast<size_t>(c->ntiles));
+  for (double2** v : {&c->A, &c->Sa, &c->Sb}) {
+    if (!e) e = alloc(v, state_bytes);
+    if (!e) e = cudaMemsetAsync(*v, 0, state_bytes, c->stream);
+  }
+  if (!e) e = alloc(&c->partial, sizeof(double) * 4 * tot_blocks);
+  if (!e) e = alloc(&c->tot, sizeof(double) * 4);
+  if (!e) e = alloc(&c->W, sizeof(double) * Np);
+  if (!e) e = cudaMemcpyAsync(c->W, W.data(), sizeof(double) * Np, cudaMemcpyHostToDevice, c->stream);
   if (!e && prm->U_initialization_type == 1) {
     e = alloc(&dtab, sizeof(double) * tab.size());
     if (!e) e = cudaMemcpyAsync(dtab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice, c->stream);
