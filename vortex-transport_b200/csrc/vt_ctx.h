@@ -43,6 +43,7 @@ struct vt_ctx {
   unsigned* flags = nullptr;
   unsigned flag_base = 0;
   bool flags_known = false, flag_launches = false;
+  int counted = 0;  // tiles of steps under way that this context is counted with (take_resident)
   int map = vt::kDefaultMap;  // form of the stage kernel
   double time = 0.0;
   vt_error_info last{};
@@ -109,6 +110,9 @@ int ensure_aos(vt_ctx* c);
 // AoS (K x Np x 4, device memory) <-> the columns of a state vector.
 cudaError_t to_columns(vt_ctx* c, const double* src, double2* dst);
 cudaError_t from_columns(vt_ctx* c, const double2* src, double* dst);
+
+// The context's steps are no longer under way (take_resident, vt_solver.cu).
+void steps_are_done(vt_ctx* c);
 
 // Frees the adjoint's buffers (no-op without them).
 void adjoint_release(vt_ctx* c);

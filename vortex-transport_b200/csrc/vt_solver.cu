@@ -10,10 +10,12 @@
 // 1.28 as graphs of a step, 250 at 8 x 8, p = 3 6.18 and 6.24; the first
 // gradient of a new 128 x 128, p = 3 problem 15 to 18 ms against 27 with
 // its sweeps captured (later ones 14.7 against 14.2). Only vt_step_rk4_async,
-// whose caller does not wait for the steps, launches graphs (enqueue_graphs).
+// whose caller does not wait for the steps, and small problems beside each other
+// launch graphs (enqueue_graphs).
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -317,6 +319,7 @@ void release(vt_ctx* c) {
   if (!c) return;
   cudaSetDevice(c->device);
   vt::adjoint_release(c);
+  vt::steps_are_done(c);
   if (c->steps.exec) cudaGraphExecDestroy(c->steps.exec);
   void* bufs[] = {c->U,   c->A,   c->Sa, c->Sb,      c->R,   c->geo,   c->nbr,
                   c->err, c->aos, c->W,  c->partial, c->tot, c->elem,  c->lists, c->flags};
@@ -405,6 +408,34 @@ cudaError_t use_kernel(vt_ctx* c, int map) {
   return cudaSuccess;
 }
 
+// Tiles, per device, of the contexts that may take the resident kernel and have
+// steps under way. Resident launches share SMs only as far as each of their tiles
+// has one of its own and run one after the other beyond that, where the stage
+// kernels of several contexts hide each other's latency. So a context whose tiles
+// are not all beside those under way when its steps are called steps by a launch
+// per stage (the same numbers, bit for bit). N contexts with 100 asynchronous
+// steps each, in ms, all resident and by this rule:
+//   N                      2              4              8             16
+//   40 x 40, p = 2    1.34   1.34    2.65   2.15    5.26   3.07    10.4    5.6
+//   64 x 64, p = 2    2.62   2.59    5.22   3.64    10.4   5.5     20.8   10.4
+//   64 x 64, p = 3    3.07   3.34    6.12   4.71    12.2   7.3     24.4   14.2
+//   24 x 24, p = 1    1.23   1.23    1.26   1.26    1.32   1.32     2.5    2.9
+// (with twice as many tiles allowed as there are SMs 64 x 64, p = 2: 2.6, 4.7, 6.2, 11.1).
+constexpr int kMaxDevices = 64;
+std::atomic<int> tiles_under_way[kMaxDevices];
+
+// Counts c's tiles until steps_are_done; whether its steps may be resident.
+bool take_resident(vt_ctx* c) {
+  if (!c->resident || c->device < 0 || c->device >= kMaxDevices) return c->resident != nullptr;
+  c->counted += c->ntiles;
+  return tiles_under_way[c->device].fetch_add(c->ntiles) + c->ntiles <= c->sms;
+}
+
+void steps_are_done(vt_ctx* c) {
+  if (c->counted) tiles_under_way[c->device].fetch_sub(c->counted);
+  c->counted = 0;
+}
+
 // nsteps steps by the resident kernel, at most kResidentSteps a launch.
 constexpr int kResidentSteps = 1024;
 cudaError_t enqueue_resident(vt_ctx* c, double dt, int nsteps, bool euler) {
@@ -448,6 +479,7 @@ int finish(vt_ctx* c, int nsteps, double dt) {
   unsigned long long words[4] = {~0ull, 0, 0, 0};
   cudaError_t e = cudaMemcpyAsync(words, c->err, sizeof(words), cudaMemcpyDeviceToHost, c->stream);
   if (!e) e = cudaStreamSynchronize(c->stream);
+  steps_are_done(c);
   if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("step", e));
   for (int s = 0; s < nsteps; ++s) c->time += dt;  // Element::time += t_step per step
   c->last = vt_error_info{};
@@ -497,6 +529,8 @@ using vt::finish;
 using vt::reset_error_words;
 using vt::from_columns;
 using vt::stage_args;
+using vt::steps_are_done;
+using vt::take_resident;
 using vt::to_columns;
 
 extern "C" {
@@ -813,12 +847,14 @@ int vt_download_state(vt_ctx* c, double* U, double* F) {
 }
 
 // nsteps steps by launches of a graph of kGraphSteps (and plain launches for the
-// rest), for vt_step_rk4_async, which is to return early: 4 launches a step take
-// the host 10 us, and once about 1000 are under way it waits for the GPU. 500 and
-// 1000 steps at 384 x 384, p = 1 held the caller for 44 and 135 ms, now for 0.16
-// and 0.32 (0.5 and 0.7 where the graph has to be made); the steps take 90.5 and
-// 91.0, 181.1 and 182.0 ms. With a graph of one step 64 at 100 x 100, p = 2 take
-// 1.98 ms, of 4 1.83, of 16 1.79 (launched 1.88), and instantiating 16 takes 0.5 ms.
+// rest), for small problems beside each other (take_resident), where the launches
+// of all of them add up, and for vt_step_rk4_async, which is to return early: 4
+// launches a step take the host 10 us, and once about 1000 are under way it waits
+// for the GPU. 500 and 1000 steps at 384 x 384, p = 1 held the caller for 44 and
+// 135 ms, now for 0.16 and 0.32 (0.5 and 0.7 where the graph has to be made); the
+// steps take 90.5 and 91.0, 181.1 and 182.0 ms. With a graph of one step 64 at
+// 100 x 100, p = 2 take 1.98 ms, of 4 1.83, of 16 1.79 (launched 1.88), and
+// instantiating 16 takes 0.5 ms.
 constexpr int kGraphSteps = 4;
 static cudaError_t enqueue_graphs(vt_ctx* c, double dt, int nsteps) {
   vt_ctx::StepsGraph& g = c->steps;
@@ -853,13 +889,16 @@ static int rk4_enqueue(vt_ctx* c, double dt, int nsteps, bool async) {
   // A caller that captures the context's stream may replay the steps. A
   // resident launch waits for the flags' numbers of its first time, which a
   // replay finds passed already, so captured steps are a launch per stage.
-  if (c->resident && !captured)
+  if (!captured && take_resident(c))
     e = enqueue_resident(c, dt, nsteps, false);
-  else if (async && !captured && nsteps >= 2 * kGraphSteps)
+  else if ((async || c->resident) && !captured && nsteps >= 2 * kGraphSteps)
     e = enqueue_graphs(c, dt, nsteps);
   else
     for (int s = 0; s < nsteps && !e; ++s) e = enqueue_rk4_step(c, dt);
-  if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("rk4 launch", e));
+  if (e) {
+    steps_are_done(c);
+    return fail(VT_ERR_CUDA, vt::cuda_msg("rk4 launch", e));
+  }
   c->pending_steps += nsteps;
   c->pending_dt = dt;
   return VT_OK;
@@ -899,14 +938,18 @@ int vt_step_euler(vt_ctx* c, double dt, int nsteps) {
   cudaSetDevice(c->device);
   if (c->pending_steps) return fail(VT_ERR_INVALID, "a previous async step is not synchronised");
   cudaError_t e = reset_error_words(c);
-  if (c->resident && !e) e = enqueue_resident(c, dt, nsteps, true);
-  for (int s = 0; s < nsteps && !e && !c->resident; ++s) {
+  const bool resident = !e && take_resident(c);
+  if (resident) e = enqueue_resident(c, dt, nsteps, true);
+  for (int s = 0; s < nsteps && !e && !resident; ++s) {
     // double buffer: the neighbours of an element read the old state
     e = c->launch(stage_args(c, c->U, c->U, c->A, c->Sa, vt::kStageEuler, 0.0, dt), c->block.data(),
                   c->max_blocks, c->stream);
     std::swap(c->U, c->Sa);
   }
-  if (e) return fail(VT_ERR_CUDA, vt::cuda_msg("euler", e));
+  if (e) {
+    steps_are_done(c);
+    return fail(VT_ERR_CUDA, vt::cuda_msg("euler", e));
+  }
   return finish(c, nsteps, dt);
 }
 
