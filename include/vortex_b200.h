@@ -178,7 +178,8 @@ int vt_step_rk4(vt_ctx* ctx, double dt, int nsteps);
 int vt_step_euler(vt_ctx* ctx, double dt, int nsteps);
 
 /* Same as vt_step_rk4 but only enqueues the work on the context's stream and
- * returns; vt_synchronize() waits and reports the status. */
+ * returns; vt_synchronize() waits and reports the status. The stream may be
+ * captured around the call, and the captured steps replayed. */
 int vt_step_rk4_async(vt_ctx* ctx, double dt, int nsteps);
 int vt_synchronize(vt_ctx* ctx);
 
@@ -250,7 +251,8 @@ int vt_test_bulk_wait(vt_ctx* ctx, unsigned tries, int issue_no_copies);
 
 /* Device time of each kernel kind of one RK4 step, measured with CUDA events
  * around individual launches: ms[0..3] = stages 0..3, averaged over
- * `reps` steps of size dt. Advances the state by `reps` steps. */
+ * `reps` steps of size dt. Advances the state by `reps` steps. (Also for small
+ * problems, whose steps vt_step_rk4 makes in one launch where it can.) */
 int vt_profile_rk4_stages(vt_ctx* ctx, double dt, int reps, float* ms);
 
 /* ---- batched ensemble --------------------------------------------------- */
@@ -259,7 +261,8 @@ int vt_profile_rk4_stages(vt_ctx* ctx, double dt, int reps, float* ms);
  * `n` calls of rk4 (Timestepping.cpp:85-306) sharing each kernel launch.
  * Instances with the same p and reference tables form a group stored as one
  * ragged element array; one stage launch per group advances all its
- * instances, and the groups' launches run side by side. Each instance keeps
+ * instances, and the groups' launches run side by side (with several groups of
+ * small meshes as one CUDA graph per step). Each instance keeps
  * its own time step, and its elements see exactly the arithmetic of a
  * vt_ctx built from the same descriptor. */
 typedef struct vt_batch vt_batch;

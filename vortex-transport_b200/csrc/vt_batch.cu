@@ -9,7 +9,8 @@
 // instance would get, so the arithmetic per element is identical) listed one
 // after another, each tile carrying its instance's time step. One launch of the
 // stage kernel per group and stage advances every instance of the group; the
-// groups' launches run side by side on a stream each.
+// groups' launches run side by side on a stream each, or, where they would wait
+// for the host, as a captured step (enqueue_steps).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -654,7 +655,7 @@ static int batch_backward(vt_batch* b, const double* dJdU_T, double* dJdU_0, int
     if (device_pointers && vt::aligned_to(dJdU_T, 16) && vt::aligned_to(dJdU_0, 16)) {
       // Every instance straight from and to its place in the caller's arrays.
       // Twelve instances of 64 x 64 cells at p = 2, 20 steps forward and back:
-      // 9.7 ms, where gathering the group into an array allocated for the call,
+      // 9.3 ms, where gathering the group into an array allocated for the call,
       // and scattering from it, gave 10.7 to 14.7 ms with the allocator's mood.
       b->views[gi]->all_instances = true;
       const int st = vt_adjoint_backward(b->views[gi], dJdU_T, dJdU_0, 1);
@@ -814,7 +815,7 @@ int vt_batch_set_mapping(vt_batch* b, const int* mapping) {
   drop_graph(b);
   for (size_t gi = 0; gi < b->groups.size(); ++gi) {
     if (mapping[gi] != vt::kMapComponent && mapping[gi] != vt::kMapDefault)
-      return fail(VT_ERR_INVALID, "vt_batch_set_mapping: mapping must be 0 (component) or 1 (pair)");
+      return fail(VT_ERR_INVALID, "vt_batch_set_mapping: mapping must be 0 (operators as they are) or 1 (folded)");
     vt::Group& G = b->groups[gi];
     const vt::StageKernel k = vt::select_kernel(G.p, G.nfq, G.ops.data(), G.far, mapping[gi]);
     int limit = 0;

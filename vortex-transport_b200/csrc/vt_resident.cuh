@@ -15,6 +15,8 @@
 //   50 RK4 steps,   64 x 64, p = 2       1.12         0.97        0.86
 //   100 Euler steps, 27 x 18, p = 1      0.51         0.42        0.37
 //
+// (3.96, 0.826 and 0.351 since the loop for faces without a slot has kernels of
+// its own.)
 // (768 threads, which leave 80 registers each: 4.43, 0.93 and 0.40 ms.) What is
 // left of a stage at 8 x 8, p = 3, in cycles of 7900: lift and volume, with the
 // wait for the slowest faces, 2300, faces 2000, waiting for the neighbours and

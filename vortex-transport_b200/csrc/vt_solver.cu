@@ -1100,7 +1100,7 @@ void* vt_stream(vt_ctx* c) { return c ? static_cast<void*>(c->stream) : nullptr;
 
 int vt_set_stage_mapping(vt_ctx* c, int mapping) {
   if (!c || (mapping != vt::kMapComponent && mapping != vt::kMapDefault))
-    return fail(VT_ERR_INVALID, "vt_set_stage_mapping: mapping must be 0 (component) or 1 (pair)");
+    return fail(VT_ERR_INVALID, "vt_set_stage_mapping: mapping must be 0 (operators as they are) or 1 (folded)");
   std::lock_guard<std::mutex> lk(c->mu);
   cudaSetDevice(c->device);
   const cudaError_t e = vt::use_kernel(c, mapping);
